@@ -225,6 +225,8 @@ def decay_scan(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign: float, beta
     assert z.shape == (t, heads if head_decay else heads * dk) and (not head_decay or (z.dtype == torch.float32 and not delta))
     assert q.dtype == k.dtype == v.dtype and (beta is None or beta.dtype == z.dtype)
     assert v_scale is None or v_scale.shape == (t, heads)
+    if walk_ok(q, k, v, dk, ctx, head_decay, ones_column, bonus):
+        return _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx, heads, dk, dv, q_scale, delta, head_decay, v_scale)
     if not delta and not ctx.decode_only and t >= SEGMENT_MIN_TOKENS and SEGMENTS > 1 and dk <= SEGMENT_MAX_DK:
         return _decay_scan_segmented(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, ctx, heads, dk, dv, q_scale, head_decay,
                                      v_scale, dv_in, bonus)
@@ -274,6 +276,45 @@ def conv_state_update(conv_state, x, ctx, taps: int) -> None:
     native.recurrence_check(native.recurrence().ms_conv_state_update(
         _ptr(conv_state), _ptr(x), _rows(x), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.state_slot), ctx.num_rows, x.shape[1],
         taps, _dt(x.dtype), ctx.stream))
+
+
+WALK_MIN_TOKENS = 64  # steps with fewer tokens stay on the token-by-token walk
+
+
+def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool = False, bonus=None) -> bool:
+    """Whether ``decay_scan`` walks the step by chunks of 16 tokens (``csrc/chunk_walk.cu``): a step that is not all single tokens, heads of up
+    to 128 key channels; with one decay per head float32 operands whose rows start on 16 bytes, 32, 64 or 128 key channels."""
+    if ctx.decode_only or q.shape[0] < WALK_MIN_TOKENS or ones_column or bonus is not None or dk > 128:
+        return False
+    if not head_decay:
+        return True
+    return (dk in (32, 64, 128) and q.dtype == torch.float32 and all(x.data_ptr() % 16 == 0 and x.stride(0) % 4 == 0 for x in (q, k)))
+
+
+def _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx, heads, dk, dv, q_scale, delta, head_decay, v_scale) -> None:
+    t, dev, rows = o_out.shape[0], o_out.device, ctx.num_rows
+    lib = native.recurrence()
+    most = int(lib.ms_walk_max(t, rows))
+    table = ctx.step_cache.get("walk.table") if hasattr(ctx, "step_cache") else None
+    if table is None:  # the same for every layer of the step
+        ints = torch.empty(2 * most + rows + 1, dtype=torch.int32, device=dev)
+        table = (ints[:2 * most], ints[2 * most:])
+        native.recurrence_check(lib.ms_walk_table(_ptr(table[0]), _ptr(table[1]), _ptr(ctx.cu_q), rows, ctx.stream))
+        if hasattr(ctx, "step_cache"):
+            ctx.step_cache["walk.table"] = table
+    scratch = ctx.buffer("walk.scratch", (int(lib.ms_walk_scratch(most, heads, dk, dv, int(delta), int(head_decay))),), torch.float32, dev)
+    groups = q.shape[1] // dk
+    rest = (_ptr(v_scale), _ptr(scratch), _ptr(table[0]), _ptr(table[1]), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.state_slot), rows, most, heads,
+            dk, dv, float(q_scale))
+    if head_decay:
+        native.recurrence_check(lib.ms_walk_scan_head(
+            _ptr(o_out), _ptr(state), _ptr(q), _rows(q), _ptr(k), _rows(k), heads // groups, _ptr(v), _rows(v), _ptr(z), _rows(z), *rest,
+            ctx.stream), launches=2)
+        return
+    native.recurrence_check(lib.ms_walk_scan(
+        _ptr(o_out), _ptr(state), _ptr(q), _rows(q), _ptr(k), _rows(k), heads // groups, _ptr(v), _rows(v), _ptr(z), _rows(z), _ptr(z_bias),
+        _ptr(decay_coef), float(z_sign), _ptr(beta), 0 if beta is None else _rows(beta), *rest, int(delta), _dt(q.dtype), _dt(z.dtype), ctx.stream),
+        launches=2)
 
 
 # The decay rule is linear in the state with a diagonal factor, so the rows of a step with many tokens are cut into
