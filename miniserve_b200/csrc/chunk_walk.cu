@@ -34,11 +34,12 @@ __device__ __forceinline__ float wk_softplus(float x) { return fmaxf(x, 0.f) + l
 struct Tf32x2 {
   uint32_t hi, lo;
 };
+// hi: x rounded to 11 bits of significand, lo: what is left (12 bits and a sign, of which the last is cut off). Integer adds and masks: a
+// conversion instruction takes several times their issue slots. A NaN stays one in lo whatever the addition makes of it in hi.
 __device__ __forceinline__ Tf32x2 wk_split(float x) {
   Tf32x2 r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r.hi) : "f"(x));
-  const float rest = x - __uint_as_float(r.hi);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r.lo) : "f"(rest));
+  r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  r.lo = __float_as_uint(x - __uint_as_float(r.hi)) & 0xffffe000u;
   return r;
 }
 __device__ __forceinline__ void wk_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
