@@ -1,0 +1,85 @@
+"""The four-channels-a-thread forms of the convolution, the per-head norm and the grouped norm against the forms for any operand, which
+the same numbers take when their rows do not start on whole vectors: sizes around the edges of a thread, a warp and a run of tokens."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from miniserve_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda")
+
+
+def _rows(lens, started):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    return SimpleNamespace(cu_q=torch.tensor(cu, **i32), q_start=torch.tensor(started, **i32), state_slot=torch.arange(len(lens) - 1, -1, -1, **i32),
+                           row_of_token=torch.tensor([r for r, n in enumerate(lens) for _ in range(n)], **i32), num_rows=len(lens),
+                           stream=torch.cuda.current_stream().cuda_stream)
+
+
+def _view(gen, t, width, ahead, dtype):
+    """[T, width] behind ``ahead`` columns of rows as wide as whole fours allow (ahead odd: no whole vectors)."""
+    full = torch.randn(t, -(-(width + ahead) // 4) * 4 + 4, generator=gen).to(dtype).to(DEV)
+    return full[:, ahead:ahead + width]
+
+
+def _near(a, b, dtype):
+    # the two forms add a norm's squares in other orders: a few units in the last place of float32, then one rounding
+    tol = 2e-6 if dtype == torch.float32 else 2.0 ** -7
+    assert not torch.isnan(b).any() and ((a.float() - b.float()).abs() <= tol * b.float().abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps, unit, dk, others, dv", [(4, 4, 64, 5, 36), (3, 2, 16, 3, 8), (2, 1, 128, 1, 4), (4, 0, 1, 6, 700), (2, 3, 4, 2, 6)])
+@pytest.mark.parametrize("lens, started", [((1, 1, 1), (0, 3, 1)), ((5, 1, 8, 700, 2, 3), (0, 9, 2, 1, 0, 5)), ((2048,), (0,))])
+def test_convolution_in_fours(dtype, taps, unit, dk, others, dv, lens, started):
+    gen = torch.Generator().manual_seed(taps * 100 + unit)
+    ctx, t, c = _rows(lens, started), sum(lens), unit * dk + others * dv
+    x = _view(gen, t, c, 4, dtype)
+    odd = torch.empty(t, c + 7, dtype=dtype, device=DEV)[:, 1:1 + c]
+    odd.copy_(x)
+    state = torch.randn(len(lens), taps - 1, c, generator=gen).to(dtype).to(DEV)
+    w, bias = torch.randn(c, taps, generator=gen).to(DEV), torch.randn(c, generator=gen).to(DEV)
+    got, want = (torch.full((t, c), float("nan"), device=DEV) for _ in range(2))
+    for b in (None, bias):
+        ops.conv_silu_unit(got, x, state, w, ctx, unit, dk, others, dv, 1e-6, bias=b)
+        ops.conv_silu_unit(want, odd, state, w, ctx, unit, dk, others, dv, 1e-6, bias=b)
+        _near(got, want, torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("t, heads, dv", [(1, 1, 64), (37, 3, 32), (130, 5, 128), (3, 7, 64)])
+@pytest.mark.parametrize("kind, own", [("silu", False), ("sigmoid", True)])
+def test_head_norm_in_fours(dtype, t, heads, dv, kind, own):
+    gen = torch.Generator().manual_seed(t + dv)
+    o, w = torch.randn(t, heads, dv, generator=gen).to(DEV), torch.randn(heads * dv if own else dv, generator=gen).to(DEV)
+    gate = _view(gen, t, heads * dv, 4, dtype)
+    odd = torch.empty(t, heads * dv + 3, dtype=dtype, device=DEV)[:, 1:1 + heads * dv]
+    odd.copy_(gate)
+    got, want = (torch.full((t, heads * dv), float("nan"), dtype=dtype, device=DEV) for _ in range(2))
+    ops.head_norm_gate(got, o, w, gate, 1e-5, 0.7, kind)
+    ops.head_norm_gate(want, o, w, odd, 1e-5, 0.7, kind)
+    _near(got, want, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("t, parts, size, dv, skip", [(1, 1, 4, 4, True), (9, 8, 512, 64, True), (5, 3, 260, 52, False), (3, 2, 1024, 128, True),
+                                                      (2, 1, 252, 12, True)])
+def test_group_norm_in_fours(dtype, t, parts, size, dv, skip):
+    gen = torch.Generator().manual_seed(size)
+    width = parts * size
+    o, w = torch.randn(t, width, generator=gen).to(DEV), torch.randn(width, generator=gen).to(DEV)
+    x = _view(gen, t, width, 4, torch.float32) if skip else None
+    s = torch.randn(width // dv, generator=gen).to(DEV) if skip else None
+    gate = _view(gen, t, width, 4, dtype)
+    odd = torch.empty(t, width + 3, dtype=dtype, device=DEV)[:, 1:1 + width]
+    odd.copy_(gate)
+    got, want = (torch.full((t, width), float("nan"), dtype=dtype, device=DEV) for _ in range(2))
+    ops.gated_group_norm(got, o, x, s, gate, w, parts, dv, 1e-6)
+    ops.gated_group_norm(want, o, x, s, odd, w, parts, dv, 1e-6)
+    _near(got, want, dtype)
