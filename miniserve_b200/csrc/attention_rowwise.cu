@@ -15,6 +15,7 @@
 // first keep_first keys of the request stay visible behind the window (their tiles are walked first, in order). A
 // distance bias takes r1_h * ln(1 + r2_h * (p - j)) off the scaled score of key j.
 #include <cfloat>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -125,6 +126,280 @@ attention_rowwise_kernel(T* __restrict__ out,            // [T, nq, d]
   }
 }
 
+// ---------------------------------------------------------------- the same for prompts, 64 query rows of a request at a time
+// The arithmetic of every (token, head) is the one above, operation by operation (the same bits); what differs is who does it: a CTA
+// takes 64 query rows (tokens of one request times the query heads of a kv head) and walks the key tiles once for all of them, keys and
+// values staged in shared memory by asynchronous copies a tile ahead. A warp has 16 rows from the scores to the output: a lane 4 x 4
+// scores, then the rows one after the other with a lane per key (the same exchanges as above), then 4 rows x 4 MD columns of the output.
+// A tile in which a row sees nothing leaves the row as it is (alpha = 1, p = 0), so all rows may walk the tiles that any of them sees.
+// Bound by shared-memory reads (32 floats read for 64 products of a score tile): 700 tokens of 16 heads of 128 on 8
+// kv heads take 346 us where a warp per token and head takes 2,183 (every lane walking its own key's row in global memory).
+constexpr int TW_ROWS = 64, TW_KEYS = 32, TW_THREADS = 128, TW_LDS = TW_KEYS + 4;
+
+__device__ __forceinline__ void tw_cp16(void* dst, const void* src, bool in) {
+  const int bytes = in ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+template <int MD>  // head sizes of up to 32 MD, whole fours
+__global__ void __launch_bounds__(TW_THREADS)
+attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
+                           const int* __restrict__ cu_q, const int* __restrict__ q_start, const int* __restrict__ page_indptr,
+                           const int* __restrict__ page_indices, int num_rows, int nq, int nkv, int d, float scale, int window, int sink,
+                           int page_shift, int num_pages, int* __restrict__ status, const float* __restrict__ sink_values, float softcap, int chunk,
+                           const float* __restrict__ dist_r1, const float* __restrict__ dist_r2, int keep_first) {
+  constexpr int LD = 32 * MD + 4;
+  extern __shared__ __align__(16) float tw_smem[];
+  float* qs = tw_smem;                        // [64][LD]
+  float* ks = qs + TW_ROWS * LD;              // [2][32][LD]
+  float* vs = ks + 2 * TW_KEYS * LD;          // [2][32][LD]
+  float* ss = vs + 2 * TW_KEYS * LD;          // [64][TW_LDS]
+  float* alphas = ss + TW_ROWS * TW_LDS;      // [64]
+  unsigned* seen = reinterpret_cast<unsigned*>(alphas + TW_ROWS);  // [64]
+  __shared__ int s_row, s_tile;
+  __shared__ int usable[2][TW_KEYS];
+  pdl_prologue();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int group = nq / nkv, per_tile = TW_ROWS / group, kvh = blockIdx.y;
+  if (warp == 0) {  // which request and which of its tiles: the late (long) tiles first
+    int want = gridDim.x - 1 - blockIdx.x, row = -1, base = 0;
+    for (int r0 = 0; r0 < num_rows && row < 0; r0 += 32) {
+      const int r = r0 + lane;
+      const int mine = r < num_rows ? (cu_q[r + 1] - cu_q[r] + per_tile - 1) / per_tile : 0;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, want < base + upto);
+      if (hit) {
+        const int at = __ffs(hit) - 1;
+        row = r0 + at;
+        want -= base + __shfl_sync(0xffffffffu, upto - mine, at);
+      } else {
+        base += __shfl_sync(0xffffffffu, upto, 31);
+      }
+    }
+    if (lane == 0) {
+      s_row = row;
+      s_tile = want;
+    }
+  }
+  __syncthreads();
+  const int row = s_row;
+  if (row < 0) return;
+  const int t0 = cu_q[row] + s_tile * per_tile, n_tok = min(per_tile, cu_q[row + 1] - t0);
+  const int pos0 = q_start[row] + s_tile * per_tile, pos_last = pos0 + n_tok - 1;
+  const int rows = n_tok * group;  // of the 64
+  const int* pages = page_indices + page_indptr[row];
+  const int page_size = 1 << page_shift;
+  const float inv_cap = softcap > 0.f ? 1.0f / softcap : 0.f;
+  auto first_key = [&](int pos) {
+    int lo = window > 0 ? max(0, pos - window + 1) : 0;
+    if (chunk > 0) lo = max(lo, (pos / chunk) * chunk);
+    return lo;
+  };
+  const int lo_tile = (first_key(pos0) >> 5) << 5;  // (the first token's window begins first)
+  const int kept_end = keep_first > 0 ? min((keep_first + 31) & ~31, lo_tile) : 0;
+  const int vec = d / 4;
+  for (int idx = tid; idx < TW_ROWS * vec; idx += TW_THREADS) {
+    const int r = idx / vec, c = (idx - r * vec) * 4;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < rows) x = *reinterpret_cast<const float4*>(q + ((size_t)(t0 + r / group) * nq + kvh * group + r % group) * d + c);
+    *reinterpret_cast<float4*>(qs + r * LD + c) = x;
+  }
+  auto stage = [&](int tile, int buf) {
+    if (tile <= pos_last) {
+      for (int idx = tid; idx < TW_KEYS * vec; idx += TW_THREADS) {
+        const int j = idx / vec, c = (idx - j * vec) * 4, kj = tile + j;
+        bool in = kj <= pos_last;
+        const int page = in ? pages[kj >> page_shift] : -1;
+        in = page >= 0;
+        MS_DEBUG_ONLY(if (in && page >= num_pages) {
+          atomicExch(status, 5);
+          in = false;
+        })
+        const size_t base = in ? (((size_t)page * nkv + kvh) * page_size + (kj & (page_size - 1))) * d + c : 0;
+        tw_cp16(ks + (buf * TW_KEYS + j) * LD + c, k_pool + base, in);
+        tw_cp16(vs + (buf * TW_KEYS + j) * LD + c, v_pool + base, in);
+        if (c == 0) usable[buf][j] = in;
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  auto next_tile = [&](int tile) { return tile + TW_KEYS == kept_end ? lo_tile : tile + TW_KEYS; };
+
+  const int r0 = warp * 16;            // the warp's rows
+  const int qg = lane >> 3, kg = lane & 7;  // a lane's four rows r0 + 4 qg + i; its keys kg + 8 jj, its columns 4 kg + 32 m
+  float m[16], l[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+  }
+  float acc[4][MD][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int mm = 0; mm < MD; ++mm)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][mm][e] = 0.f;
+
+  int tile = kept_end > 0 ? 0 : lo_tile, buf = 0;
+  stage(tile, 0);
+#pragma unroll 1
+  for (; tile <= pos_last; tile = next_tile(tile), buf ^= 1) {
+    stage(next_tile(tile), buf ^ 1);
+    asm volatile("cp.async.wait_group 1;\n" ::);
+    __syncthreads();
+    if (r0 < rows) {
+      const float* kb = ks + buf * TW_KEYS * LD;
+      const float* vb = vs + buf * TW_KEYS * LD;
+      {
+        float s[4][4] = {};
+        const float* qp = qs + (r0 + 4 * qg) * LD;
+        for (int c = 0; c < d; c += 4) {
+          float4 a[4], b[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qp + i * LD + c);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(kb + (kg + 8 * j) * LD + c);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+              s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+              s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+              s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ss[(r0 + 4 * qg + i) * TW_LDS + kg + 8 * j] = s[i][j];
+      }
+      __syncwarp();
+      const int kj = tile + lane;
+      const bool there = kj <= pos_last && usable[buf][lane];
+      bool all_see = true;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int r = r0 + i;
+        if (r >= rows) break;
+        const int qpos = pos0 + r / group, h = kvh * group + r % group, lo = first_key(qpos);
+        float s = -INFINITY;
+        if (kj <= qpos && (kj >= lo || kj < keep_first)) {
+          if (there) {
+            s = ss[r * TW_LDS + lane] * scale;
+            if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
+            if (dist_r1) s -= dist_r1[h] * logf(1.0f + dist_r2[h] * (float)(qpos - kj));
+          } else {
+            atomicExch(status, 3);
+          }
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, s != -INFINITY);
+        const float m_new = fmaxf(m[i], warp_max(s));
+        const float alpha = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_new);
+        const float p = (s == -INFINITY) ? 0.f : expf(s - m_new);
+        l[i] = l[i] * alpha + warp_sum(p);
+        m[i] = m_new;
+        ss[r * TW_LDS + lane] = p;
+        if (lane == 0) {
+          alphas[r] = alpha;
+          seen[r] = mask;
+        }
+        all_see = all_see && mask == 0xffffffffu;
+      }
+      __syncwarp();
+      float al[4];
+      unsigned mk[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + 4 * qg + i;
+        al[i] = r < rows ? alphas[r] : 0.f;
+        mk[i] = r < rows ? seen[r] : 0u;
+#pragma unroll
+        for (int mm = 0; mm < MD; ++mm)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[i][mm][e] *= al[i];
+      }
+      const float* pr = ss + (r0 + 4 * qg) * TW_LDS;
+      auto values = [&](auto whole) {
+#pragma unroll 1
+        for (int j0 = 0; j0 < TW_KEYS; j0 += 4) {
+          float4 p[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pr + i * TW_LDS + j0);
+#pragma unroll
+          for (int jj = 0; jj < 4; ++jj) {
+            float4 v[MD];
+#pragma unroll
+            for (int mm = 0; mm < MD; ++mm) v[mm] = *reinterpret_cast<const float4*>(vb + (j0 + jj) * LD + 4 * kg + 32 * mm);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
+              // (a key that a row does not see may hold anything: the row's sums must not meet it)
+              if (whole.value || ((mk[i] >> (j0 + jj)) & 1u)) {
+#pragma unroll
+                for (int mm = 0; mm < MD; ++mm) {
+                  acc[i][mm][0] = fmaf(pj, v[mm].x, acc[i][mm][0]);
+                  acc[i][mm][1] = fmaf(pj, v[mm].y, acc[i][mm][1]);
+                  acc[i][mm][2] = fmaf(pj, v[mm].z, acc[i][mm][2]);
+                  acc[i][mm][3] = fmaf(pj, v[mm].w, acc[i][mm][3]);
+                }
+              }
+            }
+          }
+        }
+      };
+      if (all_see) values(std::true_type());
+      else values(std::false_type());
+    }
+    __syncthreads();
+  }
+  if (r0 >= rows) return;
+  // (m and l of a row are the same in all lanes: the sink's term is the row's own, as above)
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int r = r0 + i;
+    if (r >= rows) break;
+    float a = 1.f;
+    if (sink) {
+      const float s0 = sink_values ? sink_values[kvh * group + r % group] : 0.f;
+      const float m_all = fmaxf(m[i], s0);
+      a = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_all);
+      l[i] = l[i] * a + expf(s0 - m_all);
+    }
+    if (lane == 0) {
+      alphas[r] = a;
+      ss[r * TW_LDS] = l[i];
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + 4 * qg + i;
+    if (r >= rows) continue;
+    const float a = alphas[r], sum = ss[r * TW_LDS];
+    float* o = out + ((size_t)(t0 + r / group) * nq + kvh * group + r % group) * d;
+#pragma unroll
+    for (int mm = 0; mm < MD; ++mm) {
+      const int c = 4 * kg + 32 * mm;
+      if (c < d) {
+        float4 x;
+        if (sink) {
+          x.x = acc[i][mm][0] * a / sum; x.y = acc[i][mm][1] * a / sum; x.z = acc[i][mm][2] * a / sum; x.w = acc[i][mm][3] * a / sum;
+        } else {
+          x.x = acc[i][mm][0] / sum; x.y = acc[i][mm][1] / sum; x.z = acc[i][mm][2] / sum; x.w = acc[i][mm][3] / sum;
+        }
+        *reinterpret_cast<float4*>(o + c) = x;
+      }
+    }
+  }
+}
+
 }  // namespace ms
 
 using namespace ms;
@@ -160,5 +435,42 @@ MS_EXPORT int ms_attention_rowwise(void* out, const void* q, const void* k_pool,
     else MS_ROWWISE_LAUNCH(__nv_bfloat16, 16);
   }
 #undef MS_ROWWISE_LAUNCH
+  return 0;
+}
+
+// 1 if ms_attention_tiled_f32 takes these sizes: head sizes of whole fours up to 128, groups of up to 64 query heads.
+MS_EXPORT int ms_attention_tiled_f32_supports(int head_dim, int nq, int nkv) {
+  return head_dim >= 4 && head_dim <= 128 && head_dim % 4 == 0 && nkv > 0 && nq % nkv == 0 && nq / nkv <= TW_ROWS && nkv <= 65535;
+}
+
+// ms_attention_rowwise for float32 and a step of whole rows: cu_q [rows + 1], q_start [rows]. The same results, bit for bit.
+MS_EXPORT int ms_attention_tiled_f32(float* out, const float* q, const float* k_pool, const float* v_pool, const int* cu_q, const int* q_start,
+                                     const int* page_indptr, const int* page_indices, int num_tokens, int num_rows, int nq, int nkv, int head_dim,
+                                     float scale, int window, int sink, int page_size, int num_pages, int* status, cudaStream_t stream,
+                                     const float* sink_values, float softcap, int chunk, const float* dist_r1, const float* dist_r2, int keep_first) {
+  if (num_tokens == 0) return 0;
+  MS_CHECK_ARG(ms_attention_tiled_f32_supports(head_dim, nq, nkv), "attention: %d/%d heads of %d", nq, nkv, head_dim);
+  MS_CHECK_ARG(keep_first >= 0 && (dist_r1 == nullptr) == (dist_r2 == nullptr), "attention: keep_first=%d, and both numbers of a distance bias",
+               keep_first);
+  MS_CHECK_ARG(softcap >= 0.f && chunk >= 0, "attention: softcap=%g and chunk=%d must not be negative", softcap, chunk);
+  MS_CHECK_ARG(page_size > 0 && (page_size & (page_size - 1)) == 0, "attention: page_size=%d must be a power of two", page_size);
+  MS_CHECK_ARG((uintptr_t)q % 16 == 0 && (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0 && (uintptr_t)out % 16 == 0,
+               "attention: operands must start on 16 bytes");
+  int page_shift = 0;
+  while ((1 << page_shift) < page_size) ++page_shift;
+  const dim3 grid(num_tokens / (TW_ROWS / (nq / nkv)) + num_rows, nkv);
+#define MS_TILED_LAUNCH(MD)                                                                                                                     \
+  do {                                                                                                                                          \
+    auto kernel = attention_tiled_f32_kernel<MD>;                                                                                               \
+    constexpr size_t smem = ((TW_ROWS + 4 * TW_KEYS) * (32 * MD + 4) + TW_ROWS * TW_LDS + 2 * TW_ROWS) * 4;                                     \
+    static const cudaError_t asked = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                      \
+    MS_CHECK_CUDA(asked);                                                                                                                       \
+    MS_LAUNCH(kernel, grid, TW_THREADS, smem, stream, out, q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, num_rows, nq, nkv, head_dim, \
+              scale, window, sink, page_shift, num_pages, status, sink_values, softcap, chunk, dist_r1, dist_r2, keep_first);                   \
+  } while (0)
+  if (head_dim <= 32) MS_TILED_LAUNCH(1);
+  else if (head_dim <= 64) MS_TILED_LAUNCH(2);
+  else MS_TILED_LAUNCH(4);
+#undef MS_TILED_LAUNCH
   return 0;
 }

@@ -541,6 +541,35 @@ def attention_rowwise(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, 
         int(extras.chunk or 0), _ptr(extras.dist_r1), _ptr(extras.dist_r2), int(extras.keep_first or 0)))
 
 
+def attention_tiled_ok(q: torch.Tensor, k_pool: torch.Tensor, ctx) -> bool:
+    """Whether a float32 step runs ``attention_tiled``: a step that is not all single tokens (those keep a warp per token and head), head
+    sizes of whole fours up to 128."""
+    if q.dtype != torch.float32 or getattr(ctx, "decode_only", False) or q.shape[0] <= ctx.num_rows:
+        return False
+    return (bool(native.kernels().ms_attention_tiled_f32_supports(q.shape[2], q.shape[1], k_pool.shape[1]))
+            and q.data_ptr() % 16 == 0 and k_pool.data_ptr() % 16 == 0)
+
+
+def attention_tiled(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx, group: int, scale: float,
+                    window: int | None, sink: bool = False, extras: "AttentionExtras | None" = None) -> None:
+    """``attention_rowwise`` for a step of whole rows, 64 query rows of a request at a time: the same float32 operations in the same
+    order for every (token, head), so the same bits."""
+    _check_dev(out, q, k_pool, v_pool)
+    extras = extras or NO_EXTRAS
+    for r in (extras.sink_values, extras.dist_r1, extras.dist_r2):
+        assert r is None or (r.dtype == torch.float32 and r.numel() == q.shape[1] and r.is_cuda and r.is_contiguous())
+    assert (extras.dist_r1 is None) == (extras.dist_r2 is None)
+    t, nq, d = q.shape
+    nkv, page_size = k_pool.shape[1], k_pool.shape[2]
+    assert out.shape == q.shape and k_pool.shape[3] == d and out.dtype == q.dtype == k_pool.dtype == v_pool.dtype == torch.float32
+    native.kernel_check(native.kernels().ms_attention_tiled_f32(
+        _ptr(out), _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.page_indptr[group]),
+        _ptr(ctx.page_indices[group]), t, ctx.num_rows, nq, nkv, d, float(scale), int(window or 0),
+        int(sink or extras.sink_values is not None), page_size, k_pool.shape[0], _ptr(ctx.status), _stream(ctx.stream),
+        _ptr(extras.sink_values), float(extras.softcap or 0.0), int(extras.chunk or 0), _ptr(extras.dist_r1), _ptr(extras.dist_r2),
+        int(extras.keep_first or 0)))
+
+
 def nucleus_bytes() -> int:
     return native.kernels().ms_nucleus_bytes()
 
@@ -574,11 +603,14 @@ def attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: 
     ``sink``: one more term of score 0 in the softmax's denominator, which carries no value.
     ``extras``: learned sink scores, a cap on the scores, a mask by blocks of positions (``AttentionExtras``).
 
-    float32 runs the row-wise kernel (bit-identical however the step was cut). bfloat16 runs the
+    float32 runs the row-wise kernel, prompts its tiled form (bit-identical however the step was cut). bfloat16 runs the
     tensor-core kernels when they take this head size, else the row-wise kernel too."""
     from . import attention_bf16
 
     extras = extras if extras is not None and extras.any else None
+    if attention_tiled_ok(q, k_pool, ctx):
+        attention_tiled(out, q, k_pool, v_pool, ctx, group, scale, window, sink, extras)
+        return
     if extras is not None and not (q.dtype == torch.bfloat16 and attention_bf16.takes_extras(q.shape[2], k_pool.shape[2])):
         attention_rowwise(out, q, k_pool, v_pool, ctx.positions, ctx.row_of_token, ctx.page_indptr[group],
                           ctx.page_indices[group], scale, window, ctx.status, stream=ctx.stream, sink=sink, extras=extras)

@@ -114,6 +114,9 @@ def kernels():
     _declare(lib, "ms_gemm_f32_batched", [_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _p])
     _declare(lib, "ms_attention_rowwise",
              [_p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _f, _i, _i, _i, _i, _p, _i, _p, _p, _f, _i, _p, _p, _i])
+    _declare(lib, "ms_attention_tiled_f32_supports", [_i, _i, _i])
+    _declare(lib, "ms_attention_tiled_f32",
+             [_p] * 8 + [_i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _p, _p, _p, _f, _i, _p, _p, _i])
     _declare(lib, "ms_nucleus_bytes", [])
     _declare(lib, "ms_sample_scratch_bytes", [_i, _i], _ll)
     _declare(lib, "ms_sample", [_p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _p])
