@@ -133,13 +133,36 @@ attention_rowwise_kernel(T* __restrict__ out,            // [T, nq, d]
 // scores, then the rows one after the other with a lane per key (the same exchanges as above), then 4 rows x 4 MD columns of the output.
 // A tile in which a row sees nothing leaves the row as it is (alpha = 1, p = 0), so all rows may walk the tiles that any of them sees.
 // Bound by shared-memory reads (32 floats read for 64 products of a score tile): 700 tokens of 16 heads of 128 on 8
-// kv heads take 346 us where a warp per token and head takes 2,183 (every lane walking its own key's row in global memory).
+// kv heads take 262 us where a warp per token and head takes 2,183 (every lane walking its own key's row in global memory).
 constexpr int TW_ROWS = 64, TW_KEYS = 32, TW_THREADS = 128, TW_LDS = TW_KEYS + 4;
 
 __device__ __forceinline__ void tw_cp16(void* dst, const void* src, bool in) {
   const int bytes = in ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
+
+// Folds 16 values over the lanes of a warp, all sixteen in one go: lane l comes back with the fold of v[tw_row(l)]. The pairs are those of
+// the exchange by 16, 8, 4, 2, 1 that folds one value (warp_sum), so the result is the same bit for bit.
+template <typename F>
+__device__ __forceinline__ float tw_fold16(float (&v)[16], F fold) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int n = 8; n > 0; n >>= 1) {
+    const bool up = lane & (2 * n);
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+      v[i] = fold(keep, __shfl_xor_sync(0xffffffffu, send, 2 * n));
+    }
+  }
+  return fold(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
+}
+__device__ __forceinline__ unsigned long long tw_twice(float x) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ int tw_row(int lane) { return lane >> 1; }
 
 template <int MD>  // head sizes of up to 32 MD, whole fours
 __global__ void __launch_bounds__(TW_THREADS)
@@ -232,19 +255,14 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
 
   const int r0 = warp * 16;            // the warp's rows
   const int qg = lane >> 3, kg = lane & 7;  // a lane's four rows r0 + 4 qg + i; its keys kg + 8 jj, its columns 4 kg + 32 m
-  float m[16], l[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
-  }
-  float acc[4][MD][4];
+  float m = -INFINITY, l = 0.f;        // of row r0 + tw_row(lane)
+  unsigned long long acc[4][MD][2];    // two columns each: fma.rn.f32x2 rounds each half as fmaf does
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int mm = 0; mm < MD; ++mm)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][mm][e] = 0.f;
+      for (int e = 0; e < 2; ++e) acc[i][mm][e] = 0ull;
 
   int tile = kept_end > 0 ? 0 : lo_tile, buf = 0;
   stage(tile, 0);
@@ -259,6 +277,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
       {
         float s[4][4] = {};
         const float* qp = qs + (r0 + 4 * qg) * LD;
+#pragma unroll 4
         for (int c = 0; c < d; c += 4) {
           float4 a[4], b[4];
 #pragma unroll
@@ -283,71 +302,82 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
       __syncwarp();
       const int kj = tile + lane;
       const bool there = kj <= pos_last && usable[buf][lane];
-      bool all_see = true;
+      float sc[16];
+      bool all_see = true, missing = false;
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int r = r0 + i;
-        if (r >= rows) break;
         const int qpos = pos0 + r / group, h = kvh * group + r % group, lo = first_key(qpos);
+        const bool sees = r < rows && kj <= qpos && (kj >= lo || kj < keep_first);
         float s = -INFINITY;
-        if (kj <= qpos && (kj >= lo || kj < keep_first)) {
-          if (there) {
-            s = ss[r * TW_LDS + lane] * scale;
-            if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
-            if (dist_r1) s -= dist_r1[h] * logf(1.0f + dist_r2[h] * (float)(qpos - kj));
-          } else {
-            atomicExch(status, 3);
-          }
+        if (sees && there) {
+          s = ss[r * TW_LDS + lane] * scale;
+          if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
+          if (dist_r1) s -= dist_r1[h] * logf(1.0f + dist_r2[h] * (float)(qpos - kj));
         }
-        const unsigned mask = __ballot_sync(0xffffffffu, s != -INFINITY);
-        const float m_new = fmaxf(m[i], warp_max(s));
-        const float alpha = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_new);
-        const float p = (s == -INFINITY) ? 0.f : expf(s - m_new);
-        l[i] = l[i] * alpha + warp_sum(p);
-        m[i] = m_new;
-        ss[r * TW_LDS + lane] = p;
-        if (lane == 0) {
-          alphas[r] = alpha;
-          seen[r] = mask;
-        }
-        all_see = all_see && mask == 0xffffffffu;
+        missing = missing || (sees && !there);
+        all_see = all_see && (r >= rows || s != -INFINITY);
+        sc[i] = s;
       }
+      if (missing) atomicExch(status, 3);
+      all_see = __all_sync(0xffffffffu, all_see);
+      if (!all_see) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const unsigned mask = __ballot_sync(0xffffffffu, sc[i] != -INFINITY);
+          if (lane == i) seen[r0 + i] = mask;
+        }
+      }
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = sc[i];
+      const float m_new = fmaxf(m, tw_fold16(v, [](float x, float y) { return fmaxf(x, y); }));
+      const float alpha = (m == -INFINITY) ? 0.f : expf(m - m_new);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float mi = __shfl_sync(0xffffffffu, m_new, 2 * i);
+        v[i] = (sc[i] == -INFINITY) ? 0.f : expf(sc[i] - mi);
+        ss[(r0 + i) * TW_LDS + lane] = v[i];
+      }
+      l = l * alpha + tw_fold16(v, [](float x, float y) { return x + y; });
+      m = m_new;
+      if (!(lane & 1)) alphas[r0 + tw_row(lane)] = alpha;
       __syncwarp();
       float al[4];
       unsigned mk[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = r0 + 4 * qg + i;
-        al[i] = r < rows ? alphas[r] : 0.f;
-        mk[i] = r < rows ? seen[r] : 0u;
+        al[i] = alphas[r];
+        mk[i] = all_see ? 0xffffffffu : seen[r];
+        const unsigned long long twice = tw_twice(al[i]);
 #pragma unroll
         for (int mm = 0; mm < MD; ++mm)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[i][mm][e] *= al[i];
+          for (int e = 0; e < 2; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][mm][e]) : "l"(twice));
       }
       const float* pr = ss + (r0 + 4 * qg) * TW_LDS;
       auto values = [&](auto whole) {
-#pragma unroll 1
+#pragma unroll 2
         for (int j0 = 0; j0 < TW_KEYS; j0 += 4) {
           float4 p[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pr + i * TW_LDS + j0);
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj) {
-            float4 v[MD];
+            ulonglong2 v[MD];
 #pragma unroll
-            for (int mm = 0; mm < MD; ++mm) v[mm] = *reinterpret_cast<const float4*>(vb + (j0 + jj) * LD + 4 * kg + 32 * mm);
+            for (int mm = 0; mm < MD; ++mm) v[mm] = *reinterpret_cast<const ulonglong2*>(vb + (j0 + jj) * LD + 4 * kg + 32 * mm);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
               // (a key that a row does not see may hold anything: the row's sums must not meet it)
               if (whole.value || ((mk[i] >> (j0 + jj)) & 1u)) {
+                const unsigned long long twice = tw_twice(pj);
 #pragma unroll
                 for (int mm = 0; mm < MD; ++mm) {
-                  acc[i][mm][0] = fmaf(pj, v[mm].x, acc[i][mm][0]);
-                  acc[i][mm][1] = fmaf(pj, v[mm].y, acc[i][mm][1]);
-                  acc[i][mm][2] = fmaf(pj, v[mm].z, acc[i][mm][2]);
-                  acc[i][mm][3] = fmaf(pj, v[mm].w, acc[i][mm][3]);
+                  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][mm][0]) : "l"(twice), "l"(v[mm].x));
+                  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][mm][1]) : "l"(twice), "l"(v[mm].y));
                 }
               }
             }
@@ -360,21 +390,18 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
     __syncthreads();
   }
   if (r0 >= rows) return;
-  // (m and l of a row are the same in all lanes: the sink's term is the row's own, as above)
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int r = r0 + i;
-    if (r >= rows) break;
+  {  // the sink's term of the lane's row, as above
+    const int r = r0 + tw_row(lane);
     float a = 1.f;
     if (sink) {
       const float s0 = sink_values ? sink_values[kvh * group + r % group] : 0.f;
-      const float m_all = fmaxf(m[i], s0);
-      a = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_all);
-      l[i] = l[i] * a + expf(s0 - m_all);
+      const float m_all = fmaxf(m, s0);
+      a = (m == -INFINITY) ? 0.f : expf(m - m_all);
+      l = l * a + expf(s0 - m_all);
     }
-    if (lane == 0) {
+    if (!(lane & 1)) {
       alphas[r] = a;
-      ss[r * TW_LDS] = l[i];
+      ss[r * TW_LDS] = l;
     }
   }
   __syncwarp();
@@ -389,11 +416,12 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
       const int c = 4 * kg + 32 * mm;
       if (c < d) {
         float4 x;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x.x), "=f"(x.y) : "l"(acc[i][mm][0]));
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x.z), "=f"(x.w) : "l"(acc[i][mm][1]));
         if (sink) {
-          x.x = acc[i][mm][0] * a / sum; x.y = acc[i][mm][1] * a / sum; x.z = acc[i][mm][2] * a / sum; x.w = acc[i][mm][3] * a / sum;
-        } else {
-          x.x = acc[i][mm][0] / sum; x.y = acc[i][mm][1] / sum; x.z = acc[i][mm][2] / sum; x.w = acc[i][mm][3] / sum;
+          x.x *= a; x.y *= a; x.z *= a; x.w *= a;
         }
+        x.x /= sum; x.y /= sum; x.z /= sum; x.w /= sum;
         *reinterpret_cast<float4*>(o + c) = x;
       }
     }

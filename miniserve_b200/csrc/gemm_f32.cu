@@ -64,61 +64,68 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
   }
 }
 
-// The same products in larger tiles: BM x BN outputs a CTA, 8 x 8 a thread (two runs of four rows by two of four columns), k in steps of
-// 16 through two shared-memory buffers, the next step's operands on their way in registers. The order of an element's sum is the same.
+// The same products in larger tiles: BM x 128 outputs a CTA, 8 x 8 a thread, k in steps of 16 through two shared-memory buffers, the next
+// step's operands on their way in registers, two neighbouring columns a multiply-add instruction (fma.rn.f32x2: each half rounds as fmaf
+// does). The order of an element's sum is the same. Needs rows that start on 16 bytes.
 // Bound by FFMA issue (34 TFMA/s on the whole GPU) beside shared-memory reads: a thread's 16 operands for 64 products are what keeps
-// the two even; at 4 x 4 the reads take twice the products' time.
-constexpr int GK = 16;
-template <int BM, int BN>
-__global__ void __launch_bounds__(BM * BN / 64)
+// the two even; at 4 x 4 the reads take twice the products' time. 700 rows: 1024 -> 4096
+// columns 151 us against 262 at 4 x 4, 2048 -> 1024 113 / 208, 1024 -> 6144 207 / 401, 3072 -> 1024 165 / 311; one column an instruction: 184, 172,
+// 224, 255 (a warp alone on its scheduler issues every second cycle).
+constexpr int GK = 16, GBN2 = 128;
+template <int BM>
+__global__ void __launch_bounds__(BM * 2, BM == 128 ? 2 : 3)
 gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K, int lda, int ldw, int ldc,
-                      long long stride_a, long long stride_w, long long stride_c, int vec) {
-  constexpr int THREADS = BM * BN / 64, TX = BN / 8, LA = BM * GK / 4 / THREADS, LW = BN * GK / 4 / THREADS;  // float4 a thread brings in
-  static_assert(LA * THREADS * 4 == BM * GK && LW * THREADS * 4 == BN * GK, "whole float4 a thread");
+                      long long stride_a, long long stride_w, long long stride_c) {
+  constexpr int THREADS = BM * 2, LA = BM * GK / 4 / THREADS, LW = GBN2 * GK / 4 / THREADS;  // pieces of 16 bytes a thread
+  static_assert(LA * THREADS * 4 == BM * GK && LW * THREADS * 4 == GBN2 * GK, "whole pieces a thread");
+  __shared__ __align__(16) float as[2][GK][BM + 4], ws[2][GK][GBN2 + 4];
+  pdl_prologue();
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * GBN2;
   A += blockIdx.z * stride_a;
   W += blockIdx.z * stride_w;
   C += blockIdx.z * stride_c;
-  __shared__ __align__(16) float as[2][GK][BM + 4], ws[2][GK][BN + 4];
-  pdl_prologue();
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  auto fetch = [&](const float* src, int ld, int row, int rows, int k) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);  // (zeros behind the ends: fma(0, 0, x) is x)
-    if (row < rows) {
-      const float* p = src + (size_t)row * ld + k;
-      if (vec && k + 4 <= K) return *reinterpret_cast<const float4*>(p);
-      if (k < K) v.x = p[0];
-      if (k + 1 < K) v.y = p[1];
-      if (k + 2 < K) v.z = p[2];
-      if (k + 3 < K) v.w = p[3];
-    }
-    return v;
-  };
+  const int pr = tid >> 2, pk = (tid & 3) * 4;
+  const float *ap[LA], *wp[LW];  // (rows behind the end read the last one: what comes of them is not stored)
+#pragma unroll
+  for (int i = 0; i < LA; ++i) ap[i] = A + (size_t)min(m0 + pr + i * (THREADS / 4), M - 1) * lda + pk;
+#pragma unroll
+  for (int i = 0; i < LW; ++i) wp[i] = W + (size_t)min(n0 + pr + i * (THREADS / 4), N - 1) * ldw + pk;
   float4 ra[LA], rw[LW];
   auto load = [&](int k0) {
+    if (k0 + GK <= K) {
 #pragma unroll
-    for (int i = 0; i < LA; ++i) ra[i] = fetch(A, lda, m0 + (tid + i * THREADS) / 4, M, k0 + (tid & 3) * 4);
+      for (int i = 0; i < LA; ++i) ra[i] = *reinterpret_cast<const float4*>(ap[i] + k0);
 #pragma unroll
-    for (int i = 0; i < LW; ++i) rw[i] = fetch(W, ldw, n0 + (tid + i * THREADS) / 4, N, k0 + (tid & 3) * 4);
+      for (int i = 0; i < LW; ++i) rw[i] = *reinterpret_cast<const float4*>(wp[i] + k0);
+    } else {  // zeros behind the last k: fma(0, 0, x) is x
+      auto piece = [&](const float* p) {
+        const int k = k0 + pk;
+        return make_float4(k < K ? p[k0] : 0.f, k + 1 < K ? p[k0 + 1] : 0.f, k + 2 < K ? p[k0 + 2] : 0.f, k + 3 < K ? p[k0 + 3] : 0.f);
+      };
+#pragma unroll
+      for (int i = 0; i < LA; ++i) ra[i] = piece(ap[i]);
+#pragma unroll
+      for (int i = 0; i < LW; ++i) rw[i] = piece(wp[i]);
+    }
   };
   auto put = [&](int buf) {
-    const int k = (tid & 3) * 4;
 #pragma unroll
     for (int i = 0; i < LA; ++i) {
-      const int r = (tid + i * THREADS) / 4;
-      as[buf][k][r] = ra[i].x; as[buf][k + 1][r] = ra[i].y; as[buf][k + 2][r] = ra[i].z; as[buf][k + 3][r] = ra[i].w;
+      float* p = &as[buf][pk][pr + i * (THREADS / 4)];
+      p[0] = ra[i].x; p[BM + 4] = ra[i].y; p[2 * (BM + 4)] = ra[i].z; p[3 * (BM + 4)] = ra[i].w;
     }
 #pragma unroll
     for (int i = 0; i < LW; ++i) {
-      const int r = (tid + i * THREADS) / 4;
-      ws[buf][k][r] = rw[i].x; ws[buf][k + 1][r] = rw[i].y; ws[buf][k + 2][r] = rw[i].z; ws[buf][k + 3][r] = rw[i].w;
+      float* p = &ws[buf][pk][pr + i * (THREADS / 4)];
+      p[0] = rw[i].x; p[GBN2 + 4] = rw[i].y; p[2 * (GBN2 + 4)] = rw[i].z; p[3 * (GBN2 + 4)] = rw[i].w;
     }
   };
-  float acc[8][8];
+  unsigned long long acc[8][4];  // two columns each
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
   load(0);
   put(0);
   __syncthreads();
@@ -128,32 +135,49 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
     if (more) load(k0 + GK);
 #pragma unroll
     for (int kk = 0; kk < GK; ++kk) {
-      float a[8], w[8];
+      float a[8];
+      ulonglong2 w[2];
       *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&as[buf][kk][ty * 4]);
       *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&as[buf][kk][BM / 2 + ty * 4]);
-      *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(&ws[buf][kk][tx * 4]);
-      *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(&ws[buf][kk][BN / 2 + tx * 4]);
+      w[0] = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][tx * 4]);
+      w[1] = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][GBN2 / 2 + tx * 4]);
+      const unsigned long long wj[4] = {w[0].x, w[0].y, w[1].x, w[1].y};
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 8; ++i) {
+        unsigned long long twice;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(twice) : "f"(a[i]));
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(twice), "l"(wj[j]));
+      }
     }
     if (more) put(buf ^ 1);
     __syncthreads();
   }
+  const bool wide = ldc % 4 == 0 && stride_c % 4 == 0 && (uintptr_t)C % 16 == 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int m = m0 + (i >> 2) * (BM / 2) + ty * 4 + (i & 3);
     if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int n = n0 + (j >> 2) * (BN / 2) + tx * 4 + (j & 3);
-      if (n < N) C[(size_t)m * ldc + n] = acc[i][j];
+    for (int half = 0; half < 2; ++half) {
+      const int n = n0 + half * (GBN2 / 2) + tx * 4;
+      float f[4];
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(f[0]), "=f"(f[1]) : "l"(acc[i][2 * half]));
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(f[2]), "=f"(f[3]) : "l"(acc[i][2 * half + 1]));
+      float* p = C + (size_t)m * ldc + n;
+      if (wide && n + 4 <= N) {
+        *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (n + e < N) p[e] = f[e];
+      }
     }
   }
 }
 
-// Which tile: what takes the fewest outputs on the busiest SM. GBM x GBN (4 x 4 a thread, half the rate) where there are few rows.
+// The rows of a tile: what leaves the busiest SM the fewest outputs. GBM x GBN (4 x 4 a thread, half the rate) where there are few rows
+// or columns, or rows that do not start on 16 bytes.
 inline int launch_gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int batch, long long stride_a,
                            long long stride_w, long long stride_c, cudaStream_t stream) {
   static int sms = 0;
@@ -162,21 +186,22 @@ inline int launch_gemm_f32(float* C, const float* A, const float* W, int M, int 
     MS_CHECK_CUDA(cudaGetDevice(&dev));
     MS_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   }
-  const int vec = lda % 4 == 0 && ldw % 4 == 0 && stride_a % 4 == 0 && stride_w % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
-  auto cost = [&](int bm, int bn, int slower) {
+  const bool rows16 = lda % 4 == 0 && ldw % 4 == 0 && stride_a % 4 == 0 && stride_w % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+  auto cost = [&](int bm, int bn) {
     const long long tiles = (long long)ceil_div(M, bm) * ceil_div(N, bn) * batch;
-    return (tiles + sms - 1) / sms * bm * bn * slower;
+    return (tiles + sms - 1) / sms * bm * bn;
   };
-  const long long small = cost(GBM, GBN, 2), wide = cost(64, 128, 1), large = cost(128, 128, 1), narrow = cost(64, 64, 1) * 5 / 4;
-#define MS_GEMM_F32(BM, BN)                                                                                                                    \
-  MS_LAUNCH((gemm_f32_tiled_kernel<BM, BN>), dim3(ceil_div(N, BN), ceil_div(M, BM), batch), BM * BN / 64, 0, stream, C, A, W, M, N, K, lda, ldw, ldc, \
-            stride_a, stride_w, stride_c, vec)
-  if (M <= 32 || small < wide) {
+  const long long large = cost(128, GBN2), small = cost(64, GBN2);
+  if (!rows16 || M <= 32 || 2 * cost(GBM, GBN) < (large < small ? large : small)) {
     MS_LAUNCH(gemm_f32_kernel, dim3(ceil_div(N, GBN), ceil_div(M, GBM), batch), 256, 0, stream, C, A, W, M, N, K, lda, ldw, ldc, stride_a, stride_w,
               stride_c);
-  } else if (large <= wide && large <= narrow) MS_GEMM_F32(128, 128);
-  else if (wide <= narrow) MS_GEMM_F32(64, 128);
-  else MS_GEMM_F32(64, 64);
+    return 0;
+  }
+#define MS_GEMM_F32(BM)                                                                                                                         \
+  MS_LAUNCH(gemm_f32_tiled_kernel<BM>, dim3(ceil_div(N, GBN2), ceil_div(M, BM), batch), BM * 2, 0, stream, C, A, W, M, N, K, lda, ldw, ldc, stride_a, \
+            stride_w, stride_c)
+  if (large <= small) MS_GEMM_F32(128);
+  else MS_GEMM_F32(64);
 #undef MS_GEMM_F32
   return 0;
 }
