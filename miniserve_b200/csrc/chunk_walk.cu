@@ -687,14 +687,17 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
   }
 }
 
-// Dynamic shared memory beyond 48 KB is asked for once per kernel.
+// Dynamic shared memory beyond 48 KB is asked for once per kernel. Not a dependent launch: CTAs that become resident while the kernel
+// before drains gather on the SMs that are free first, and two chains on one SM walk at half the rate (16 heads of 64 x 64 with the delta
+// rule over 2,048 tokens, both kernels: 140 us against 188; 32 heads of 128 x 64 with a decay per head 134 against 238).
 #define MS_WALK_LAUNCH(MODE, N, MT, grid, ...)                                                                            \
   do {                                                                                                                    \
     auto walk = walk_kernel<MODE, N, MT>;                                                                                 \
     constexpr size_t bytes = WalkItems<MODE, N, MT>::bytes;                                                               \
     static const cudaError_t asked = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
     MS_CHECK_CUDA(asked);                                                                                                 \
-    MS_LAUNCH(walk, grid, WK_THREADS, bytes, stream, __VA_ARGS__);                                                        \
+    walk<<<grid, WK_THREADS, bytes, stream>>>(__VA_ARGS__);                                                               \
+    MS_CHECK_LAUNCH();                                                                                                    \
   } while (0)
 
 template <typename TIn, typename TZ, bool DELTA, int N>
