@@ -493,8 +493,8 @@ MS_EXPORT int ms_attention_tiled_f32(float* out, const float* q, const float* k_
     constexpr size_t smem = ((TW_ROWS + 4 * TW_KEYS) * (32 * MD + 4) + TW_ROWS * TW_LDS + 2 * TW_ROWS) * 4;                                     \
     static const cudaError_t asked = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                      \
     MS_CHECK_CUDA(asked);                                                                                                                       \
-    MS_LAUNCH(kernel, grid, TW_THREADS, smem, stream, out, q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, num_rows, nq, nkv, head_dim, \
-              scale, window, sink, page_shift, num_pages, status, sink_values, softcap, chunk, dist_r1, dist_r2, keep_first);                   \
+    MS_LAUNCH_APART(kernel, grid, TW_THREADS, smem, stream, out, q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, num_rows, nq, nkv, \
+                    head_dim, scale, window, sink, page_shift, num_pages, status, sink_values, softcap, chunk, dist_r1, dist_r2, keep_first);                   \
   } while (0)
   if (head_dim <= 32) MS_TILED_LAUNCH(1);
   else if (head_dim <= 64) MS_TILED_LAUNCH(2);

@@ -696,8 +696,7 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
     constexpr size_t bytes = WalkItems<MODE, N, MT>::bytes;                                                               \
     static const cudaError_t asked = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
     MS_CHECK_CUDA(asked);                                                                                                 \
-    walk<<<grid, WK_THREADS, bytes, stream>>>(__VA_ARGS__);                                                               \
-    MS_CHECK_LAUNCH();                                                                                                    \
+    MS_LAUNCH_APART(walk, grid, WK_THREADS, bytes, stream, __VA_ARGS__);                                                  \
   } while (0)
 
 template <typename TIn, typename TZ, bool DELTA, int N>

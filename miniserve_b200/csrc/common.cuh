@@ -203,5 +203,12 @@ enum MsDtype : int { MS_F32 = 0, MS_BF16 = 1 };
   MS_EXPORT void name(int on) { ::ms::pdl_switch() = on; }
 #define MS_LAUNCH(kernel, grid, block, smem, stream, ...) \
   MS_CHECK_CUDA(::ms::launch(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__))
+// Not a dependent launch: for a long kernel with few or uneven CTAs. CTAs that become resident while the kernel before drains gather on
+// the SMs that are free first, and share them until they end.
+#define MS_LAUNCH_APART(kernel, grid, block, smem, stream, ...)                                     \
+  do {                                                                                              \
+    (kernel)<<<dim3(grid), dim3(block), (size_t)(smem), stream>>>(__VA_ARGS__);                     \
+    MS_CHECK_LAUNCH();                                                                              \
+  } while (0)
 #define MS_LAUNCH_CLUSTERED(kernel, grid, block, smem, stream, cluster_x, ...) \
   MS_CHECK_CUDA(::ms::launch_clustered(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, (unsigned)(cluster_x), __VA_ARGS__))

@@ -198,8 +198,8 @@ inline int launch_gemm_f32(float* C, const float* A, const float* W, int M, int 
     return 0;
   }
 #define MS_GEMM_F32(BM)                                                                                                                         \
-  MS_LAUNCH(gemm_f32_tiled_kernel<BM>, dim3(ceil_div(N, GBN2), ceil_div(M, BM), batch), BM * 2, 0, stream, C, A, W, M, N, K, lda, ldw, ldc, stride_a, \
-            stride_w, stride_c)
+  MS_LAUNCH_APART(gemm_f32_tiled_kernel<BM>, dim3(ceil_div(N, GBN2), ceil_div(M, BM), batch), BM * 2, 0, stream, C, A, W, M, N, K, lda, ldw, ldc, \
+                  stride_a, stride_w, stride_c)
   if (large <= small) MS_GEMM_F32(128);
   else MS_GEMM_F32(64);
 #undef MS_GEMM_F32
