@@ -14,7 +14,8 @@
 // The second walks a row's chunks in order, a CTA per (16 value columns, head, row): the products of a chunk against the state
 // that stays in registers. Both keep 32 bits: sums and the state are float32, and a factor of a tensor-core product is given as two
 // tf32 numbers, hi = round(x) and lo = round(x - hi) (22 bits and more of x), of which the three products that matter are made.
-// Against 64-bit sums the results are as far off as the token-by-token walk's (a few 1e-8 of the terms' size).
+// Against 64-bit sums the results are as far off as the token-by-token walk's (a few 1e-8 of the terms' size). A value that is not
+// finite makes its column of the whole chunk NaN, in the tokens ahead of it too (a pair that is left out counts zero times it).
 //
 // What bounds it: the walk is a chain of tokens / 16 steps, each a few dependent tensor-core products and two barriers (one without
 // the delta rule); the token-by-token walk is a chain of `tokens` steps of two lane-group sums each.
@@ -790,7 +791,7 @@ MS_EXPORT int ms_walk_scan(float* o, float* state, const void* q, int ld_q, cons
   if (num_rows == 0 || max_chunks == 0) return 0;
   MS_CHECK_ARG(dk >= 1 && dk <= 128 && dv >= 1 && H >= 1 && H <= 65535 && num_rows <= 65535, "walk_scan: %d heads of %d x %d, %d rows", H, dk, dv, num_rows);
   MS_CHECK_ARG(qk_group > 0 && H % qk_group == 0, "walk_scan: %d heads are not a multiple of the group of %d", H, qk_group);
-  MS_CHECK_ARG(!delta || (beta != nullptr && v_scale == nullptr), "walk_scan: the delta rule needs beta and takes no factor on the values");
+  MS_CHECK_ARG(!delta || beta != nullptr, "walk_scan: the delta rule needs beta");
   MS_CHECK_ARG((uintptr_t)scratch % 16 == 0, "walk_scan: scratch must start on 16 bytes");
   const int2* tb = reinterpret_cast<const int2*>(tab);
 #define MS_WALK(TIN, TZZ)                                                                                                                      \

@@ -541,13 +541,13 @@ def attention_rowwise(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, 
         int(extras.chunk or 0), _ptr(extras.dist_r1), _ptr(extras.dist_r2), int(extras.keep_first or 0)))
 
 
-def attention_tiled_ok(q: torch.Tensor, k_pool: torch.Tensor, ctx) -> bool:
+def attention_tiled_ok(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx) -> bool:
     """Whether a float32 step runs ``attention_tiled``: a step that is not all single tokens (those keep a warp per token and head), head
-    sizes of whole fours up to 128."""
+    sizes of whole fours up to 128, tensors that start on 16 bytes."""
     if q.dtype != torch.float32 or getattr(ctx, "decode_only", False) or q.shape[0] <= ctx.num_rows:
         return False
     return (bool(native.kernels().ms_attention_tiled_f32_supports(q.shape[2], q.shape[1], k_pool.shape[1]))
-            and q.data_ptr() % 16 == 0 and k_pool.data_ptr() % 16 == 0)
+            and all(x.data_ptr() % 16 == 0 for x in (out, q, k_pool, v_pool)))
 
 
 def attention_tiled(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx, group: int, scale: float,
@@ -608,7 +608,7 @@ def attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: 
     from . import attention_bf16
 
     extras = extras if extras is not None and extras.any else None
-    if attention_tiled_ok(q, k_pool, ctx):
+    if attention_tiled_ok(out, q, k_pool, v_pool, ctx):
         attention_tiled(out, q, k_pool, v_pool, ctx, group, scale, window, sink, extras)
         return
     if extras is not None and not (q.dtype == torch.bfloat16 and attention_bf16.takes_extras(q.shape[2], k_pool.shape[2])):

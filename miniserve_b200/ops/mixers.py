@@ -286,8 +286,9 @@ WALK_MIN_TOKENS = 16
 
 def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool = False, bonus=None) -> bool:
     """Whether ``decay_scan`` walks the step by chunks of 16 tokens (``csrc/chunk_walk.cu``): a step that is not all single tokens, heads of up
-    to 128 key channels; with one decay per head float32 operands whose rows start on 16 bytes, 32, 64 or 128 key channels."""
-    if ctx.decode_only or q.shape[0] < WALK_MIN_TOKENS or ones_column or bonus is not None or dk > 128:
+    to 128 key channels, no more rows than a grid's last dimension; with one decay per head float32 operands whose rows start on 16 bytes, 32, 64
+    or 128 key channels."""
+    if ctx.decode_only or q.shape[0] < WALK_MIN_TOKENS or ctx.num_rows > 65535 or ones_column or bonus is not None or dk > 128:
         return False
     if not head_decay:
         return True

@@ -72,7 +72,7 @@ def _both(run, q, k, v, dk, head_decay, want, size, last, state, heads, dv):
 @pytest.mark.parametrize("dtype, z_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16)])
 @pytest.mark.parametrize("rule", ["decay", "delta"])
 @pytest.mark.parametrize("heads, groups, dk, dv, pad", [(2, 1, 64, 64, 8), (3, 3, 10, 6, 3), (4, 2, 24, 40, 8), (1, 1, 72, 136, 1), (2, 2, 128, 16, 8),
-                                                        (1, 1, 32, 17, 4), (1, 1, 1, 1, 0)])
+                                                        (1, 1, 32, 17, 4), (1, 1, 1, 1, 0), (6, 2, 40, 20, 0)])
 def test_channel_decays_by_chunks(dtype, z_dtype, rule, heads, groups, dk, dv, pad):
     gen = torch.Generator().manual_seed(dk * 1000 + dv)
     t, delta = sum(n for _, n in ROWS), rule == "delta"
@@ -87,13 +87,16 @@ def test_channel_decays_by_chunks(dtype, z_dtype, rule, heads, groups, dk, dv, p
     z = z.to(z_dtype).to(DEV)
     bias, coef = (torch.randn(heads * dk, generator=gen) * 0.3).to(DEV), (torch.rand(heads, generator=gen) + 0.2).to(DEV)
     beta = torch.randn(t, heads + 3, generator=gen).to(z_dtype).to(DEV)[:, 2:2 + heads] if delta else None
+    scale = torch.rand(t, heads, generator=gen).to(DEV) if pad == 0 else None  # (a factor per token and head on the values)
     state = torch.randn(len(ROWS), heads, dv, dk, generator=gen).to(DEV)
+    vd = v.double().cpu().view(t, heads, dv) * (1.0 if scale is None else scale.double().cpu()[:, :, None])
     wide = lambda x: x.double().cpu().view(t, groups, dk).repeat_interleave(heads // groups, dim=1)  # noqa: E731
     soft = torch.nn.functional.softplus(z.double().cpu() + bias.double().cpu(), threshold=1e9).view(t, heads, dk)
     decay = torch.exp(-coef.double().cpu()[None, :, None] * soft)
-    exact = _exact(wide(q) * 0.3, wide(k), v.double().cpu().view(t, heads, dv), decay, torch.sigmoid(beta.double().cpu()) if delta else None,
+    exact = _exact(wide(q) * 0.3, wide(k), vd, decay, torch.sigmoid(beta.double().cpu()) if delta else None,
                    ROWS, SLOTS, state.double().cpu())
-    _both(lambda o, st, ctx: ops.decay_scan(o, st, q, k, v, z, bias, coef, 1.0, beta, ctx, heads, dk, dv, 0.3, delta=delta),
+    _both(lambda o, st, ctx: ops.decay_scan(o, st, q, k, v, z, bias, coef, 1.0, beta, ctx, heads, dk, dv, 0.3, delta=delta,
+                                            v_scale=scale),
           q, k, v, dk, False, *exact, state, heads, dv)
 
 

@@ -66,7 +66,7 @@ def test_prompt_attention_in_tiles_is_the_row_wise_one_bit_for_bit(extra, nq, nk
     want, got = (torch.full_like(q, float("nan")) for _ in range(2))
     ops.attention_rowwise(want, q, pb.k_pool, pb.v_pool, ctx.positions, ctx.row_of_token, ctx.page_indptr[0], ctx.page_indices[0], d ** -0.5, window,
                           ctx.status, sink=e.get("sink", False), extras=extras)
-    assert ops.attention_tiled_ok(q, pb.k_pool, ctx)
+    assert ops.attention_tiled_ok(got, q, pb.k_pool, pb.v_pool, ctx)
     ops.attention(got, q, pb.k_pool, pb.v_pool, ctx, 0, d ** -0.5, window, e.get("sink", False), extras)
     assert ctx.status.item() == 0 and not torch.isnan(want).any() and torch.equal(got, want)
 
