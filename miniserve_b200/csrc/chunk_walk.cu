@@ -88,40 +88,36 @@ __device__ __forceinline__ void wk_load(float (&f)[N], const float* p) {
 }
 
 // ---------------------------------------------------------------- the chunks of a step
-// tab[c] = (row, first flat token) of chunk c, row_first[r] the row's first chunk (row_first[num_rows]: how many chunks there are). One CTA.
-__global__ void __launch_bounds__(256)
-walk_table_kernel(int2* __restrict__ tab, int* __restrict__ row_first, const int* __restrict__ cu_q, int num_rows) {
-  pdl_prologue();
-  __shared__ int first[257], begin[256];
+// A row of n tokens has ceil(n / 16) chunks, numbered row by row. Every warp finds its own by adding up over the rows, 32 at a time: a table
+// made by a launch of its own costs a small step more on the host (4 us) than these sums cost on the device.
+
+// (row, first flat token) of a chunk, the same in every lane; row -1 behind the last chunk
+__device__ __forceinline__ int2 wk_at(int chunk, const int* __restrict__ cu_q, int num_rows) {
+  const int lane = threadIdx.x & 31;
   int base = 0;
-  for (int r0 = 0; r0 < num_rows; r0 += 256) {
-    const int r = r0 + threadIdx.x;
-    const int t0 = r < num_rows ? cu_q[r] : 0, len = r < num_rows ? cu_q[r + 1] - t0 : 0;
-    begin[threadIdx.x] = t0;
-    first[threadIdx.x + 1] = (len + WK_TOK - 1) / WK_TOK;
-    if (threadIdx.x == 0) first[0] = 0;
-    __syncthreads();
-    for (int o = 1; o < 256; o <<= 1) {  // sums up to and including each row
-      const int add = (int)threadIdx.x >= o ? first[threadIdx.x + 1 - o] : 0;
-      __syncthreads();
-      first[threadIdx.x + 1] += add;
-      __syncthreads();
+  for (int r0 = 0; r0 < num_rows; r0 += 32) {
+    const int r = r0 + lane;
+    const int begin = r < num_rows ? cu_q[r] : 0, mine = r < num_rows ? (cu_q[r + 1] - begin + WK_TOK - 1) / WK_TOK : 0;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += x;
     }
-    if (r < num_rows) row_first[r] = base + first[threadIdx.x];
-    const int rows = min(256, num_rows - r0), total = first[rows];
-    for (int c = threadIdx.x; c < total; c += 256) {
-      int lo = 0, hi = rows - 1;  // the last row whose first chunk is at most c
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (first[mid] <= c) lo = mid;
-        else hi = mid - 1;
-      }
-      tab[base + c] = make_int2(r0 + lo, begin[lo] + (c - first[lo]) * WK_TOK);
+    const unsigned hit = __ballot_sync(0xffffffffu, chunk < base + upto);
+    if (hit) {
+      const int at = __ffs(hit) - 1;
+      return make_int2(r0 + at, __shfl_sync(0xffffffffu, begin, at) + (chunk - base - __shfl_sync(0xffffffffu, upto - mine, at)) * WK_TOK);
     }
-    base += total;
-    __syncthreads();
+    base += __shfl_sync(0xffffffffu, upto, 31);
   }
-  if (threadIdx.x == 0) row_first[num_rows] = base;
+  return make_int2(-1, 0);
+}
+// how many chunks the rows ahead of `row` have
+__device__ __forceinline__ int wk_first(int row, const int* __restrict__ cu_q) {
+  int sum = 0;
+  for (int r = threadIdx.x & 31; r < row; r += 32) sum += (cu_q[r + 1] - cu_q[r] + WK_TOK - 1) / WK_TOK;
+  return __reduce_add_sync(0xffffffffu, sum);
 }
 
 // ---------------------------------------------------------------- what a chunk needs beside the state (a decay per key channel)
@@ -136,16 +132,16 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
                     float* __restrict__ u0_out, float* __restrict__ pairs, const TIn* __restrict__ q, int ld_q, const TIn* __restrict__ k,
                     int ld_k, int qk_group, const TIn* __restrict__ v, int ld_v, const TZ* __restrict__ z, int ld_z,
                     const float* __restrict__ z_bias, const float* __restrict__ decay_coef, float z_sign, const TZ* __restrict__ beta,
-                    int ld_beta, const float* __restrict__ v_scale, const int2* __restrict__ tab, const int* __restrict__ row_first,
-                    const int* __restrict__ cu_q, int num_rows, int H, int dk, int dv, int dvp, float q_scale) {
+                    int ld_beta, const float* __restrict__ v_scale, const int* __restrict__ cu_q, int num_rows, int H, int dk, int dv, int dvp,
+                    float q_scale) {
   constexpr int DKP = 32 * N;
   __shared__ __align__(16) float qs[WK_TOK][DKP], ks[WK_TOK][DKP], ds[WK_TOK][DKP];
   __shared__ __align__(16) float am[DELTA ? WK_TOK : 1][WK_TOK + 4];
   __shared__ float bs[WK_TOK], vsc[WK_TOK];
   pdl_prologue();
   const int chunk = blockIdx.x, h = blockIdx.y;
-  if (chunk >= row_first[num_rows]) return;
-  const int2 at = tab[chunk];
+  const int2 at = wk_at(chunk, cu_q, num_rows);
+  if (at.x < 0) return;
   const int t0 = at.y, n = min(WK_TOK, cu_q[at.x + 1] - t0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t qk_at = (size_t)(h / qk_group) * dk;
@@ -302,8 +298,8 @@ template <int MODE, int N, int MT>
 __global__ void __launch_bounds__(WK_THREADS)
 walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __restrict__ qp, int ld_q, const float* __restrict__ wp,
             const float* __restrict__ kp, int ld_k, int qk_group, const float* __restrict__ dec, const float* __restrict__ v, int ld_v,
-            const float* __restrict__ v_scale, const float* __restrict__ pairs, const int* __restrict__ row_first, const int* __restrict__ cu_q,
-            const int* __restrict__ q_start, const int* __restrict__ state_slot, int H, int dk, int dv) {
+            const float* __restrict__ v_scale, const float* __restrict__ pairs, const int* __restrict__ cu_q, const int* __restrict__ q_start,
+            const int* __restrict__ state_slot, int H, int dk, int dv) {
   using I = WalkItems<MODE, N, MT>;
   constexpr int DKP = 32 * N, COLS = I::cols, LD = I::ld, LDU = I::ldu, ST = I::stages;
   extern __shared__ __align__(16) float wk_smem[];
@@ -314,9 +310,11 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
   pdl_prologue();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int v0 = blockIdx.x * COLS, h = blockIdx.y, r = blockIdx.z;
-  const int c0 = row_first[r], c1 = row_first[r + 1];
-  if (c1 <= c0) return;
   const int row_begin = cu_q[r], row_end = cu_q[r + 1];
+  const int c0 = wk_first(r, cu_q);
+  int c1 = c0 + (row_end - row_begin + WK_TOK - 1) / WK_TOK;
+  asm volatile("" : "+r"(c1));  // (a number of chunks that the compiler can see to be above zero has it order the loop for fewer registers)
+  if (c1 <= c0) return;
   const int slice = warp * 8 * N;      // the warp's key channels
   const int mine = slice + 2 * N * t;  // the lane's 2 N of them as a product's operand,
   const int mine_n = slice + N * g;    // and its N as an accumulator's columns
@@ -626,14 +624,14 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
 template <int DK>
 __global__ void __launch_bounds__(WK_THREADS)
 walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const float* __restrict__ q, int ld_q, const float* __restrict__ k,
-                 int ld_k, int qk_group, const float* __restrict__ decay, int ld_decay, const int2* __restrict__ tab,
-                 const int* __restrict__ row_first, const int* __restrict__ cu_q, int num_rows, int H, float q_scale) {
+                 int ld_k, int qk_group, const float* __restrict__ decay, int ld_decay, const int* __restrict__ cu_q, int num_rows, int H,
+                 float q_scale) {
   __shared__ __align__(16) float qs[WK_TOK][DK + 4], ks[WK_TOK][DK + 4];
   __shared__ float dot[WK_TOK][WK_TOK + 1], as[WK_TOK][33];
   pdl_prologue();
   const int chunk = blockIdx.x, grp = blockIdx.y;
-  if (chunk >= row_first[num_rows]) return;
-  const int2 at = tab[chunk];
+  const int2 at = wk_at(chunk, cu_q, num_rows);
+  if (at.x < 0) return;
   const int t0 = at.y, n = min(WK_TOK, cu_q[at.x + 1] - t0);
   const int tid = threadIdx.x;
 #pragma unroll
@@ -703,8 +701,7 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
 template <typename TIn, typename TZ, bool DELTA, int N>
 int launch_walk(float* o, float* state, const TIn* q, int ld_q, const TIn* k, int ld_k, int qk_group, const TIn* v, int ld_v, const TZ* z,
                 int ld_z, const float* z_bias, const float* decay_coef, float z_sign, const TZ* beta, int ld_beta, const float* v_scale,
-                float* scratch, const int2* tab, const int* row_first, const int* cu_q, const int* q_start, const int* state_slot, int num_rows,
-                int max_chunks, int H, int dk, int dv, float q_scale, cudaStream_t stream) {
+                float* scratch, const int* cu_q, const int* q_start, const int* state_slot, int num_rows, int max_chunks, int H, int dk, int dv, float q_scale, cudaStream_t stream) {
   constexpr int DKP = 32 * N;
   const size_t items = (size_t)max_chunks * H;
   const int dvp = ceil_div(dv, WK_COLS) * WK_COLS;
@@ -716,9 +713,9 @@ int launch_walk(float* o, float* state, const TIn* q, int ld_q, const TIn* k, in
   float* wp = u0 + items * WK_TOK * dvp;
   auto prepare = walk_prepare_kernel<TIn, TZ, DELTA, N>;
   MS_LAUNCH(prepare, dim3(max_chunks, H), WK_THREADS, 0, stream, wp, qp, kp, last, u0, pairs, q, ld_q, k, ld_k, qk_group, v, ld_v, z, ld_z, z_bias,
-            decay_coef, z_sign, beta, ld_beta, v_scale, tab, row_first, cu_q, num_rows, H, dk, dv, dvp, q_scale);
+            decay_coef, z_sign, beta, ld_beta, v_scale, cu_q, num_rows, H, dk, dv, dvp, q_scale);
   MS_WALK_LAUNCH(DELTA ? WALK_DELTA : WALK_CHANNEL, N, 1, dim3(dvp / WK_COLS, H, num_rows), o, state, qp, DKP, wp, kp, DKP, 1, last, u0, dvp,
-                 (const float*)nullptr, pairs, row_first, cu_q, q_start, state_slot, H, dk, dv);
+                 (const float*)nullptr, pairs, cu_q, q_start, state_slot, H, dk, dv);
   return 0;
 }
 
@@ -737,9 +734,8 @@ int launch_walk_for(int delta, int dk, Args... args) {
 
 template <int N>
 int launch_walk_head(float* o, float* state, const float* q, int ld_q, const float* k, int ld_k, int qk_group, const float* v, int ld_v,
-                     const float* decay, int ld_decay, const float* v_scale, float* scratch, const int2* tab, const int* row_first,
-                     const int* cu_q, const int* q_start, const int* state_slot, int num_rows, int max_chunks, int H, int dv, float q_scale,
-                     cudaStream_t stream) {
+                     const float* decay, int ld_decay, const float* v_scale, float* scratch, const int* cu_q, const int* q_start,
+                     const int* state_slot, int num_rows, int max_chunks, int H, int dv, float q_scale, cudaStream_t stream) {
   constexpr int DK = 32 * N;
   static int sm_count = 0;
   if (sm_count == 0) {
@@ -750,15 +746,15 @@ int launch_walk_head(float* o, float* state, const float* q, int ld_q, const flo
   float* pairs = scratch;
   float* decays = pairs + (size_t)max_chunks * H * WK_TOK * WK_TOK;
   auto prepare = walk_head_kernel<DK>;
-  MS_LAUNCH(prepare, dim3(max_chunks, H / qk_group), WK_THREADS, 0, stream, pairs, decays, q, ld_q, k, ld_k, qk_group, decay, ld_decay, tab, row_first,
-            cu_q, num_rows, H, q_scale);
+  MS_LAUNCH(prepare, dim3(max_chunks, H / qk_group), WK_THREADS, 0, stream, pairs, decays, q, ld_q, k, ld_k, qk_group, decay, ld_decay, cu_q,
+            num_rows, H, q_scale);
   // 32 value columns a CTA share what they load and split of q and k, where that leaves two CTAs an SM
   if ((long long)num_rows * H * ceil_div(dv, 2 * WK_COLS) >= 2LL * sm_count)
     MS_WALK_LAUNCH(WALK_HEAD, N, 2, dim3(ceil_div(dv, WK_COLS * 2), H, num_rows), o, state, q, ld_q, (const float*)nullptr, k, ld_k, qk_group, decays, v,
-                   ld_v, v_scale, pairs, row_first, cu_q, q_start, state_slot, H, DK, dv);
+                   ld_v, v_scale, pairs, cu_q, q_start, state_slot, H, DK, dv);
   else
     MS_WALK_LAUNCH(WALK_HEAD, N, 1, dim3(ceil_div(dv, WK_COLS), H, num_rows), o, state, q, ld_q, (const float*)nullptr, k, ld_k, qk_group, decays, v,
-                   ld_v, v_scale, pairs, row_first, cu_q, q_start, state_slot, H, DK, dv);
+                   ld_v, v_scale, pairs, cu_q, q_start, state_slot, H, DK, dv);
   return 0;
 }
 
@@ -767,17 +763,11 @@ int launch_walk_head(float* o, float* state, const float* q, int ld_q, const flo
 using namespace ms;
 
 // The most chunks that a step of so many tokens in so many rows can have.
-MS_EXPORT int ms_walk_max(int tokens, int rows) { return tokens / WK_TOK + rows; }
+static inline int walk_max(int tokens, int rows) { return tokens / WK_TOK + rows; }
 
-MS_EXPORT int ms_walk_table(int* tab, int* row_first, const int* cu_q, int num_rows, cudaStream_t stream) {
-  if (num_rows == 0) return 0;
-  MS_LAUNCH(walk_table_kernel, 1, 256, 0, stream, reinterpret_cast<int2*>(tab), row_first, cu_q, num_rows);
-  return 0;
-}
-
-// Floats of scratch for a step of so many chunks. per_head: one decay per head.
-MS_EXPORT long long ms_walk_scratch(int chunks, int H, int dk, int dv, int delta, int per_head) {
-  const long long items = (long long)chunks * H, dkp = dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
+// Floats of scratch for a step of so many tokens in so many rows. per_head: one decay per head.
+MS_EXPORT long long ms_walk_scratch(int tokens, int rows, int H, int dk, int dv, int delta, int per_head) {
+  const long long items = (long long)walk_max(tokens, rows) * H, dkp = dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
   if (per_head) return items * (WK_TOK * WK_TOK + 3 * WK_TOK);
   return items * (WK_TOK * dkp * (delta ? 3 : 2) + dkp + WK_TOK * WK_TOK + (long long)WK_TOK * (ceil_div(dv, WK_COLS) * WK_COLS));
 }
@@ -785,18 +775,18 @@ MS_EXPORT long long ms_walk_scratch(int chunks, int H, int dk, int dv, int delta
 // The decay rule (delta 0) or the delta rule with a decay per key channel; operands as ms_decay_scan's, dk up to 128. o [T, H, dv] float32.
 MS_EXPORT int ms_walk_scan(float* o, float* state, const void* q, int ld_q, const void* k, int ld_k, int qk_group, const void* v, int ld_v,
                            const void* z, int ld_z, const float* z_bias, const float* decay_coef, float z_sign, const void* beta, int ld_beta,
-                           const float* v_scale, float* scratch, const int* tab, const int* row_first, const int* cu_q, const int* q_start,
-                           const int* state_slot, int num_rows, int max_chunks, int H, int dk, int dv, float q_scale, int delta, int in_dtype,
-                           int z_dtype, cudaStream_t stream) {
-  if (num_rows == 0 || max_chunks == 0) return 0;
+                           const float* v_scale, float* scratch, const int* cu_q, const int* q_start, const int* state_slot,
+                           int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, int delta, int in_dtype, int z_dtype,
+                           cudaStream_t stream) {
+  if (num_rows == 0 || num_tokens == 0) return 0;
   MS_CHECK_ARG(dk >= 1 && dk <= 128 && dv >= 1 && H >= 1 && H <= 65535 && num_rows <= 65535, "walk_scan: %d heads of %d x %d, %d rows", H, dk, dv, num_rows);
   MS_CHECK_ARG(qk_group > 0 && H % qk_group == 0, "walk_scan: %d heads are not a multiple of the group of %d", H, qk_group);
   MS_CHECK_ARG(!delta || beta != nullptr, "walk_scan: the delta rule needs beta");
   MS_CHECK_ARG((uintptr_t)scratch % 16 == 0, "walk_scan: scratch must start on 16 bytes");
-  const int2* tb = reinterpret_cast<const int2*>(tab);
+  const int max_chunks = walk_max(num_tokens, num_rows);
 #define MS_WALK(TIN, TZZ)                                                                                                                      \
   return launch_walk_for<TIN, TZZ>(delta, dk, o, state, (const TIN*)q, ld_q, (const TIN*)k, ld_k, qk_group, (const TIN*)v, ld_v, (const TZZ*)z, ld_z, \
-                                   z_bias, decay_coef, z_sign, (const TZZ*)beta, ld_beta, v_scale, scratch, tb, row_first, cu_q, q_start,      \
+                                   z_bias, decay_coef, z_sign, (const TZZ*)beta, ld_beta, v_scale, scratch, cu_q, q_start,      \
                                    state_slot, num_rows, max_chunks, H, dk, dv, q_scale, stream)
   if (in_dtype == MS_F32 && z_dtype == MS_F32) MS_WALK(float, float);
   if (in_dtype == MS_F32 && z_dtype == MS_BF16) MS_WALK(float, __nv_bfloat16);
@@ -809,17 +799,16 @@ MS_EXPORT int ms_walk_scan(float* o, float* state, const void* q, int ld_q, cons
 // The decay rule with one decay per head ([T, ld_decay] float32): q, k, v float32, dk 32, 64 or 128, rows of q and k that start on 16
 // bytes.
 MS_EXPORT int ms_walk_scan_head(float* o, float* state, const float* q, int ld_q, const float* k, int ld_k, int qk_group, const float* v, int ld_v,
-                                const float* decay, int ld_decay, const float* v_scale, float* scratch, const int* tab, const int* row_first,
-                                const int* cu_q, const int* q_start, const int* state_slot, int num_rows, int max_chunks, int H, int dk, int dv,
-                                float q_scale, cudaStream_t stream) {
-  if (num_rows == 0 || max_chunks == 0) return 0;
+                                const float* decay, int ld_decay, const float* v_scale, float* scratch, const int* cu_q, const int* q_start,
+                                const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, cudaStream_t stream) {
+  if (num_rows == 0 || num_tokens == 0) return 0;
   MS_CHECK_ARG((dk == 32 || dk == 64 || dk == 128) && dv >= 1 && H >= 1 && H <= 65535 && num_rows <= 65535, "walk_scan_head: %d heads of %d x %d", H, dk, dv);
   MS_CHECK_ARG(qk_group > 0 && H % qk_group == 0, "walk_scan_head: %d heads are not a multiple of the group of %d", H, qk_group);
   MS_CHECK_ARG((uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 && ld_q % 4 == 0 && ld_k % 4 == 0 && (uintptr_t)scratch % 16 == 0,
                "walk_scan_head: rows of q and k must start on 16 bytes");
-  const int2* tb = reinterpret_cast<const int2*>(tab);
+  const int max_chunks = walk_max(num_tokens, num_rows);
 #define MS_WALK(N)                                                                                                                            \
-  return launch_walk_head<N>(o, state, q, ld_q, k, ld_k, qk_group, v, ld_v, decay, ld_decay, v_scale, scratch, tb, row_first, cu_q, q_start, \
+  return launch_walk_head<N>(o, state, q, ld_q, k, ld_k, qk_group, v, ld_v, decay, ld_decay, v_scale, scratch, cu_q, q_start, \
                              state_slot, num_rows, max_chunks, H, dv, q_scale, stream)
   if (dk == 32) MS_WALK(1);
   if (dk == 64) MS_WALK(2);

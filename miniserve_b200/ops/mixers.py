@@ -205,7 +205,7 @@ def sum_bias(out, a, b=None, vec=None, stream=None) -> None:
 
 def decay_scan(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign: float, beta, ctx, heads: int, dk: int, dv: int,
                q_scale: float, delta: bool, head_decay: bool = False, v_scale=None, ones_column: bool = False, bonus=None) -> None:
-    """The token-by-token recurrence of every row of the step (``csrc/recurrence.cu``), from each
+    """The recurrence of every row of the step, token by token (``csrc/recurrence.cu``) or by chunks of 16 (``walk_ok``), from each
     request's slot of ``state`` [slots, heads, dv, dk] float32 (zero where a row starts at position 0)
     and back into it; o_out [T, heads, dv] float32. q, k [T, groups*dk], v [T, heads*dv], z [T, heads*dk]
     and beta [T, heads] are 2-d views; z_bias [heads*dk], decay_coef [heads] float32.
@@ -280,7 +280,7 @@ def conv_state_update(conv_state, x, ctx, taps: int) -> None:
 
 # Steps with fewer tokens stay on the token-by-token walk. Measured alone, chunks against walk in us: 16 heads of 64 x 64 with the delta rule 10 / 13
 # at 16 tokens, 13 / 37 at 64, 32 / 137 at 256 (58 / 62 for 63 single tokens beside 65); 8 of 64 x 128 with the decay rule 9 / 11, 14 / 29, 30 / 104;
-# 32 of 128 x 64 with a decay per head 10 / 16, 16 / 48, 38 / 179. The table of the chunks (3 us) is made once per step.
+# 32 of 128 x 64 with a decay per head 10 / 16, 16 / 48, 38 / 179.
 WALK_MIN_TOKENS = 16
 
 
@@ -296,20 +296,12 @@ def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool =
 
 
 def _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx, heads, dk, dv, q_scale, delta, head_decay, v_scale) -> None:
-    t, dev, rows = o_out.shape[0], o_out.device, ctx.num_rows
+    t, rows = o_out.shape[0], ctx.num_rows
     lib = native.recurrence()
-    most = int(lib.ms_walk_max(t, rows))
-    table = ctx.step_cache.get("walk.table") if hasattr(ctx, "step_cache") else None
-    if table is None:  # the same for every layer of the step
-        ints = torch.empty(2 * most + rows + 1, dtype=torch.int32, device=dev)
-        table = (ints[:2 * most], ints[2 * most:])
-        native.recurrence_check(lib.ms_walk_table(_ptr(table[0]), _ptr(table[1]), _ptr(ctx.cu_q), rows, ctx.stream))
-        if hasattr(ctx, "step_cache"):
-            ctx.step_cache["walk.table"] = table
-    scratch = ctx.buffer("walk.scratch", (int(lib.ms_walk_scratch(most, heads, dk, dv, int(delta), int(head_decay))),), torch.float32, dev)
+    scratch = ctx.buffer("walk.scratch", (int(lib.ms_walk_scratch(t, rows, heads, dk, dv, int(delta), int(head_decay))),), torch.float32,
+                         o_out.device)
     groups = q.shape[1] // dk
-    rest = (_ptr(v_scale), _ptr(scratch), _ptr(table[0]), _ptr(table[1]), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.state_slot), rows, most, heads,
-            dk, dv, float(q_scale))
+    rest = (_ptr(v_scale), _ptr(scratch), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.state_slot), t, rows, heads, dk, dv, float(q_scale))
     if head_decay:
         native.recurrence_check(lib.ms_walk_scan_head(
             _ptr(o_out), _ptr(state), _ptr(q), _rows(q), _ptr(k), _rows(k), heads // groups, _ptr(v), _rows(v), _ptr(z), _rows(z), *rest,
@@ -321,7 +313,7 @@ def _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx,
         launches=2)
 
 
-# The decay rule is linear in the state with a diagonal factor, so the rows of a step with many tokens are cut into
+# The decay rule is linear in the state with a diagonal factor, so the rows of a step with many tokens that ``walk_ok`` leaves are cut into
 # SEGMENTS pieces that are walked at the same time (``csrc/recurrence.cu``). Whether a step is cut follows from its
 # number of tokens alone (what a captured graph is keyed by), never from how the tokens are shared among rows.
 SEGMENTS = 8

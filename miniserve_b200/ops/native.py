@@ -180,11 +180,9 @@ def recurrence():
     _declare(lib, "ms_mlstm_output", [_p, _i, _p, _i, _p, _p, _p, _i, _i, _i, _i, _f, _f, _i, _p])
     _declare(lib, "ms_conv_bias", [_p, _p, _i, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p])
     _declare(lib, "ms_chunk_max", [_i, _i])
-    _declare(lib, "ms_walk_max", [_i, _i])
-    _declare(lib, "ms_walk_table", [_p, _p, _p, _i, _p])
-    _declare(lib, "ms_walk_scratch", [_i] * 6, _ll)
-    _declare(lib, "ms_walk_scan", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p, _f, _p, _i, _p, _p] + [_p] * 5 + [_i] * 5 + [_f, _i, _i, _i, _p])
-    _declare(lib, "ms_walk_scan_head", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p] + [_p] * 5 + [_i] * 5 + [_f, _p])
+    _declare(lib, "ms_walk_scratch", [_i] * 7, _ll)
+    _declare(lib, "ms_walk_scan", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p, _f, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _i, _i, _i, _p])
+    _declare(lib, "ms_walk_scan_head", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _p])
     _declare(lib, "ms_chunk_supports", [_i, _i])
     _declare(lib, "ms_chunk_table", [_p, _p, _p, _i, _p])
     _declare(lib, "ms_chunk_scan", [_p, _i, _p, _p, _i, _p, _i, _i, _p, _i] + [_p] * 11 + [_i] * 5 + [_f, _i, _p])

@@ -117,3 +117,22 @@ def test_head_decays_by_chunks(heads, groups, dk, dv, scaled):
     exact = _exact(wide(q) * 0.7, wide(k), vd, a.double().cpu()[:, :, None].expand(t, heads, dk), None, ROWS, SLOTS, state.double().cpu())
     _both(lambda o, st, ctx: ops.decay_scan(o, st, q, k, v, a, None, None, 0.0, None, ctx, heads, dk, dv, 0.7, delta=False, head_decay=True,
                                             v_scale=scale), q, k, v, dk, True, *exact, state, heads, dv)
+
+
+def test_many_rows():
+    """More rows than a warp has lanes, empty ones among them (also the first and the last)."""
+    gen = torch.Generator().manual_seed(7)
+    lens = [0, 1, 16, 17, 0, 0, 33] * 11 + [1] * 70 + [50, 0]
+    rows, slots = [(3 * (i % 2), n) for i, n in enumerate(lens)], torch.randperm(len(lens), generator=gen).tolist()
+    t, heads, d = sum(lens), 2, 32
+    q, k, v = (torch.randn(t, heads * d, generator=gen).to(DEV) for _ in range(3))
+    a, state = torch.rand(t, heads, generator=gen).to(DEV), torch.randn(len(rows), heads, d, d, generator=gen).to(DEV)
+    wide = lambda x: x.double().cpu().view(t, heads, d)  # noqa: E731
+    want, size, last = _exact(wide(q), wide(k), wide(v), a.double().cpu()[:, :, None].expand(t, heads, d), None, rows, slots, state.double().cpu())
+    for (start, n), slot in zip(rows, slots):
+        if n == 0:  # an empty row is no step of its request
+            last[slot] = state[slot].double().cpu()
+    ctx = _ctx(rows, slots)
+    o, st = torch.full((t, heads, d), float("nan"), device=DEV), state.clone()
+    ops.decay_scan(o, st, q, k, v, a, None, None, 0.0, None, ctx, heads, d, d, 1.0, delta=False, head_decay=True)
+    assert ((o.double().cpu() - want).abs() / size).max() < 1e-6 and ((st.double().cpu() - last).abs().max() / last.abs().max()) < 4e-6
