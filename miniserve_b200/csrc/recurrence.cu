@@ -14,9 +14,9 @@
 // fixed order. Tokens are taken in chunks: the CTA stages the chunk's q, k, v, decays (and beta) in
 // float32, all threads at once, then walks the chunk token by token. The decays of a prompt portion are
 // worked out beforehand by a kernel of their own (exponentials and logarithms for every token and
-// channel at once, instead of inside the serial walk); a decode step works them out while staging. A request's result
-// is the same bit for bit however its tokens are cut into steps and whatever else the step holds: the
-// state is carried in float32 and nothing in a token's arithmetic depends on the chunking.
+// channel at once, instead of inside the serial walk); a decode step works them out while staging. The state is carried in
+// float32 and nothing in a token's arithmetic depends on this chunking. Prompts with up to 128 key channels run the decay and the
+// delta rule in chunks of 16 tokens on the tensor cores instead (chunk_walk.cu).
 //
 // The decay is d = exp(-c_h * softplus(sign * (z + bias))) with z the output of a projection:
 // sign = -1, c_h = 1/tau gives sigmoid(z + bias)^(1/tau); sign = +1, c_h = exp(A_h) gives
@@ -481,13 +481,15 @@ __device__ __forceinline__ void store4(float* p, const float4& f) { *reinterpret
 // inputs in registers, so an input is read once. Bound by memory (2 bytes in, 4 out per channel and token): 2,048 x 6,144 bfloat16 take 38 us
 // (2.0 TB/s) where a warp per token and head takes 97; 2,048 x 2,048 with unit heads of 64 19 against 40. Heads
 // of dk channels that are divided by their length are dk / 4 neighbouring lanes (a power of two).
+// `update` (every row has one token): the thread that read a row's history leaves it one token further, which saves a decode step the
+// launch that does it for rows of any length.
 constexpr int CONV_RUN = 8, CONV_THREADS = 128;
 template <typename T, int TAPS, int RUN>
 __global__ void __launch_bounds__(CONV_THREADS)
-conv_silu_unit_x4_kernel(float* __restrict__ out, const T* __restrict__ proj, int ld, const T* __restrict__ conv_state, const float* __restrict__ w,
+conv_silu_unit_x4_kernel(float* __restrict__ out, const T* __restrict__ proj, int ld, T* conv_state, const float* __restrict__ w,
                          const int* __restrict__ row_of_token, const int* __restrict__ cu_q, const int* __restrict__ q_start,
                          const int* __restrict__ state_slot, int num_tokens, int C, int unit_channels, int lanes_per_head, float unit_eps,
-                         const float* __restrict__ bias) {
+                         const float* __restrict__ bias, int update) {
   pdl_prologue();
   const int ch = (blockIdx.x * CONV_THREADS + threadIdx.x) * 4;
   const int t0 = blockIdx.y * RUN;
@@ -525,6 +527,11 @@ conv_silu_unit_x4_kernel(float* __restrict__ out, const T* __restrict__ proj, in
 #pragma unroll
     for (int j = 0; j + 1 < TAPS; ++j) win[j] = win[j + 1];
     win[TAPS - 1] = x[i];
+    if (update && in) {
+      T* st = conv_state + (size_t)state_slot[current] * (TAPS - 1) * C + c;
+#pragma unroll
+      for (int j = 0; j + 1 < TAPS; ++j) store4(st + (size_t)j * C, win[j + 1]);
+    }
     float4 acc = b;
 #pragma unroll
     for (int j = 0; j < TAPS; ++j) {
@@ -801,10 +808,25 @@ MS_EXPORT int ms_segment_finish(float* o, float* state, const float* ends, float
   return 0;
 }
 
-MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, const void* conv_state, const float* w,
+MS_EXPORT int ms_conv_state_update(void* conv_state, const void* proj, int ld, const int* cu_q, const int* q_start,
+                                   const int* state_slot, int num_rows, int C, int taps, int dtype, cudaStream_t stream) {
+  if (num_rows == 0 || taps <= 1) return 0;
+  const long long items = (long long)num_rows * C;
+  const unsigned blocks = (unsigned)((items + 255) / 256);
+  if (dtype == MS_F32)
+    MS_LAUNCH(conv_state_update_kernel<float>, blocks, 256, 0, stream, (float*)conv_state, (const float*)proj, ld, cu_q, q_start,
+              state_slot, num_rows, C, taps);
+  else
+    MS_LAUNCH(conv_state_update_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (__nv_bfloat16*)conv_state,
+              (const __nv_bfloat16*)proj, ld, cu_q, q_start, state_slot, num_rows, C, taps);
+  return 0;
+}
+
+// update: 0 leaves the slots' histories as they are, 1 makes them those behind the step, 2 the same where every row has one token.
+MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, void* conv_state, const float* w,
                                 const int* row_of_token, const int* cu_q, const int* q_start, const int* state_slot,
                                 int num_tokens, int C, int taps, int unit_heads, int dk, int other_heads, int dv, float unit_eps,
-                                int dtype, const float* bias, cudaStream_t stream) {
+                                int dtype, const float* bias, int num_rows, int update, cudaStream_t stream) {
   if (num_tokens == 0) return 0;
   MS_CHECK_ARG(taps >= 1 && C == unit_heads * dk + other_heads * dv, "conv_silu_unit: %d channels are not %d x %d + %d x %d", C,
                unit_heads, dk, other_heads, dv);
@@ -822,8 +844,8 @@ MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, const void
     else MS_CONV_RUN(T, TAPS, 1);                       \
   } while (0)
 #define MS_CONV_RUN(T, TAPS, RUN)                                                                                                                      \
-  MS_LAUNCH((conv_silu_unit_x4_kernel<T, TAPS, RUN>), grid, CONV_THREADS, 0, stream, out, (const T*)proj, ld, (const T*)conv_state, w, row_of_token, cu_q, q_start, \
-            state_slot, num_tokens, C, unit_heads * dk, lanes, unit_eps, bias)
+  MS_LAUNCH((conv_silu_unit_x4_kernel<T, TAPS, RUN>), grid, CONV_THREADS, 0, stream, out, (const T*)proj, ld, (T*)conv_state, w, row_of_token, cu_q, q_start, \
+            state_slot, num_tokens, C, unit_heads * dk, lanes, unit_eps, bias, (int)(update == 2))
     if (dtype == MS_F32) {
       if (taps == 2) MS_CONV(float, 2);
       else if (taps == 3) MS_CONV(float, 3);
@@ -835,7 +857,7 @@ MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, const void
     }
 #undef MS_CONV
 #undef MS_CONV_RUN
-    return 0;
+    return update == 1 ? ms_conv_state_update(conv_state, proj, ld, cu_q, q_start, state_slot, num_rows, C, taps, dtype, stream) : 0;
   }
   const long long items = (long long)num_tokens * (unit_heads + other_heads);
   const int warps = 8;
@@ -847,21 +869,7 @@ MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, const void
     MS_LAUNCH(conv_silu_unit_kernel<__nv_bfloat16>, blocks, warps * 32, 0, stream, out, (const __nv_bfloat16*)proj, ld,
               (const __nv_bfloat16*)conv_state, w, row_of_token, cu_q, q_start, state_slot, num_tokens, C, taps, unit_heads, dk,
               other_heads, dv, unit_eps, bias);
-  return 0;
-}
-
-MS_EXPORT int ms_conv_state_update(void* conv_state, const void* proj, int ld, const int* cu_q, const int* q_start,
-                                   const int* state_slot, int num_rows, int C, int taps, int dtype, cudaStream_t stream) {
-  if (num_rows == 0 || taps <= 1) return 0;
-  const long long items = (long long)num_rows * C;
-  const unsigned blocks = (unsigned)((items + 255) / 256);
-  if (dtype == MS_F32)
-    MS_LAUNCH(conv_state_update_kernel<float>, blocks, 256, 0, stream, (float*)conv_state, (const float*)proj, ld, cu_q, q_start,
-              state_slot, num_rows, C, taps);
-  else
-    MS_LAUNCH(conv_state_update_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (__nv_bfloat16*)conv_state,
-              (const __nv_bfloat16*)proj, ld, cu_q, q_start, state_slot, num_rows, C, taps);
-  return 0;
+  return update ? ms_conv_state_update(conv_state, proj, ld, cu_q, q_start, state_slot, num_rows, C, taps, dtype, stream) : 0;
 }
 
 MS_EXPORT int ms_head_norm_gate(void* out, int ld_out, const float* o, const float* w, const void* gate, int ld_gate,

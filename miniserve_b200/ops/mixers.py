@@ -7,6 +7,8 @@ such an operand is passed as a 2-d view whose last stride is 1; its row stride g
 
 from __future__ import annotations
 
+from functools import lru_cache
+
 import torch
 
 from . import native
@@ -253,11 +255,12 @@ def decay_scan(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign: float, beta
 
 
 def conv_silu_unit(out, x, conv_state, weight, ctx, unit_heads: int, dk: int, other_heads: int, dv: int, unit_eps: float,
-                   bias=None) -> None:
+                   bias=None, update: bool = False) -> None:
     """out [T, C] float32 = SiLU(causal convolution over time of the C channels ``x`` [T, C], a view),
     the first ``unit_heads`` heads of dk channels then divided by sqrt(sum of squares + unit_eps).
     ``weight`` [C, taps] float32 (``bias`` [C] float32 is added if given); ``conv_state`` [slots, taps - 1, C] holds each
-    request's last inputs."""
+    request's last inputs; with ``update`` they become those behind the step (``conv_state_update``), in the same launch where every row
+    has one token."""
     t, c = out.shape
     taps = weight.shape[1]
     _f32(out, weight, bias)
@@ -266,7 +269,8 @@ def conv_silu_unit(out, x, conv_state, weight, ctx, unit_heads: int, dk: int, ot
     assert conv_state.shape[1:] == (max(taps - 1, 0), c)
     native.recurrence_check(native.recurrence().ms_conv_silu_unit(
         _ptr(out), _ptr(x), _rows(x), _ptr(conv_state), _ptr(weight), _ptr(ctx.row_of_token), _ptr(ctx.cu_q), _ptr(ctx.q_start),
-        _ptr(ctx.state_slot), t, c, taps, unit_heads, dk, other_heads, dv, float(unit_eps), _dt(x.dtype), _ptr(bias), ctx.stream))
+        _ptr(ctx.state_slot), t, c, taps, unit_heads, dk, other_heads, dv, float(unit_eps), _dt(x.dtype), _ptr(bias), ctx.num_rows,
+        (2 if ctx.decode_only else 1) if update else 0, ctx.stream), launches=2 if update and not ctx.decode_only else 1)
 
 
 def conv_state_update(conv_state, x, ctx, taps: int) -> None:
@@ -292,14 +296,18 @@ def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool =
         return False
     if not head_decay:
         return True
-    return (dk in (32, 64, 128) and q.dtype == torch.float32 and all(x.data_ptr() % 16 == 0 and x.stride(0) % 4 == 0 for x in (q, k)))
+    return (dk in (32, 64, 128) and q.dtype == torch.float32 and (q.data_ptr() | k.data_ptr()) % 16 == 0 and (q.stride(0) | k.stride(0)) % 4 == 0)
+
+
+@lru_cache(maxsize=256)
+def _walk_floats(*sizes) -> int:
+    return int(native.recurrence().ms_walk_scratch(*map(int, sizes)))
 
 
 def _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx, heads, dk, dv, q_scale, delta, head_decay, v_scale) -> None:
     t, rows = o_out.shape[0], ctx.num_rows
     lib = native.recurrence()
-    scratch = ctx.buffer("walk.scratch", (int(lib.ms_walk_scratch(t, rows, heads, dk, dv, int(delta), int(head_decay))),), torch.float32,
-                         o_out.device)
+    scratch = ctx.buffer("walk.scratch", (_walk_floats(t, rows, heads, dk, dv, delta, head_decay),), torch.float32, o_out.device)
     groups = q.shape[1] // dk
     rest = (_ptr(v_scale), _ptr(scratch), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.state_slot), t, rows, heads, dk, dv, float(q_scale))
     if head_decay:

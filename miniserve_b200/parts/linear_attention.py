@@ -1,6 +1,6 @@
 """Linear-attention mixers: a matrix state per head and request instead of keys and values of every
-past token, or a vector (the gated linear recurrence at the end). The matrix states run the token-by-token recurrence of
-``csrc/recurrence.cu`` (prompt portions and decoded tokens alike). All keep the state in float32 in the request's slot, and
+past token, or a vector (the gated linear recurrence at the end). The matrix states run the recurrences of
+``csrc/recurrence.cu`` token by token, prompts where ``ops.decay_scan`` says so by chunks (``csrc/chunk_walk.cu``). All keep the state in float32 in the request's slot, and
 start from zero where a row's first token is at position 0."""
 
 from __future__ import annotations
@@ -197,11 +197,10 @@ class GatedDeltaRule(Part):
         zg = ops.linear(low, self.w_up, stream=ctx.stream, out=ctx.buffer("delta.zg", (t, self.w_up.shape[0]), dt, dev))
         qkv = ctx.buffer("delta.qkv", (t, c), torch.float32, dev)
         conv_state = conv.state if conv is not None else ctx.buffer("delta.noconv", (1, 0, c), dt, dev)
-        ops.conv_silu_unit(qkv, proj[:, :c], conv_state, self.w_conv, ctx, 2 * g, dk, h, dv, self.unit_eps)
-        if conv is not None:
-            ops.conv_state_update(conv_state, proj[:, :c], ctx, self.taps)
+        ops.conv_silu_unit(qkv, proj[:, :c], conv_state, self.w_conv, ctx, 2 * g, dk, h, dv, self.unit_eps, update=conv is not None)
         o = ctx.buffer("delta.o", (t, h, dv), torch.float32, dev)
-        ops.decay_scan(o, state.state, qkv[:, :g * dk], qkv[:, g * dk:2 * g * dk], qkv[:, 2 * g * dk:], zg[:, :h * dk],
+        q, k, v = torch.split_with_sizes(qkv, (g * dk, g * dk, h * dv), 1)
+        ops.decay_scan(o, state.state, q, k, v, zg[:, :h * dk],
                        self.w_dt_bias, self.decay_coef, 1.0, proj[:, c:c + h], ctx, h, dk, dv, dk ** -0.5, delta=True)
         ops.head_norm_gate(out, o, self.w_norm, zg[:, h * dk:h * dk + h * dv], self.eps, scale, "sigmoid", stream=ctx.stream)
 
@@ -299,13 +298,12 @@ class SelectiveStateSpace(Part):
         xbc = ctx.buffer("ssm.xbc", (t, c), torch.float32, dev)
         conv_state = conv.state if conv is not None else ctx.buffer("ssm.noconv", (1, 0, c), dt, dev)
         unit = _conv_unit(c)
-        ops.conv_silu_unit(xbc, xbc_in, conv_state, self.w_conv, ctx, 0, 1, c // unit, unit, 0.0, bias=self.w_conv_bias)
-        if conv is not None:
-            ops.conv_state_update(conv_state, xbc_in, ctx, self.taps)
+        ops.conv_silu_unit(xbc, xbc_in, conv_state, self.w_conv, ctx, 0, 1, c // unit, unit, 0.0, bias=self.w_conv_bias,
+                           update=conv is not None)
         steps = ctx.buffer("ssm.dt", (2, t, h), torch.float32, dev)  # step sizes, then decays
         ops.ssm_step_decay(steps, proj[:, inner + c:inner + c + h], self.w_dt_bias, self.decay_coef, stream=ctx.stream)
         o = ctx.buffer("ssm.o", (t, h, dv), torch.float32, dev)
-        xs, bs, cs = xbc[:, :inner], xbc[:, inner:inner + g * n], xbc[:, inner + g * n:]
+        xs, bs, cs = torch.split_with_sizes(xbc, (inner, g * n, g * n), 1)
         ops.decay_scan(o, state.state, cs, bs, xs, steps[1], None, self.decay_coef, 1.0, None, ctx, h, n, dv, 1.0, delta=False,
                        head_decay=True, v_scale=steps[0])
         ops.gated_group_norm(out, o.view(t, inner), xs, self.w_skip, proj[:, :inner], self.w_norm, self.norm_groups, dv, self.eps,

@@ -50,6 +50,15 @@ def test_convolution_in_fours(dtype, taps, unit, dk, others, dv, lens, started):
         ops.conv_silu_unit(got, x, state, w, ctx, unit, dk, others, dv, 1e-6, bias=b)
         ops.conv_silu_unit(want, odd, state, w, ctx, unit, dk, others, dv, 1e-6, bias=b)
         _near(got, want, torch.float32)
+    # the histories behind the step, made with the outputs (in one launch where every row has one token) and by the launch for any rows
+    left = state.clone()
+    ops.conv_state_update(left, x, ctx, taps)
+    ctx.decode_only = max(lens) == 1
+    for operand in (x, odd):
+        moved = state.clone()
+        ops.conv_silu_unit(want, operand, moved, w, ctx, unit, dk, others, dv, 1e-6, bias=bias, update=True)
+        assert torch.equal(moved, left)
+        _near(got, want, torch.float32)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
