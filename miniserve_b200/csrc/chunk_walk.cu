@@ -1,4 +1,4 @@
-// The recurrences of ``recurrence.cu`` over a prompt by chunks of 16 tokens, in 32-bit accuracy on the tensor cores.
+// The recurrences of ``recurrence.cu`` over a prompt by chunks of 16 tokens, in float32.
 //
 //   decay rule:  S <- diag(d_t) S + k_t v_t^T;                                                   o_t = S^T q_t
 //   delta rule:  S <- diag(d_t) S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;           o_t = S^T q_t
@@ -10,81 +10,57 @@
 //   (I + A) U = diag(beta) (V - (G k) S):   U = U0 - W S   with   (I + A) U0 = diag(beta) V,  (I + A) W = diag(beta) (G k)
 //   O = (G q) S + P U,          S_behind = G_last S + (D_(last, .) k)^T U.
 //
+// (The triangular system of a chunk: the WY form of products of Householder-like factors, C. Bischof and C. Van Loan, 1987, as chunked
+// linear recurrences use it.)
+//
 // The first kernel works out, for all chunks at once, what does not need the state: W, q' = G q, k' = D_(last, .) k, U0, P.
-// The second walks a row's chunks in order, a CTA per (16 value columns, head, row): the products of a chunk against the state
-// that stays in registers. Both keep 32 bits: sums and the state are float32, and a factor of a tensor-core product is given as two
-// tf32 numbers, hi = round(x) and lo = round(x - hi) (22 bits and more of x), of which the three products that matter are made.
-// Against 64-bit sums the results are as far off as the token-by-token walk's (a few 1e-8 of the terms' size). A value that is not
-// finite makes its column of the whole chunk NaN, in the tokens ahead of it too (a pair that is left out counts zero times it).
+// The second walks a row's chunks in order, a warp per 4 value columns: the products of a chunk against the state that stays in registers.
 //
-// What bounds it: the walk is a chain of tokens / 16 steps, each a few dependent tensor-core products and two barriers (one without
-// the delta rule); the token-by-token walk is a chain of `tokens` steps of two lane-group sums each.
+// Accuracy: every sum is made of float32 multiply-adds that round to nearest, as the token-by-token walk's; products of decays, the
+// last steps of the pairs' sums and the triangular system are worked out in 64 bits and rounded once. (A running product of 16 decays just
+// below one is rounded down every time: in 32 bits the state of a slowly decaying head comes out three times as far off as the walk's.
+// Tensor cores were further off too: a factor as two tf32 numbers loses a bit, and their sums are cut, not rounded.) Against 64-bit sums
+// outputs and states are no further off than the walk's: root mean squares of the errors over 2,048 tokens 0.76 to 1.0 of the walk's
+// (outputs) and 0.7 to 1.05 (states: few numbers), decays from 0.02 to 1; 0.27 to 0.4 with the delta rule and no decay.
+// A token sees nothing of the tokens behind it, whatever they hold: a value that is not finite reaches its own token and the later
+// ones. (With one decay per head the sums against the state are scaled behind the sum: a state within q's size of the largest float
+// overflows.)
 //
-// The accumulator of a product is the next product's operand as it lies in the registers: a warp's slice of 8 N key channels is
-// taken as N tiles of 8 of which tile i has the channels N n + i (n = 0..7), so that accumulator columns (2 t, 2 t + 1) of a lane are
-// its operand's (t, t + 4), and everything a lane loads of q', W (2 N channels) or k' (N channels) is contiguous.
+// What bounds it: the walk is a chain of tokens / 16 steps, each the products against W, an exchange among the 16 lanes of a column
+// and the state's update; the token-by-token walk is a chain of `tokens` steps of two lane-group sums each.
+#include <cfloat>
+
 #include "chunk_mma.cuh"
 
 namespace ms {
 
-constexpr int WK_TOK = 16, WK_THREADS = 128, WK_WARPS = 4, WK_COLS = 16;
+constexpr int WK_TOK = 16, WK_THREADS = 128, WK_COLS = 16;  // (WK_THREADS: of the kernels ahead of the walk; WK_COLS: what u0 is padded to)
+constexpr int WK_CHAIN = 2, WK_OUT = 4, WK_OWN = 8;          // warps of the walk's chain, of its outputs, an output warp's tokens
 enum WalkMode : int { WALK_CHANNEL = 0, WALK_DELTA = 1, WALK_HEAD = 2 };
 
 __device__ __forceinline__ float wk_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
-struct Tf32x2 {
-  uint32_t hi, lo;
-};
-// hi: x rounded to 11 bits of significand, lo: what is left (12 bits and a sign, of which the last is cut off). Integer adds and masks: a
-// conversion instruction takes several times their issue slots. A NaN stays one in lo whatever the addition makes of it in hi.
-__device__ __forceinline__ Tf32x2 wk_split(float x) {
-  Tf32x2 r;
-  r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  r.lo = __float_as_uint(x - __uint_as_float(r.hi)) & 0xffffe000u;
+// two neighbouring floats in a register pair: each half rounds as the plain instruction does
+using wk_f2 = unsigned long long;
+__device__ __forceinline__ void wk_fma2(wk_f2& d, wk_f2 a, wk_f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ wk_f2 wk_mul2(wk_f2 a, wk_f2 b) {
+  wk_f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-__device__ __forceinline__ void wk_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ wk_f2 wk_pair(float x, float y) {
+  wk_f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
 }
-struct FragA {
-  uint32_t hi[4], lo[4];
-};
-__device__ __forceinline__ FragA wk_frag(float x0, float x1, float x2, float x3) {
-  FragA f;
-  const float x[4] = {x0, x1, x2, x3};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const Tf32x2 s = wk_split(x[e]);
-    f.hi[e] = s.hi;
-    f.lo[e] = s.lo;
-  }
-  return f;
+__device__ __forceinline__ float2 wk_halves(wk_f2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
 }
-// A product in the accuracy of float32: main += hi hi, rest += lo hi + hi lo (an accumulator of their own: shorter chains). PART 0..2 in turn.
-template <int PART>
-__device__ __forceinline__ void wk_part(float (&main)[4], float (&rest)[4], const FragA& a, const Tf32x2 (&b)[2]) {
-  if constexpr (PART == 0) wk_mma(rest, a.lo, b[0].hi, b[1].hi);
-  else if constexpr (PART == 1) wk_mma(main, a.hi, b[0].hi, b[1].hi);
-  else wk_mma(rest, a.hi, b[0].lo, b[1].lo);
-}
-
-// N consecutive floats (an address that is a multiple of their size up to 16 bytes)
-template <int N>
-__device__ __forceinline__ void wk_load(float (&f)[N], const float* p) {
-  if constexpr (N % 4 == 0) {
-#pragma unroll
-    for (int e = 0; e < N; e += 4) {
-      const float4 v = *reinterpret_cast<const float4*>(p + e);
-      f[e] = v.x; f[e + 1] = v.y; f[e + 2] = v.z; f[e + 3] = v.w;
-    }
-  } else if constexpr (N == 2) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    f[0] = v.x; f[1] = v.y;
-  } else {
-    f[0] = *p;
-  }
+__device__ __forceinline__ float wk_sum2(wk_f2 x) {
+  const float2 h = wk_halves(x);
+  return h.x + h.y;
 }
 
 // ---------------------------------------------------------------- the chunks of a step
@@ -125,9 +101,10 @@ __device__ __forceinline__ int wk_first(int row, const int* __restrict__ cu_q) {
 // [chunks, H, 16, dvp] (dvp: dv in whole sixteens, zeros behind; without the delta rule v itself), pairs = P [chunks, H, 16, 16]. z: the
 // decays' logits (bias, coef, sign as in recurrence.cu); beta likewise logits.
 // Bound by instruction issue: 16 x 16 pairs over dk channels with a decay each. A warp takes four tokens j at once, eight lanes
-// over the channels of each, lets their keys decay from j on, and adds up over the lanes at the end (28 exchanges for four tokens).
+// over the channels of each (two channels an instruction), lets their keys decay from j on, and adds up over the lanes at the end (28
+// exchanges for four tokens). The sum over the lanes, products of decays and the triangular system in 64 bits (above).
 template <typename TIn, typename TZ, bool DELTA, int N>
-__global__ void __launch_bounds__(WK_THREADS)
+__global__ void __launch_bounds__(WK_THREADS, 4)
 walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float* __restrict__ k_out, float* __restrict__ last_out,
                     float* __restrict__ u0_out, float* __restrict__ pairs, const TIn* __restrict__ q, int ld_q, const TIn* __restrict__ k,
                     int ld_k, int qk_group, const TIn* __restrict__ v, int ld_v, const TZ* __restrict__ z, int ld_z,
@@ -136,7 +113,7 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
                     float q_scale) {
   constexpr int DKP = 32 * N;
   __shared__ __align__(16) float qs[WK_TOK][DKP], ks[WK_TOK][DKP], ds[WK_TOK][DKP];
-  __shared__ __align__(16) float am[DELTA ? WK_TOK : 1][WK_TOK + 4];
+  __shared__ __align__(16) double am[DELTA ? WK_TOK : 1][WK_TOK];  // A, a column j in am[j]
   __shared__ float bs[WK_TOK], vsc[WK_TOK];
   pdl_prologue();
   const int chunk = blockIdx.x, h = blockIdx.y;
@@ -171,32 +148,34 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
   const size_t item = (size_t)chunk * H + h;
   {
     const int cl = lane & 7, j = warp * 4 + (lane >> 3);
-    float p[4 * N] = {}, val[32];
+    wk_f2 p[2 * N] = {};
+    double val[32];
 #pragma unroll
     for (int i = 0; i < WK_TOK; ++i) {
-      float a = 0.f, b = 0.f;
+      wk_f2 a = 0ull, b = 0ull;
 #pragma unroll
       for (int m = 0; m < N; ++m) {
-        float fk[4], fq[4], fd[4];
-        wk_load<4>(fk, &ks[i][cl * 4 + 32 * m]);
-        wk_load<4>(fq, &qs[i][cl * 4 + 32 * m]);
-        wk_load<4>(fd, &ds[i][cl * 4 + 32 * m]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          p[4 * m + e] = i == j ? fk[e] : p[4 * m + e] * fd[e];  // (nothing ahead of token j)
-          if (DELTA) a = fmaf(fk[e], p[4 * m + e], a);
-          b = fmaf(fq[e], p[4 * m + e], b);
+        const ulonglong2 fk = *reinterpret_cast<const ulonglong2*>(&ks[i][cl * 4 + 32 * m]);
+        const ulonglong2 fq = *reinterpret_cast<const ulonglong2*>(&qs[i][cl * 4 + 32 * m]);
+        const ulonglong2 fd = *reinterpret_cast<const ulonglong2*>(&ds[i][cl * 4 + 32 * m]);
+        p[2 * m] = i == j ? fk.x : wk_mul2(p[2 * m], fd.x);  // (nothing ahead of token j)
+        p[2 * m + 1] = i == j ? fk.y : wk_mul2(p[2 * m + 1], fd.y);
+        if (DELTA) {
+          wk_fma2(a, fk.x, p[2 * m]);
+          wk_fma2(a, fk.y, p[2 * m + 1]);
         }
+        wk_fma2(b, fq.x, p[2 * m]);
+        wk_fma2(b, fq.y, p[2 * m + 1]);
       }
-      val[i] = a;
-      val[16 + i] = b;
+      val[i] = wk_sum2(a);
+      val[16 + i] = wk_sum2(b);
     }
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
       const bool up = cl & o;
 #pragma unroll
       for (int i = 0; i < 4 * o; ++i) {
-        const float send = up ? val[i] : val[i + 4 * o], keep = up ? val[i + 4 * o] : val[i];
+        const double send = up ? val[i] : val[i + 4 * o], keep = up ? val[i + 4 * o] : val[i];
         val[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
@@ -204,29 +183,29 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int i = i0 + e;
-      if (cl >= 4) pairs[(item * WK_TOK + i) * WK_TOK + j] = i >= j ? val[e] : 0.f;
-      else if (DELTA) am[i][j] = i > j ? val[e] * bs[i] : 0.f;
+      if (cl >= 4) pairs[(item * WK_TOK + i) * WK_TOK + j] = i >= j ? (float)val[e] : 0.f;
+      else if (DELTA) am[j][i] = i > j ? val[e] * (double)bs[i] : 0.0;
     }
   }
   if (DELTA) __syncthreads();
   // a thread per key channel: q', W (forward substitution), k', the decay of the whole chunk; and one per value column: U0 likewise
 #pragma unroll 1
   for (int c = tid; c < DKP + dvp; c += WK_THREADS) {
-    float x[WK_TOK];
+    double x[WK_TOK];
     if (c < DKP) {
-      float passed = 1.f;
+      double passed = 1.0;
 #pragma unroll
       for (int i = 0; i < WK_TOK; ++i) {
-        passed *= ds[i][c];
-        q_out[(item * WK_TOK + i) * DKP + c] = passed * qs[i][c];
-        x[i] = passed * ks[i][c];
+        passed *= (double)ds[i][c];
+        q_out[(item * WK_TOK + i) * DKP + c] = (float)(passed * (double)qs[i][c]);
+        x[i] = passed * (double)ks[i][c];
       }
-      last_out[item * DKP + c] = passed;
-      float behind = 1.f;
+      last_out[item * DKP + c] = (float)passed;
+      double behind = 1.0;
 #pragma unroll
       for (int i = WK_TOK - 1; i >= 0; --i) {
-        k_out[(item * WK_TOK + i) * DKP + c] = ks[i][c] * behind;
-        behind *= ds[i][c];
+        k_out[(item * WK_TOK + i) * DKP + c] = (float)((double)ks[i][c] * behind);
+        behind *= (double)ds[i][c];
       }
     } else {
       const int col = c - DKP;
@@ -237,36 +216,37 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
     if (!DELTA && c < DKP) continue;
     float* out = c < DKP ? w_out + item * WK_TOK * DKP + c : u0_out + item * WK_TOK * dvp + (c - DKP);
     const int step = c < DKP ? DKP : dvp;
+    if (DELTA) {
+      asm volatile("" ::: "memory");  // (A is read again for every column: kept over the columns it takes 240 registers)
 #pragma unroll
-    for (int i = 0; i < WK_TOK; ++i) {
-      if (DELTA) {
-        float y = bs[i] * x[i];
+      for (int i = 0; i < WK_TOK; ++i) x[i] *= (double)bs[i];
 #pragma unroll
-        for (int j = 0; j < i; ++j) y = fmaf(-am[i][j], x[j], y);
-        x[i] = y;
-      }
-      out[(size_t)i * step] = x[i];
+      for (int j = 0; j + 1 < WK_TOK; ++j)
+#pragma unroll
+        for (int i = j + 1; i < WK_TOK; ++i) x[i] = fma(-am[j][i], x[j], x[i]);
     }
+#pragma unroll
+    for (int i = 0; i < WK_TOK; ++i) out[(size_t)i * step] = (float)x[i];
   }
 }
 
 // ---------------------------------------------------------------- the walk over a row's chunks
-// grid (value column tiles, H, rows). The four warps share the key channels out among themselves (8 N each): a product over the key
-// channels is four partial sums that meet in shared memory, the state's own update stays inside a warp.
+// grid (value column tiles, H, rows), 4 C columns a CTA. A column's DKP key channels lie with 16 lanes, 2 N each, in registers; a lane has
+// C columns, a warp 2 C: an operand read from shared memory makes products for all of them. A product against 16 tokens' vectors is 16 sums a
+// lane and column, folded over the 16 lanes all at once (lane l keeps token l's).
+// The first warps carry the chain (W, u, the state behind the chunk); the others, beside them on the SM's other schedulers, make the
+// outputs from the state that the chain left in shared memory, eight tokens a warp, the chunk's own tokens' part one chunk later, when u is
+// there. One barrier a chunk.
 // Channel mode and the delta rule read what walk_prepare_kernel left (qp, wp, kp, dec, u0, pairs). Head mode reads q, k and v
 // themselves, and the pairs and decays of walk_head_kernel.
-// A chunk's operands come through a ring in shared memory that every lane fills and reads for itself alone (cp.async): a chunk takes
-// less time than a load from L2.
-template <int MODE, int N, int MT>
-struct WalkItems {  // floats of one lane and chunk
-  static constexpr int q = 0, w = 4 * N, k = w + (MODE == WALK_DELTA ? 4 * N : 0), last = k + 4 * N,
-                       pair = last + (MODE == WALK_HEAD ? 8 : 2 * N), u = pair + 2, more = u + 2 * MT,
-                       floats = (more + (MODE == WALK_HEAD ? 2 : 0) + 3) / 4 * 4;
-  static constexpr int stages = MODE == WALK_HEAD ? 3 : 4;
-  static constexpr int cols = MT * WK_COLS, ld = cols + 4, ldu = WK_TOK + 4;
-  static constexpr int ring = stages * floats * WK_THREADS, xs = MODE == WALK_DELTA ? WK_WARPS * WK_TOK * ld : 0, os = 2 * WK_WARPS * WK_TOK * ld,
-                       us = (MODE == WALK_DELTA ? 1 : 2) * cols * ldu;
-  static constexpr size_t bytes = (size_t)(ring + xs + os + us) * 4;
+// A chunk's operands come through a ring in shared memory (cp.async), two or three chunks ahead: a chunk takes less time than a load from L2.
+template <int MODE, int N, int C>
+struct WalkStage {  // floats
+  static constexpr int dkp = 32 * N, cols = 2 * C * WK_CHAIN, ldp = WK_TOK + 4, decays = MODE == WALK_HEAD ? 3 * WK_TOK : dkp;
+  static constexpr int q = 0, k = WK_TOK * dkp, w = 2 * WK_TOK * dkp, last = w + (MODE == WALK_DELTA ? WK_TOK * dkp : 0), pair = last + decays,
+                       u = pair + WK_TOK * ldp, scale = u + WK_TOK * cols, floats = scale + (MODE == WALK_HEAD ? WK_TOK : 0);
+  static constexpr int stages = C == 4 ? 3 : 4, states = 2 * cols * dkp, us = 2 * cols * WK_TOK, decayed = MODE == WALK_HEAD ? cols * WK_TOK : 0;
+  static constexpr size_t bytes = (size_t)(stages * floats + states + us + decayed) * 4;
 };
 
 // BYTES from global memory into shared memory, zeros where not `in`
@@ -275,346 +255,306 @@ __device__ __forceinline__ void wk_cp(float* dst, const float* src, bool in) {
   const int n = in ? BYTES : 0;
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(cs_smem(dst)), "l"(src), "n"(BYTES), "r"(n) : "memory");
 }
-// COUNT consecutive floats of one lane: pieces of 16 bytes (or what there is) whose places in a stage are 128 lanes wide
-template <int COUNT>
-__device__ __forceinline__ void wk_ring_fill(float* stage, int item, const float* src, bool in, const float* any) {
-  constexpr int W = COUNT % 4 == 0 ? 4 : COUNT;
+
+// a lane's 2 N channels of a row of DKP in shared memory: two for N = 1, else fours that are 64 apart
+template <int N>
+__device__ __forceinline__ void wk_row(wk_f2 (&x)[N], const float* row, int l) {
+  if constexpr (N == 1) {
+    x[0] = *reinterpret_cast<const wk_f2*>(row + 2 * l);
+  } else {
 #pragma unroll
-  for (int e = 0; e < COUNT; e += W) wk_cp<W * 4>(stage + (item + e) * WK_THREADS + threadIdx.x * W, in ? src + e : any, in);
-}
-template <int COUNT>
-__device__ __forceinline__ void wk_ring_read(float (&f)[COUNT], const float* stage, int item) {
-  constexpr int W = COUNT % 4 == 0 ? 4 : COUNT;
-#pragma unroll
-  for (int e = 0; e < COUNT; e += W) {
-    float x[W];
-    wk_load<W>(x, stage + (item + e) * WK_THREADS + threadIdx.x * W);
-#pragma unroll
-    for (int i = 0; i < W; ++i) f[e + i] = x[i];
+    for (int m = 0; m < N / 2; ++m) {
+      const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(row + 64 * m + 4 * l);
+      x[2 * m] = y.x;
+      x[2 * m + 1] = y.y;
+    }
   }
 }
+template <int N>
+__device__ __forceinline__ int wk_channel(int l, int pair, int half) {
+  return N == 1 ? 2 * l + half : 64 * (pair >> 1) + 4 * l + 2 * (pair & 1) + half;
+}
 
-template <int MODE, int N, int MT>
-__global__ void __launch_bounds__(WK_THREADS)
+// The products of a lane's columns with ROWS rows, summed over the column's lanes: lane l comes back with row l's. (Eight rows: lanes l and l ^ 8
+// with two parts of row l & 7's.) A lane takes row i ^ l as its i-th, so that what it keeps of an exchange is always the first half of its sums.
+template <int N, int C, int ROWS>
+__device__ __forceinline__ void wk_against(float (&d)[C], const wk_f2 (&S)[C][N], const float* rows, int l) {
+  float val[C][ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    wk_f2 x[N], a[C] = {};
+    wk_row<N>(x, rows + (i ^ (l & (ROWS - 1))) * (32 * N), l);
+#pragma unroll
+    for (int p = 0; p < N; ++p)
+#pragma unroll
+      for (int c = 0; c < C; ++c) wk_fma2(a[c], S[c][p], x[p]);
+#pragma unroll
+    for (int c = 0; c < C; ++c) val[c][i] = wk_sum2(a[c]);
+  }
+#pragma unroll
+  for (int o = ROWS / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+      for (int i = 0; i < o; ++i) val[c][i] += __shfl_xor_sync(0xffffffffu, val[c][i + o], o);
+#pragma unroll
+  for (int c = 0; c < C; ++c) d[c] = val[c][0];
+}
+
+template <int MODE, int N, int C>
+__global__ void __launch_bounds__((WK_CHAIN + WK_OUT) * 32, C == 4 ? 2 : 1)
 walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __restrict__ qp, int ld_q, const float* __restrict__ wp,
             const float* __restrict__ kp, int ld_k, int qk_group, const float* __restrict__ dec, const float* __restrict__ v, int ld_v,
             const float* __restrict__ v_scale, const float* __restrict__ pairs, const int* __restrict__ cu_q, const int* __restrict__ q_start,
             const int* __restrict__ state_slot, int H, int dk, int dv) {
-  using I = WalkItems<MODE, N, MT>;
-  constexpr int DKP = 32 * N, COLS = I::cols, LD = I::ld, LDU = I::ldu, ST = I::stages;
+  using I = WalkStage<MODE, N, C>;
+  constexpr int DKP = I::dkp, COLS = I::cols, ST = I::stages, FETCHERS = WK_OUT * 32;
   extern __shared__ __align__(16) float wk_smem[];
-  float* ring = wk_smem;
-  float* xs = ring + I::ring;  // [warp][token][LD]
-  float* os = xs + I::xs;      // [2][warp][token][LD]
-  float* us = os + I::os;      // [1 or 2][column][LDU]
-  pdl_prologue();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = lane & 15;
   const int v0 = blockIdx.x * COLS, h = blockIdx.y, r = blockIdx.z;
   const int row_begin = cu_q[r], row_end = cu_q[r + 1];
   const int c0 = wk_first(r, cu_q);
-  int c1 = c0 + (row_end - row_begin + WK_TOK - 1) / WK_TOK;
-  asm volatile("" : "+r"(c1));  // (a number of chunks that the compiler can see to be above zero has it order the loop for fewer registers)
+  const int c1 = c0 + (row_end - row_begin + WK_TOK - 1) / WK_TOK;
   if (c1 <= c0) return;
-  const int slice = warp * 8 * N;      // the warp's key channels
-  const int mine = slice + 2 * N * t;  // the lane's 2 N of them as a product's operand,
-  const int mine_n = slice + N * g;    // and its N as an accumulator's columns
-  const int tok_u = tid >> 3, col_u = (tid & 7) * 2;  // the (token, two columns) that a thread brings in and adds up
-  const size_t head = (size_t)(h / qk_group) * dk;
+  const bool chain = warp < WK_CHAIN;
+  const int mine = (warp % WK_CHAIN) * (2 * C) + (lane >> 4) * C;  // the lane's first column of the CTA's
+  float* states = wk_smem + ST * I::floats + mine * DKP;                  // [2][COLS][DKP]: the state ahead of a chunk
+  float* us = wk_smem + ST * I::floats + I::states + mine * WK_TOK;       // [2][COLS][16]: u of a chunk
+  float* decayed = wk_smem + ST * I::floats + I::states + I::us + mine * WK_TOK;  // (head mode) [COLS][16]: u decayed to the chunk's end
 
+  const int ft = tid - WK_CHAIN * 32;  // (the output warps fetch)
   auto fetch = [&](int c) {  // (nothing behind the row's last chunk; the group is committed all the same)
     if (c < c1) {
-      float* st = ring + (size_t)((c - c0) % ST) * (I::floats * WK_THREADS);
+      float* st = wk_smem + (size_t)((c - c0) % ST) * I::floats;
       const int tok0 = row_begin + (c - c0) * WK_TOK;
       const size_t item = (size_t)c * H + h;
       if constexpr (MODE == WALK_HEAD) {
+        const size_t head = (size_t)(h / qk_group) * dk;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int tok = tok0 + j * 8 + g;
-          wk_ring_fill<2 * N>(st, I::q + j * 2 * N, qp + (size_t)tok * ld_q + head + mine, tok < row_end, qp);
+        for (int idx = ft; idx < WK_TOK * DKP / 4; idx += FETCHERS) {
+          const int i = idx / (DKP / 4), ch = (idx % (DKP / 4)) * 4, tok = tok0 + i;
+          const bool in = tok < row_end;
+          wk_cp<16>(st + I::q + i * DKP + ch, in ? qp + (size_t)tok * ld_q + head + ch : qp, in);
+          wk_cp<16>(st + I::k + i * DKP + ch, in ? kp + (size_t)tok * ld_k + head + ch : kp, in);
         }
+        if (ft < 3 * WK_TOK / 4) wk_cp<16>(st + I::last + ft * 4, dec + item * (3 * WK_TOK) + ft * 4, true);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int tok = tok0 + 4 * t + j;
-          wk_ring_fill<N>(st, I::k + j * N, kp + (size_t)tok * ld_k + head + mine_n, tok < row_end, kp);
+        for (int idx = ft; idx < WK_TOK * COLS; idx += FETCHERS) {
+          const int i = idx / COLS, col = v0 + idx % COLS, tok = tok0 + i;
+          const bool in = tok < row_end && col < dv;
+          wk_cp<4>(st + I::u + idx, in ? v + (size_t)tok * ld_v + (size_t)h * dv + col : v, in);
         }
-        const float* d = dec + item * (3 * WK_TOK);
-        wk_ring_fill<2>(st, I::last, d + 2 * t, true, dec);
-        wk_ring_fill<2>(st, I::last + 2, d + 8 + 2 * t, true, dec);
-        wk_ring_fill<4>(st, I::last + 4, d + WK_TOK + 4 * t, true, dec);
-        wk_ring_fill<1>(st, I::more, d + 2 * WK_TOK, true, dec);
-        const int tok = tok0 + tok_u;
-        const bool in = tok < row_end;
-        if (v_scale) wk_ring_fill<1>(st, I::more + 1, v_scale + (size_t)tok * H + h, in, v_scale);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int col = v0 + mt * 16 + col_u + e;
-            wk_ring_fill<1>(st, I::u + mt * 2 + e, v + (size_t)tok * ld_v + (size_t)h * dv + col, in && col < dv, v);
-          }
+        if (v_scale && ft < WK_TOK) {
+          const bool in = tok0 + ft < row_end;
+          wk_cp<4>(st + I::scale + ft, in ? v_scale + (size_t)(tok0 + ft) * H + h : v_scale, in);
+        }
       } else {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          wk_ring_fill<2 * N>(st, I::q + j * 2 * N, qp + (item * WK_TOK + j * 8 + g) * DKP + mine, true, qp);
-          if constexpr (MODE == WALK_DELTA) wk_ring_fill<2 * N>(st, I::w + j * 2 * N, wp + (item * WK_TOK + j * 8 + g) * DKP + mine, true, wp);
+        for (int idx = ft; idx < WK_TOK * DKP / 4; idx += FETCHERS) {
+          const int at = idx * 4;
+          const size_t from = item * (WK_TOK * DKP) + at;
+          wk_cp<16>(st + I::q + at, qp + from, true);
+          wk_cp<16>(st + I::k + at, kp + from, true);
+          if constexpr (MODE == WALK_DELTA) wk_cp<16>(st + I::w + at, wp + from, true);
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) wk_ring_fill<N>(st, I::k + j * N, kp + (item * WK_TOK + 4 * t + j) * DKP + mine_n, true, kp);
-        wk_ring_fill<2 * N>(st, I::last, dec + item * DKP + mine, true, dec);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) wk_ring_fill<2>(st, I::u + mt * 2, v + (item * WK_TOK + tok_u) * ld_v + v0 + mt * 16 + col_u, true, v);
+        if (ft < DKP / 4) wk_cp<16>(st + I::last + ft * 4, dec + item * DKP + ft * 4, true);
+        for (int idx = ft; idx < WK_TOK * COLS / 4; idx += FETCHERS) {
+          const int i = idx / (COLS / 4), col = (idx % (COLS / 4)) * 4;
+          wk_cp<16>(st + I::u + i * COLS + col, v + (item * WK_TOK + i) * ld_v + v0 + col, true);
+        }
       }
-      wk_ring_fill<2>(st, I::pair, pairs + (item * WK_TOK + (warp & 1) * 8 + g) * WK_TOK + 4 * t + 2 * (warp >> 1), true, pairs);
+      if (ft < WK_TOK * WK_TOK / 4) wk_cp<16>(st + I::pair + (ft >> 2) * I::ldp + (ft & 3) * 4, pairs + item * (WK_TOK * WK_TOK) + ft * 4, true);
     }
     cs_commit();
   };
-  // o of the chunk that begins at tok0: the four warps' partial sums
-  auto put_out = [&](int tok0, int buf) {
-    const int tok = tok0 + tok_u;
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      float x[2] = {0.f, 0.f};
-#pragma unroll
-      for (int w = 0; w < WK_WARPS; ++w) {
-        const float2 y = *reinterpret_cast<const float2*>(os + ((buf * WK_WARPS + w) * WK_TOK + tok_u) * LD + mt * 16 + col_u);
-        x[0] += y.x;
-        x[1] += y.y;
-      }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int col = v0 + mt * 16 + col_u + e;
-        if (tok < row_end && col < dv) o[((size_t)tok * H + h) * dv + col] = x[e];
-      }
-    }
-  };
 
+  if (!chain) {
 #pragma unroll
-  for (int s = 0; s < ST - 1; ++s) fetch(c0 + s);
-  float S[MT][N][4];
+    for (int s = 0; s < ST - 1; ++s) fetch(c0 + s);
+  }
+  wk_f2 S[C][N];
   float* slot = state + ((size_t)state_slot[r] * H + h) * (size_t)dv * dk;
-  const bool fresh = q_start[r] == 0;
+  // the chain's state into shared memory for the outputs, and from there
+  auto leave = [&](int buf) {
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
+    for (int e = 0; e < C; ++e)
 #pragma unroll
-    for (int nt = 0; nt < N; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int col = v0 + mt * 16 + g + (e >= 2 ? 8 : 0), c = mine + N * (e & 1) + nt;
-        S[mt][nt][e] = !fresh && col < dv && c < dk ? slot[(size_t)col * dk + c] : 0.f;
+      for (int p = 0; p < N; p += 2) {
+        float* to = states + (buf * COLS + e) * DKP + wk_channel<N>(l, p, 0);
+        if constexpr (N == 1) *reinterpret_cast<wk_f2*>(to) = S[e][0];
+        else *reinterpret_cast<ulonglong2*>(to) = make_ulonglong2(S[e][p], S[e][p + 1]);
       }
+  };
+  if (chain) {
+    const bool fresh = q_start[r] == 0;
+#pragma unroll
+    for (int e = 0; e < C; ++e)
+#pragma unroll
+      for (int p = 0; p < N; ++p) {
+        float x[2];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int col = v0 + mine + e, ch = wk_channel<N>(l, p, half);
+          x[half] = !fresh && col < dv && ch < dk ? slot[(size_t)col * dk + ch] : 0.f;
+        }
+        S[e][p] = wk_pair(x[0], x[1]);
+      }
+    leave(0);
+  }
+  float out[C] = {};
+  wk_f2 P[WK_OWN / 2] = {};
+  const int tk0 = warp >= 2 * WK_CHAIN ? WK_OWN : 0, tk = tk0 + (l & 7), j0 = l & 8;  // an output lane's token, of whose earlier ones it takes j0 .. j0 + 7
 
 #pragma unroll 1
-  for (int c = c0; c < c1; ++c) {
-    const int tok0 = row_begin + (c - c0) * WK_TOK, buf = (c - c0) & 1;
-    fetch(c + ST - 1);
-    cs_wait<ST - 1>();
-    const float* st = ring + (size_t)((c - c0) % ST) * (I::floats * WK_THREADS);
-    float fu[MT * 2];
+  for (int c = c0; c <= c1; ++c) {  // (one more trip for the last chunk's outputs)
+    const int buf = (c - c0) & 1, tok0 = row_begin + (c - c0) * WK_TOK;
+    if (!chain) cs_wait<ST - 2>();
+    __syncthreads();  // the chunk has come, and every warp is done with the stage that the next fetch fills
+    const float* st = wk_smem + (size_t)((c - c0) % ST) * I::floats;
+    if (chain) {
+      if (c == c1) break;
+      float u[C];
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      if constexpr (MODE == WALK_HEAD) {  // (two pieces of their own)
-        float x0[1], x1[1];
-        wk_ring_read<1>(x0, st, I::u + 2 * mt);
-        wk_ring_read<1>(x1, st, I::u + 2 * mt + 1);
-        fu[2 * mt] = x0[0];
-        fu[2 * mt + 1] = x1[0];
+      for (int e = 0; e < C; e += 2) {
+        const float2 given = *reinterpret_cast<const float2*>(st + I::u + l * COLS + mine + e);
+        u[e] = given.x;
+        u[e + 1] = given.y;
+      }
+      if constexpr (MODE == WALK_DELTA) {
+        float d[C];
+        wk_against<N, C, WK_TOK>(d, S, st + I::w, l);
+#pragma unroll
+        for (int e = 0; e < C; ++e) u[e] -= d[e];
+      }
+      if constexpr (MODE == WALK_HEAD) {
+        const float f = v_scale ? st[I::scale + l] : 1.f;
+#pragma unroll
+        for (int e = 0; e < C; ++e) u[e] *= f;
+      }
+      const float* uk = us + buf * COLS * WK_TOK;
+#pragma unroll
+      for (int e = 0; e < C; ++e) {
+        if (tok0 + l >= row_end) u[e] = 0.f;  // (what a state that is not finite makes of a token behind the row's end)
+        us[(buf * COLS + e) * WK_TOK + l] = u[e];
+      }
+      if constexpr (MODE == WALK_HEAD) {
+        const float f = st[I::last + WK_TOK + l];
+#pragma unroll
+        for (int e = 0; e < C; ++e) decayed[e * WK_TOK + l] = u[e] * f;
+        uk = decayed;
+      }
+      wk_f2 keep[N];
+      if constexpr (MODE == WALK_HEAD) {
+        const float f = st[I::last + 2 * WK_TOK];
+#pragma unroll
+        for (int p = 0; p < N; ++p) keep[p] = wk_pair(f, f);
       } else {
-        float x[2];
-        wk_ring_read<2>(x, st, I::u + 2 * mt);
-        fu[2 * mt] = x[0];
-        fu[2 * mt + 1] = x[1];
+        wk_row<N>(keep, st + I::last, l);
       }
-    }
-    if constexpr (MODE == WALK_HEAD) {
-      if (v_scale) {
-        float x[1];
-        wk_ring_read<1>(x, st, I::more + 1);
+      __syncwarp();
+      // the first half of the tokens by itself, then the state ahead of the chunk, then the other tokens one by one: half the roundings
+      // of a long-lived state, and none more of one that decays fast (whose last token, then, must come behind it)
+      const bool half = row_end - tok0 <= WK_TOK / 2;
+      wk_f2 next[C][N];
 #pragma unroll
-        for (int e = 0; e < MT * 2; ++e) fu[e] *= x[0];
-      }
-    }
-    FragA a[MT][N];
+      for (int e = 0; e < C; ++e)
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+        for (int p = 0; p < N; ++p) next[e][p] = half ? wk_mul2(S[e][p], keep[p]) : 0ull;
 #pragma unroll
-      for (int nt = 0; nt < N; ++nt) a[mt][nt] = wk_frag(S[mt][nt][0], S[mt][nt][2], S[mt][nt][1], S[mt][nt][3]);
-    // d = the state against the two rows of 2 N channels that a lane holds of q' or W
-    auto against = [&](float (&d)[MT][2][4], int item) {
-      float rest[MT][2][4] = {};
+      for (int j = 0; j < WK_TOK; j += 4) {
+        if (j == WK_TOK / 2 && !half) {
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+          for (int e = 0; e < C; ++e)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) d[mt][j][e] = 0.f;
-      float f[2][2 * N];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) wk_ring_read<2 * N>(f[j], st, item + j * 2 * N);
-#pragma unroll
-      for (int nt = 0; nt < N; ++nt) {
-        Tf32x2 b[2][2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) b[j][e] = wk_split(f[j][N * e + nt]);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) wk_part<0>(d[mt][j], rest[mt][j], a[mt][nt], b[j]);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) wk_part<1>(d[mt][j], rest[mt][j], a[mt][nt], b[j]);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) wk_part<2>(d[mt][j], rest[mt][j], a[mt][nt], b[j]);
-      }
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) d[mt][j][e] += rest[mt][j][e];
-    };
-    float acc[MT][2][4];
-    if constexpr (MODE == WALK_DELTA) {
-      float x[MT][2][4];
-      against(x, I::w);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) xs[(warp * WK_TOK + j * 8 + 2 * t + (e & 1)) * LD + mt * 16 + g + (e >= 2 ? 8 : 0)] = x[mt][j][e];
-      __syncthreads();
-      float2 y[MT][WK_WARPS];
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int w = 0; w < WK_WARPS; ++w) y[mt][w] = *reinterpret_cast<const float2*>(xs + (w * WK_TOK + tok_u) * LD + mt * 16 + col_u);
-      against(acc, I::q);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        us[(mt * 16 + col_u) * LDU + tok_u] = fu[2 * mt] - ((y[mt][0].x + y[mt][1].x) + (y[mt][2].x + y[mt][3].x));
-        us[(mt * 16 + col_u + 1) * LDU + tok_u] = fu[2 * mt + 1] - ((y[mt][0].y + y[mt][1].y) + (y[mt][2].y + y[mt][3].y));
-      }
-    } else {
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) us[(buf * COLS + mt * 16 + col_u + e) * LDU + tok_u] = fu[2 * mt + e];
-      against(acc, I::q);
-    }
-    __syncthreads();
-    // the chunk before: its partial sums are all there (they have two buffers)
-    if (c > c0) put_out(tok0 - WK_TOK, buf ^ 1);
-    // ---- the state's update, and the chunk's own tokens (a quarter of those products a warp)
-    float keep[2 * N], suf[4], total = 1.f;
-    if constexpr (MODE == WALK_HEAD) {
-      float p0[2], p1[2], x[1];
-      wk_ring_read<2>(p0, st, I::last);
-      wk_ring_read<2>(p1, st, I::last + 2);
-      wk_ring_read<4>(suf, st, I::last + 4);
-      wk_ring_read<1>(x, st, I::more);
-      total = x[0];
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          acc[mt][0][e] *= p0[e & 1];
-          acc[mt][1][e] *= p1[e & 1];
+            for (int p = 0; p < N; ++p) wk_fma2(next[e][p], S[e][p], keep[p]);
         }
-    } else {
-      wk_ring_read<2 * N>(keep, st, I::last);
-    }
-    float fp[2];
-    wk_ring_read<2>(fp, st, I::pair);
-    const Tf32x2 bp[2] = {wk_split(fp[0]), wk_split(fp[1])};
-    float rest[MT][N][4] = {};
-    FragA au[MT][2];
+        float4 uj[C];
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      float ua[4], ub[4];
-      const float* ut = us + ((MODE == WALK_DELTA ? 0 : buf) * COLS + mt * 16 + g) * LDU + 4 * t;
-      wk_load<4>(ua, ut);
-      wk_load<4>(ub, ut + 8 * LDU);
+        for (int e = 0; e < C; ++e) uj[e] = *reinterpret_cast<const float4*>(uk + e * WK_TOK + j);
 #pragma unroll
-      for (int s = 0; s < 2; ++s) au[mt][s] = wk_frag(ua[2 * s], ub[2 * s], ua[2 * s + 1], ub[2 * s + 1]);
+        for (int i = 0; i < 4; ++i) {
+          wk_f2 x[N];
+          wk_row<N>(x, st + I::k + (j + i) * DKP, l);
 #pragma unroll
-      for (int nt = 0; nt < N; ++nt)
+          for (int e = 0; e < C; ++e) {
+            const float f = i == 0 ? uj[e].x : i == 1 ? uj[e].y : i == 2 ? uj[e].z : uj[e].w;
+            const wk_f2 twice = wk_pair(f, f);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[mt][nt][e] *= MODE == WALK_HEAD ? total : keep[N * (e & 1) + nt];
-    }
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      float fk[2][N];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        wk_ring_read<N>(fk[e], st, I::k + (2 * s + e) * N);
-        if constexpr (MODE == WALK_HEAD) {
-#pragma unroll
-          for (int nt = 0; nt < N; ++nt) fk[e][nt] *= suf[2 * s + e];
+            for (int p = 0; p < N; ++p) wk_fma2(next[e][p], twice, x[p]);
+          }
         }
       }
-      Tf32x2 b[N][2];
 #pragma unroll
-      for (int nt = 0; nt < N; ++nt)
+      for (int e = 0; e < C; ++e)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) b[nt][e] = wk_split(fk[e][nt]);
+        for (int p = 0; p < N; ++p) S[e][p] = next[e][p];
+      leave(buf ^ 1);
+      __syncwarp();  // (u is read to the end before the next chunk's takes its place)
+    } else {
+      fetch(c + ST - 1);
+      if (c > c0) {  // the chunk before: P U
+        const float* uc = us + (buf ^ 1) * COLS * WK_TOK;
+        bool finite = true;
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+        for (int e = 0; e < C; ++e) finite = finite && fabsf(uc[e * WK_TOK + l]) <= FLT_MAX;
+        finite = __all_sync(0xffffffffu, finite);
+        if (finite) {
+          wk_f2 a[C];
 #pragma unroll
-        for (int nt = 0; nt < N; ++nt) wk_part<0>(S[mt][nt], rest[mt][nt], au[mt][s], b[nt]);
+          for (int e = 0; e < C; ++e) a[e] = wk_pair(out[e], 0.f);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+          for (int j = 0; j < WK_OWN; j += 4)
 #pragma unroll
-        for (int nt = 0; nt < N; ++nt) wk_part<1>(S[mt][nt], rest[mt][nt], au[mt][s], b[nt]);
+            for (int e = 0; e < C; ++e) {
+              const ulonglong2 uj = *reinterpret_cast<const ulonglong2*>(uc + e * WK_TOK + j0 + j);
+              wk_fma2(a[e], P[j / 2], uj.x);
+              wk_fma2(a[e], P[j / 2 + 1], uj.y);
+            }
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+          for (int e = 0; e < C; ++e) out[e] = wk_sum2(a[e]);
+        } else {  // (zero times a later token's infinity is no zero)
 #pragma unroll
-        for (int nt = 0; nt < N; ++nt) wk_part<2>(S[mt][nt], rest[mt][nt], au[mt][s], b[nt]);
-    }
+          for (int j = 0; j < WK_OWN; ++j) {
+            const float2 x = wk_halves(P[j / 2]);
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      float own[4] = {}, rest_own[4] = {};
-      FragA f;
+            for (int e = 0; e < C; ++e)
+              if (j0 + j <= tk) out[e] = fmaf(j & 1 ? x.y : x.x, uc[e * WK_TOK + j0 + j], out[e]);
+          }
+        }
+        const int tok = tok0 - WK_TOK + tk;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        f.hi[e] = warp >> 1 ? au[mt][1].hi[e] : au[mt][0].hi[e];
-        f.lo[e] = warp >> 1 ? au[mt][1].lo[e] : au[mt][0].lo[e];
+        for (int e = 0; e < C; ++e) {
+          out[e] += __shfl_xor_sync(0xffffffffu, out[e], 8);
+          if ((e & 1) == (l >> 3) && tok < row_end && v0 + mine + e < dv) o[((size_t)tok * H + h) * dv + v0 + mine + e] = out[e];
+        }
       }
-      wk_part<0>(own, rest_own, f, bp);
-      wk_part<1>(own, rest_own, f, bp);
-      wk_part<2>(own, rest_own, f, bp);
+      if (c == c1) break;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        own[e] += rest_own[e];
-        acc[mt][0][e] += warp & 1 ? 0.f : own[e];
-        acc[mt][1][e] += warp & 1 ? own[e] : 0.f;
+      for (int e = 0; e < C; ++e) wk_row<N>(S[e], states + (buf * COLS + e) * DKP, l);
+#pragma unroll
+      for (int j = 0; j < WK_OWN; j += 4) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(st + I::pair + tk * I::ldp + j0 + j);
+        P[j / 2] = x.x;
+        P[j / 2 + 1] = x.y;
       }
+      wk_against<N, C, WK_OWN>(out, S, st + I::q + tk0 * DKP, l);
+      if constexpr (MODE == WALK_HEAD) {
+        const float f = st[I::last + tk];
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          os[((buf * WK_WARPS + warp) * WK_TOK + j * 8 + 2 * t + (e & 1)) * LD + mt * 16 + g + (e >= 2 ? 8 : 0)] = acc[mt][j][e];
-#pragma unroll
-      for (int nt = 0; nt < N; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) S[mt][nt][e] += rest[mt][nt][e];
+        for (int e = 0; e < C; ++e) out[e] *= f;
+      }
     }
   }
-  __syncthreads();
-  put_out(row_begin + (c1 - 1 - c0) * WK_TOK, (c1 - 1 - c0) & 1);
+  if (!chain) return;
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
+  for (int e = 0; e < C; ++e)
 #pragma unroll
-    for (int nt = 0; nt < N; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int col = v0 + mt * 16 + g + (e >= 2 ? 8 : 0), c = mine + N * (e & 1) + nt;
-        if (col < dv && c < dk) slot[(size_t)col * dk + c] = S[mt][nt][e];
-      }
+    for (int p = 0; p < N; ++p) {
+      const float2 x = wk_halves(S[e][p]);
+      const int col = v0 + mine + e, ch = wk_channel<N>(l, p, 0);
+      if (col < dv && ch < dk) slot[(size_t)col * dk + ch] = x.x;
+      if (col < dv && ch + 1 < dk) slot[(size_t)col * dk + ch + 1] = x.y;
+    }
 }
 
 // ---------------------------------------------------------------- one decay per head: the pairs of a chunk's tokens
@@ -627,7 +567,8 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
                  int ld_k, int qk_group, const float* __restrict__ decay, int ld_decay, const int* __restrict__ cu_q, int num_rows, int H,
                  float q_scale) {
   __shared__ __align__(16) float qs[WK_TOK][DK + 4], ks[WK_TOK][DK + 4];
-  __shared__ float dot[WK_TOK][WK_TOK + 1], as[WK_TOK][33];
+  __shared__ double dot[WK_TOK][WK_TOK + 1];
+  __shared__ float as[WK_TOK][33];
   pdl_prologue();
   const int chunk = blockIdx.x, grp = blockIdx.y;
   const int2 at = wk_at(chunk, cu_q, num_rows);
@@ -648,16 +589,27 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
   __syncthreads();
   {  // a thread's two dot products: token i with j and with j + 8
     const int i = tid >> 3, j = tid & 7;
-    float s0[4] = {}, s1[4] = {};
-#pragma unroll 4
-    for (int c = 0; c < DK; c += 4) {
-      const float4 a = *reinterpret_cast<const float4*>(&qs[i][c]), b = *reinterpret_cast<const float4*>(&ks[j][c]),
-                   d = *reinterpret_cast<const float4*>(&ks[j + 8][c]);
-      s0[0] = fmaf(a.x, b.x, s0[0]); s0[1] = fmaf(a.y, b.y, s0[1]); s0[2] = fmaf(a.z, b.z, s0[2]); s0[3] = fmaf(a.w, b.w, s0[3]);
-      s1[0] = fmaf(a.x, d.x, s1[0]); s1[1] = fmaf(a.y, d.y, s1[1]); s1[2] = fmaf(a.z, d.z, s1[2]); s1[3] = fmaf(a.w, d.w, s1[3]);
+    wk_f2 s0[16] = {}, s1[16] = {};  // (sums of DK / 32 products, added up in 64 bits)
+#pragma unroll 1
+    for (int c = 0; c < DK; c += 32)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&qs[i][c + 4 * e]), b = *reinterpret_cast<const ulonglong2*>(&ks[j][c + 4 * e]),
+                         d = *reinterpret_cast<const ulonglong2*>(&ks[j + 8][c + 4 * e]);
+        wk_fma2(s0[2 * e], a.x, b.x);
+        wk_fma2(s0[2 * e + 1], a.y, b.y);
+        wk_fma2(s1[2 * e], a.x, d.x);
+        wk_fma2(s1[2 * e + 1], a.y, d.y);
+      }
+    double x0 = 0.0, x1 = 0.0;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const float2 a = wk_halves(s0[e]), b = wk_halves(s1[e]);
+      x0 += (double)a.x + (double)a.y;
+      x1 += (double)b.x + (double)b.y;
     }
-    dot[i][j] = ((s0[0] + s0[1]) + (s0[2] + s0[3])) * q_scale;
-    dot[i][j + 8] = ((s1[0] + s1[1]) + (s1[2] + s1[3])) * q_scale;
+    dot[i][j] = x0;
+    dot[i][j + 8] = x1;
   }
   for (int h0 = 0; h0 < qk_group; h0 += 32) {
     const int heads = min(32, qk_group - h0), first = grp * qk_group + h0;
@@ -670,32 +622,40 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
     for (int idx = tid; idx < heads * WK_TOK; idx += WK_THREADS) {  // (head, token j): the pairs that j's write is in, running over i
       const int e = idx >> 4, j = idx & 15;
       float* out = pairs + ((size_t)chunk * H + first + e) * (WK_TOK * WK_TOK) + j;
-      float run = 1.f, before = 1.f;
+      double run = 1.0, before = 1.0;
 #pragma unroll
       for (int i = 0; i < WK_TOK; ++i) {
-        const float a = as[i][e];
+        const double a = (double)as[i][e];
         if (i > j) run *= a;
         if (i <= j) before *= a;
-        out[i * WK_TOK] = i >= j ? dot[i][j] * run : 0.f;
+        out[i * WK_TOK] = i >= j ? (float)(dot[i][j] * (run * (double)q_scale)) : 0.f;
       }
       float* dec = decays + ((size_t)chunk * H + first + e) * (3 * WK_TOK);
-      dec[j] = before * q_scale;
-      dec[WK_TOK + j] = run;
-      if (j == WK_TOK - 1) dec[2 * WK_TOK] = before;
+      dec[j] = (float)(before * (double)q_scale);
+      dec[WK_TOK + j] = (float)run;
+      if (j == WK_TOK - 1) dec[2 * WK_TOK] = (float)before;
     }
   }
 }
 
-// Dynamic shared memory beyond 48 KB is asked for once per kernel. Not a dependent launch: CTAs that become resident while the kernel
-// before drains gather on the SMs that are free first, and two chains on one SM walk at half the rate (16 heads of 64 x 64 with the delta
-// rule over 2,048 tokens, both kernels: 140 us against 188; 32 heads of 128 x 64 with a decay per head 134 against 238).
-#define MS_WALK_LAUNCH(MODE, N, MT, grid, ...)                                                                            \
-  do {                                                                                                                    \
-    auto walk = walk_kernel<MODE, N, MT>;                                                                                 \
-    constexpr size_t bytes = WalkItems<MODE, N, MT>::bytes;                                                               \
-    static const cudaError_t asked = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
-    MS_CHECK_CUDA(asked);                                                                                                 \
-    MS_LAUNCH_APART(walk, grid, WK_THREADS, bytes, stream, __VA_ARGS__);                                                  \
+// Dynamic shared memory beyond 48 KB is asked for once per kernel and device. Not a dependent launch: CTAs that become resident while the kernel
+// before drains gather on the SMs that are free first, and two chains on one SM walk at half the rate.
+#define MS_WALK_LAUNCH(MODE, N, C, ...)                                                                                     \
+  do {                                                                                                                      \
+    auto walk = walk_kernel<MODE, N, C>;                                                                                    \
+    constexpr size_t bytes = WalkStage<MODE, N, C>::bytes;                                                                  \
+    static const cudaError_t asked = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);   \
+    MS_CHECK_CUDA(asked);                                                                                                   \
+    MS_LAUNCH_APART(walk, dim3(ceil_div(dv, WalkStage<MODE, N, C>::cols), H, num_rows), (WK_CHAIN + WK_OUT) * 32, bytes, stream, __VA_ARGS__); \
+  } while (0)
+// Four columns a lane take half the reads from shared memory of two, but half the CTAs too: two until 16 columns a CTA leave two SMs of three
+// one. Both kernels, 2,048 tokens, two columns against four, us: 64 CTAs of 16 columns (16 heads of 64 x 64, delta rule) 140 / 169, (8 of 64 x 128,
+// decay rule) 107 / 126; 128 of them (32 of 64 x 64, delta rule) 242 / 221, (32 of 128 x 64, a decay per head) 219 / 191; 768 (three rows, 64
+// of 128 x 64) 396 / 254.
+#define MS_WALK_LAUNCH_FOR(MODE, N, ...)                                                                                            \
+  do {                                                                                                                              \
+    if (3ll * num_rows * H * ceil_div(dv, WalkStage<MODE, N, 4>::cols) >= 2ll * sms) MS_WALK_LAUNCH(MODE, N, 4, __VA_ARGS__);       \
+    else MS_WALK_LAUNCH(MODE, N, 2, __VA_ARGS__);                                                                                   \
   } while (0)
 
 template <typename TIn, typename TZ, bool DELTA, int N>
@@ -714,8 +674,9 @@ int launch_walk(float* o, float* state, const TIn* q, int ld_q, const TIn* k, in
   auto prepare = walk_prepare_kernel<TIn, TZ, DELTA, N>;
   MS_LAUNCH(prepare, dim3(max_chunks, H), WK_THREADS, 0, stream, wp, qp, kp, last, u0, pairs, q, ld_q, k, ld_k, qk_group, v, ld_v, z, ld_z, z_bias,
             decay_coef, z_sign, beta, ld_beta, v_scale, cu_q, num_rows, H, dk, dv, dvp, q_scale);
-  MS_WALK_LAUNCH(DELTA ? WALK_DELTA : WALK_CHANNEL, N, 1, dim3(dvp / WK_COLS, H, num_rows), o, state, qp, DKP, wp, kp, DKP, 1, last, u0, dvp,
-                 (const float*)nullptr, pairs, cu_q, q_start, state_slot, H, dk, dv);
+  const int sms = sm_count();
+  MS_WALK_LAUNCH_FOR((DELTA ? WALK_DELTA : WALK_CHANNEL), N, o, state, qp, DKP, wp, kp, DKP, 1, last, u0, dvp, (const float*)nullptr, pairs, cu_q,
+                     q_start, state_slot, H, dk, dv);
   return 0;
 }
 
@@ -737,24 +698,14 @@ int launch_walk_head(float* o, float* state, const float* q, int ld_q, const flo
                      const float* decay, int ld_decay, const float* v_scale, float* scratch, const int* cu_q, const int* q_start,
                      const int* state_slot, int num_rows, int max_chunks, int H, int dv, float q_scale, cudaStream_t stream) {
   constexpr int DK = 32 * N;
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0;
-    MS_CHECK_CUDA(cudaGetDevice(&dev));
-    MS_CHECK_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
-  }
   float* pairs = scratch;
   float* decays = pairs + (size_t)max_chunks * H * WK_TOK * WK_TOK;
   auto prepare = walk_head_kernel<DK>;
   MS_LAUNCH(prepare, dim3(max_chunks, H / qk_group), WK_THREADS, 0, stream, pairs, decays, q, ld_q, k, ld_k, qk_group, decay, ld_decay, cu_q,
             num_rows, H, q_scale);
-  // 32 value columns a CTA share what they load and split of q and k, where that leaves two CTAs an SM
-  if ((long long)num_rows * H * ceil_div(dv, 2 * WK_COLS) >= 2LL * sm_count)
-    MS_WALK_LAUNCH(WALK_HEAD, N, 2, dim3(ceil_div(dv, WK_COLS * 2), H, num_rows), o, state, q, ld_q, (const float*)nullptr, k, ld_k, qk_group, decays, v,
-                   ld_v, v_scale, pairs, cu_q, q_start, state_slot, H, DK, dv);
-  else
-    MS_WALK_LAUNCH(WALK_HEAD, N, 1, dim3(ceil_div(dv, WK_COLS), H, num_rows), o, state, q, ld_q, (const float*)nullptr, k, ld_k, qk_group, decays, v,
-                   ld_v, v_scale, pairs, cu_q, q_start, state_slot, H, DK, dv);
+  const int sms = sm_count();
+  MS_WALK_LAUNCH_FOR(WALK_HEAD, N, o, state, q, ld_q, (const float*)nullptr, k, ld_k, qk_group, decays, v, ld_v, v_scale, pairs, cu_q, q_start,
+                     state_slot, H, DK, dv);
   return 0;
 }
 

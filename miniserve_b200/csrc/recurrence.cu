@@ -16,7 +16,7 @@
 // worked out beforehand by a kernel of their own (exponentials and logarithms for every token and
 // channel at once, instead of inside the serial walk); a decode step works them out while staging. The state is carried in
 // float32 and nothing in a token's arithmetic depends on this chunking. Prompts with up to 128 key channels run the decay and the
-// delta rule in chunks of 16 tokens on the tensor cores instead (chunk_walk.cu).
+// delta rule in chunks of 16 tokens instead (chunk_walk.cu).
 //
 // The decay is d = exp(-c_h * softplus(sign * (z + bias))) with z the output of a projection:
 // sign = -1, c_h = 1/tau gives sigmoid(z + bias)^(1/tau); sign = +1, c_h = exp(A_h) gives

@@ -50,23 +50,41 @@ def _columns(gen, t, width, dtype, pad):
     return torch.randn(t, width + 2 * pad, generator=gen).to(torch.bfloat16).to(dtype).to(DEV)[:, pad:pad + width]
 
 
-def _both(run, q, k, v, dk, head_decay, want, size, last, state, heads, dv):
-    """Runs by chunks and token by token: (largest error over the terms' size, its root mean square, the states' largest error) of each."""
+ROUTES = {"chunks": dict(WALK_MIN_TOKENS=1), "walk": dict(WALK_MIN_TOKENS=1 << 30, SEGMENTS=1),
+          "segments": dict(WALK_MIN_TOKENS=1 << 30, SEGMENT_MIN_TOKENS=1)}
+
+
+def _by(route, run, q, k, v, dk, head_decay, rows, slots, state, heads, dv):
+    """(outputs, the state behind) of one route."""
+    kept = {name: getattr(mixers, name) for name in ROUTES[route]}
+    try:
+        for name, value in ROUTES[route].items():
+            setattr(mixers, name, value)
+        ctx = _ctx(rows, slots)
+        assert mixers.walk_ok(q, k, v, dk, ctx, head_decay=head_decay) == (route == "chunks")
+        st, o = state.clone(), torch.full((q.shape[0], heads, dv), float("nan"), device=DEV)
+        run(o, st, ctx)
+    finally:
+        for name, value in kept.items():
+            setattr(mixers, name, value)
+    return o, st
+
+
+def _both(run, q, k, v, dk, head_decay, want, size, last, state, heads, dv, delta=False):
+    """By chunks, token by token, and (the decay rule) in segments: largest error over the terms' size, root mean square of it, of the states'."""
     errors = {}
-    for name, least in (("chunks", 1), ("walk", 1 << 30)):
-        kept, mixers.WALK_MIN_TOKENS = mixers.WALK_MIN_TOKENS, least
-        try:
-            ctx = _ctx(ROWS, SLOTS)
-            assert mixers.walk_ok(q, k, v, dk, ctx, head_decay=head_decay) == (name == "chunks")
-            st, o = state.clone(), torch.full((q.shape[0], heads, dv), float("nan"), device=DEV)
-            run(o, st, ctx)
-        finally:
-            mixers.WALK_MIN_TOKENS = kept
-        off = (o.double().cpu() - want).abs() / size
-        errors[name] = (off.max().item(), off.pow(2).mean().sqrt().item(), ((st.double().cpu() - last).abs().max() / last.abs().max()).item())
+    for route in ("chunks", "walk") if delta else ("chunks", "walk", "segments"):
+        o, st = _by(route, run, q, k, v, dk, head_decay, ROWS, SLOTS, state, heads, dv)
+        off, behind = (o.double().cpu() - want).abs() / size, (st.double().cpu() - last).abs()
+        errors[route] = (off.max().item(), off.pow(2).mean().sqrt().item(), (behind.max() / last.abs().max()).item(), behind.pow(2).mean().sqrt().item())
     print(dk, dv, errors)
-    # factors of 22 bits (2.4e-7 a product) and float32 sums: below 1e-6 of the terms' sizes
-    assert errors["chunks"][0] < 1e-6 and errors["chunks"][2] < 4e-6, errors
+    # a float32 sum in any order: a few roundings of 6e-8 of the terms' sizes, at most one for each of them
+    for route, e in errors.items():
+        assert e[0] < 1e-6 and e[2] < 1e-6, (route, errors)
+    # and chunks are no less accurate than the walk: two root mean squares over n numbers of like size differ by chance by 1 / sqrt(n) of
+    # themselves, and these numbers' sizes differ
+    for at, n in ((1, want.numel()), (3, last.numel())):
+        assert errors["chunks"][at] < (1.05 + 10 / n ** 0.5) * errors["walk"][at], errors
 
 
 @pytest.mark.parametrize("dtype, z_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16)])
@@ -97,7 +115,7 @@ def test_channel_decays_by_chunks(dtype, z_dtype, rule, heads, groups, dk, dv, p
                    ROWS, SLOTS, state.double().cpu())
     _both(lambda o, st, ctx: ops.decay_scan(o, st, q, k, v, z, bias, coef, 1.0, beta, ctx, heads, dk, dv, 0.3, delta=delta,
                                             v_scale=scale),
-          q, k, v, dk, False, *exact, state, heads, dv)
+          q, k, v, dk, False, *exact, state, heads, dv, delta)
 
 
 @pytest.mark.parametrize("heads, groups, dk, dv, scaled", [(8, 2, 128, 64, True), (4, 4, 64, 16, True), (2, 1, 32, 33, False), (160, 2, 32, 70, True),
@@ -136,3 +154,64 @@ def test_many_rows():
     o, st = torch.full((t, heads, d), float("nan"), device=DEV), state.clone()
     ops.decay_scan(o, st, q, k, v, a, None, None, 0.0, None, ctx, heads, d, d, 1.0, delta=False, head_decay=True)
     assert ((o.double().cpu() - want).abs() / size).max() < 1e-6 and ((st.double().cpu() - last).abs().max() / last.abs().max()) < 4e-6
+
+
+def _operands(rule, gen, t, heads, dk, dv, lo, hi):
+    """Operands whose decays are uniform in [lo, hi], and how to run them: (run, q, k, v, exact decays, beta, factor on the values)."""
+    rnd, uni = (lambda *s: torch.randn(*s, generator=gen).to(DEV)), (lambda *s: torch.rand(*s, generator=gen).to(DEV))
+    q, k, v = rnd(t, heads * dk), rnd(t, heads, dk), rnd(t, heads * dv)
+    k = (k / k.norm(dim=-1, keepdim=True)).reshape(t, -1).contiguous()
+    if rule == "head":
+        a, scale = lo + (hi - lo) * uni(t, heads), uni(t, heads) * 0.1 + 0.01
+        return (lambda o, st, ctx: ops.decay_scan(o, st, q, k, v, a, None, None, 0.0, None, ctx, heads, dk, dv, 0.25, delta=False, head_decay=True,
+                                                  v_scale=scale)), q, k, v, a.double().cpu()[:, :, None].expand(t, heads, dk), None, scale, a
+    coef, bias = uni(heads) * 0.5 + 0.2, torch.zeros(heads * dk, device=DEV)
+    decay = (lo + (hi - lo) * uni(t, heads * dk).double()).clamp(max=1 - 2.0 ** -22)
+    z = torch.log(torch.expm1(-torch.log(decay) / coef.double().repeat_interleave(dk))).float()
+    soft = torch.nn.functional.softplus(z.double().cpu(), threshold=1e9)
+    exact = torch.exp(-coef.double().cpu().repeat_interleave(dk) * soft).view(t, heads, dk)
+    beta = rnd(t, heads) if rule == "delta" else None
+    return (lambda o, st, ctx: ops.decay_scan(o, st, q, k, v, z, bias, coef, 1.0, beta, ctx, heads, dk, dv, 0.25, delta=rule == "delta")), \
+        q, k, v, exact, None if beta is None else torch.sigmoid(beta.double().cpu()), None, z
+
+
+@pytest.mark.parametrize("rule, heads, dk, dv", [("decay", 2, 64, 64), ("delta", 2, 64, 64), ("head", 2, 128, 64)])
+@pytest.mark.parametrize("lo, hi", [(0.02, 0.6), (0.7, 0.99), (0.999, 1.0), (0.9999, 1.0)])
+def test_long_rows_by_chunks_are_as_accurate_as_the_walk(rule, heads, dk, dv, lo, hi):
+    """2,048 tokens behind a stored state: states of a token or two, and states that last from the first token to the last."""
+    gen = torch.Generator().manual_seed(int(hi * 100) + dk)
+    rows, slots, t = [(9, 2048), (0, 40)], [1, 0], 2088
+    run, q, k, v, decay, beta, scale, _ = _operands(rule, gen, t, heads, dk, dv, lo, hi)
+    state = torch.randn(2, heads, dv, dk, generator=gen).to(DEV)
+    wide = lambda x: x.double().cpu().view(t, heads, -1)  # noqa: E731
+    vd = wide(v) * (1.0 if scale is None else scale.double().cpu()[:, :, None])
+    want, _, last = _exact(wide(q) * 0.25, wide(k), vd, decay, beta, rows, slots, state.double().cpu())
+    errors = {}
+    for route in ("chunks", "walk"):
+        o, st = _by(route, run, q, k, v, dk, rule == "head", rows, slots, state, heads, dv)
+        off, behind = o.double().cpu() - want, (st.double().cpu() - last) / last.pow(2).mean().sqrt()
+        errors[route] = (off.pow(2).mean().sqrt() / want.pow(2).mean().sqrt()).item(), behind.pow(2).mean().sqrt().item()
+    print(rule, lo, hi, errors)
+    assert all(c < 1.05 * w for c, w in zip(errors["chunks"], errors["walk"])), errors
+
+
+@pytest.mark.parametrize("rule, heads, dk, dv", [("decay", 2, 64, 24), ("delta", 2, 40, 64), ("head", 2, 32, 33)])
+@pytest.mark.parametrize("where, bad", [(w, float(b)) for w in ("v", "k", "q", "state") for b in ("inf", "nan")]
+                         + [("decay", float("nan")), ("v", -3.4e38), ("state", -1e37)])
+def test_values_that_are_not_finite_stay_with_their_token_and_the_later_ones(rule, heads, dk, dv, where, bad):
+    """The same outputs and states are finite as token by token (also beside numbers near the largest), the others what they are without."""
+    gen = torch.Generator().manual_seed(3)
+    rows, slots, t = [(4, 37), (0, 20)], [1, 0], 57
+    run, q, k, v, _, _, _, z = _operands(rule, gen, t, heads, dk, dv, 0.7, 0.99)
+    state = torch.randn(2, heads, dv, dk, generator=gen).to(DEV)
+    args = q, k, v, dk, rule == "head", rows, slots
+    plain = _by("chunks", run, *args, state, heads, dv)
+    if where == "state":
+        state[1, 0, 3, 5] = bad
+    else:
+        dict(v=v, k=k, q=q, decay=z)[where][21, 1] = bad
+    got, want = (_by(route, run, *args, state, heads, dv) for route in ("chunks", "walk"))
+    for g, w, p in zip(got, want, plain):
+        assert torch.equal(torch.isfinite(g), torch.isfinite(w))
+        own = (w - p).abs() <= 1e-5 * p.abs().max()  # (what the number does not reach; the walk says which)
+        assert own.float().mean() > 0.5 and ((g - p).abs()[own] <= 2e-5 * p.abs().max()).all()
