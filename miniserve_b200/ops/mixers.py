@@ -206,7 +206,8 @@ def sum_bias(out, a, b=None, vec=None, stream=None) -> None:
 
 
 def decay_scan(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign: float, beta, ctx, heads: int, dk: int, dv: int,
-               q_scale: float, delta: bool, head_decay: bool = False, v_scale=None, ones_column: bool = False, bonus=None) -> None:
+               q_scale: float, delta: bool, head_decay: bool = False, v_scale=None, ones_column: bool = False, bonus=None,
+               exact: bool = False) -> None:
     """The recurrence of every row of the step, token by token (``csrc/recurrence.cu``) or by chunks of 16 (``walk_ok``), from each
     request's slot of ``state`` [slots, heads, dv, dk] float32 (zero where a row starts at position 0)
     and back into it; o_out [T, heads, dv] float32. q, k [T, groups*dk], v [T, heads*dv], z [T, heads*dk]
@@ -216,7 +217,9 @@ def decay_scan(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign: float, beta
     ``ones_column``: v has heads * (dv - 1) columns and every head's last value is one (times v_scale): that column of the state is
     the decayed sum of the keys, that entry of the output its product with the query (the decay rule only).
     ``bonus`` [heads * dk] float32: the read-out sees the state before the token's own write, and that write times ``bonus`` per key channel;
-    z [T, heads*dk] float32 then holds the decays themselves."""
+    z [T, heads*dk] float32 then holds the decays themselves.
+    ``exact``: never by chunks (what 32-bit models ask for: how a prompt is cut into steps, and what else a step holds, then changes no
+    bits of short steps, and of long ones no more than the segments do)."""
     t = o_out.shape[0]
     dv_in = dv - int(ones_column)
     _f32(o_out, state, z_bias, decay_coef, v_scale, bonus)
@@ -227,7 +230,7 @@ def decay_scan(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign: float, beta
     assert z.shape == (t, heads if head_decay else heads * dk) and (not head_decay or (z.dtype == torch.float32 and not delta))
     assert q.dtype == k.dtype == v.dtype and (beta is None or beta.dtype == z.dtype)
     assert v_scale is None or v_scale.shape == (t, heads)
-    if walk_ok(q, k, v, dk, ctx, head_decay, ones_column, bonus):
+    if not exact and walk_ok(q, k, v, dk, ctx, head_decay, ones_column, bonus):
         return _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx, heads, dk, dv, q_scale, delta, head_decay, v_scale)
     if not delta and not ctx.decode_only and t >= SEGMENT_MIN_TOKENS and SEGMENTS > 1 and dk <= SEGMENT_MAX_DK:
         return _decay_scan_segmented(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, ctx, heads, dk, dv, q_scale, head_decay,

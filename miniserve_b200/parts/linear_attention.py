@@ -94,7 +94,7 @@ class DecayLinearAttention(Part):
         at_k, at_v, at_g = h * dk, 2 * h * dk, 2 * h * dk + h * dv
         # sigmoid(z)^(1/tau) = exp(-softplus(-z) / tau)
         ops.decay_scan(o, cache.state, proj[:, :at_k], proj[:, at_k:at_v], proj[:, at_v:at_g], z, self.w_a_bias, self.decay_coef,
-                       -1.0, None, ctx, h, dk, dv, dk ** -0.5, delta=False)
+                       -1.0, None, ctx, h, dk, dv, dk ** -0.5, delta=False, exact=dt == torch.float32)
         ops.head_norm_gate(out, o, self.w_norm, proj[:, at_g:at_g + h * dv], self.eps, scale, "silu", stream=ctx.stream)
 
     def forward(self, x, ctx, cache):
@@ -201,7 +201,7 @@ class GatedDeltaRule(Part):
         o = ctx.buffer("delta.o", (t, h, dv), torch.float32, dev)
         q, k, v = torch.split_with_sizes(qkv, (g * dk, g * dk, h * dv), 1)
         ops.decay_scan(o, state.state, q, k, v, zg[:, :h * dk],
-                       self.w_dt_bias, self.decay_coef, 1.0, proj[:, c:c + h], ctx, h, dk, dv, dk ** -0.5, delta=True)
+                       self.w_dt_bias, self.decay_coef, 1.0, proj[:, c:c + h], ctx, h, dk, dv, dk ** -0.5, delta=True, exact=dt == torch.float32)
         ops.head_norm_gate(out, o, self.w_norm, zg[:, h * dk:h * dk + h * dv], self.eps, scale, "sigmoid", stream=ctx.stream)
 
     def forward(self, x, ctx, cache):
@@ -305,7 +305,7 @@ class SelectiveStateSpace(Part):
         o = ctx.buffer("ssm.o", (t, h, dv), torch.float32, dev)
         xs, bs, cs = torch.split_with_sizes(xbc, (inner, g * n, g * n), 1)
         ops.decay_scan(o, state.state, cs, bs, xs, steps[1], None, self.decay_coef, 1.0, None, ctx, h, n, dv, 1.0, delta=False,
-                       head_decay=True, v_scale=steps[0])
+                       head_decay=True, v_scale=steps[0], exact=dt == torch.float32)
         ops.gated_group_norm(out, o.view(t, inner), xs, self.w_skip, proj[:, :inner], self.w_norm, self.norm_groups, dv, self.eps,
                              stream=ctx.stream)
 

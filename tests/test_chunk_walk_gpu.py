@@ -215,3 +215,32 @@ def test_values_that_are_not_finite_stay_with_their_token_and_the_later_ones(rul
         assert torch.equal(torch.isfinite(g), torch.isfinite(w))
         own = (w - p).abs() <= 1e-5 * p.abs().max()  # (what the number does not reach; the walk says which)
         assert own.float().mean() > 0.5 and ((g - p).abs()[own] <= 2e-5 * p.abs().max()).all()
+
+
+@pytest.mark.parametrize("kind", ["decay", "delta", "state_space"])
+def test_cuts_change_no_bit_of_a_32_bit_layer(kind):
+    """The 32-bit mode stays on the token-by-token walk: the same bits however a prompt is cut into portions, and whatever comes with it."""
+    from miniserve_b200.config import PartSpec
+    from miniserve_b200.parts import BuildEnv, build_part
+    from tests import test_fekulix_gpu as fekulix
+    from tests import test_rofozen_gpu as rofozen
+
+    torch.manual_seed(5)
+    if kind == "state_space":
+        part, _ = rofozen._ssm(torch.float32, 4, 16, 32, 2, 4, 2)
+        rofozen._bind(part, torch.float32, change=rofozen._ssm_weights)
+    else:
+        names = dict(q="q", k="k", v="v", g="g", o="o", norm="norm", a1="a1", a2="a2", a_bias="a2.b")
+        spec = PartSpec("decay_linear_attention", dict(hidden=48, heads=2, key_dim=24, value_dim=40, tau=5.0, decay_rank=8, eps=1e-5, names=names))
+        if kind == "delta":
+            spec = PartSpec("gated_delta_rule", dict(
+                hidden=48, heads=4, kv_heads=2, key_dim=16, value_dim=24, conv=3, decay_rank=8, gate_rank=16, eps=1e-5,
+                names=dict(q="q", k="k", v="v", q_conv="q.conv", k_conv="k.conv", v_conv="v.conv", beta="b", a_log="A_log", norm="norm", a1="a1",
+                           a2="a2", dt_bias="dt_bias", g1="g1", g2="g2", o="o")))
+        part = build_part("mixer", spec, BuildEnv(torch.float32, DEV))
+        fekulix._bind(part, torch.float32)
+    width = rofozen.HIDDEN if kind == "state_space" else 48
+    views, x = fekulix._state_views(part), torch.randn(60, width, device=DEV)
+    whole = fekulix._portions(part, views, x, (60,), 1, torch.float32)
+    for cuts in ((20, 3, 37), (15, 15, 15, 15), (44, 16)):
+        assert torch.equal(fekulix._portions(part, views, x, cuts, 1, torch.float32), whole), cuts
