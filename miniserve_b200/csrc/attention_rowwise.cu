@@ -491,8 +491,8 @@ MS_EXPORT int ms_attention_tiled_f32(float* out, const float* q, const float* k_
   do {                                                                                                                                          \
     auto kernel = attention_tiled_f32_kernel<MD>;                                                                                               \
     constexpr size_t smem = ((TW_ROWS + 4 * TW_KEYS) * (32 * MD + 4) + TW_ROWS * TW_LDS + 2 * TW_ROWS) * 4;                                     \
-    static const cudaError_t asked = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                      \
-    MS_CHECK_CUDA(asked);                                                                                                                       \
+    static std::atomic<unsigned long long> allowed{0};                                                                                          \
+    MS_CHECK_CUDA(allow_shared_memory((const void*)kernel, (int)smem, allowed));                                                                \
     MS_LAUNCH_APART(kernel, grid, TW_THREADS, smem, stream, out, q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, num_rows, nq, nkv, \
                     head_dim, scale, window, sink, page_shift, num_pages, status, sink_values, softcap, chunk, dist_r1, dist_r2, keep_first);                   \
   } while (0)

@@ -645,8 +645,8 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
   do {                                                                                                                      \
     auto walk = walk_kernel<MODE, N, C>;                                                                                    \
     constexpr size_t bytes = WalkStage<MODE, N, C>::bytes;                                                                  \
-    static const cudaError_t asked = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);   \
-    MS_CHECK_CUDA(asked);                                                                                                   \
+    static std::atomic<unsigned long long> allowed{0};                                                                      \
+    MS_CHECK_CUDA(allow_shared_memory((const void*)walk, (int)bytes, allowed));                                             \
     MS_LAUNCH_APART(walk, dim3(ceil_div(dv, WalkStage<MODE, N, C>::cols), H, num_rows), (WK_CHAIN + WK_OUT) * 32, bytes, stream, __VA_ARGS__); \
   } while (0)
 // Four columns a lane take half the reads from shared memory of two, but half the CTAs too: two until 16 columns a CTA leave two SMs of three

@@ -5,9 +5,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <atomic>
 #include <cstdio>
 #include <cstring>
+
+#include "per_device.cuh"
 
 namespace ms {
 
@@ -131,17 +132,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
       else if (now - began > limit_ns) return false;
     }
   }
-}
-
-// Multiprocessors of the calling thread's device, asked for once per device (0 if it cannot be had: only the choice of a form hangs on it).
-inline int sm_count() {
-  static std::atomic<int> known[64] = {};
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
-  if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
-  return n;
 }
 
 inline int& pdl_switch() {
