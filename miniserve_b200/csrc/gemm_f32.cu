@@ -180,12 +180,7 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
 // or columns, or rows that do not start on 16 bytes.
 inline int launch_gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int batch, long long stride_a,
                            long long stride_w, long long stride_c, cudaStream_t stream) {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    MS_CHECK_CUDA(cudaGetDevice(&dev));
-    MS_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  }
+  const int known = sm_count(), sms = known > 0 ? known : 148;
   const bool rows16 = lda % 4 == 0 && ldw % 4 == 0 && stride_a % 4 == 0 && stride_w % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
   auto cost = [&](int bm, int bn) {
     const long long tiles = (long long)ceil_div(M, bm) * ceil_div(N, bn) * batch;

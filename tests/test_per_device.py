@@ -50,3 +50,8 @@ def test_every_device_is_asked_once(tmp_path):
 def test_no_kernel_keeps_one_devices_answer():
     for source in sorted(CSRC.glob("*.cu*")):
         assert not re.search(r"static[^;{]*\bcudaError_t\b[^;]*=\s*cudaFuncSetAttribute", source.read_text()), source.name
+
+
+@pytest.mark.parametrize("source", ["gemm_f32.cu", "chunk_walk.cu"])
+def test_no_multiprocessor_count_of_one_device(source):
+    assert "cudaDevAttrMultiProcessorCount" not in (CSRC / source).read_text()
