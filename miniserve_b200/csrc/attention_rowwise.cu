@@ -249,7 +249,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
         if (c == 0) usable[buf][j] = in;
       }
     }
-    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   auto next_tile = [&](int tile) { return tile + TW_KEYS == kept_end ? lo_tile : tile + TW_KEYS; };
 
@@ -269,7 +269,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
 #pragma unroll 1
   for (; tile <= pos_last; tile = next_tile(tile), buf ^= 1) {
     stage(next_tile(tile), buf ^ 1);
-    asm volatile("cp.async.wait_group 1;\n" ::);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();
     if (r0 < rows) {
       const float* kb = ks + buf * TW_KEYS * LD;

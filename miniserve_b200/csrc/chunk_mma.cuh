@@ -9,11 +9,11 @@ constexpr int CS_TOK = 64, CS_THREADS = 256;
 __device__ __forceinline__ uint32_t cs_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cs_cp16(void* dst, const void* src, bool in) {
   const int bytes = in ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(cs_smem(dst)), "l"(src), "r"(bytes));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(cs_smem(dst)), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cs_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+__device__ __forceinline__ void cs_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
-__device__ __forceinline__ void cs_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+__device__ __forceinline__ void cs_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cs_ldsm(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(cs_smem(p)));
 }
