@@ -285,21 +285,26 @@ def conv_state_update(conv_state, x, ctx, taps: int) -> None:
         taps, _dt(x.dtype), ctx.stream))
 
 
-# Steps with fewer tokens stay on the token-by-token walk. Measured alone, chunks against walk in us: 16 heads of 64 x 64 with the delta rule 10 / 13
-# at 16 tokens, 13 / 37 at 64, 32 / 137 at 256 (58 / 62 for 63 single tokens beside 65); 8 of 64 x 128 with the decay rule 9 / 11, 14 / 29, 30 / 104;
-# 32 of 128 x 64 with a decay per head 10 / 16, 16 / 48, 38 / 179.
+# Rows with fewer tokens (steps, with a decay per head) stay on the token-by-token walk. Measured alone, chunks against walk in us: 16 heads of
+# 64 x 64 with the delta rule 11 / 14 at 16 tokens, 13 / 38 at 64, 24 / 137 at 256; 8 of 64 x 128 with the decay rule 11 / 11, 13 / 29, 21 / 102;
+# 32 of 128 x 64 with a decay per head 8 / 16, 13 / 49, 30 / 179. A single token costs a whole chunk: 64 rows of 2 tokens 57 / 38, 44 / 38, 95 / 123.
 WALK_MIN_TOKENS = 16
 
 
 def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool = False, bonus=None) -> bool:
     """Whether ``decay_scan`` walks the step by chunks of 16 tokens (``csrc/chunk_walk.cu``): a step that is not all single tokens, heads of up
     to 128 key channels, no more rows than a grid's last dimension; with one decay per head float32 operands whose rows start on 16 bytes, 32, 64
-    or 128 key channels."""
-    if ctx.decode_only or q.shape[0] < WALK_MIN_TOKENS or ctx.num_rows > 65535 or ones_column or bonus is not None or dk > 128:
+    or 128 key channels, else rows long enough."""
+    t = q.shape[0]
+    if ctx.decode_only or t < WALK_MIN_TOKENS or ctx.num_rows > 65535 or ones_column or bonus is not None or dk > 128:
         return False
-    if not head_decay:
-        return True
-    return (dk in (32, 64, 128) and q.dtype == torch.float32 and (q.data_ptr() | k.data_ptr()) % 16 == 0 and (q.stride(0) | k.stride(0)) % 4 == 0)
+    if head_decay:
+        return (dk in (32, 64, 128) and q.dtype == torch.float32 and (q.data_ptr() | k.data_ptr()) % 16 == 0 and (q.stride(0) | k.stride(0)) % 4 == 0)
+    # Every decoding row ahead of the prompts costs 0.4 to 0.75 us more by chunks, every token of the longest row 0.4 less; that row has at least
+    # the others' mean (what a captured graph is keyed by says no more of the lengths). 64 decoding rows beside 16, 64 and 512 tokens, us, chunks
+    # against walk: 16 heads with the delta rule 57 / 40, 59 / 60, 79 / 249; 32 heads 108 / 70, 115 / 100, 162 / 412.
+    singles = getattr(ctx, "leading_single_rows", 0)
+    return t - singles >= max(WALK_MIN_TOKENS, 2 * singles) * (ctx.num_rows - singles)
 
 
 @lru_cache(maxsize=256)
