@@ -543,8 +543,13 @@ def attention_rowwise(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, 
 
 def attention_tiled_ok(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx) -> bool:
     """Whether a float32 step runs ``attention_tiled``: a step that is not all single tokens (those keep a warp per token and head), head
-    sizes of whole fours up to 128, tensors that start on 16 bytes."""
+    sizes of whole fours up to 128, tensors that start on 16 bytes, contexts of more than a tile of keys."""
     if q.dtype != torch.float32 or getattr(ctx, "decode_only", False) or q.shape[0] <= ctx.num_rows:
+        return False
+    # A CTA's staging costs more than a few keys do: 2 tokens behind nothing 18 us tiled against 8, a prompt of 40 tokens 30 against 38 (16 heads
+    # of 128 on 8), 24 / 27 (32 of 64 on 4), 22 / 20 (4 of 64). A captured step is replayed for contexts of any length.
+    keys = getattr(ctx, "max_kv_len", 1 << 30) if getattr(ctx, "recorder", None) is None else 1 << 30
+    if keys <= (32 if q.shape[1] * q.shape[2] >= 1024 else 64):
         return False
     return (bool(native.kernels().ms_attention_tiled_f32_supports(q.shape[2], q.shape[1], k_pool.shape[1]))
             and all(x.data_ptr() % 16 == 0 for x in (out, q, k_pool, v_pool)))
