@@ -835,8 +835,9 @@ MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, void* conv
   if (taps >= 2 && taps <= 4 && C % 4 == 0 && ld % 4 == 0 && (uintptr_t)proj % item == 0 && (uintptr_t)conv_state % item == 0 && (uintptr_t)out % 16 == 0 &&
       (!bias || (uintptr_t)bias % 16 == 0) && (unit_heads == 0 || (dk % 4 == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0)) &&
       num_tokens <= 65535) {
-    // runs of eight tokens read an input once; a step that does not fill the GPU with them (decoding rows) takes one token a thread
-    const bool runs = (long long)ceil_div(C / 4, CONV_THREADS) * ceil_div(num_tokens, CONV_RUN) >= 2LL * scan_sm_count();
+    // runs of eight tokens read an input once; one token a thread, which looks up its row and reads a window of its own, where those CTAs are
+    // few enough to be on the GPU at once (decoding rows)
+    const bool runs = (long long)ceil_div(C / 4, CONV_THREADS) * num_tokens > 4LL * scan_sm_count();
     const dim3 grid(ceil_div(C / 4, CONV_THREADS), ceil_div(num_tokens, runs ? CONV_RUN : 1));
 #define MS_CONV(T, TAPS)                                \
   do {                                                  \
