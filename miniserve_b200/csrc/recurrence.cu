@@ -1024,8 +1024,9 @@ MS_EXPORT int ms_gated_group_norm(void* out, int ld_out, const float* o, const f
   MS_CHECK_ARG(parts >= 1 && width % parts == 0 && dv >= 1, "gated_group_norm: %d channels in %d parts", width, parts);
   const int item = dtype == MS_F32 ? 16 : 8, size = width / parts;
   // a warp per part reads up to 256 channels in two steps; wider parts, which it reads in up to eight, only where there are warps enough to
-  // fill the GPU: 32 tokens of 4,096 channels in 8 parts 4.5 us against 4.1 with a CTA a part, 2,048 in 2 parts 7.0 against 6.1
-  const bool warps_enough = size <= 256 || (long long)num_tokens * parts > 3LL * scan_sm_count();
+  // fill the GPU: 32 tokens of 4,096 channels in 8 parts 4.5 us against 4.1 with a CTA a part, 2,048 in 2 parts 7.0 against 6.1. (The two add a
+  // part's squares up in different orders: in float32 a token's bits must not hang on how many tokens the step has.)
+  const bool warps_enough = size <= 256 || dtype == MS_F32 || (long long)num_tokens * parts > 3LL * scan_sm_count();
   if (warps_enough && size % 4 == 0 && size <= 1024 && dv % 4 == 0 && ld_out % 4 == 0 && ld_gate % 4 == 0 && ld_x % 4 == 0 && (uintptr_t)out % item == 0 &&
       (uintptr_t)gate % item == 0 && (uintptr_t)o % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 && (long long)num_tokens * parts < (1 << 30)) {
     const int items = num_tokens * parts;

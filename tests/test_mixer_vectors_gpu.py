@@ -78,7 +78,7 @@ def test_head_norm_in_fours(dtype, t, heads, dv, kind, own):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("t, parts, size, dv, skip", [(1, 1, 4, 4, True), (9, 8, 512, 64, True), (5, 3, 260, 52, False), (3, 2, 1024, 128, True),
-                                                      (2, 1, 252, 12, True)])
+                                                      (2, 1, 252, 12, True), (500, 1, 1024, 64, True), (460, 1, 260, 52, False)])
 def test_group_norm_in_fours(dtype, t, parts, size, dv, skip):
     gen = torch.Generator().manual_seed(size)
     width = parts * size
@@ -92,3 +92,17 @@ def test_group_norm_in_fours(dtype, t, parts, size, dv, skip):
     ops.gated_group_norm(got, o, x, s, gate, w, parts, dv, 1e-6)
     ops.gated_group_norm(want, o, x, s, odd, w, parts, dv, 1e-6)
     _near(got, want, dtype)
+
+
+@pytest.mark.parametrize("size, parts", [(512, 2), (1024, 1), (64, 4)])
+def test_float32_norms_of_a_token_are_the_same_bits_in_any_step(size, parts):
+    """One token, a few and many: what the step holds beside a token picks no other order of its sums."""
+    gen = torch.Generator().manual_seed(size)
+    t, width = 600, size * parts
+    o, gate, w = (torch.randn(*s, generator=gen).to(DEV) for s in ((t, width), (t, width), (width,)))
+    whole = torch.empty(t, width, device=DEV)
+    ops.gated_group_norm(whole, o, None, None, gate, w, parts, 32, 1e-6)
+    for n in (1, 7, 150):
+        part = torch.empty(n, width, device=DEV)
+        ops.gated_group_norm(part, o[:n].contiguous(), None, None, gate[:n].contiguous(), w, parts, 32, 1e-6)
+        assert torch.equal(part, whole[:n])
