@@ -832,12 +832,17 @@ MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, void* conv
                unit_heads, dk, other_heads, dv);
   // four channels a thread where heads and rows are whole fours (and a normed head is a power of two of lanes of one warp)
   const int item = dtype == MS_F32 ? 16 : 8, lanes = dk / 4;
-  if (taps >= 2 && taps <= 4 && C % 4 == 0 && ld % 4 == 0 && (uintptr_t)proj % item == 0 && (uintptr_t)conv_state % item == 0 && (uintptr_t)out % 16 == 0 &&
-      (!bias || (uintptr_t)bias % 16 == 0) && (unit_heads == 0 || (dk % 4 == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0)) &&
-      num_tokens <= 65535) {
-    // runs of eight tokens read an input once; one token a thread, which looks up its row and reads a window of its own, where those CTAs are
-    // few enough to be on the GPU at once (decoding rows)
-    const bool runs = (long long)ceil_div(C / 4, CONV_THREADS) * num_tokens > 4LL * scan_sm_count();
+  // One token a thread, which looks up its row and reads a window of its own, where those CTAs are on the GPU at once (decoding rows); runs of
+  // eight tokens, which read an input once, where they give every multiprocessor threads enough. Between the two a warp per token and head is
+  // faster: with normed heads 201 tokens of 2,048 channels 5 us against 7 in runs and 8 one by one, 2,048 of 96 4 against 7 and 6; without, 64
+  // of 6,144 7.2 against 5.7 and 7.2. (Not in float32: the forms add a head's squares up in different orders, and a token's bits must not hang
+  // on how many tokens the step has.)
+  const int sms = scan_sm_count();
+  const bool single = (long long)ceil_div(C / 4, CONV_THREADS) * num_tokens <= 4LL * sms;
+  const bool runs = !single && (dtype == MS_F32 || (long long)(C / 4) * ceil_div(num_tokens, CONV_RUN) >= (long long)(unit_heads > 0 ? 128 : 64) * sms);
+  if ((runs || single) && taps >= 2 && taps <= 4 && C % 4 == 0 && ld % 4 == 0 && (uintptr_t)proj % item == 0 && (uintptr_t)conv_state % item == 0 &&
+      (uintptr_t)out % 16 == 0 && (!bias || (uintptr_t)bias % 16 == 0) &&
+      (unit_heads == 0 || (dk % 4 == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0)) && num_tokens <= 65535) {
     const dim3 grid(ceil_div(C / 4, CONV_THREADS), ceil_div(num_tokens, runs ? CONV_RUN : 1));
 #define MS_CONV(T, TAPS)                                \
   do {                                                  \

@@ -106,3 +106,16 @@ def test_float32_norms_of_a_token_are_the_same_bits_in_any_step(size, parts):
         part = torch.empty(n, width, device=DEV)
         ops.gated_group_norm(part, o[:n].contiguous(), None, None, gate[:n].contiguous(), w, parts, 32, 1e-6)
         assert torch.equal(part, whole[:n])
+
+
+@pytest.mark.parametrize("c, unit, dk", [(96, 1, 32), (2048, 16, 64)])
+def test_float32_convolutions_of_a_token_are_the_same_bits_in_any_step(c, unit, dk):
+    gen = torch.Generator().manual_seed(c)
+    t = 800
+    x, w, state = torch.randn(t, c, generator=gen).to(DEV), torch.randn(c, 4, generator=gen).to(DEV), torch.zeros(1, 3, c, device=DEV)
+    outs = []
+    for n in (t, 201, 40, 1):
+        out = torch.empty(n, c, device=DEV)
+        ops.conv_silu_unit(out, x[:n], state, w, _rows((n,), (0,)), unit, dk, c // dk - unit, dk, 1e-6)
+        outs.append(out)
+    assert all(torch.equal(o, outs[0][:o.shape[0]]) for o in outs)
