@@ -23,7 +23,7 @@ def _ctx(rows, slots):
     held = {}
     return SimpleNamespace(
         cu_q=torch.tensor(cu, **i32), q_start=torch.tensor([s for s, _ in rows], **i32), state_slot=torch.tensor(slots, **i32),
-        num_rows=len(rows), decode_only=False, stream=torch.cuda.current_stream().cuda_stream, step_cache={},
+        num_rows=len(rows), decode_only=False, held=held, stream=torch.cuda.current_stream().cuda_stream, step_cache={},
         buffer=lambda role, shape, dtype, dev: held.setdefault((role, shape, dtype), torch.empty(shape, dtype=dtype, device=dev)))
 
 
@@ -116,6 +116,28 @@ def test_channel_decays_by_chunks(dtype, z_dtype, rule, heads, groups, dk, dv, p
     _both(lambda o, st, ctx: ops.decay_scan(o, st, q, k, v, z, bias, coef, 1.0, beta, ctx, heads, dk, dv, 0.3, delta=delta,
                                             v_scale=scale),
           q, k, v, dk, False, *exact, state, heads, dv, delta)
+
+
+@pytest.mark.parametrize("rule, heads, dk, dv, exact", [("decay", 2, 136, 24, False), ("delta", 2, 136, 24, False), ("delta", 1, 256, 6, False),
+                                                        ("decay", 2, 24, 40, True), ("delta", 3, 64, 20, True)])
+def test_prompts_that_stay_on_the_walk(rule, heads, dk, dv, exact):
+    """More than 128 key channels, and what 32-bit models ask for: token by token over prompts (the decay rule of 531 tokens in segments)."""
+    gen = torch.Generator().manual_seed(dk)
+    t = sum(n for _, n in ROWS)
+    q, k, v = torch.randn(t, heads * dk, generator=gen).to(DEV), torch.randn(t, heads, dk, generator=gen), torch.randn(t, heads * dv, generator=gen).to(DEV)
+    k = (k / k.norm(dim=-1, keepdim=True)).reshape(t, -1).to(DEV)
+    z, bias, coef = torch.randn(t, heads * dk, generator=gen).to(DEV), torch.zeros(heads * dk, device=DEV), torch.ones(heads, device=DEV)
+    beta = torch.randn(t, heads, generator=gen).to(DEV) if rule == "delta" else None
+    state, ctx = torch.randn(len(ROWS), heads, dv, dk, generator=gen).to(DEV), _ctx(ROWS, SLOTS)
+    wide = lambda x: x.double().cpu().view(t, heads, -1)  # noqa: E731
+    decay = torch.exp(-torch.nn.functional.softplus(wide(z)))
+    want, size, last = _exact(wide(q) * 0.25, wide(k), wide(v), decay, None if beta is None else torch.sigmoid(beta.double().cpu()), ROWS, SLOTS,
+                              state.double().cpu())
+    assert exact or not mixers.walk_ok(q, k, v, dk, ctx)
+    o, st = torch.full((t, heads, dv), float("nan"), device=DEV), state.clone()
+    ops.decay_scan(o, st, q, k, v, z, bias, coef, 1.0, beta, ctx, heads, dk, dv, 0.25, delta=rule == "delta", exact=exact)
+    assert not any(role.startswith("walk") for role, *_ in ctx.held)
+    assert ((o.double().cpu() - want).abs() / size).max() < 1e-6 and ((st.double().cpu() - last).abs().max() / last.abs().max()) < 1e-6
 
 
 @pytest.mark.parametrize("heads, groups, dk, dv, scaled", [(8, 2, 128, 64, True), (4, 4, 64, 16, True), (2, 1, 32, 33, False), (160, 2, 32, 70, True),
