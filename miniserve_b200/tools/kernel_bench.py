@@ -5,7 +5,7 @@ summaries under ``profiles/`` were measured and captured with.
     python -m miniserve_b200.tools.kernel_bench attn_prefill --tokens 2048
     python -m miniserve_b200.tools.kernel_bench skinny --m 8 --n 4096 --k 1024
     python -m miniserve_b200.tools.kernel_bench sample --batch 8 --top-p 0.9
-    python -m miniserve_b200.tools.kernel_bench decay_scan --tokens 2048 --heads 8 --key-dim 64 --value-dim 128 [--delta]
+    python -m miniserve_b200.tools.kernel_bench decay_scan --tokens 2048 --heads 8 --key-dim 64 --value-dim 128 [--delta] [--exact]
     python -m miniserve_b200.tools.kernel_bench attn_prefill --tokens 2048 --softcap 30 --chunk 1024 --learned-sink
     python -m miniserve_b200.tools.kernel_bench add_rmsnorm --m 2048 --n 1024 --offset
     python -m miniserve_b200.tools.kernel_bench pointwise --op channel_gate --tokens 2048 --heads 16 --head-dim 128
@@ -131,6 +131,7 @@ def main(argv=None) -> int:
                                      "expert_combine"],
                     default="channel_gate", help="pointwise: which kernel (--tokens rows; --heads x --head-dim, or --n, columns)")
     ap.add_argument("--head-decay", action="store_true", help="decay_scan: one decay per head, worked out beforehand (float32), a column of ones")
+    ap.add_argument("--exact", action="store_true", help="decay_scan: token by token, as 32-bit models run it")
     ap.add_argument("--chunks", action="store_true", help="decay_scan --head-decay: by chunks on the tensor cores")
     ap.add_argument("--blocks", type=int, default=4, help="recurrent: equal parts of the --n channels, a gate matrix each")
     ap.add_argument("--taps", type=int, default=4, help="recurrent: taps of the convolution")
@@ -490,7 +491,8 @@ def main(argv=None) -> int:
             if args.head_decay:
                 return ops.decay_scan(o, state, q, k, v, decay, None, None, 0.0, None, ctx, hh, dk, dv + 1, dk ** -0.5, delta=False, head_decay=True,
                                       v_scale=write, ones_column=True)
-            ops.decay_scan(o, state, q, k, v, z, bias, coef, -1.0, beta, ctx, hh, dk, dv, dk ** -0.5, delta=args.delta)
+            ops.decay_scan(o, state, q, k, v, z, bias, coef, -1.0, beta, ctx, hh, dk, dv, dk ** -0.5, delta=args.delta,
+                           exact=args.exact)
     us = _time(calls, copies, args.launches)
     if us is not None:
         out.update(us_per_launch=round(us, 2), copies=copies)
