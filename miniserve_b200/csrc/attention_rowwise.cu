@@ -133,7 +133,7 @@ attention_rowwise_kernel(T* __restrict__ out,            // [T, nq, d]
 // scores, then the rows one after the other with a lane per key (the same exchanges as above), then 4 rows x 4 MD columns of the output.
 // A tile in which a row sees nothing leaves the row as it is (alpha = 1, p = 0), so all rows may walk the tiles that any of them sees.
 // Bound by shared-memory reads (32 floats read for 64 products of a score tile): 700 tokens of 16 heads of 128 on 8
-// kv heads take 262 us where a warp per token and head takes 2,183 (every lane walking its own key's row in global memory).
+// kv heads take 254 us where a warp per token and head takes 2,291, both inside a layer (every lane walking its own key's row in global memory).
 constexpr int TW_ROWS = 64, TW_KEYS = 32, TW_THREADS = 128, TW_LDS = TW_KEYS + 4;
 
 __device__ __forceinline__ void tw_cp16(void* dst, const void* src, bool in) {

@@ -21,8 +21,9 @@
 // below one is rounded down every time: in 32 bits the state of a slowly decaying head comes out three times as far off as the walk's.
 // Tensor cores are further off too, factors as two tf32 numbers: 1.3 to 2.3 times the walk's errors over a few tokens, and growing with the
 // row where a state lasts, 24 times at 8,192 tokens: their sums are not rounded to nearest.) Against 64-bit sums
-// outputs and states are no further off than the walk's: root mean squares of the errors over 2,048 tokens 0.76 to 1.0 of the walk's
-// (outputs) and 0.7 to 1.05 (states: few numbers), decays from 0.02 to 1; 0.27 to 0.4 with the delta rule and no decay.
+// outputs and states are no further off than the walk's: root mean squares of the errors over 2,048 tokens 0.75 to 1.0 of the walk's
+// (outputs) and 0.7 to 1.1 (states: few independent numbers), decays from 0.02 to 1; 0.27 to 0.57 with the delta rule and no decay, 1.2 where
+// that rule has fewer than 16 key channels, fewer than a chunk has tokens.
 // A token sees nothing of the tokens behind it, whatever they hold: a value that is not finite reaches its own token and the later
 // ones. (With one decay per head the sums against the state are scaled behind the sum: a state within q's size of the largest float
 // overflows.)
