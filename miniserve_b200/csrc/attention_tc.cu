@@ -27,6 +27,7 @@
 namespace ms {
 
 constexpr int AT_D = 128, AT_ROWS = 128, AT_KEYS = 128;
+constexpr int AT_FIRST = 96;  // so many of a tile's probabilities are handed over before the rest
 constexpr float AT_LOG2E = 1.4426950408889634f;
 constexpr int AT_BLOCK = 128 * 64 * 2;  // one [128 rows][64 bf16] swizzled block: 16 KB
 
@@ -41,10 +42,10 @@ __device__ __forceinline__ void at_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(at_smem(bar)) : "memory");
 }
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity) { return mbar_wait_bounded(at_smem(bar), parity); }
-__device__ __forceinline__ void at_tma_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
+__device__ __forceinline__ void at_tma_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c3) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
-      ::"r"(at_smem(dst)), "l"(map), "r"(at_smem(bar)), "r"(c0), "r"(c1) : "memory");
+      "cp.async.bulk.tensor.4d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %4}], [%2];\n"
+      ::"r"(at_smem(dst)), "l"(map), "r"(at_smem(bar)), "r"(0), "r"(c3) : "memory");
 }
 __device__ __forceinline__ void at_tma_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(
@@ -104,23 +105,21 @@ __device__ __forceinline__ float at_ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
   return y;
 }
-// 2^x on the FMA pipes (for x <= 8): round to the nearest integer with the 1.5 * 2^23 trick, a
-// cubic for 2^fraction on [-0.5, 0.5] (relative error 1e-4, far below the bfloat16 rounding of P),
-// and the integer part added to the exponent bits. Used for a share of the elements so that the
-// special-function unit (16 ex2 per clock per SM) would not limit the softmax. Measured on B200 it
-// is not the limit here (0, 2, 3 or 4 of every 8 emulated: 411, 427, 421, 431 us for 8,192 tokens).
-__device__ __forceinline__ float at_ex2_poly(float x) {
-  x = fmaxf(x, -125.f);
-  const float t = x + 12582912.f;
-  const float f = x - (t - 12582912.f);
-  float p = fmaf(f, 0.0558382829f, 0.2426394785f);
-  p = fmaf(p, f, 0.6931367339f);
-  p = fmaf(p, f, 0.9999245570f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
+// The larger of three; two multiply-adds and two sums in one instruction (the same roundings as one by one).
+__device__ __forceinline__ float at_max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
-#ifndef AT_EMULATED_OF_8
-#define AT_EMULATED_OF_8 0  // of every 8 exponentials, this many go to the FMA pipes (measured: no gain, so none)
-#endif
+__device__ __forceinline__ void at_fma2(float& x0, float& x1, float a0, float a1, float b, float c) {
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 c, {%5, %5};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}\n"
+      : "=f"(x0), "=f"(x1) : "f"(a0), "f"(a1), "f"(b), "f"(c));
+}
+__device__ __forceinline__ void at_add2(float& x0, float& x1, float a0, float a1) {
+  asm("{\n\t.reg .b64 a, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 d, {%0, %1};\n\tadd.rn.f32x2 d, d, a;\n\tmov.b64 {%0, %1}, d;\n\t}\n"
+      : "+f"(x0), "+f"(x1) : "f"(a0), "f"(a1));
+}
 #define AT_FENCE_BEFORE() asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory")
 #define AT_FENCE_AFTER() asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory")
 
@@ -137,14 +136,31 @@ __host__ __device__ constexpr uint32_t at_idesc(bool b_mn) {
 // the tensor-memory columns its S tile occupied, and the second product takes its A operand from
 // there. Tensor memory: S/P of A [0,128), S/P of B [128,256), O of A [256,384), O of B [384,512).
 // Warps 0-3: softmax A, 4-7: softmax B, 8: TMA, 9: MMA, 10-11: idle (registers are handed over by groups of four warps).
+//
+// Every role walks the CTA's items with counters of its own that run on from item to item, so nothing stops at an
+// item's end: while a group writes its rows out of tensor memory, the tensor cores work on the other group or on the
+// next item's first scores, and the next item's queries and keys are on their way. K and V have a ring of two tiles
+// each with barriers of their own: K of a tile is free as soon as both groups' scores of it are done, V a softmax later.
+// A copy brings a whole page of one head (4 KB at 16 tokens), both halves of its rows.
+//
+// What bounds it: per tile of 128 keys both groups have 4,096 cycles of tensor-core work at cuBLAS's rate (32 products of
+// 128x128x16), 2,048 of ex2 in the special-function unit and about 1,100 of issue, in two chains S -> softmax -> P V that
+// each wait for themselves. Measured (one B200, 16 heads of 8 kv heads, pages of 16, us for 512 / 2,048 / 4,096 / 8,192
+// tokens): 20.6 / 38.1 / 96 / 333 with barriers armed anew at every item and one barrier for K and V of a tile;
+// 17.4 / 34.7 / 78 / 261 as it is described above; 16.5 / 32.7 / 72 / 242 with two multiply-adds or sums an
+// instruction; 15.9 / 32.2 / 67 / 229 with the first three quarters of P handed over before the last (a quarter: 233 at
+// 8,192, half: 230). 8,192 tokens: 1,203 TFLOP/s. A share of the exponentials on the FMA pipes instead was slower (250 against
+// 242), as were fewer or more registers for the two issuing warps than 104 (56: 620 bytes of spills there).
 constexpr int AT_THREADS = 384;  // 8 softmax warps, 1 TMA warp, 1 MMA warp, 2 warps that only make up the third group of four
 
 struct AtSmem {
   static constexpr int q = 0;                     // group A: 2 blocks, group B: 2 blocks
-  static constexpr int kv = 4 * AT_BLOCK;         // 2 stages x (K: 2 blocks, V: 2 blocks)
-  static constexpr int stage = 4 * AT_BLOCK;
-  static constexpr int total = kv + 2 * stage;    // 12 blocks = 192 KB
+  static constexpr int slot = 2 * AT_BLOCK;       // a tile of K or V: [16 groups of 8 keys][2 halves of a row][8 keys][64]
+  static constexpr int k = 4 * AT_BLOCK;          // 2 slots
+  static constexpr int v = k + 2 * slot;          // 2 slots
+  static constexpr int total = v + 2 * slot;      // 12 blocks = 192 KB
 };
+constexpr int AT_GROUP8 = 2048;                   // 8 keys: two swizzled blocks [8 rows][64 bf16], one per half of a row
 
 __device__ __forceinline__ void at_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, bool accumulate) {
   const uint32_t acc = accumulate ? 1u : 0u;
@@ -233,16 +249,13 @@ __device__ __forceinline__ void at_rescale(uint32_t t_o, float alpha) {
   }
 }
 // The softmax step of one row for a tile in which the row sees only the keys at offsets
-// [seen_lo, seen_hi]. The scores are read twice, 32 columns at a time: once for the maximum, once for
-// the exponentials (chunk c of P, 16 columns, lies below chunk c + 1 of S, so chunks are read and
-// written in turn). A function of its own: inlined beside the all-in-registers form of interior tiles
-// it cost that form its registers. The one-pass form (the whole row in registers here too) was tried in
-// this function and measured slower inside a prompt step (3.60 against 3.53 ms for 2,048 tokens): its
-// 128 live values cost the kernel around the call more than the second read costs here.
+// [seen_lo, seen_hi], with what EXTRAS brings. The scores are read twice, 32 columns at a time: once for the
+// maximum, once for the exponentials (chunk c of P, 16 columns, lies below chunk c + 1 of S, so chunks are read
+// and written in turn). A function of its own: inlined beside the all-in-registers form of interior tiles it cost
+// that form its registers. (Without extras a mask is one select per score, made in registers at the call's place.)
 // Returns the sum of the row's exponentials.
 // `keep_off`: offsets below it are seen whatever seen_lo says (the kept first keys of a request). `dist_c`, `dist_r2`,
 // `dist_0`: the distance bias's factor in raw units (0: none), its second number, and the distance of offset 0.
-template <bool CAP>
 __device__ __noinline__ float at_softmax_masked(uint32_t t_s, uint32_t t_o, int seen_lo, int seen_hi, float scale_log2,
                                                 float& m_used, float& l_sum, float cap_raw, float cap_c2, int keep_off,
                                                 float dist_c, float dist_r2, int dist_0) {
@@ -255,9 +268,9 @@ __device__ __noinline__ float at_softmax_masked(uint32_t t_s, uint32_t t_o, int 
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       const int off = c * 32 + i;
-      float sc = CAP && cap_c2 > 0.f ? at_cap(v[i], cap_raw, cap_c2) : v[i];
-      const bool seen = off <= seen_hi && (off >= seen_lo || (CAP && off < keep_off));
-      if (CAP && dist_c != 0.f && seen) sc -= at_distance(dist_c, dist_r2, dist_0 - off);
+      float sc = cap_c2 > 0.f ? at_cap(v[i], cap_raw, cap_c2) : v[i];
+      const bool seen = off <= seen_hi && (off >= seen_lo || (off < keep_off));
+      if (dist_c != 0.f && seen) sc -= at_distance(dist_c, dist_r2, dist_0 - off);
       mx[i & 3] = fmaxf(mx[i & 3], seen ? sc : -INFINITY);
     }
   }
@@ -274,16 +287,16 @@ __device__ __noinline__ float at_softmax_masked(uint32_t t_s, uint32_t t_o, int 
     at_tmem_ld32(t_s + (uint32_t)(c * 32), v);
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
     uint32_t pk[16];
-    if (CAP && cap_c2 > 0.f) {
+    if (cap_c2 > 0.f) {
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = at_cap(v[i], cap_raw, cap_c2);
     }
 #pragma unroll
     for (int i = 0; i < 32; i += 2) {
       const int off = c * 32 + i;
-      const bool seen0 = off <= seen_hi && (off >= seen_lo || (CAP && off < keep_off));
-      const bool seen1 = off + 1 <= seen_hi && (off + 1 >= seen_lo || (CAP && off + 1 < keep_off));
-      if (CAP && dist_c != 0.f) {
+      const bool seen0 = off <= seen_hi && (off >= seen_lo || (off < keep_off));
+      const bool seen1 = off + 1 <= seen_hi && (off + 1 >= seen_lo || (off + 1 < keep_off));
+      if (dist_c != 0.f) {
         if (seen0) v[i] -= at_distance(dist_c, dist_r2, dist_0 - off);
         if (seen1) v[i + 1] -= at_distance(dist_c, dist_r2, dist_0 - off - 1);
       }
@@ -299,8 +312,8 @@ __device__ __noinline__ float at_softmax_masked(uint32_t t_s, uint32_t t_o, int 
 }
 
 // What one work item (a tile of 2 x 128 query rows, one group of heads, one split of the keys)
-// has to do. All threads of a CTA compute it from the item's index; the scheduler warp also
-// uses it to tell empty items from real ones.
+// has to do. The scheduler warp computes it from the item's index and hands it to the other roles
+// through a ring of two in shared memory; it also tells empty items from real ones.
 struct AtItem {
   int r, rank, tok0, q_len, m0, start, kv_len, head0, split;
   int n_tiles[2], q_first[2], q_last[2], lo_g[2], lo_max[2], shares[2];
@@ -308,7 +321,7 @@ struct AtItem {
   // Kept first keys: the walk over key tiles runs over virtual tiles; those below `first_tile` (the window's first
   // tile) are the request's tiles 0, 1, ... that hold kept keys: virtual tile v is real tile v - walk_shift there.
   int first_tile, walk_shift;
-  bool has_b;
+  int has_b, alive;  // alive 0: no item, the CTA is done
   __device__ __forceinline__ int real_tile(int v) const { return v < first_tile ? v - walk_shift : v; }
 };
 
@@ -378,8 +391,9 @@ __device__ __forceinline__ bool at_item(AtItem& it, int idx, const AtGrid& gr, c
 // past a short key range) are stepped over: the lanes look at the 32 items from the claimed one
 // on, so a run of empty items costs one round trip. When nothing is left, the CTA signs off on a
 // second counter, and the last one to do so puts both back to zero for the next launch.
-__device__ __forceinline__ int at_claim(int* __restrict__ queue, const AtGrid& gr, const int* __restrict__ cu_q,
-                                        const int* __restrict__ q_start, int lane, bool first) {
+// Lane 0's `item` is the one claimed.
+__device__ __forceinline__ bool at_claim(AtItem& item, int* __restrict__ queue, const AtGrid& gr, const int* __restrict__ cu_q,
+                                         const int* __restrict__ q_start, int lane, bool first) {
   const int total = gr.total();
   for (;;) {
     int idx = (int)blockIdx.x;
@@ -392,12 +406,11 @@ __device__ __forceinline__ int at_claim(int* __restrict__ queue, const AtGrid& g
         queue[0] = 0;
         queue[1] = 0;
       }
-      return -1;
+      return false;
     }
-    AtItem probe;
-    const bool work = idx + lane < total && at_item(probe, idx + lane, gr, cu_q, q_start);
+    const bool work = idx + lane < total && at_item(item, idx + lane, gr, cu_q, q_start);
     const unsigned mask = __ballot_sync(0xffffffffu, work);
-    if (mask & 1u) return idx;
+    if (mask & 1u) return true;
     const int run = mask ? __ffs(mask) - 1 : 32;  // this many items from idx on are empty
     if (!first && lane == 0 && run > 1) atomicMax(queue, idx + run - (int)gridDim.x);
     first = false;
@@ -417,14 +430,43 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         int* __restrict__ tickets, const int* __restrict__ plan, const AtExtras ex) {
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t q_full, kv_full[2], kv_empty[2], s_full[2], p_full[2], o_final[2];
+  __shared__ uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_first[2], p_full[2], o_final[2];
+  __shared__ uint64_t item_full[2], item_empty[2], drained;
+  __shared__ AtItem items[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int ticket_of[2];
-  __shared__ int item_slot;       // the item the CTA works on (-1: none left)
-  __shared__ int failed;          // a bounded wait gave up somewhere: the CTA winds down
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  pdl_prologue();
+  // what needs nothing of the kernels before goes before the wait for them
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      at_mbar_init(&q_full[i], 1);
+      at_mbar_init(&q_empty[i], 1);
+      at_mbar_init(&k_full[i], 1);
+      at_mbar_init(&k_empty[i], 1);
+      at_mbar_init(&v_full[i], 1);
+      at_mbar_init(&v_empty[i], 1);
+      at_mbar_init(&s_full[i], 1);
+      at_mbar_init(&p_first[i], 128);
+      at_mbar_init(&p_full[i], 128);
+      at_mbar_init(&o_final[i], 1);
+      at_mbar_init(&item_full[i], 1);
+      at_mbar_init(&item_empty[i], 9);  // 8 softmax warps and the thread that issues products
+    }
+    at_mbar_init(&drained, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(at_smem(&tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  AT_FENCE_BEFORE();
+  __syncthreads();
+  AT_FENCE_AFTER();
+  const uint32_t tmem = tmem_slot;
+  pdl_wait();
+
   // A launch that was captured into a CUDA graph takes what follows from the rows' lengths (tiles per
   // row, rows, key splits) from device memory, where the host puts it before every replay: the
   // launch itself (a CTA per SM, these arguments) is then the same for every step of its size.
@@ -438,206 +480,292 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   }
   const int G = gr.G, window = gr.window;
   const int tpc = AT_ROWS / G;
-  int next_item = -1;  // held by the scheduler warp
-  if (warp == 8) {
-    next_item = at_claim(queue, gr, cu_q, q_start, lane, true);
-    if (lane == 0) item_slot = next_item;
-  }
-  auto init_barriers = [&]() {
-    at_mbar_init(&q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      at_mbar_init(&kv_full[i], 1);
-      at_mbar_init(&kv_empty[i], 1);
-      at_mbar_init(&s_full[i], 1);
-      at_mbar_init(&p_full[i], 128);
-      at_mbar_init(&o_final[i], 1);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  };
-  if (threadIdx.x == 0) {
-    failed = 0;
-    init_barriers();
-  }
-  if (warp == 9) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(at_smem(&tmem_slot)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-  }
-  AT_FENCE_BEFORE();
-  __syncthreads();
-  AT_FENCE_AFTER();
-  const uint32_t tmem = tmem_slot;
 
-  // The roles part for good here, each with its own loop over the items, because they part in registers
-  // too: 12 warps of 168 registers fill the register file, the softmax warps (a whole row of scores each,
+  // The roles part for good here, and in registers too: 12 warps of 168 registers fill the register file, the softmax warps (a whole row of scores each,
   // 128 values) want more and the two warps that issue copies and products, and their two idle
   // companions, need few. Warps 8 to 11 give theirs up, warps 0 to 7 take them.
   if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n");
-    for (;;) {
-      const int cur = item_slot;
-      if (cur < 0) break;
-      AtItem it;
-      at_item(it, cur, gr, cu_q, q_start);
-      const int r = it.r, tok0 = it.tok0, m0 = it.m0, kv_len = it.kv_len;
-      const int head0 = it.head0, kvh = head0 / (nq / nkv), tile_begin = it.tile_begin, n_all = it.n_all;
-      const bool has_b = it.has_b;
-      if (warp == 8) {
-        // ---------------------------------------------------------- TMA producer (and scheduler)
-        if (lane == 0) {
-          at_expect_tx(&q_full, (has_b ? 4 : 2) * AT_BLOCK);
-          at_tma_3d(smem + AtSmem::q, &map_q, &q_full, 0, head0, tok0 + m0);
-          at_tma_3d(smem + AtSmem::q + AT_BLOCK, &map_q, &q_full, 64, head0, tok0 + m0);
-          if (has_b) {
-            at_tma_3d(smem + AtSmem::q + 2 * AT_BLOCK, &map_q, &q_full, 0, head0, tok0 + m0 + tpc);
-            at_tma_3d(smem + AtSmem::q + 3 * AT_BLOCK, &map_q, &q_full, 64, head0, tok0 + m0 + tpc);
-          }
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;\n");
+    if (warp == 8) {
+      // ---------------------------------------------------------- TMA producer and scheduler
+      // Loads go out in the order in which they are needed: queries of A, first keys, queries of B, first values,
+      // then keys and values of each tile. `tiles` counts the tiles of all items; tile c lies in slot c & 1.
+      const int page_size = 1 << page_shift;
+      const int box_rows = min(page_size, AT_KEYS);
+      int tiles = 0, queries[2] = {0, 0};
+      bool ok = true;
+      auto wait_free = [&](uint64_t* bar, int use) {  // before use number `use` of a slot
+        if (use > 0) {
+          if (lane == 0) ok = at_wait(bar, (use - 1) & 1);
+          ok = __shfl_sync(0xffffffffu, ok, 0);
         }
-        const int* pages = page_indices + page_indptr[r];
-        const int page_size = 1 << page_shift;
-        const int box_rows = min(page_size, AT_KEYS);
-        bool ok = true;
-        for (int j = 0; j < n_all; ++j) {
-          const int s = j & 1;
-          const int key0 = it.real_tile(tile_begin + j) * AT_KEYS;
+        return ok;
+      };
+      for (int i = 0; ok; ++i) {
+        AtItem mine;
+        const bool alive = at_claim(mine, queue, gr, cu_q, q_start, lane, i == 0);
+        if (!wait_free(&item_empty[i & 1], i >> 1)) break;
+        AtItem& it = items[i & 1];
+        if (lane == 0) {
+          mine.alive = alive;
+          it = mine;
+          at_arrive(&item_full[i & 1]);
+        }
+        __syncwarp();
+        if (!alive) break;
+        const int* pages = page_indices + page_indptr[it.r];
+        const int kv_len = it.kv_len, head0 = it.head0, kvh = head0 / (nq / nkv), n_all = it.n_all;
+        auto load_q = [&](int g) {
+          if (it.n_tiles[g] == 0 || !wait_free(&q_empty[g], queries[g])) return;
+          ++queries[g];
+          if (lane == 0) {
+            unsigned char* dst = smem + AtSmem::q + g * 2 * AT_BLOCK;
+            at_expect_tx(&q_full[g], 2 * AT_BLOCK);
+            at_tma_3d(dst, &map_q, &q_full[g], 0, head0, it.tok0 + it.m0 + g * tpc);
+            at_tma_3d(dst + AT_BLOCK, &map_q, &q_full[g], 64, head0, it.tok0 + it.m0 + g * tpc);
+          }
+        };
+        for (int j = 0; j < n_all && ok; ++j, ++tiles) {
+          const int s = tiles & 1;
+          const int key0 = it.real_tile(it.tile_begin + j) * AT_KEYS;
           const int boxes = min(AT_KEYS, ((kv_len - key0 + box_rows - 1) / box_rows) * box_rows) / box_rows;
-          int my_row = 0;
+          int group8 = 0;  // where this lane's keys begin, in groups of 8 rows of the pool
           if (lane < boxes) {
             const int key = key0 + lane * box_rows;
             const int page = pages[key >> page_shift];
-            my_row = (max(page, 0) * nkv + kvh) * page_size + (key & (page_size - 1));
+            group8 = ((max(page, 0) * nkv + kvh) * page_size + (key & (page_size - 1))) >> 3;
           }
-          if (j >= 2) {
-            if (lane == 0) ok = at_wait(&kv_empty[s], ((j >> 1) - 1) & 1);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) {
-              if (lane == 0) {
-                atomicExch(status, 31);
-                failed = 1;
-              }
-              break;
-            }
-          }
-          unsigned char* kt = smem + AtSmem::kv + s * AtSmem::stage;
-          unsigned char* vt = kt + 2 * AT_BLOCK;
-          if (lane == 0) at_expect_tx(&kv_full[s], (uint32_t)boxes * box_rows * 128 * 4);
+          const uint32_t bytes = (uint32_t)boxes * box_rows * (AT_D * 2);
+          if (j == 0) load_q(0);
+          if (!ok || !wait_free(&k_empty[s], tiles >> 1)) break;
+          if (lane == 0) at_expect_tx(&k_full[s], bytes);
           __syncwarp();
-          if (lane < boxes) {
-            const int off = lane * box_rows * 128;
-            at_tma_2d(kt + off, &map_k, &kv_full[s], 0, my_row);
-            at_tma_2d(kt + AT_BLOCK + off, &map_k, &kv_full[s], 64, my_row);
-            at_tma_2d(vt + off, &map_v, &kv_full[s], 0, my_row);
-            at_tma_2d(vt + AT_BLOCK + off, &map_v, &kv_full[s], 64, my_row);
-          }
+          if (lane < boxes) at_tma_4d(smem + AtSmem::k + s * AtSmem::slot + lane * box_rows * (AT_D * 2), &map_k, &k_full[s], group8);
+          if (j == 0) load_q(1);
+          if (!ok || !wait_free(&v_empty[s], tiles >> 1)) break;
+          if (lane == 0) at_expect_tx(&v_full[s], bytes);
+          __syncwarp();
+          if (lane < boxes) at_tma_4d(smem + AtSmem::v + s * AtSmem::slot + lane * box_rows * (AT_D * 2), &map_v, &v_full[s], group8);
         }
-        // all loads of this item are on their way: find the next one while the others compute
         __syncwarp();
-        next_item = at_claim(queue, gr, cu_q, q_start, lane, false);
-      } else if (warp == 9) {
-        // ---------------------------------------------------------- MMA issuer
-        if (at_elect()) {
-          constexpr uint32_t idesc_s = at_idesc(false), idesc_o = at_idesc(true);
-          bool ok = at_wait(&q_full, 0);
-          int kv_ready = -1;  // the last tile whose kv_full this thread has waited for
-          auto need_kv = [&](int j) -> bool {
-            if (j <= kv_ready) return true;
-            if (!at_wait(&kv_full[j & 1], (j >> 1) & 1)) return false;
-            kv_ready = j;
+      }
+      if (!ok && lane == 0) {
+        atomicExch(status, 31);
+        // copies in flight must not outlive the CTA: a shorter wait for each barrier's last one
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const int uses = (tiles + 1 - s) >> 1;
+          if (queries[s] > 0) mbar_wait_bounded(at_smem(&q_full[s]), (queries[s] - 1) & 1, MS_WAIT_NS / 64);
+          if (uses > 0) mbar_wait_bounded(at_smem(&k_full[s]), (uses - 1) & 1, MS_WAIT_NS / 64);
+          if (uses > 0) mbar_wait_bounded(at_smem(&v_full[s]), (uses - 1) & 1, MS_WAIT_NS / 64);
+        }
+      }
+    } else if (warp == 9) {
+      // ---------------------------------------------------------- MMA issuer
+      if (at_elect()) {
+        constexpr uint32_t idesc_s = at_idesc(false), idesc_o = at_idesc(true);
+        bool ok = true;
+        int k_seen0 = -1, k_seen1 = -1, k_used = 0;    // per slot: the last tile waited for; bits: one group has used the tile in it
+        int queries[2] = {0, 0}, steps[2] = {0, 0};    // per group: items begun, tiles whose P was taken
+        int base = 0;                                  // tiles of the items before the current one
+        struct Some {
+          int n[2], n_all, alive;
+        } cur, next;
+        int fetched = 0;
+        auto fetch = [&](Some& to) {
+          ok = ok && at_wait(&item_full[fetched & 1], (fetched >> 1) & 1);
+          if (!ok) {
+            to.alive = 0;
+            return;
+          }
+          const AtItem& it = items[fetched & 1];
+          to.n[0] = it.n_tiles[0];
+          to.n[1] = it.n_tiles[1];
+          to.n_all = it.n_all;
+          to.alive = it.alive;
+          at_arrive(&item_empty[fetched & 1]);
+          ++fetched;
+        };
+        // the scores of group g over tile j of an item whose first tile is number `first`
+        auto issue_s = [&](int g, const Some& of, int first, int j) {
+          const int c = first + j, s = c & 1;
+          if ((s ? k_seen1 : k_seen0) < c) {
+            ok = at_wait(&k_full[s], (c >> 1) & 1);
+            if (!ok) return;
+            if (s) k_seen1 = c;
+            else k_seen0 = c;
             AT_FENCE_AFTER();
-            return true;
-          };
-          auto issue_s = [&](int g, int j) -> bool {
-            if (!need_kv(j)) return false;
-            const unsigned char* kt = smem + AtSmem::kv + (j & 1) * AtSmem::stage;
-            const unsigned char* qt = smem + AtSmem::q + g * 2 * AT_BLOCK;
+          }
+          const unsigned char* kt = smem + AtSmem::k + s * AtSmem::slot;
+          const unsigned char* qt = smem + AtSmem::q + g * 2 * AT_BLOCK;
   #pragma unroll
-            for (int kk = 0; kk < AT_D / 16; ++kk) {
-              const uint64_t da = at_desc(qt + (kk >> 2) * AT_BLOCK, 16, 1024) + (uint64_t)(2 * (kk & 3));
-              const uint64_t db = at_desc(kt + (kk >> 2) * AT_BLOCK, 16, 1024) + (uint64_t)(2 * (kk & 3));
-              at_mma(tmem + (uint32_t)(g * 128), da, db, idesc_s, kk != 0);
-            }
-            at_commit(&s_full[g]);
-            return true;
-          };
-          if (ok && it.n_tiles[0] > 0) ok = issue_s(0, 0);
-          if (ok && it.n_tiles[1] > 0) ok = issue_s(1, 0);
-          for (int j = 0; j < n_all && ok; ++j) {
-            const unsigned char* vt = smem + AtSmem::kv + (j & 1) * AtSmem::stage + 2 * AT_BLOCK;
-  #pragma unroll 1
-            for (int g = 0; g < 2 && ok; ++g) {
-              if (j >= it.n_tiles[g]) continue;
-              if (!at_wait(&p_full[g], j & 1)) { ok = false; break; }
+          for (int kk = 0; kk < AT_D / 16; ++kk) {
+            const uint64_t da = at_desc(qt + (kk >> 2) * AT_BLOCK, 16, 1024) + (uint64_t)(2 * (kk & 3));
+            const uint64_t db = at_desc(kt + (kk >> 2) * 1024, 16, AT_GROUP8) + (uint64_t)(2 * (kk & 3));
+            at_mma(tmem + (uint32_t)(g * 128), da, db, idesc_s, kk != 0);
+          }
+          at_commit(&s_full[g]);
+          if (j + 1 == of.n[g]) at_commit(&q_empty[g]);
+          // the last of the groups that need the tile frees its slot
+          if (((k_used >> s) & 1) || !(j < of.n[0] && j < of.n[1])) {
+            k_used &= ~(1 << s);
+            at_commit(&k_empty[s]);
+          } else {
+            k_used |= 1 << s;
+          }
+        };
+        auto begin = [&](int g, const Some& of, int first) {
+          if (!ok || of.n[g] == 0) return;
+          ok = at_wait(&q_full[g], queries[g] & 1);
+          if (!ok) return;
+          ++queries[g];
+          AT_FENCE_AFTER();
+          issue_s(g, of, first, 0);
+        };
+        fetch(cur);
+        if (cur.alive) {
+          begin(0, cur, 0);
+          begin(1, cur, 0);
+        }
+        while (ok && cur.alive) {
+          bool have_next = false;
+          int begun = 0;
+          for (int j = 0; j < cur.n_all && ok; ++j) {
+            const int c = base + j, s = c & 1;
+            const unsigned char* vt = smem + AtSmem::v + s * AtSmem::slot;
+            bool v_seen = false;
+  #pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              if (!ok || j >= cur.n[g]) continue;
+              ok = at_wait(&p_first[g], steps[g] & 1);
+              if (ok && !v_seen) ok = at_wait(&v_full[s], (c >> 1) & 1);
+              if (!ok) continue;
+              v_seen = true;
               AT_FENCE_AFTER();
   #pragma unroll
               for (int kk = 0; kk < AT_KEYS / 16; ++kk) {
+                if (kk == AT_FIRST / 16) {
+                  ok = at_wait(&p_full[g], steps[g] & 1);
+                  if (!ok) break;
+                  AT_FENCE_AFTER();
+                }
                 // A = P of this group in tensor memory: 16 keys = 8 columns of packed bf16 pairs;
                 // B = V [keys][d], MN-major
-                const uint64_t db = at_desc(vt + kk * 2048, AT_BLOCK, 1024);
+                const uint64_t db = at_desc(vt + kk * 2 * AT_GROUP8, 1024, AT_GROUP8);
                 at_mma_ts(tmem + (uint32_t)(256 + g * 128), tmem + (uint32_t)(g * 128 + kk * 8), db, idesc_o, (j | kk) != 0);
               }
-              if (j + 1 < it.n_tiles[g]) {
-                ok = issue_s(g, j + 1);  // overwrites this group's S/P columns: ordered after the product above
+              if (!ok) continue;
+              ++steps[g];
+              // the next scores overwrite this group's S/P columns: ordered after the product above
+              if (j + 1 < cur.n[g]) {
+                issue_s(g, cur, base, j + 1);
               } else {
                 at_commit(&o_final[g]);
+                // on to the next item, unless the other group has more than one tile to go (its keys come first)
+                if (cur.n_all - (j + 1) <= 1) {
+                  if (!have_next) fetch(next);
+                  have_next = true;
+                  if (next.alive) begin(g, next, base + cur.n_all);
+                  begun |= 1 << g;
+                }
               }
             }
-            // the producer waits for this only before tile j + 2: an arrival that nobody waits for
-            // must not be in flight when the barriers are set up again for the next item
-            if (ok && j + 2 < n_all) at_commit(&kv_empty[j & 1]);
+            if (ok) at_commit(&v_empty[s]);
           }
-          if (!ok) {
-            atomicExch(status, 33);
-            failed = 1;
+          if (!have_next) fetch(next);
+          base += cur.n_all;
+          if (next.alive) {
+  #pragma unroll
+            for (int g = 0; g < 2; ++g)
+              if (!(begun & (1 << g))) begin(g, next, base);
+          }
+          cur = next;
+        }
+        // arrivals that nobody else waits for must not outlive the CTA, nor products
+        if (ok) {
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            const int uses = (base + 1 - s) >> 1;
+            if (ok && queries[s] > 0) ok = at_wait(&q_empty[s], (queries[s] - 1) & 1);
+            if (ok && uses > 0) ok = at_wait(&k_empty[s], (uses - 1) & 1) && at_wait(&v_empty[s], (uses - 1) & 1);
           }
         }
+        if (!ok) {
+          atomicExch(status, 33);
+          at_commit(&drained);
+          at_wait(&drained, 0);
+        }
       }
-      // ------------------------------------------------------------ between items
-      // Everything of this item is over: every product has completed (the softmax groups waited for
-      // the last ones), every arrival that was asked for has been waited for. The barriers start
-      // again from phase 0 and the scheduler publishes the next item.
-      AT_FENCE_BEFORE();
-      __syncthreads();
-      if (failed) break;
-      if (threadIdx.x == 0) init_barriers();
-      if (warp == 8 && lane == 0) item_slot = next_item;
-      __syncthreads();
-      AT_FENCE_AFTER();
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;\n");
-    for (;;) {
-      const int cur = item_slot;
-      if (cur < 0) break;
-      AtItem it;
-      at_item(it, cur, gr, cu_q, q_start);
-      const int r = it.r, tok0 = it.tok0, q_len = it.q_len, m0 = it.m0, start = it.start, kv_len = it.kv_len;
-      const int head0 = it.head0, split = it.split, tile_begin = it.tile_begin;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;\n");
+    const int g = warp >> 2;
+    const int row = threadIdx.x & 127;                // row within the group = tensor-memory lane
+    const int tok = row / G, hd = row - tok * G;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t t_s = tmem + (uint32_t)(g * 128) + lane_base, t_o = tmem + (uint32_t)(256 + g * 128) + lane_base;
+    int tiles = 0, steps = 0, finals = 0;  // tiles of the items before; this group's own tiles; its items
+    for (int i = 0;; ++i) {
+      // ---------------------------------------------------------- softmax, thread = row of its group
+      bool ok = at_wait(&item_full[i & 1], (i >> 1) & 1);
+      if (at_group_any(1 + g, !ok)) {
+        if (row == 0) atomicExch(status, 34);
+        break;
+      }
+      const AtItem& it = items[i & 1];
+      const int r = it.r, rank = it.rank, tok0 = it.tok0, q_len = it.q_len, m0 = it.m0, start = it.start, kv_len = it.kv_len;
+      const int head0 = it.head0, split = it.split, tile_begin = it.tile_begin, first_tile = it.first_tile, walk_shift = it.walk_shift;
+      const int lo_mine = it.lo_g[g], lo_max_mine = it.lo_max[g], q_first_mine = it.q_first[g], lo_item = it.lo_g[0];
+      const int n_mine = it.n_tiles[g], n_all = it.n_all, shares = it.shares[g], alive = it.alive;
+      __syncwarp();
+      if (lane == 0) at_arrive(&item_empty[i & 1]);  // (what follows reads the copies)
+      if (!alive) break;
+      const int tile_first = tiles;
+      tiles += n_all;
+      if (n_mine == 0) continue;
       {
-        // ---------------------------------------------------------- softmax, thread = row of its group
-        const int g = warp >> 2;
-        const int row = threadIdx.x & 127;                // row within the group = tensor-memory lane
-        const int tok = row / G, hd = row - tok * G;
         const int tok_in_req = m0 + g * tpc + tok;
         const int qpos = start + tok_in_req;
-        const int lo_mine = it.lo_g[g], lo_max_mine = it.lo_max[g], q_first_mine = it.q_first[g];
         const int block_lo = EXTRAS && gr.chunk > 0 ? (qpos / gr.chunk) * gr.chunk : 0;
         // the sink's score in units of log2 (it is neither scaled nor capped)
         const float sink_l2 = EXTRAS && ex.sink_values != nullptr ? ex.sink_values[head0 + hd] * AT_LOG2E : 0.f;
         const float dist_c = EXTRAS && ex.dist_r1 != nullptr ? ex.dist_r1[head0 + hd] / scale_log2 : 0.f;
         const float dist_r2 = EXTRAS && ex.dist_r1 != nullptr ? ex.dist_r2[head0 + hd] : 0.f;
-        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        const uint32_t t_s = tmem + (uint32_t)(g * 128) + lane_base, t_o = tmem + (uint32_t)(256 + g * 128) + lane_base;
-        const int n_mine = it.n_tiles[g];
         float m_used = -INFINITY, l_sum = 0.f;
-        bool ok = true;
-        for (int j = 0; j < n_mine && ok; ++j) {
-          if (!at_wait(&s_full[g], j & 1)) { ok = false; break; }
+        auto hand_over = [&](uint64_t* bar) {  // this row's stores of P so far are done
+          asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+          AT_FENCE_BEFORE();
+          at_arrive(bar);
+        };
+        for (int j = 0; j < n_mine; ++j, ++steps) {
+          ok = __all_sync(0xffffffffu, ok && at_wait(&s_full[g], steps & 1));  // (a warp stops as one)
+          if (!ok) break;
           AT_FENCE_AFTER();
-          const int key0 = it.real_tile(tile_begin + j) * AT_KEYS;
+          const int key0 = (tile_begin + j - (tile_begin + j < first_tile ? walk_shift : 0)) * AT_KEYS;
           const bool interior = key0 + AT_KEYS - 1 <= q_first_mine && key0 >= lo_max_mine;
+          // Rows of V that no query may weigh: keys beyond the request's end, and keys that the window of every row of
+          // this item has passed and that are not kept first keys. Their pages may have been given back and hold
+          // anything (a probability of zero times a NaN is a NaN), so they are made zero.
+          const int valid_keys = kv_len - key0;
+          const bool passed = key0 + row < lo_item && key0 + row >= gr.keep;
+          if ((valid_keys < AT_KEYS && row >= valid_keys) || passed) {
+            const int c = tile_first + j;
+            ok = at_wait(&v_full[c & 1], (c >> 1) & 1);  // (the copy must not land on top of the zeros)
+            unsigned char* vt = smem + AtSmem::v + (c & 1) * AtSmem::slot + (row >> 3) * AT_GROUP8 + (row & 7) * 128;
+  #pragma unroll
+            for (int h = 0; h < 2; ++h)
+  #pragma unroll
+              for (int cc = 0; cc < 8; ++cc) *reinterpret_cast<uint4*>(vt + h * 1024 + cc * 16) = make_uint4(0u, 0u, 0u, 0u);
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+          }
+          __syncwarp();
           float part[4] = {0.f, 0.f, 0.f, 0.f};
-          if (interior) {
-            // every key of the tile is seen by every row of the group: the whole row of scores in
-            // registers, four loads in flight, one wait
+          // a tile on the diagonal, at a window's edge or at the request's end: the keys of the tile that this row
+          // sees are those at offsets [seen_lo, seen_hi]
+          const int seen_hi = qpos - key0;
+          const int seen_lo = max(max(lo_mine, block_lo), window > 0 ? qpos - window + 1 : 0) - key0;
+          if (!EXTRAS || interior) {
+            // the whole row of scores in registers, four loads in flight, one wait
             float sv[4][32];
   #pragma unroll
             for (int c = 0; c < 4; ++c) at_tmem_ld32(t_s + (uint32_t)(c * 32), sv[c]);
@@ -655,11 +783,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   #pragma unroll
                 for (int i = 0; i < 32; ++i) sv[c][i] -= at_distance(dist_c, dist_r2, d0 - (c * 32 + i));
             }
+            if (!EXTRAS && !interior) {
+  #pragma unroll
+              for (int c = 0; c < 4; ++c)
+  #pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                  const int off = c * 32 + i;
+                  sv[c][i] = off <= seen_hi && off >= seen_lo ? sv[c][i] : -INFINITY;
+                }
+            }
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   #pragma unroll
             for (int c = 0; c < 4; ++c)
   #pragma unroll
-              for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], sv[c][i]);
+              for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = at_max3(mx[(i >> 1) & 3], sv[c][i], sv[c][i + 1]);
             const float alpha = at_new_maximum(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), m_used, scale_log2);
             if (__any_sync(0xffffffffu, alpha != 1.f)) {
               at_rescale(t_o, alpha);
@@ -672,52 +809,38 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               uint32_t pk[16];
   #pragma unroll
               for (int i = 0; i < 32; i += 2) {
-                const float x0 = fmaf(sv[c][i], scale_log2, -m_sub), x1 = fmaf(sv[c][i + 1], scale_log2, -m_sub);
-                const float e0 = (i & 7) < AT_EMULATED_OF_8 ? at_ex2_poly(x0) : at_ex2(x0);
-                const float e1 = ((i + 1) & 7) < AT_EMULATED_OF_8 ? at_ex2_poly(x1) : at_ex2(x1);
-                part[(i >> 1) & 3] += e0 + e1;
+                // (natural pairs of registers: sums of pairs as in the masked form cost moves, 249 against 229 us at 8,192 tokens)
+                float x0, x1;
+                at_fma2(x0, x1, sv[c][i], sv[c][i + 1], scale_log2, -m_sub);
+                const float e0 = at_ex2(x0), e1 = at_ex2(x1);
+                at_add2(part[i & 2], part[(i & 2) + 1], e0, e1);
                 __nv_bfloat162 p2 = __floats2bfloat162_rn(e0, e1);
                 pk[i >> 1] = *reinterpret_cast<uint32_t*>(&p2);
               }
               at_tmem_st16(t_s + (uint32_t)(c * 16), pk);
+              if (c == AT_FIRST / 32 - 1) hand_over(&p_first[g]);
             }
           } else {
-            // a tile on the diagonal, at a window's edge or at the request's end: the keys of the tile
-            // that this row sees are those at offsets [seen_lo, seen_hi]
-            const int seen_hi = qpos - key0;
-            const int seen_lo = max(max(lo_mine, block_lo), window > 0 ? qpos - window + 1 : 0) - key0;
-            part[0] = at_softmax_masked<EXTRAS>(t_s, t_o, seen_lo, seen_hi, scale_log2, m_used, l_sum, ex.cap_raw, ex.cap_c2,
-                                                EXTRAS ? gr.keep - key0 : 0, dist_c, dist_r2, qpos - key0);
+            part[0] = at_softmax_masked(t_s, t_o, seen_lo, seen_hi, scale_log2, m_used, l_sum, ex.cap_raw, ex.cap_c2,
+                                        gr.keep - key0, dist_c, dist_r2, qpos - key0);
+            hand_over(&p_first[g]);
           }
           l_sum += (part[0] + part[1]) + (part[2] + part[3]);
-          // Rows of V that no query may weigh: keys beyond the request's end, and keys that the window of every row of
-          // this item has passed and that are not kept first keys. Their pages may have been given back and hold
-          // anything (a probability of zero times a NaN is a NaN), so they are made zero.
-          const int valid_keys = kv_len - key0;
-          const bool passed = key0 + row < it.lo_g[0] && key0 + row >= gr.keep;
-          if ((valid_keys < AT_KEYS && row >= valid_keys) || passed) {
-            unsigned char* vt = smem + AtSmem::kv + (j & 1) * AtSmem::stage + 2 * AT_BLOCK;
-  #pragma unroll
-            for (int h = 0; h < 2; ++h)
-  #pragma unroll
-              for (int cc = 0; cc < 8; ++cc) *reinterpret_cast<uint4*>(vt + h * AT_BLOCK + row * 128 + cc * 16) = make_uint4(0u, 0u, 0u, 0u);
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-          }
-          asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-          AT_FENCE_BEFORE();
-          at_arrive(&p_full[g]);
+          hand_over(&p_full[g]);
         }
-        if (ok && n_mine > 0) ok = at_wait(&o_final[g], 0);
-        if (!ok) {
-          atomicExch(status, 34);
-          failed = 1;
+        if (ok) ok = at_wait(&o_final[g], finals & 1);
+        ++finals;
+        // all 128 threads of the group meet here, also after a wait that gave up: all of them stop then
+        if (at_group_any(1 + g, !ok)) {
+          if (row == 0) atomicExch(status, 34);
+          break;
         }
         AT_FENCE_AFTER();
         const bool store = tok_in_req < q_len;
         const size_t item = (size_t)(tok0 + (store ? tok_in_req : 0)) * nq + head0 + hd;  // (token, head) of this row
         __nv_bfloat16* dst = out + item * AT_D;
-        if (it.shares[g] <= 1) {
-          if (ok && n_mine > 0) {
+        if (shares <= 1) {
+          {
             // a sink: one more term of score 0 in the denominator, with no value
             const float inv = 1.0f / (l_sum + (sink ? at_ex2(sink_l2 - m_used * scale_log2) : 0.f));
   #pragma unroll 1
@@ -731,7 +854,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               }
             }
           }
-        } else if (n_mine > 0) {
+        } else {
           // One of several splits of this group's keys. Each takes a ticket when it is done. All but the
           // last leave their partial result (unnormalised O, the maximum it is scaled by, the sum) and
           // count themselves done; the last waits until the others are (they took their tickets before
@@ -739,17 +862,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           // partial results up in the order of the splits, its own from tensor memory, and writes the
           // rows. Partial results are laid out [group of rows][split][4 columns][row], so that the 128
           // threads of a group (one row each) write and read whole 512-byte lines together.
-          const size_t unit = ((size_t)(it.rank * gr.rows + r) * gr.head_groups + head0 / G) * 2 + g;
+          const size_t unit = ((size_t)(rank * gr.rows + r) * gr.head_groups + head0 / G) * 2 + g;
           float4* po = reinterpret_cast<float4*>(part_o) + (unit * gr.splits + split) * (32 * 128) + row;
           float2* pml = part_ml + unit * gr.splits * 128 + row;
           int* ticket = tickets + unit;
           int* done = tickets + (size_t)gr.q_tiles * gr.rows * gr.head_groups * 2 + unit;
-          // all 128 threads of the group meet here, also after a wait that gave up: then nobody takes a ticket
-          const bool bad = at_group_any(1 + g, !ok);
-          if (row == 0 && !bad) ticket_of[g] = atomicAdd(ticket, 1);
+          if (row == 0) ticket_of[g] = atomicAdd(ticket, 1);
           at_group_sync(1 + g);
-          const bool last = !bad && ticket_of[g] == it.shares[g] - 1;
-          if (!bad && !last) {
+          const bool last = ticket_of[g] == shares - 1;
+          if (!last) {
   #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
               float ov[32];
@@ -762,13 +883,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             __threadfence();
             at_group_sync(1 + g);
             if (row == 0) atomicAdd(done, 1);
-          } else if (last) {
+          } else {
             if (row == 0) {
               // bounded like every wait: a split that took its ticket and never finishes is an error, not a hang
               unsigned long long began = 0;
               bool there = false;
               for (uint32_t polls = 1; !there; ++polls) {
-                there = *reinterpret_cast<volatile int*>(done) >= it.shares[g] - 1;
+                there = *reinterpret_cast<volatile int*>(done) >= shares - 1;
                 if (!there && (polls & 63u) == 0) {
                   unsigned long long now;
                   asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(now));
@@ -784,10 +905,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             at_group_sync(1 + g);
             const float4* pall = reinterpret_cast<const float4*>(part_o) + unit * gr.splits * (32 * 128) + row;
             float m_all = m_used;
-            for (int sp = 0; sp < it.shares[g]; ++sp)
+            for (int sp = 0; sp < shares; ++sp)
               if (sp != split) m_all = fmaxf(m_all, __ldcg(&pml[sp * 128]).x);
             float l_all = 0.f;
-            for (int sp = 0; sp < it.shares[g]; ++sp) {
+            for (int sp = 0; sp < shares; ++sp) {
               const float2 ml = sp == split ? make_float2(m_used, l_sum) : __ldcg(&pml[sp * 128]);
               l_all += ml.y == 0.f ? 0.f : at_ex2((ml.x - m_all) * scale_log2) * ml.y;
             }
@@ -800,7 +921,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
   #pragma unroll
               for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-              for (int sp = 0; sp < it.shares[g]; ++sp) {
+              for (int sp = 0; sp < shares; ++sp) {
                 if (sp == split) {
                   const float w = l_sum == 0.f ? 0.f : at_ex2((m_used - m_all) * scale_log2);
   #pragma unroll
@@ -828,20 +949,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           at_group_sync(1 + g);  // ticket_of[g] is free for the next item
         }
       }
-      // ------------------------------------------------------------ between items
-      // Everything of this item is over: every product has completed (the softmax groups waited for
-      // the last ones), every arrival that was asked for has been waited for. The barriers start
-      // again from phase 0 and the scheduler publishes the next item.
-      AT_FENCE_BEFORE();
-      __syncthreads();
-      if (failed) break;
-      if (threadIdx.x == 0) init_barriers();
-      __syncthreads();
-      AT_FENCE_AFTER();
     }
   }
   AT_FENCE_BEFORE();
   __syncthreads();
+  AT_FENCE_AFTER();
   if (warp == 9) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
   }
@@ -980,13 +1092,14 @@ MS_EXPORT int ms_attn_tc_prefill(void* out, const void* q, const void* k_pool, c
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     MS_CHECK_ARG(res == CUDA_SUCCESS, "attention_tc: encoding the query map failed with code %d", (int)res);
   }
-  const cuuint64_t rows = (cuuint64_t)pool_pages * nkv * page_size;
-  const cuuint64_t kdims[2] = {(cuuint64_t)AT_D, rows};
-  const cuuint64_t kstrides[1] = {(cuuint64_t)AT_D * 2};
-  const cuuint32_t kbox[2] = {64, (cuuint32_t)(page_size < AT_KEYS ? page_size : AT_KEYS)};
-  const cuuint32_t kelem[2] = {1, 1};
+  // The cache as [groups of 8 rows][2 halves of a row][8 rows][64]: one copy brings a page's keys (or values) of one head, in the
+  // order in which the products' descriptors walk them (a swizzled block is 8 rows of 128 bytes; a group's two blocks lie side by side).
+  const cuuint64_t kdims[4] = {64, 8, 2, (cuuint64_t)pool_pages * nkv * page_size / 8};
+  const cuuint64_t kstrides[3] = {(cuuint64_t)AT_D * 2, 128, (cuuint64_t)AT_D * 2 * 8};
+  const cuuint32_t kbox[4] = {64, 8, 2, (cuuint32_t)(page_size < AT_KEYS ? page_size : AT_KEYS) / 8};
+  const cuuint32_t kelem[4] = {1, 1, 1, 1};
   for (int i = 0; i < 2; ++i) {
-    const CUresult res = encode(i == 0 ? &map_k : &map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+    const CUresult res = encode(i == 0 ? &map_k : &map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
                                 const_cast<void*>(i == 0 ? k_pool : v_pool), kdims, kstrides, kbox, kelem,
                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

@@ -506,6 +506,22 @@ def test_attention_tcgen05_prompts_and_mixed_steps(nq, nkv, d, page, key_splits)
     assert torch.allclose(out.float(), ref, **BF16_TOL)
 
 
+@pytest.mark.parametrize("page", [8, 16, 128])
+@pytest.mark.parametrize("window", [None, 150])
+def test_attention_tcgen05_takes_several_items_a_cta(page, window, key_splits):
+    """More items than CTAs, of one to six key tiles, with and without a second group of rows: rings and barriers run on
+    from item to item, whatever the parity at which an item begins."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = [((37 * i) % 600, 1 + (i * 11) % 30 + (90 if i % 5 == 0 else 0)) for i in range(2 * sms + 25)]
+    pb, q, ref, scale = _attention_case(torch.bfloat16, rows, 2, 1, 128, page, window=window)
+    out = torch.full_like(q, float("nan"))
+    for _ in range(2):  # the second launch finds the queue as the first one left it
+        ops.attention_tc_prefill(out, q, pb.k_pool, pb.v_pool, make_context(pb), 0, scale, window)
+    torch.cuda.synchronize()
+    assert ops.device_status("cuda").item() == 0
+    assert torch.allclose(out.float(), ref, **BF16_TOL)
+
+
 @pytest.mark.parametrize("window", [1, 7, 128, 129, 200])
 def test_attention_tcgen05_window_edge(window, key_splits):
     rows = [(0, 400), (130, 3), (399, 1), (256, 128)]
