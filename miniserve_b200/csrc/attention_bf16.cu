@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "tensor_map.cuh"
 
 #ifndef MS_HEAD_DIM
 #error "compile with -DMS_HEAD_DIM=<head size>"
@@ -47,6 +48,14 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
 }
+__device__ __forceinline__ void ldmatrix_x4_at(uint32_t (&r)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans_at(uint32_t (&r)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
@@ -75,11 +84,11 @@ struct PagedKV {
   const __nv_bfloat16* v;
   const int* pages;  // this request's page ids
   int kv_head, nkv, page_shift;
-  __device__ __forceinline__ size_t row_offset(int key) const {
-    const int page = pages[key >> page_shift];
+  __device__ __forceinline__ size_t row_in(int page, int key) const {
     const int page_size = 1 << page_shift;
-    return (((size_t)max(page, 0) * nkv + kv_head) * page_size + (key & (page_size - 1))) * D;
+    return ((size_t)max(page, 0) * nkv + kv_head) * page_size + (key & (page_size - 1));
   }
+  __device__ __forceinline__ size_t row_offset(int key) const { return row_in(pages[key >> page_shift], key) * D; }
 };
 
 // Copy keys [key0, key0 + ROWS) of K and V into padded tiles; rows outside [lo, hi) are zero-filled.
@@ -318,24 +327,193 @@ struct DecodeSmem {
   static constexpr size_t bytes_pipe = (size_t)(q_elems + pipe_elems) * 2;
   static constexpr size_t bytes_merge = (size_t)DC_WARPS * 16 * (D + 2) * 4 + (size_t)q_elems * 2;
   static constexpr size_t bytes = bytes_pipe > bytes_merge ? bytes_pipe : bytes_merge;
+  // stages filled by tensor copies: [2 groups of 8 keys][D / 64 parts of a row][8 keys][64] of K, then of V, in blocks swizzled in 128 bytes
+  static constexpr size_t q_bytes_tma = ((size_t)q_elems * 2 + 1023) / 1024 * 1024;
+  static constexpr int stage_bytes_tma = 2 * DC_SLICE * D * 2;
+  static constexpr size_t bytes_pipe_tma = 1024 + (size_t)DC_WARPS * DC_STAGES * stage_bytes_tma;  // (1024: to align it)
+  static constexpr size_t bytes_tma = q_bytes_tma + bytes_pipe_tma > bytes_merge ? q_bytes_tma + bytes_pipe_tma : bytes_merge;
+};
+constexpr bool DC_TMA = D == 64 || D == 128;  // head sizes whose slices tensor copies can bring
+
+// One warp's ring of stages filled by tensor copies, two a slice (a page's 16 keys of one head), instead of 16 bytes a lane: the copies
+// were 300 of the 520 instructions that a slice took, and the warps' instructions were what the kernel waited for (64 requests of
+// 2,048 keys: 0.34 instructions a cycle and scheduler with two warps each; 97.7 us at 5.5 TB/s, now 89.4 at 6.05). The page of the
+// next slice is looked up a slice ahead. Waits are bounded.
+struct DecodeRing {
+  uint32_t stages, bars;  // shared-memory addresses
+  __device__ __forceinline__ void init(uint32_t stages_at, uint32_t bars_at, int lane) {
+    stages = stages_at;
+    bars = bars_at;
+    if (lane < DC_STAGES) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bars + lane * 8));
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    __syncwarp();
+  }
+  // (one lane) group8: the first of the slice's two groups of 8 rows of the pool
+  __device__ __forceinline__ void load(int stage, const CUtensorMap* map_k, const CUtensorMap* map_v, int group8) const {
+    const uint32_t st = stages + stage * DecodeSmem::stage_bytes_tma, bar = bars + stage * 8;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(DecodeSmem::stage_bytes_tma) : "memory");
+    tma_load_4d(st, map_k, bar, group8);
+    tma_load_4d(st + DecodeSmem::stage_bytes_tma / 2, map_v, bar, group8);
+  }
+  __device__ __forceinline__ bool wait(int stage, uint32_t parity, unsigned long long limit = MS_WAIT_NS) const {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bars + stage * 8, parity, limit));
+  }
+  // Rows of V that must not be weighed, not even by zero (they may hold anything): made zero.
+  __device__ __forceinline__ void clear(int stage, int key0, int lo, int hi, int lane) const {
+    if (key0 < lo || key0 + DC_SLICE > hi) {
+      const uint32_t vt = stages + stage * DecodeSmem::stage_bytes_tma + DecodeSmem::stage_bytes_tma / 2;
+      for (int idx = lane; idx < DC_SLICE * CHUNKS; idx += 32) {
+        const int row = idx / CHUNKS, chunk = idx - row * CHUNKS;
+        if (key0 + row < lo || key0 + row >= hi)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n"
+                       ::"r"(vt + (row >> 3) * (D * 16) + (chunk >> 3) * 1024 + (row & 7) * 128 + (((chunk ^ row) & 7) << 4)), "r"(0) : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // before the stage's next copy
+      __syncwarp();
+    }
+  }
 };
 
+// One slice (16 keys from key0 on) of K and V on its way into `st`; rows outside [lo_load, kv_len) are zero-filled.
+__device__ __forceinline__ void decode_load_slice(__nv_bfloat16* st, const PagedKV& kv, int key0, int lo_load, int kv_len, int lane) {
+  if (kv.page_shift >= 4) {
+    // pages of at least 16 tokens: the whole slice lies in one page, one lookup per slice
+    const int page = kv.pages[key0 >> kv.page_shift];
+    const size_t base = ((((size_t)max(page, 0) * kv.nkv + kv.kv_head) << kv.page_shift) + (key0 & ((1 << kv.page_shift) - 1))) * D;
+#pragma unroll
+    for (int it = 0; it < DC_SLICE * CHUNKS / 32; ++it) {
+      const int idx = it * 32 + lane, row = idx / CHUNKS, chunk = idx - row * CHUNKS;
+      const bool valid = key0 + row >= lo_load && key0 + row < kv_len;
+      const size_t off = valid ? base + row * D + chunk * 8 : 0;
+      cp_async16(st + row * DPAD + chunk * 8, kv.k + off, valid);
+      cp_async16(st + (DC_SLICE + row) * DPAD + chunk * 8, kv.v + off, valid);
+    }
+  } else {
+    load_kv_tile<DC_SLICE, 32>(st, st + DC_SLICE * DPAD, kv, key0, lo_load, kv_len, lane);
+  }
+}
+
+// One slice's scores, softmax step and share of the output for up to 16 query heads (rows g and g + 8 of the tile). TMA: `st` is
+// a stage of a DecodeRing, else K and V lie in padded tiles at kt and vt. EX: with what AttnExtras brings.
+template <bool TMA, bool EX>
+__device__ __forceinline__ void decode_slice(float (&o)[DTILES][4], float (&m_run)[2], float (&l_run)[2],
+                                             const uint32_t (&qf)[Q_IN_REGS ? KSTEPS : 1][4], const __nv_bfloat16* qs,
+                                             const __nv_bfloat16* kt, const __nv_bfloat16* vt, uint32_t st, int key0, int lo, int keep, int kv_len,
+                                             float scale_log2, const AttnExtras& ex, const float (&dr1)[2], const float (&dr2)[2], int lane) {
+  const int t = lane & 3;
+  float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+  for (int kk = 0; kk < KSTEPS; ++kk) {
+    uint32_t a[4], b[4];
+    if (Q_IN_REGS) {
+      a[0] = qf[kk][0]; a[1] = qf[kk][1]; a[2] = qf[kk][2]; a[3] = qf[kk][3];
+    } else {
+      ldmatrix_x4(a, qs + (lane & 15) * DPAD + kk * 16 + (lane >> 4) * 8);
+    }
+    if (TMA) {
+      ldmatrix_x4_at(b, st + (lane >> 4) * (D * 16) + (kk >> 2) * 1024 + (lane & 7) * 128 + (((kk & 3) * 32) ^ ((((lane >> 3) & 1) ^ (lane & 7)) << 4)));
+    } else {
+      ldmatrix_x4(b, kt + ((lane & 7) + ((lane >> 4) << 3)) * DPAD + kk * 16 + ((lane >> 3) & 1) * 8);
+    }
+    mma_bf16(s[0], a, b[0], b[1]);
+    mma_bf16(s[1], a, b[2], b[3]);
+  }
+  const bool inside = !EX && key0 >= lo && key0 + DC_SLICE <= kv_len;  // every key is seen: no mask
+  const int key_base = key0 + 2 * t;
+  float m_new[2] = {m_run[0], m_run[1]};
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int key = key_base + nt * 8 + (e & 1);
+      const bool ok = inside || ((key >= lo || (EX && key < keep)) && key < kv_len);
+      // rows of the tile are query heads (g and g + 8 of this CTA's sixteen), all at position kv_len - 1
+      s[nt][e] = ok ? !EX ? s[nt][e] * scale_log2 : shaped_score(s[nt][e], scale_log2, ex) - (ex.dist_r1 ? distance_bias(dr1[e >> 1], dr2[e >> 1], kv_len - 1 - key) : 0.f)
+                    : -INFINITY;
+      m_new[e >> 1] = fmaxf(m_new[e >> 1], s[nt][e]);
+    }
+  float alpha[2], m_use[2], row_sum[2] = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    m_new[j] = quad_max(m_new[j]);
+    m_use[j] = m_new[j] == -INFINITY ? 0.f : m_new[j];
+    alpha[j] = exp2f(m_run[j] - m_use[j]);
+    m_run[j] = m_new[j];
+  }
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      s[nt][e] = exp2f(s[nt][e] - m_use[e >> 1]);
+      row_sum[e >> 1] += s[nt][e];
+    }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) l_run[j] = l_run[j] * alpha[j] + row_sum[j];
+  uint32_t a[4];
+  a[0] = pack_bf16(s[0][0], s[0][1]);
+  a[1] = pack_bf16(s[0][2], s[0][3]);
+  a[2] = pack_bf16(s[1][0], s[1][1]);
+  a[3] = pack_bf16(s[1][2], s[1][3]);
+  // the running maximum rarely moves after the first slices: rescale only when it did
+  if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+    for (int dt = 0; dt < DTILES; ++dt) {
+      o[dt][0] *= alpha[0]; o[dt][1] *= alpha[0]; o[dt][2] *= alpha[1]; o[dt][3] *= alpha[1];
+    }
+  }
+#pragma unroll
+  for (int dp = 0; dp < DTILES / 2; ++dp) {
+    uint32_t b[4];
+    if (TMA) {
+      ldmatrix_x4_trans_at(b, st + DC_SLICE * D * 2 + ((lane >> 3) & 1) * (D * 16) + (dp >> 2) * 1024 + (lane & 7) * 128 +
+                                  (((dp & 3) * 32) ^ (((lane >> 4) ^ (lane & 7)) << 4)));
+    } else {
+      ldmatrix_x4_trans(b, vt + ((lane & 7) + ((lane >> 3) & 1) * 8) * DPAD + dp * 16 + (lane >> 4) * 8);
+    }
+    mma_bf16(o[2 * dp], a, b[0], b[1]);
+    mma_bf16(o[2 * dp + 1], a, b[2], b[3]);
+  }
+}
+
+template <bool TMA, bool EX>
 __global__ void __launch_bounds__(DC_THREADS)
-attn_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
+attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int* __restrict__ status,
+                   __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
                    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_pool,
                    const __nv_bfloat16* __restrict__ v_pool, const int* __restrict__ kv_len_ptr,
                    const int* __restrict__ page_indptr, const int* __restrict__ page_indices, int nq, int nkv,
                    float scale_log2, int window, int sink, int page_shift, int num_splits, int* __restrict__ counters,
-                   int cluster_merge, AttnExtras ex) {
+                   int cluster_merge, int longest_first, AttnExtras ex) {
   // Until pdl_wait() below, only data written before this step is touched: the step's metadata and
   // the keys and values of older tokens. So the CTA may start streaming them while the kernels
   // before it (the q/k/v projection, the rotation and cache write) are still running.
   pdl_launch_dependents();
-  const int split = blockIdx.x, r = blockIdx.y;
   const int group = nq / nkv, chunks_per_group = (group + 15) / 16;
-  const int kvh = blockIdx.z / chunks_per_group, head0 = kvh * group + (blockIdx.z % chunks_per_group) * 16;
-  const int heads_here = min(16, kvh * group + group - head0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int split = blockIdx.x;
+  int r = blockIdx.y, z = blockIdx.z;
+  if (longest_first) {
+    // One CTA per item and more items than fit the GPU at once: CTAs start in the order of their index, so the longest
+    // request's items come first and the shortest fill the end. Thread i finds request i's rank.
+    __shared__ __align__(16) int lens[DC_THREADS];
+    __shared__ int found;
+    const int rows = gridDim.y, index = blockIdx.z * rows + blockIdx.y, rank = index / (int)gridDim.z;
+    z = index - rank * gridDim.z;
+    const int mine = tid < rows ? kv_len_ptr[tid] : -1;
+    lens[tid] = mine;
+    __syncthreads();
+    int ahead = 0;
+    for (int i = 0; i < rows; i += 4) {
+      const int4 v = *reinterpret_cast<const int4*>(lens + i);
+      ahead += (v.x > mine || (v.x == mine && i < tid)) + (v.y > mine || (v.y == mine && i + 1 < tid)) +
+               (v.z > mine || (v.z == mine && i + 2 < tid)) + (v.w > mine || (v.w == mine && i + 3 < tid));
+    }
+    if (tid < rows && ahead == rank) found = tid;
+    __syncthreads();
+    r = found;
+  }
+  const int kvh = z / chunks_per_group, head0 = kvh * group + (z % chunks_per_group) * 16;
+  const int heads_here = min(16, kvh * group + group - head0);
   const int kv_len = kv_len_ptr[r];
   int lo = window > 0 ? max(0, kv_len - window) : 0;
   if (ex.chunk > 0) lo = max(lo, ((kv_len - 1) / ex.chunk) * ex.chunk);  // the one query sits at position kv_len - 1
@@ -354,6 +532,12 @@ attn_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o, 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   __nv_bfloat16* pipe = qs + DecodeSmem::q_elems + warp * DC_STAGES * DecodeSmem::stage_elems;
+  DecodeRing ring;
+  if (TMA) {
+    __shared__ uint64_t bars[DC_WARPS][DC_STAGES];
+    ring.init(((smem_addr(smem_raw) + (uint32_t)DecodeSmem::q_elems * 2 + 1023) & ~1023u) + warp * DC_STAGES * DecodeSmem::stage_bytes_tma,
+              smem_addr(bars[warp]), lane);
+  }
 
   PagedKV kv{k_pool, v_pool, page_indices + page_indptr[r], kvh, nkv, page_shift};
 
@@ -365,25 +549,21 @@ attn_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o, 
   // this warp's slices: s_begin + warp, + DC_WARPS, ...
   const int my_first = s_begin + warp;
   const int my_count = my_first < s_end ? (s_end - my_first + DC_WARPS - 1) / DC_WARPS : 0;
+  int page_ahead = 0;  // the page of the next slice to be asked for: looked up a slice before its copies go out
+  if (TMA && my_count > 0) page_ahead = kv.pages[(MS_DC_SLICE(my_first) * DC_SLICE) >> page_shift];
   auto issue = [&](int i) {
+    if (TMA) {
+      if (i < my_count && lane == 0) {
+        const int key0 = MS_DC_SLICE(my_first + i * DC_WARPS) * DC_SLICE;
+        ring.load(i % DC_STAGES, &map_k, &map_v, (int)(kv.row_in(page_ahead, key0) >> 3));
+        if (i + 1 < my_count) page_ahead = kv.pages[(MS_DC_SLICE(my_first + (i + 1) * DC_WARPS) * DC_SLICE) >> page_shift];
+      }
+      return;
+    }
     if (i < my_count) {
       __nv_bfloat16* st = pipe + (i % DC_STAGES) * DecodeSmem::stage_elems;
       const int key0 = MS_DC_SLICE(my_first + i * DC_WARPS) * DC_SLICE;
-      if (page_shift >= 4) {
-        // pages of at least 16 tokens: the whole slice lies in one page, one lookup per slice
-        const int page = kv.pages[key0 >> page_shift];
-        const size_t base = ((((size_t)max(page, 0) * nkv + kvh) << page_shift) + (key0 & ((1 << page_shift) - 1))) * D;
-#pragma unroll
-        for (int it = 0; it < DC_SLICE * CHUNKS / 32; ++it) {
-          const int idx = it * 32 + lane, row = idx / CHUNKS, chunk = idx - row * CHUNKS;
-          const bool valid = key0 + row >= lo_load && key0 + row < kv_len;
-          const size_t off = valid ? base + row * D + chunk * 8 : 0;
-          cp_async16(st + row * DPAD + chunk * 8, kv.k + off, valid);
-          cp_async16(st + (DC_SLICE + row) * DPAD + chunk * 8, kv.v + off, valid);
-        }
-      } else {
-        load_kv_tile<DC_SLICE, 32>(st, st + DC_SLICE * DPAD, kv, key0, lo_load, kv_len, lane);
-      }
+      decode_load_slice(st, kv, key0, lo_load, kv_len, lane);
     }
     cp_async_commit();
   };
@@ -422,72 +602,21 @@ attn_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o, 
   }
   for (int i = 0; i < my_count; ++i) {
     issue(i + DC_STAGES - 1);
-    cp_async_wait<DC_STAGES - 1>();
-    __syncwarp();
-    const __nv_bfloat16* kt = pipe + (i % DC_STAGES) * DecodeSmem::stage_elems;
-    const __nv_bfloat16* vt = kt + DC_SLICE * DPAD;
-    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-    for (int kk = 0; kk < KSTEPS; ++kk) {
-      uint32_t a[4], b[4];
-      if (Q_IN_REGS) {
-        a[0] = qf[kk][0]; a[1] = qf[kk][1]; a[2] = qf[kk][2]; a[3] = qf[kk][3];
-      } else {
-        ldmatrix_x4(a, qs + (lane & 15) * DPAD + kk * 16 + (lane >> 4) * 8);
+    const int stage = i % DC_STAGES, key0 = MS_DC_SLICE(my_first + i * DC_WARPS) * DC_SLICE;
+    if (TMA) {
+      if (!ring.wait(stage, (i / DC_STAGES) & 1)) {
+        if (lane == 0) atomicExch(status, 36);
+        for (int k = i + 1; k < min(i + DC_STAGES, my_count); ++k) ring.wait(k % DC_STAGES, (k / DC_STAGES) & 1, MS_WAIT_NS / 64);  // (copies in flight)
+        break;
       }
-      ldmatrix_x4(b, kt + ((lane & 7) + ((lane >> 4) << 3)) * DPAD + kk * 16 + ((lane >> 3) & 1) * 8);
-      mma_bf16(s[0], a, b[0], b[1]);
-      mma_bf16(s[1], a, b[2], b[3]);
+      ring.clear(stage, key0, lo_load, kv_len, lane);
+    } else {
+      cp_async_wait<DC_STAGES - 1>();
+      __syncwarp();
     }
-    const int key_base = MS_DC_SLICE(my_first + i * DC_WARPS) * DC_SLICE + 2 * t;
-    float m_new[2] = {m_run[0], m_run[1]};
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int key = key_base + nt * 8 + (e & 1);
-        const bool ok = (key >= lo || key < keep) && key < kv_len;
-        // rows of the tile are query heads (g and g + 8 of this CTA's sixteen), all at position kv_len - 1
-        s[nt][e] = ok ? shaped_score(s[nt][e], scale_log2, ex) - (ex.dist_r1 ? distance_bias(dr1[e >> 1], dr2[e >> 1], kv_len - 1 - key) : 0.f)
-                      : -INFINITY;
-        m_new[e >> 1] = fmaxf(m_new[e >> 1], s[nt][e]);
-      }
-    float alpha[2], m_use[2], row_sum[2] = {0.f, 0.f};
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      m_new[j] = quad_max(m_new[j]);
-      m_use[j] = m_new[j] == -INFINITY ? 0.f : m_new[j];
-      alpha[j] = exp2f(m_run[j] - m_use[j]);
-      m_run[j] = m_new[j];
-    }
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        s[nt][e] = exp2f(s[nt][e] - m_use[e >> 1]);
-        row_sum[e >> 1] += s[nt][e];
-      }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) l_run[j] = l_run[j] * alpha[j] + row_sum[j];
-    uint32_t a[4];
-    a[0] = pack_bf16(s[0][0], s[0][1]);
-    a[1] = pack_bf16(s[0][2], s[0][3]);
-    a[2] = pack_bf16(s[1][0], s[1][1]);
-    a[3] = pack_bf16(s[1][2], s[1][3]);
-    // the running maximum rarely moves after the first slices: rescale only when it did
-    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
-#pragma unroll
-      for (int dt = 0; dt < DTILES; ++dt) {
-        o[dt][0] *= alpha[0]; o[dt][1] *= alpha[0]; o[dt][2] *= alpha[1]; o[dt][3] *= alpha[1];
-      }
-    }
-#pragma unroll
-    for (int dp = 0; dp < DTILES / 2; ++dp) {
-      uint32_t b[4];
-      ldmatrix_x4_trans(b, vt + ((lane & 7) + ((lane >> 3) & 1) * 8) * DPAD + dp * 16 + (lane >> 4) * 8);
-      mma_bf16(o[2 * dp], a, b[0], b[1]);
-      mma_bf16(o[2 * dp + 1], a, b[2], b[3]);
-    }
+    const __nv_bfloat16* kt = pipe + stage * DecodeSmem::stage_elems;
+    decode_slice<TMA, EX>(o, m_run, l_run, qf, qs, kt, kt + DC_SLICE * DPAD, ring.stages + stage * DecodeSmem::stage_bytes_tma, key0, lo, keep, kv_len,
+                          scale_log2, ex, dr1, dr2, lane);
     __syncwarp();
   }
   cp_async_wait<0>();
@@ -712,19 +841,41 @@ MS_EXPORT int MS_ATTN_FN(decode_fused)(void* out, void* part_o, void* part_ml, i
                                        const int* page_indptr, const int* page_indices, int num_rows, int nq, int nkv,
                                        float scale, int window, int sink, int page_size, int num_splits, cudaStream_t stream,
                                        const float* sink_values, float softcap, int chunk, const float* dist_r1, const float* dist_r2,
-                                       int keep_first);
+                                       int keep_first, long long pool_pages, int* status, int max_kv_len);
 
-// The decode kernel's shared-memory attribute belongs to a device: set once for each.
+// Which form of the decode kernel a launch takes: slices by tensor copies where a slice lies in one page and the pool is known
+// (`pool_pages` > 0), else 16 bytes a lane; without extras the form that carries none of their code.
+using DecodeKernel = void (*)(const CUtensorMap, const CUtensorMap, int*, __nv_bfloat16*, float*, float*, const __nv_bfloat16*, const __nv_bfloat16*,
+                              const __nv_bfloat16*, const int*, const int*, const int*, int, int, float, int, int, int, int, int*, int, int, AttnExtras);
+static bool decode_takes_tma(const void* k_pool, const void* v_pool, long long pool_pages, int page_size, const int* status) {
+  return DC_TMA && pool_pages > 0 && page_size >= DC_SLICE && status != nullptr && (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0;
+}
+static bool has_extras(const AttnExtras& ex) { return ex.cap_inv > 0.f || ex.chunk > 0 || ex.dist_r1 != nullptr || ex.keep_first > 0; }
+static DecodeKernel decode_form(bool tma, const AttnExtras& ex) {
+  return !tma ? attn_decode_kernel<false, true> : has_extras(ex) ? attn_decode_kernel<DC_TMA, true> : attn_decode_kernel<DC_TMA, !DC_TMA>;
+}
+static constexpr size_t decode_smem(bool tma) { return tma ? DecodeSmem::bytes_tma : DecodeSmem::bytes; }
+
+// The decode kernels' shared-memory attribute belongs to a device: set once for each.
 static int configure_decode() {
   static bool configured[64] = {};
   int dev = 0;
   MS_CHECK_CUDA(cudaGetDevice(&dev));
   MS_CHECK_ARG(dev >= 0 && dev < 64, "attention: device index %d is not supported", dev);
   if (!configured[dev]) {
-    MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes));
+    MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes));
+    if (DC_TMA) {
+      MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<DC_TMA, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes_tma));
+      MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<DC_TMA, !DC_TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes_tma));
+    }
     configured[dev] = true;
   }
   return 0;
+}
+static int decode_maps(CUtensorMap* map_k, CUtensorMap* map_v, bool tma, const void* k_pool, const void* v_pool, long long pool_pages, int nkv, int page_size) {
+  if (!tma) return 0;
+  if (int rc = cache_tensor_map(map_k, k_pool, pool_pages * nkv * page_size, D, DC_SLICE)) return rc;
+  return cache_tensor_map(map_v, v_pool, pool_pages * nkv * page_size, D, DC_SLICE);
 }
 
 // Scratch for num_splits > 1: part_o [rows, nq, splits, D] floats and part_ml [rows, nq, splits, 2] floats.
@@ -733,7 +884,7 @@ MS_EXPORT int MS_ATTN_FN(decode)(void* out, void* part_o, void* part_ml, const v
                                  const int* page_indices, int num_rows, int nq, int nkv, float scale, int window, int sink,
                                  int page_size, int num_splits, cudaStream_t stream) {
   return MS_ATTN_FN(decode_fused)(out, part_o, part_ml, nullptr, q, k_pool, v_pool, kv_len, page_indptr, page_indices,
-                                  num_rows, nq, nkv, scale, window, sink, page_size, num_splits, stream, nullptr, 0.f, 0, nullptr, nullptr, 0);
+                                  num_rows, nq, nkv, scale, window, sink, page_size, num_splits, stream, nullptr, 0.f, 0, nullptr, nullptr, 0, 0, nullptr, 0);
 }
 
 // As above; with `counters` (num_rows * kv_heads * ceil(group / 16) ints, zero before the first
@@ -744,7 +895,7 @@ MS_EXPORT int MS_ATTN_FN(decode_fused)(void* out, void* part_o, void* part_ml, i
                                        const int* page_indptr, const int* page_indices, int num_rows, int nq, int nkv,
                                        float scale, int window, int sink, int page_size, int num_splits, cudaStream_t stream,
                                        const float* sink_values, float softcap, int chunk, const float* dist_r1, const float* dist_r2,
-                                       int keep_first) {
+                                       int keep_first, long long pool_pages, int* status, int max_kv_len) {
   if (num_rows == 0) return 0;
   MS_CHECK_ARG(softcap >= 0.f && chunk >= 0, "attention: softcap=%g and chunk=%d must not be negative", softcap, chunk);
   sink = sink || sink_values != nullptr;
@@ -756,11 +907,18 @@ MS_EXPORT int MS_ATTN_FN(decode_fused)(void* out, void* part_o, void* part_ml, i
   MS_CHECK_ARG(num_rows <= 65535, "attention: too many rows (%d) for one launch", num_rows);
   const int group = nq / nkv;
   if (int rc = configure_decode()) return rc;
+  CUtensorMap map_k = {}, map_v = {};
+  const bool tma = decode_takes_tma(k_pool, v_pool, pool_pages, page_size, status);
+  if (int rc = decode_maps(&map_k, &map_v, tma, k_pool, v_pool, pool_pages, nkv, page_size)) return rc;
   dim3 grid(num_splits, num_rows, nkv * ceil_div(group, 16));
-  MS_LAUNCH(attn_decode_kernel, grid, DC_THREADS, DecodeSmem::bytes, stream,
-      (__nv_bfloat16*)out, (float*)part_o, (float*)part_ml, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
+  // By length where items wait for others to end: each CTA then compares all lengths, a thread a request, which takes about a
+  // microsecond (64 requests, us: 1,025 to 3,986 keys 149 -> 119, 100 keys each 18.5 -> 20.5), so not where no row is long.
+  // max_kv_len 0: not known, inside a graph, where that microsecond passes while the kernels before still run.
+  const int longest_first = (max_kv_len == 0 || max_kv_len > 512) && num_splits == 1 && num_rows > 1 && num_rows <= DC_THREADS && num_rows * (int)grid.z > sm_count();
+  MS_LAUNCH(decode_form(tma, ex), grid, DC_THREADS, decode_smem(tma), stream,
+      map_k, map_v, status, (__nv_bfloat16*)out, (float*)part_o, (float*)part_ml, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
       (const __nv_bfloat16*)v_pool, kv_len, page_indptr, page_indices, nq, nkv, scale * LOG2E, window, sink,
-      shift_of(page_size), num_splits, counters, 0, ex);
+      shift_of(page_size), num_splits, counters, 0, longest_first, ex);
   if (num_splits > 1 && counters == nullptr) {
     MS_LAUNCH(attn_decode_merge_kernel, num_rows * nq, D >= 128 ? 128 : 64, 0, stream, (__nv_bfloat16*)out,
               (const float*)part_o, (const float*)part_ml, num_splits, sink, nq, ex);
@@ -775,7 +933,7 @@ MS_EXPORT int MS_ATTN_FN(decode_cluster)(void* out, const void* q, const void* k
                                          const int* page_indptr, const int* page_indices, int num_rows, int nq, int nkv,
                                          float scale, int window, int sink, int page_size, int num_splits, cudaStream_t stream,
                                          const float* sink_values, float softcap, int chunk, const float* dist_r1,
-                                         const float* dist_r2, int keep_first) {
+                                         const float* dist_r2, int keep_first, long long pool_pages, int* status) {
   if (num_rows == 0) return 0;
   MS_CHECK_ARG(softcap >= 0.f && chunk >= 0, "attention: softcap=%g and chunk=%d must not be negative", softcap, chunk);
   sink = sink || sink_values != nullptr;
@@ -786,11 +944,14 @@ MS_EXPORT int MS_ATTN_FN(decode_cluster)(void* out, const void* q, const void* k
   MS_CHECK_ARG(num_rows <= 65535, "attention: too many rows (%d) for one launch", num_rows);
   const int group = nq / nkv;
   if (int rc = configure_decode()) return rc;
+  CUtensorMap map_k = {}, map_v = {};
+  const bool tma = decode_takes_tma(k_pool, v_pool, pool_pages, page_size, status);
+  if (int rc = decode_maps(&map_k, &map_v, tma, k_pool, v_pool, pool_pages, nkv, page_size)) return rc;
   dim3 grid(num_splits, num_rows, nkv * ceil_div(group, 16));
-  MS_LAUNCH_CLUSTERED(attn_decode_kernel, grid, DC_THREADS, DecodeSmem::bytes, stream, num_splits,
-      (__nv_bfloat16*)out, (float*)nullptr, (float*)nullptr, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
+  MS_LAUNCH_CLUSTERED(decode_form(tma, ex), grid, DC_THREADS, decode_smem(tma), stream, num_splits,
+      map_k, map_v, status, (__nv_bfloat16*)out, (float*)nullptr, (float*)nullptr, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
       (const __nv_bfloat16*)v_pool, kv_len, page_indptr, page_indices, nq, nkv, scale * LOG2E, window, sink,
-      shift_of(page_size), num_splits, (int*)nullptr, 1, ex);
+      shift_of(page_size), num_splits, (int*)nullptr, 1, 0, ex);
   return 0;
 }
 
@@ -808,7 +969,7 @@ MS_EXPORT int MS_ATTN_FN(decode_clusters_resident)(int num_splits, int* out) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_splits, 1024, 1);
     cfg.blockDim = dim3(DC_THREADS);
-    cfg.dynamicSmemBytes = DecodeSmem::bytes;
+    cfg.dynamicSmemBytes = decode_smem(DC_TMA);  // (the padded stages are no smaller; the registers of both forms allow as many)
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = num_splits;
@@ -817,7 +978,7 @@ MS_EXPORT int MS_ATTN_FN(decode_clusters_resident)(int num_splits, int* out) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    MS_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, attn_decode_kernel, &cfg));
+    MS_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, decode_form(DC_TMA, AttnExtras{}), &cfg));
     cached[dev][num_splits] = n > 0 ? n : -1;
   }
   *out = cached[dev][num_splits] > 0 ? cached[dev][num_splits] : 0;

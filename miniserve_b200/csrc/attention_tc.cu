@@ -14,8 +14,6 @@
 // only when the maximum has grown by more than 2^8 (the stale maximum is exact in the end because
 // the same one scales the sum).
 // Every mbarrier wait is bounded; on a timeout the kernel raises the status word and winds down.
-#include <cuda.h>
-
 #include <cfloat>
 #include <cstdlib>
 #include <map>
@@ -23,6 +21,7 @@
 #include <tuple>
 
 #include "common.cuh"
+#include "tensor_map.cuh"
 
 namespace ms {
 
@@ -42,11 +41,6 @@ __device__ __forceinline__ void at_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(at_smem(bar)) : "memory");
 }
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity) { return mbar_wait_bounded(at_smem(bar), parity); }
-__device__ __forceinline__ void at_tma_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %4}], [%2];\n"
-      ::"r"(at_smem(dst)), "l"(map), "r"(at_smem(bar)), "r"(0), "r"(c3) : "memory");
-}
 __device__ __forceinline__ void at_tma_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
@@ -540,12 +534,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           if (!ok || !wait_free(&k_empty[s], tiles >> 1)) break;
           if (lane == 0) at_expect_tx(&k_full[s], bytes);
           __syncwarp();
-          if (lane < boxes) at_tma_4d(smem + AtSmem::k + s * AtSmem::slot + lane * box_rows * (AT_D * 2), &map_k, &k_full[s], group8);
+          if (lane < boxes) tma_load_4d(at_smem(smem + AtSmem::k + s * AtSmem::slot + lane * box_rows * (AT_D * 2)), &map_k, at_smem(&k_full[s]), group8);
           if (j == 0) load_q(1);
           if (!ok || !wait_free(&v_empty[s], tiles >> 1)) break;
           if (lane == 0) at_expect_tx(&v_full[s], bytes);
           __syncwarp();
-          if (lane < boxes) at_tma_4d(smem + AtSmem::v + s * AtSmem::slot + lane * box_rows * (AT_D * 2), &map_v, &v_full[s], group8);
+          if (lane < boxes) tma_load_4d(at_smem(smem + AtSmem::v + s * AtSmem::slot + lane * box_rows * (AT_D * 2)), &map_v, at_smem(&v_full[s]), group8);
         }
         __syncwarp();
       }
@@ -960,23 +954,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 }
 
 // ---------------------------------------------------------------- host side
-using AtEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static int at_get_encode(AtEncodeFn* out) {
-  static AtEncodeFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    MS_CHECK_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres));
-    MS_CHECK_ARG(ptr != nullptr && qres == cudaDriverEntryPointSuccess, "attention_tc: the driver has no cuTensorMapEncodeTiled");
-    fn = reinterpret_cast<AtEncodeFn>(ptr);
-  }
-  *out = fn;
-  return 0;
-}
-
 }  // namespace ms
 
 using namespace ms;
@@ -1079,8 +1056,8 @@ MS_EXPORT int ms_attn_tc_prefill(void* out, const void* q, const void* k_pool, c
   MS_CHECK_ARG(((uintptr_t)q % 16 == 0) && ((uintptr_t)k_pool % 16 == 0) && ((uintptr_t)v_pool % 16 == 0), "attention_tc: operands must be 16-byte aligned");
   const int G = at_heads_per_cta(nq, nkv);
   const int tpc = AT_ROWS / G;
-  AtEncodeFn encode;
-  if (int rc = at_get_encode(&encode)) return rc;
+  TensorMapEncodeFn encode;
+  if (int rc = tensor_map_encoder(&encode)) return rc;
   CUtensorMap map_q, map_k, map_v;
   {
     const cuuint64_t dims[3] = {(cuuint64_t)AT_D, (cuuint64_t)nq, (cuuint64_t)num_tokens};
@@ -1092,19 +1069,10 @@ MS_EXPORT int ms_attn_tc_prefill(void* out, const void* q, const void* k_pool, c
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     MS_CHECK_ARG(res == CUDA_SUCCESS, "attention_tc: encoding the query map failed with code %d", (int)res);
   }
-  // The cache as [groups of 8 rows][2 halves of a row][8 rows][64]: one copy brings a page's keys (or values) of one head, in the
-  // order in which the products' descriptors walk them (a swizzled block is 8 rows of 128 bytes; a group's two blocks lie side by side).
-  const cuuint64_t kdims[4] = {64, 8, 2, (cuuint64_t)pool_pages * nkv * page_size / 8};
-  const cuuint64_t kstrides[3] = {(cuuint64_t)AT_D * 2, 128, (cuuint64_t)AT_D * 2 * 8};
-  const cuuint32_t kbox[4] = {64, 8, 2, (cuuint32_t)(page_size < AT_KEYS ? page_size : AT_KEYS) / 8};
-  const cuuint32_t kelem[4] = {1, 1, 1, 1};
-  for (int i = 0; i < 2; ++i) {
-    const CUresult res = encode(i == 0 ? &map_k : &map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
-                                const_cast<void*>(i == 0 ? k_pool : v_pool), kdims, kstrides, kbox, kelem,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    MS_CHECK_ARG(res == CUDA_SUCCESS, "attention_tc: encoding the cache map failed with code %d", (int)res);
-  }
+  const long long pool_rows = pool_pages * nkv * page_size;
+  const int box_rows = page_size < AT_KEYS ? page_size : AT_KEYS;
+  if (int rc = cache_tensor_map(&map_k, k_pool, pool_rows, AT_D, box_rows)) return rc;
+  if (int rc = cache_tensor_map(&map_v, v_pool, pool_rows, AT_D, box_rows)) return rc;
   int page_shift = 0;
   while ((1 << page_shift) < page_size) ++page_shift;
   constexpr size_t smem_bytes = AtSmem::total + 1024;

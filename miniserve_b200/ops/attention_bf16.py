@@ -4,14 +4,14 @@ use: a model only pays for the head size it has."""
 from __future__ import annotations
 
 import ctypes
-from ctypes import c_char_p, c_float, c_int, c_void_p
+from ctypes import c_char_p, c_float, c_int, c_longlong, c_void_p
 from functools import lru_cache
 
 import torch
 
 from . import build, native
 
-_p, _i, _f = c_void_p, c_int, c_float
+_p, _i, _f, _ll = c_void_p, c_int, c_float, c_longlong
 
 
 def _flag(name: str, default: str) -> bool:
@@ -56,8 +56,8 @@ def _lib(head_dim: int):
         ("last_error", [], c_char_p),
         ("prefill", [_p] * 8 + [_i, _i, _i, _i, _f, _i, _i, _i, _p, _p, _f, _i, _p, _p, _i], c_int),
         ("decode", [_p] * 9 + [_i, _i, _i, _f, _i, _i, _i, _i, _p], c_int),
-        ("decode_fused", [_p] * 10 + [_i, _i, _i, _f, _i, _i, _i, _i, _p, _p, _f, _i, _p, _p, _i], c_int),
-        ("decode_cluster", [_p] * 7 + [_i, _i, _i, _f, _i, _i, _i, _i, _p, _p, _f, _i, _p, _p, _i], c_int),
+        ("decode_fused", [_p] * 10 + [_i, _i, _i, _f, _i, _i, _i, _i, _p, _p, _f, _i, _p, _p, _i, _ll, _p, _i], c_int),
+        ("decode_cluster", [_p] * 7 + [_i, _i, _i, _f, _i, _i, _i, _i, _p, _p, _f, _i, _p, _p, _i, _ll, _p], c_int),
         ("decode_clusters_resident", [_i, ctypes.POINTER(c_int)], c_int),
     ):
         fn = getattr(lib, pre + name)
@@ -119,8 +119,8 @@ def choose_splits(rows: int, head_chunks: int, max_kv_len: int | None, sm_count:
     return splits
 
 
-def _scratch(ctx, rows: int, nq: int, splits: int, d: int, device) -> tuple[torch.Tensor, torch.Tensor]:
-    need = rows * nq * splits
+def _scratch(ctx, need: int, d: int, device) -> tuple[torch.Tensor, torch.Tensor]:
+    """Partial results: ``need`` rows of d floats, and of two."""
     if ctx.graph_bucket:
         # inside a CUDA graph capture: memory of the graph's own pool, alive as long as the graph
         return (torch.empty(need * d, dtype=torch.float32, device=device),
@@ -131,6 +131,17 @@ def _scratch(ctx, rows: int, nq: int, splits: int, d: int, device) -> tuple[torc
                torch.empty(need * 2, dtype=torch.float32, device=device))
         ctx.scratch["attn_decode"] = buf
     return buf
+
+
+def _counters(ctx, items: int, device) -> torch.Tensor:
+    """Tickets of the merges inside the kernels: zero before the first launch, left zero by every launch."""
+    counters = ctx.scratch.get("attn_counters")
+    if counters is None or counters.numel() < items:
+        if counters is not None:  # captured graphs may hold the smaller one's address: it stays alive
+            ctx.scratch.setdefault("retired", []).append(counters)
+        counters = torch.zeros(max(4096, items), dtype=torch.int32, device=device)
+        ctx.scratch["attn_counters"] = counters
+    return counters
 
 
 def run(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx, group: int,
@@ -145,9 +156,12 @@ def run(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.
 
 
 def run_decode(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx, group: int,
-               scale: float, window: int | None, rows: int, sink: bool = False, extras=None) -> None:
+               scale: float, window: int | None, rows: int, sink: bool = False, extras=None, form: str | None = None) -> None:
     """Rows [0, rows) of the step, one new token each (so token i belongs to row i): keys split
-    across CTAs, partial results merged by the last CTA of each (row, head group) to finish."""
+    across CTAs, partial results merged by the last CTA of each (row, head group) to finish. ``form`` (tests):
+    "general", copies of 16 bytes a lane, as head sizes other than 64 and 128 and pages of 8 tokens take."""
+    from . import device_status
+
     t, nq, d = q.shape
     nkv, page_size = k_pool.shape[1], k_pool.shape[2]
     fns = _lib(d)
@@ -156,28 +170,23 @@ def run_decode(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool:
     fit = (lambda n: clusters_resident(d, n, q.device.index or 0)) if CLUSTER_MERGE else None
     known = ctx.max_kv_len if not ctx.graph_bucket else (getattr(ctx, "graph_kv_len", 0) or None)
     splits = choose_splits(rows, chunks, known, ctx.sm_count, fit)
+    pool = (0 if form == "general" else k_pool.shape[0], device_status(q.device).data_ptr())
     if CLUSTER_MERGE and 2 <= splits <= 8:
         # the splits as one thread-block cluster: merged through distributed shared memory
         _check(fns, fns["decode_cluster"](
             out.data_ptr(), q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), ctx.kv_len.data_ptr(), indptr.data_ptr(),
             indices.data_ptr(), rows, nq, nkv, float(scale), int(window or 0), int(sink), page_size, splits, ctx.stream,
-            *_extras_args(extras)))
+            *_extras_args(extras), *pool))
         return
     part_o = part_ml = counters = None
     if splits > 1:
-        part_o, part_ml = _scratch(ctx, rows, nq, splits, d, q.device)
-        counters = ctx.scratch.get("attn_counters")
-        if counters is None or counters.numel() < rows * chunks:
-            # tickets of the fused merge: zero before the first launch, left zero by every launch
-            if counters is not None:  # captured graphs may hold the smaller one's address: it stays alive
-                ctx.scratch.setdefault("retired", []).append(counters)
-            counters = torch.zeros(max(4096, rows * chunks), dtype=torch.int32, device=q.device)
-            ctx.scratch["attn_counters"] = counters
+        part_o, part_ml = _scratch(ctx, rows * nq * splits, d, q.device)
+        counters = _counters(ctx, rows * chunks, q.device)
     _check(fns, fns["decode_fused"](
         out.data_ptr(), None if part_o is None else part_o.data_ptr(), None if part_ml is None else part_ml.data_ptr(),
         None if counters is None else counters.data_ptr(), q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), ctx.kv_len.data_ptr(), indptr.data_ptr(),
         indices.data_ptr(), rows, nq, nkv, float(scale), int(window or 0), int(sink), page_size, splits, ctx.stream,
-        *_extras_args(extras)), launches=1)
+        *_extras_args(extras), *pool, int(known or 0)), launches=1)
 
 
 def run_prefill(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx, group: int,

@@ -3,6 +3,7 @@ other than the engine's (odd widths, head sizes in steps of 16, vocabularies tha
 of two), and with inputs made so that a fault would show."""
 
 import math
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -433,6 +434,38 @@ def test_attention_bf16_decode(nq, nkv, d, page, splits, monkeypatch):
     assert ref[0, 0].mean().item() > 40  # the far key dominates row 0
     assert torch.allclose(out.float(), ref, atol=0.3, rtol=2e-2)
     assert torch.allclose(out.float()[1:3], ref[1:3], **BF16_TOL)
+
+
+@pytest.mark.parametrize("nq, nkv, d, page", [(16, 8, 128, 16), (32, 1, 64, 32), (6, 2, 64, 64), (20, 4, 128, 128)])
+@pytest.mark.parametrize("keys", [1, 17, 700, 2500])
+@pytest.mark.parametrize("extra", ["plain", "window", "shaped", "kept"])
+@pytest.mark.parametrize("splits", [1, 3, 9])
+def test_attention_bf16_decode_by_tensor_copies(nq, nkv, d, page, keys, extra, splits, monkeypatch):
+    """Against the form that copies 16 bytes a lane, whole items (the longest row's first), splits as a cluster and splits through
+    scratch memory; an empty row, rows of one key, one key beyond a slice, rows of one length, one longer than all others."""
+    torch.manual_seed(keys)
+    rows = [(0, 1), (keys - 1, 1)] + [((37 * i) % keys, 1) for i in range(38)] + [(min(4 * keys, 6000), 1), (15, 1), (16, 1), (keys // 2, 1)]
+    pb = PagedBatch(rows, page, nkv, d, torch.bfloat16, seed=2)
+    pb.k_pool = torch.randn(pb.k_pool.shape, device=DEV).bfloat16()
+    pb.v_pool = torch.randn(pb.v_pool.shape, device=DEV).bfloat16()
+    q = torch.randn(len(rows), nq, d, device=DEV).bfloat16()
+    f32 = dict(device=DEV, dtype=torch.float32)
+    extras = {"shaped": SimpleNamespace(sink_values=torch.randn(nq, **f32), softcap=3.0, chunk=300, dist_r1=None, dist_r2=None, keep_first=0),
+              "kept": SimpleNamespace(sink_values=None, softcap=0.0, chunk=0, dist_r1=torch.rand(nq, **f32), dist_r2=torch.rand(nq, **f32),
+                                      keep_first=21)}.get(extra)
+    window = {"window": 100, "kept": 40}.get(extra)
+    monkeypatch.setattr(attention_bf16, "choose_splits", lambda *a, **k: splits)
+    ctx = make_context(pb)
+    ctx.kv_len[5] = 0  # (a row of a graph that no request fills)
+    outs = []
+    for form in ("general", None, None):
+        outs.append(torch.full_like(q, -7.0))
+        attention_bf16.run_decode(outs[-1], q, pb.k_pool, pb.v_pool, ctx, 0, d ** -0.5, window, len(rows), extra == "window", extras, form)
+    assert ops.device_status("cuda").item() == 0
+    sums = [o.float() for o in outs]
+    filled = torch.arange(len(rows), device=DEV) != 5
+    for o in sums[1:]:
+        assert torch.equal(o[filled], sums[0][filled])  # the same sums in the same order
 
 
 @pytest.mark.parametrize("graph_kv_len", [0, 8192, 32768])
