@@ -142,6 +142,18 @@ __device__ __forceinline__ float clamped_glu_fast(float g, float u, const Clampe
   return __fdividef(g, 1.0f + __expf(-p.alpha * g)) * (u + p.shift);
 }
 
+// what an output is made of: the accumulator, with `up` of a gated epilogue the up half's
+template <int EPI>
+__device__ __forceinline__ float tc_activation(float x, float up, const ClampedGlu& glu) {
+  if (EPI == TC_SILU_MUL) return x / (1.0f + expf(-x)) * up;
+  if (EPI == TC_CLAMPED_GLU) return clamped_glu_fast(x, up, glu);
+  if (EPI == TC_RELU2) {
+    x = fmaxf(x, 0.f);
+    return x * x;
+  }
+  return x;
+}
+
 // The rows of A sorted into runs, one run per weight matrix (the experts of a routed feed-forward, W [E * w_rows, K]):
 // a plan on the device lists the row tiles, (matrix, first row) each, meta[0] = how many; offsets[e + 1] ends run e.
 struct TcGroups {
@@ -285,16 +297,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           } else {
             float v[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              float x = __uint_as_float(acc[j]);
-              if (EPI == TC_SILU_MUL) x = x / (1.0f + expf(-x)) * __uint_as_float(up[j]);
-              if (EPI == TC_CLAMPED_GLU) x = clamped_glu_fast(x, __uint_as_float(up[j]), grp.glu);
-              if (EPI == TC_RELU2) {
-                x = fmaxf(x, 0.f);
-                x *= x;
-              }
-              v[j] = x;
-            }
+            for (int j = 0; j < 32; ++j) v[j] = tc_activation<EPI>(__uint_as_float(acc[j]), tc_gated(EPI) ? __uint_as_float(up[j]) : 0.f, grp.glu);
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * N_out + col0;
             if (col0 + 32 <= N_out && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
@@ -331,7 +334,7 @@ __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f 
 
 template <int EPI>
 __device__ __forceinline__ void store_chunk(void* __restrict__ out, const uint32_t (&acc)[32], const uint32_t (&up)[32], int row,
-                                            int col0, int N_out) {
+                                            int col0, int N_out, const ClampedGlu& glu = ClampedGlu{}) {
   if (EPI == TC_OUT_F32) {
     float* dst = reinterpret_cast<float*>(out) + (size_t)row * N_out + col0;
     if (col0 + 32 <= N_out && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
@@ -343,11 +346,7 @@ __device__ __forceinline__ void store_chunk(void* __restrict__ out, const uint32
   } else {
   float v[32];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    float x = __uint_as_float(acc[j]);
-    if (EPI == TC_SILU_MUL) x = x / (1.0f + expf(-x)) * __uint_as_float(up[j]);
-    v[j] = x;
-  }
+  for (int j = 0; j < 32; ++j) v[j] = tc_activation<EPI>(__uint_as_float(acc[j]), __uint_as_float(up[j]), glu);
   __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * N_out + col0;
   if (col0 + 32 <= N_out && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
@@ -726,11 +725,13 @@ constexpr int PAIR_OUT_BYTES = TC_BM * 64 * 2;  // one [128][64] bfloat16 tile o
 // per CTA and stage: 128 rows of A and half of the tile's BN rows of W, 64 k each
 __host__ __device__ constexpr int pair_stage_bytes(int bn) { return (TC_BM + bn / 2) * TC_BK * 2; }
 
-template <int BN, int STAGES, int EPI>
+// GROUPED: the row tiles are the plan's (256 sorted rows of one matrix each); a tile's rows beyond its run are computed with the run's matrix and not
+// stored. Row tiles change fastest here too: a run has two or three of them, which then take a tile of W from L2 together.
+template <int BN, int STAGES, int EPI, bool GROUPED = false>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_out, void* __restrict__ out,
-                    int M, int N_out, int K, int up_row_offset, int* __restrict__ status, const QkvEpilogue qe) {
+                    int M, int N_out, int K, int up_row_offset, int* __restrict__ status, const QkvEpilogue qe, const TcGroups grp) {
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -746,14 +747,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0: the CTA that issues the products
   const int k_iters = (K + TC_BK - 1) / TC_BK;
-  const int n_tiles = (N_out + COLS - 1) / COLS, m_tiles = (M + 2 * TC_BM - 1) / (2 * TC_BM);
-  const int num_tiles = n_tiles * m_tiles;
+  const int n_tiles = (N_out + COLS - 1) / COLS;
+  int m_tiles = (M + 2 * TC_BM - 1) / (2 * TC_BM);
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   // Tiles that run at the same time share the larger operand: with fewer rows in A than in W the
   // row tiles change fastest, so that a tile of W is fetched from memory once and serves every row
   // tile while it is in L2 (24,576 x 4,096 weights do not fit L2; walking them once per row tile
   // took 339 us against the library's 271 for 2,048 rows).
-  const bool m_fastest = M <= N_out;
+  const bool m_fastest = GROUPED || M <= N_out;
   auto tile_m = [&](int tile) { return m_fastest ? tile % m_tiles : tile / n_tiles; };
   auto tile_n = [&](int tile) { return m_fastest ? tile / m_tiles : tile % n_tiles; };
 
@@ -784,14 +785,20 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   pdl_launch_dependents();
   pdl_wait();
+  if (GROUPED) m_tiles = grp.meta[0];  // (the plan is an earlier kernel's)
+  const int num_tiles = n_tiles * m_tiles;
+  // a tile's first row for this CTA, the matrix it belongs to and the end of that matrix's rows
+  auto first_row = [&](int tile) { return (GROUPED ? grp.tiles[2 * tile_m(tile) + 1] : tile_m(tile) * 2 * TC_BM) + (int)rank * TC_BM; };
+  auto matrix_of = [&](int tile) { return GROUPED ? grp.tiles[2 * tile_m(tile)] : 0; };
 
   if (warp == 0) {
     if (elect_one()) {
       int kb = 0;
       for (int tile = pair; tile < num_tiles; tile += num_pairs) {
-        const int n0 = tile_n(tile) * COLS, m0 = tile_m(tile) * 2 * TC_BM + (int)rank * TC_BM;
+        const int n0 = tile_n(tile) * COLS, m0 = first_row(tile);
         // this CTA's 128 of the tile's 256 rows of W: for SiLU * up the first CTA brings the gate rows, the second the up rows
-        const int w_row = EPI == TC_SILU_MUL ? (rank == 0 ? n0 : up_row_offset + n0) : n0 + (int)rank * (BN / 2);
+        const int w_row = (GROUPED ? matrix_of(tile) * grp.w_rows : 0) +
+                          (tc_gated(EPI) ? (rank == 0 ? n0 : up_row_offset + n0) : n0 + (int)rank * (BN / 2));
         bool ok = true;
         for (int it = 0; it < k_iters; ++it, ++kb) {
           const int s = kb % STAGES;
@@ -846,11 +853,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const bool issuer = (int)threadIdx.x == 64 + 128 * eg;
     int tc = 0, out_buf = 0;
     uint32_t cs_count = 0;  // TC_QKV_ROPE: quarters of the cos/sin table that have been through the ring before this tile
-    const bool tma_out = EPI != TC_OUT_F32 && EPI != TC_QKV_ROPE && N_out % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    const bool tma_out = (GROUPED || EPI != TC_OUT_F32) && EPI != TC_QKV_ROPE && N_out % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++tc) {
       const int buf = tc & 1;
-      const int n0 = tile_n(tile) * COLS, m0 = tile_m(tile) * 2 * TC_BM + (int)rank * TC_BM;
+      const int n0 = tile_n(tile) * COLS, m0 = first_row(tile);
       const int row = m0 + quad * 32 + lane;
+      const int rows_end = GROUPED ? min(M, grp.offsets[matrix_of(tile) + 1]) : M;
       // TC_QKV_ROPE: the rotation's cosines and sines of the tile's 128 tokens come through a ring of four
       // slots filled by bulk copies, a quarter of a half head (8 pairs) per slot, asked for four quarters
       // ahead by the first thread of the first group. Every thread reads its token's 32 + 32 bytes of a
@@ -1007,58 +1015,70 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               *reinterpret_cast<uint4*>(pool + (size_t)dst * 128 + (sub >> 3) * 64 + c * 8) = *reinterpret_cast<const uint4*>(from + rr * 128 + ((c ^ (rr & 7)) << 4));
           }
         }
-      } else if constexpr (EPI == TC_OUT_F32) {
+      } else if constexpr (EPI == TC_OUT_F32 && !GROUPED) {
 #pragma unroll 1
         for (int c = 32 * eg; c < COLS; c += 64) {
           uint32_t acc[32];
           tmem_ld32(lane_addr + (uint32_t)c, acc);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-          if (row < M) store_chunk<EPI>(out, acc, acc, row, n0 + c, N_out);
+          if (row < rows_end) store_chunk<EPI>(out, acc, acc, row, n0 + c, N_out);
         }
       } else if (!tma_out) {
 #pragma unroll 1
         for (int c = 32 * eg; c < COLS; c += 64) {
           uint32_t acc[32];
           tmem_ld32(lane_addr + (uint32_t)c, acc);
-          if constexpr (EPI == TC_SILU_MUL) {
+          if constexpr (tc_gated(EPI)) {
             uint32_t up[32];
             tmem_ld32(lane_addr + (uint32_t)(COLS + c), up);
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (row < M) store_chunk<EPI>(out, acc, up, row, n0 + c, N_out);
+            if (row < rows_end) store_chunk<EPI>(out, acc, up, row, n0 + c, N_out, grp.glu);
           } else {
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (row < M) store_chunk<EPI>(out, acc, acc, row, n0 + c, N_out);
+            if (row < rows_end) store_chunk<EPI>(out, acc, acc, row, n0 + c, N_out);
           }
         }
       } else {
-        // bfloat16 out: 64 columns at a time go through a swizzled shared-memory tile [128][64] and
-        // leave with one TMA store, which writes whole lines and clips at the matrix's edge; each
+        // 64 columns of bfloat16 (32 of float32) at a time go through a swizzled shared-memory tile of 128 rows of 128 bytes
+        // and leave with one TMA store, which writes whole lines and clips at the matrix's edge; each
         // group of warps has two such tiles that take turns, so that a store is still reading one
-        // while the next is being filled
+        // while the next is being filled. Rows that end inside the tile (GROUPED) leave row by row, eight lanes to a line:
+        // a TMA store would write the next matrix's too. (float32 straight from the registers, 16 bytes a thread and 8 KB from
+        // thread to thread, held the next tile's products up: 62.7 us for 7,600 rows of 1536 to 2048.)
+        constexpr int CW = EPI == TC_OUT_F32 ? 32 : 64;
         const int r = quad * 32 + lane;
+        const bool whole = !GROUPED || m0 + TC_BM <= rows_end;
 #pragma unroll 1
-        for (int cb = 64 * eg; cb < COLS; cb += 128) {
+        for (int cb = CW * eg; cb < COLS; cb += 2 * CW) {
           unsigned char* stage_out = smem + (size_t)STAGES * STAGE_BYTES + (size_t)(2 * eg + out_buf) * PAIR_OUT_BYTES;
           if (issuer) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");  // this tile's last store has read it
           epilogue_sync(1 + eg);
+          if constexpr (EPI == TC_OUT_F32) {
+            uint32_t acc[32];
+            tmem_ld32(lane_addr + (uint32_t)cb, acc);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
+            for (int q = 0; q < 8; ++q)
+              *reinterpret_cast<uint4*>(stage_out + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+          }
+#pragma unroll
+          for (int h = 0; h < (EPI == TC_OUT_F32 ? 0 : 2); ++h) {
             uint32_t acc[32];
             float v[32];
             tmem_ld32(lane_addr + (uint32_t)(cb + 32 * h), acc);
-            if constexpr (EPI == TC_SILU_MUL) {
+            if constexpr (tc_gated(EPI)) {
               uint32_t up[32];
               tmem_ld32(lane_addr + (uint32_t)(COLS + cb + 32 * h), up);
               asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
               for (int q = 0; q < 32; ++q) {
-                const float x = __uint_as_float(acc[q]);
-                v[q] = silu_fast(x) * __uint_as_float(up[q]);
+                const float x = __uint_as_float(acc[q]), y = __uint_as_float(up[q]);
+                v[q] = GROUPED ? tc_activation<EPI>(x, y, grp.glu) : silu_fast(x) * y;
               }
             } else {
               asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-              for (int q = 0; q < 32; ++q) v[q] = __uint_as_float(acc[q]);
+              for (int q = 0; q < 32; ++q) v[q] = tc_activation<EPI>(__uint_as_float(acc[q]), 0.f, grp.glu);
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -1074,11 +1094,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
           }
           asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-          epilogue_sync(1 + eg);
-          if (issuer) {
-            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n"
-                         ::"l"(&map_out), "r"(smem_u32(stage_out)), "r"(n0 + cb), "r"(m0) : "memory");
-            asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+          if (whole) {
+            epilogue_sync(1 + eg);
+            if (issuer) {
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n"
+                           ::"l"(&map_out), "r"(smem_u32(stage_out)), "r"(n0 + cb), "r"(m0) : "memory");
+              asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+            }
+          } else {
+            __syncwarp();  // (a warp copies the rows that it wrote itself)
+            constexpr int ITEM = EPI == TC_OUT_F32 ? 4 : 2;
+            const int chunk = lane & 7, col = n0 + cb + chunk * (16 / ITEM);
+#pragma unroll
+            for (int trip = 0; trip < 8; ++trip) {
+              const int rr = quad * 32 + 4 * trip + (lane >> 3);
+              if (m0 + rr < rows_end && col < N_out)
+                *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(out) + ((size_t)(m0 + rr) * N_out + col) * ITEM) =
+                    *reinterpret_cast<const uint4*>(stage_out + rr * 128 + ((chunk ^ (rr & 7)) << 4));
+            }
           }
           out_buf ^= 1;
         }
@@ -1126,6 +1159,21 @@ static int make_map(CUtensorMap* map, const void* base, long long rows, long lon
   const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
   const cuuint32_t elem[2] = {1, 1};
   const CUresult res = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  MS_CHECK_ARG(res == CUDA_SUCCESS, "gemm_tc: cuTensorMapEncodeTiled failed with code %d (rows=%lld cols=%lld)", (int)res, rows, cols);
+  return 0;
+}
+
+// A 2-D float32 tensor to store to, boxes of 128 rows x 32 columns.
+static int make_map_f32(CUtensorMap* map, const void* base, long long rows, long long cols) {
+  EncodeFn encode;
+  if (int rc = get_encode(&encode)) return rc;
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
+  const cuuint32_t box[2] = {32, (cuuint32_t)TC_BM};
+  const cuuint32_t elem[2] = {1, 1};
+  const CUresult res = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   MS_CHECK_ARG(res == CUDA_SUCCESS, "gemm_tc: cuTensorMapEncodeTiled failed with code %d (rows=%lld cols=%lld)", (int)res, rows, cols);
@@ -1226,7 +1274,32 @@ static int launch_tc_pair(void* out, const void* A, const void* W, int M, int N_
   MS_CHECK_ARG(tiles < (1LL << 30), "gemm_tc: too many tiles (%lld)", tiles);
   const long long pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
   MS_LAUNCH_CLUSTERED(kernel, (unsigned)(2 * pairs), PAIR_THREADS, smem, stream, 2, map_a, map_w, map_out, out, M, N_out, K,
-                      up_row_offset, status, qe);
+                      up_row_offset, status, qe, TcGroups{});
+  return 0;
+}
+
+// The grouped form of it (as launch_tc_grouped): up to max_tiles row tiles of 256, all pairs of SMs.
+template <int EPI>
+static int launch_tc_pair_grouped(void* out, const void* A, const void* W, int rows, int N_out, int matrices, int w_rows, int K, int up_row_offset,
+                                  const TcGroups& grp, int max_tiles, int* status, cudaStream_t stream) {
+  constexpr int BN = PAIR_BN, STAGES = 5, COLS = tc_gated(EPI) ? BN / 2 : BN;
+  CUtensorMap map_a, map_w, map_out;
+  if (int rc = make_map(&map_a, A, rows, K, TC_BM)) return rc;
+  if (int rc = make_map(&map_w, W, (long long)matrices * w_rows, K, BN / 2)) return rc;
+  map_out = map_a;  // (a valid map also when the kernel does not store through it)
+  if (N_out % 8 == 0 && (uintptr_t)out % 16 == 0) {
+    if (int rc = EPI == TC_OUT_F32 ? make_map_f32(&map_out, out, rows, N_out) : make_map(&map_out, out, rows, N_out, TC_BM)) return rc;
+  }
+  constexpr size_t smem = (size_t)STAGES * pair_stage_bytes(BN) + 4 * PAIR_OUT_BYTES + 1024;
+  static_assert(smem <= 227 * 1024, "the ring does not fit shared memory");
+  auto kernel = gemm_tc_pair_kernel<BN, STAGES, EPI, true>;
+  static std::atomic<unsigned long long> allowed{0};
+  MS_CHECK_CUDA(allow_shared_memory((const void*)kernel, (int)smem, allowed));
+  const long long tiles = (long long)ceil_div(N_out, COLS) * max_tiles, sms = sm_count();
+  MS_CHECK_ARG(tiles < (1LL << 30) && sms >= 2, "gemm_tc: too many tiles (%lld)", tiles);
+  const long long pairs = tiles < sms / 2 ? tiles : sms / 2;
+  MS_LAUNCH_CLUSTERED(kernel, (unsigned)(2 * pairs), PAIR_THREADS, smem, stream, 2, map_a, map_w, map_out, out, rows, N_out, K, up_row_offset, status,
+                      QkvEpilogue{}, grp);
   return 0;
 }
 
@@ -1383,9 +1456,10 @@ MS_EXPORT int ms_gemm_tc_bf16(void* out, const void* A, const void* W, int M, in
   }
 }
 
-// Rows per tile: 128, or 32 where an expert has a few rows (decode steps): then a CTA takes 64 columns of W, so that the weights are spread over
+// Rows per tile: 256, taken by pairs of CTAs, where the caller's plan has such tiles; 128; or 32 where an expert has a few rows (decode steps): then a CTA takes 64 columns of W, so that the weights are spread over
 // all SMs, and fetches 32 rows of A a stage.
-constexpr int TC_FEW_ROWS = 32;
+constexpr int TC_FEW_ROWS = 32, TC_PAIR_ROWS = 2 * TC_BM;
+// (Steps of many rows per expert are planned in tiles of 256: ops/experts.py has the line and both sides.)
 // Tiles of the grouped products of 128 rows: 1: 256 columns of W (gated) or 128, one CTA an SM; 2: 128, a shorter ring, two CTAs an SM, so that one CTA's
 // epilogue hides behind the other's products. 0: chosen from the rows per expert (measured on B200 with 16 experts, both products: 2,048 tokens x 3
 // choices at 768 of 1024: 75.6 us with 2, 87.7 with 1; at 1536 of 2048: 182 against 202; 8 tokens: 39.5 against 35.6 and 94 against 65).
@@ -1395,6 +1469,7 @@ MS_EXPORT void ms_gemm_tc_set_grouped(int config) { g_grouped_config = config; }
 template <int EPI>
 static int launch_grouped_gated(void* out, const void* A, const void* W, int rows, int N, int experts, int K, const TcGroups& grp, int tile_rows,
                                 int max_tiles, int* status, cudaStream_t stream) {
+  if (tile_rows == TC_PAIR_ROWS) return launch_tc_pair_grouped<EPI>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
   if (tile_rows == TC_FEW_ROWS) return launch_tc_grouped<64, 7, EPI, TC_FEW_ROWS>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
   const bool narrow = g_grouped_config ? g_grouped_config == 2 : rows >= 128 * experts;
   if (narrow) return launch_tc_grouped<128, 3, EPI>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
@@ -1404,13 +1479,14 @@ static int launch_grouped_gated(void* out, const void* A, const void* W, int row
 template <int EPI>
 static int launch_grouped_plain(void* out, const void* A, const void* W, int rows, int N, int experts, int K, const TcGroups& grp, int tile_rows,
                                 int max_tiles, int* status, cudaStream_t stream) {
+  if (tile_rows == TC_PAIR_ROWS) return launch_tc_pair_grouped<EPI>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
   if (tile_rows == TC_FEW_ROWS) return launch_tc_grouped<64, 7, EPI, TC_FEW_ROWS>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
   const bool narrow = g_grouped_config ? g_grouped_config == 2 : rows >= 128 * experts;
   if (narrow) return launch_tc_grouped<128, 3, EPI>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
   return launch_tc_grouped<128, 5, EPI>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
 }
 
-// The experts' products of a routed feed-forward over rows sorted by expert (tiles of 128 or 32 rows, (expert, first row)
+// The experts' products of a routed feed-forward over rows sorted by expert (tiles of 256, 128 or 32 rows, (expert, first row)
 // each; meta[0] tiles; offsets[e + 1] ends expert e's rows; at most max_tiles tiles).
 // gated = 1: W [E, 2 N, K] (an expert's gate rows, then its up rows), out [rows, N] bfloat16 = silu(A gate^T) * (A up^T);
 // gated = 0: W [E, N, K], out [rows, N] float32 = A W^T; gated = 2: W [E, N, K], out [rows, N] bfloat16 = relu(A W^T)^2;
@@ -1423,7 +1499,7 @@ MS_EXPORT int ms_gemm_tc_experts_bf16(void* out, const void* A, const void* W, i
   MS_CHECK_ARG(K % 8 == 0, "gemm_tc_experts: K=%d must be a multiple of 8 (rows must be 16-byte multiples for TMA)", K);
   MS_CHECK_ARG(((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0), "gemm_tc_experts: operands must be 16-byte aligned");
   MS_CHECK_ARG(status != nullptr && tiles != nullptr && meta != nullptr && offsets != nullptr, "gemm_tc_experts: needs a plan and a status word");
-  MS_CHECK_ARG(tile_rows == TC_BM || tile_rows == TC_FEW_ROWS, "gemm_tc_experts: tiles of %d rows", tile_rows);
+  MS_CHECK_ARG(tile_rows == TC_BM || tile_rows == TC_FEW_ROWS || tile_rows == TC_PAIR_ROWS, "gemm_tc_experts: tiles of %d rows", tile_rows);
   MS_CHECK_ARG(max_tiles <= 65535, "gemm_tc_experts: %d row tiles are too many for one launch", max_tiles);
   MS_CHECK_ARG((long long)experts * (gated == 1 || gated == 3 ? 2 : 1) * N < (1LL << 31), "gemm_tc_experts: the weights have too many rows");
   if (gated == 3) {

@@ -15,6 +15,7 @@ NO_CLAMPS = (-1.0, 1.0, 0.0)  # (limit, alpha, shift) of a clamped GLU; other ac
 SCORES = {"softmax": 0, "sigmoid": 1}
 TILE_ROWS = 64       # sorted rows per tile of the float32 and mma.sync products
 TC_TILE_ROWS = 128   # of the products on the tcgen05 tensor cores
+TC_PAIR_ROWS = 256   # of the same by pairs of CTAs
 TC_FEW_ROWS = 32     # of the same where an expert has a few rows (decode steps)
 TC_EXPERTS = os.environ.get("MINISERVE_TC_EXPERTS", "1") != "0"  # bfloat16 experts on the tcgen05 kernel where it takes the shape
 
@@ -28,10 +29,16 @@ def tc_experts_ok(dtype, hidden: int, inter: int, activation: str) -> bool:
 
 def tc_tile_rows(slots: int, experts: int) -> int:
     """Rows per tile of the tcgen05 products for a step of ``slots`` (token, choice) pairs."""
-    return TC_FEW_ROWS if slots <= FEW_ROWS_PER_EXPERT * experts else TC_TILE_ROWS
+    if slots <= FEW_ROWS_PER_EXPERT * experts:
+        return TC_FEW_ROWS
+    return TC_PAIR_ROWS if slots >= PAIR_ROWS_PER_EXPERT * experts else TC_TILE_ROWS
 
 
 FEW_ROWS_PER_EXPERT = 16  # up to so many rows per expert on average: tiles of TC_FEW_ROWS
+# From so many on: tiles of TC_PAIR_ROWS. Both products, one B200, 14 experts of 1536 at width 2048 and of 768 at 1024, us with tiles of 128 / 256
+# rows: 73 rows per expert 86.5 / 83.0 and 41 / 49, 114 rows 89.3 / 77.2 and 42.0 / 42.4, 200 rows 107.5 / 80.3 and 47.4 / 37.9, 543 rows
+# 175.7 / 122.4 and 73.7 / 49.3; 128 experts of 768 at 2048, 119 rows: 339 / 309.
+PAIR_ROWS_PER_EXPERT = 112
 
 
 def expert_route(idx, wgt, x, router, correction, top: int, group_count: int, group_keep: int, weight_scale: float,

@@ -754,3 +754,33 @@ def test_a_wait_that_nothing_answers_gives_up_raises_the_status_word_and_leaves_
     ids = torch.arange(5, device=DEV, dtype=torch.int32)
     ops.embed_gather(out, table, ids)
     assert torch.equal(out, table[:5])
+
+
+@pytest.mark.parametrize("n, k", [(128, 64), (200, 72), (72, 136), (392, 320)])
+@pytest.mark.parametrize("counts", [[256, 128, 512], [0, 1, 127, 129, 0, 255, 257, 640, 300], [700], [0, 0, 130]])
+@pytest.mark.parametrize("mode", ["silu", "clamped", "relu2", "plain"])
+def test_grouped_products_by_pairs_of_ctas(n, k, counts, mode):
+    """Tiles of 256 sorted rows against tiles of 128 (which the models' tests hold against the oracle): the same sums in the same
+    order. Runs that end inside a tile, inside its first half and at its edge; widths that are no whole tiles; rows of no run stay as they are."""
+    from miniserve_b200.ops import experts as xo
+
+    torch.manual_seed(n + len(counts))
+    e, gated = len(counts), mode in ("silu", "clamped")
+    rows = sum(counts) + 40  # (the last 40 slots chose no expert with tensors)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    idx = torch.tensor(sum(([i] * c for i, c in enumerate(counts)), []) + [e] * 40, **i32)[torch.randperm(rows, device=DEV)].view(-1, 1).contiguous()
+    a = torch.randn(rows, k, device=DEV).bfloat16()
+    w = (torch.randn(e, (2 if gated else 1) * n, k, device=DEV) * k ** -0.5).bfloat16()
+    outs = []
+    for tile_rows in (xo.TC_TILE_ROWS, xo.TC_PAIR_ROWS):
+        pos, perm, offsets = torch.empty(rows, **i32), torch.empty(rows, **i32), torch.empty(e + 1, **i32)
+        tiles, meta = torch.empty(xo.expert_max_tiles(rows, e, tile_rows), 2, **i32), torch.empty(2, **i32)
+        xo.expert_plan(pos, perm, offsets, tiles, meta, idx, e, tile_rows=tile_rows)
+        assert meta.tolist() == [sum(-(-c // tile_rows) for c in counts), sum(counts)]
+        out = torch.full((rows, n), 32768.0, device=DEV, dtype=torch.float32 if mode == "plain" else torch.bfloat16)
+        xo.expert_products_tc(out, a, w, tiles, meta, offsets, gated, relu_squared=mode == "relu2",
+                              clamps=(2.0, 1.7, 1.0) if mode == "clamped" else None, tile_rows=tile_rows)
+        outs.append(out)
+    torch.cuda.synchronize()
+    assert ops.device_status("cuda").item() == 0
+    assert torch.equal(outs[0], outs[1]) and not torch.any(outs[1][:sum(counts)] == 32768.0) and torch.all(outs[1][sum(counts):] == 32768.0)
