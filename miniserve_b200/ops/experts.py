@@ -4,6 +4,7 @@
 from __future__ import annotations
 
 import os
+from functools import lru_cache
 
 import torch
 
@@ -109,6 +110,44 @@ def expert_products_tc(out, a, w, tiles, meta, offsets, gated: bool, stream=None
                                                     _ptr(offsets), tile_rows, expert_max_tiles(slots, e, tile_rows), *map(float, clamps or NO_CLAMPS),
                                                     _ptr(device_status(a.device)), _stream(stream)),
                         lib=lib, errfn="ms_gemm_tc_last_error")
+
+
+@lru_cache(maxsize=1024)
+def _work_bytes(*sizes) -> int:
+    return int(native.experts().ms_experts_work_bytes(*sizes))
+
+
+def experts_forward(x, ctx, router, correction, logit_bias, gate_w, gate_out, w_up, w_down, shared, top: int, group_count: int, group_keep: int,
+                    group_best: int, weight_scale: float, renormalize: bool, score: str, square_weights: bool, renorm_eps: float, gated: bool,
+                    relu_squared: bool, clamps) -> torch.Tensor:
+    """A routed feed-forward in bfloat16 whose products run on the tcgen05 kernels (``tc_experts_ok``): ``expert_route``, ``expert_plan``,
+    ``expert_gather``, ``expert_products_tc`` twice and ``expert_combine`` in one native call over one piece of scratch. Operands as theirs;
+    ``shared`` [T, H], with ``gate_out`` (and ``gate_w``) its factor per token."""
+    from . import device_status
+
+    t, hidden = x.shape
+    e, w_rows, k = w_up.shape
+    inter, r = w_rows // 2 if gated else w_rows, router.shape[0]
+    _f32(router, correction, logit_bias, gate_w, gate_out)
+    assert x.dtype == w_up.dtype == w_down.dtype == torch.bfloat16 and k == hidden and w_down.shape == (e, hidden, inter)
+    assert w_up.is_contiguous() and w_down.is_contiguous() and router.shape == (r, hidden)
+    assert (correction is None or correction.numel() == r) and (logit_bias is None or logit_bias.numel() == r)
+    assert (gate_w is None) == (gate_out is None) and (gate_w is None or (gate_w.numel() == hidden and gate_out.numel() >= t))
+    assert shared is None or (shared.shape == (t, hidden) and shared.dtype == x.dtype and shared.is_contiguous())
+    slots = t * top
+    tile_rows = tc_tile_rows(slots, e)
+    out = ctx.buffer("moe.out", (t, hidden), x.dtype, x.device)
+    work = ctx.buffer("moe.work", (_work_bytes(slots, e, hidden, inter, tile_rows),), torch.uint8, x.device)
+    mode = 2 if relu_squared else (3 if clamps is not None else 1) if gated else 0
+    rc = native.experts().ms_experts_forward(
+        out.data_ptr(), x.data_ptr(), _rows(x), router.data_ptr(), _ptr(correction), _ptr(logit_bias), _ptr(gate_w), _ptr(gate_out), w_up.data_ptr(),
+        w_down.data_ptr(), _ptr(shared), work.data_ptr(), native.experts_products(), device_status(x.device).data_ptr(), t, hidden, inter, r, e, top,
+        group_count, group_keep, group_best, renormalize, SCORES[score], square_weights, mode, tile_rows, weight_scale, renorm_eps,
+        *(clamps or NO_CLAMPS), ctx.stream)
+    if rc == 2:
+        native.kernel_check(rc, lib=native.gemm_tc(), errfn="ms_gemm_tc_last_error")
+    native.experts_check(rc, launches=6)
+    return out
 
 
 def expert_gate_up(out, x, w_gate_up, perm, top: int, tiles, meta, offsets, activation: str, stream=None, clamps=None) -> None:

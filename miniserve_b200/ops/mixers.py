@@ -434,6 +434,37 @@ def ssm_step_decay(out, raw, bias, coef, stream=None) -> None:
                                                                   _dt(raw.dtype), _stream(stream)))
 
 
+@lru_cache(maxsize=256)
+def _ssm_floats(*sizes) -> int:
+    return int(native.recurrence().ms_ssm_work(*sizes))
+
+
+def ssm_features(out, proj, state, conv_state, w_conv, conv_bias, dt_bias, coef, skip, norm, ctx, heads: int, dv: int, n: int, groups: int,
+                 conv_unit: int, norm_parts: int, eps: float, exact: bool) -> bool:
+    """A selective state-space layer between its projections in one native call: ``conv_silu_unit`` (with its update), ``ssm_step_decay``,
+    ``decay_scan`` and ``gated_group_norm`` over ``proj`` [T, >= 2 heads dv + 2 groups n + heads], the columns z | x | B | C | raw dt. Steps of
+    single tokens, and the steps that ``decay_scan`` walks by chunks; for others nothing is done and False comes back."""
+    t = proj.shape[0]
+    inner, taps = heads * dv, w_conv.shape[1]
+    channels = inner + 2 * groups * n
+    decode = ctx.decode_only and n % 4 == 0
+    if not decode and (exact or ctx.decode_only or t < WALK_MIN_TOKENS or ctx.num_rows > 65535 or n not in (32, 64, 128) or inner % 4):
+        return False  # (as walk_ok has it: B and C are runs of whole fours of one buffer's rows)
+    _f32(state, w_conv, conv_bias, dt_bias, coef, skip, norm)
+    assert state.shape[1:] == (heads, dv, n) and w_conv.shape[0] == channels and out.shape == (t, inner) and out.dtype == proj.dtype
+    assert conv_bias.numel() == channels and dt_bias.numel() == coef.numel() == skip.numel() == heads and norm.numel() == inner
+    assert conv_state is None or (conv_state.shape[1:] == (taps - 1, channels) and conv_state.dtype == proj.dtype and conv_state.is_contiguous())
+    assert conv_state is not None or taps == 1
+    work = ctx.buffer("ssm.work", (_ssm_floats(t, heads, dv, n, groups),), torch.float32, proj.device)
+    walk = None if decode else ctx.buffer("walk.scratch", (_walk_floats(t, ctx.num_rows, heads, n, dv, False, True),), torch.float32, proj.device)
+    native.recurrence_check(native.recurrence().ms_ssm_features(
+        out.data_ptr(), _rows(out), proj.data_ptr(), _rows(proj), work.data_ptr(), _ptr(walk), state.data_ptr(), _ptr(conv_state), w_conv.data_ptr(),
+        conv_bias.data_ptr(), dt_bias.data_ptr(), coef.data_ptr(), skip.data_ptr(), norm.data_ptr(), ctx.row_of_token.data_ptr(), ctx.cu_q.data_ptr(),
+        ctx.q_start.data_ptr(), ctx.state_slot.data_ptr(), t, ctx.num_rows, heads, dv, n, groups, taps, conv_unit, norm_parts, decode, eps,
+        _dt(proj.dtype), ctx.stream), launches=4 if decode else 5 + (conv_state is not None))
+    return True
+
+
 def gated_group_norm(out, o, x, skip, gate, weight, parts: int, dv: int, eps: float, stream=None) -> None:
     """y = (o + skip[head] * x) * silu(gate) over the ``width`` channels of a token (head = channel // dv), then each of
     ``parts`` equal parts of y divided by its own root mean square, times ``weight`` [width]. ``o`` [T, width] float32;

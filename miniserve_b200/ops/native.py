@@ -174,6 +174,8 @@ def recurrence():
     _declare(lib, "ms_conv_silu_unit", [_p, _p, _i, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p, _i, _i, _p])
     _declare(lib, "ms_ssm_step_decay", [_p, _p, _i, _p, _p, _i, _i, _i, _p])
     _declare(lib, "ms_gated_group_norm", [_p, _i, _p, _p, _i, _p, _p, _i, _p, _i, _i, _i, _i, _f, _i, _p])
+    _declare(lib, "ms_ssm_work", [_i] * 5, _ll)
+    _declare(lib, "ms_ssm_features", [_p, _i, _p, _i] + [_p] * 14 + [_i] * 10 + [_f, _i, _p])
     _declare(lib, "ms_conv_state_update", [_p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _p])
     _declare(lib, "ms_head_norm_gate", [_p, _i, _p, _p, _p, _i, _i, _i, _i, _f, _f, _i, _i, _i, _p])
     _declare(lib, "ms_mlstm_gates", [_p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _f, _i, _i, _p])
@@ -208,7 +210,15 @@ def experts():
     _declare(lib, "ms_expert_gather", [_p, _p, _i, _p, _p, _i, _i, _i, _p])
     _declare(lib, "ms_expert_gemm", [_p, _p, _i, _p, _i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _f, _f, _i, _p])
     _declare(lib, "ms_expert_combine", [_p, _p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p, _p])
+    _declare(lib, "ms_experts_work_bytes", [_i] * 5, _ll)
+    _declare(lib, "ms_experts_forward", [_p, _p, _i] + [_p] * 11 + [_i] * 14 + [_f] * 5 + [_p])
     return lib
+
+
+@lru_cache(maxsize=None)
+def experts_products() -> int:
+    """The address of the grouped products' launcher, for the experts' library to call."""
+    return ctypes.cast(gemm_tc().ms_gemm_tc_experts_bf16, c_void_p).value
 
 
 def experts_check(rc: int, launches: int = 1) -> None:

@@ -258,6 +258,7 @@ class SelectiveStateSpace(Part):
         if self.taps < 1:
             raise ValueError(f"the convolution needs at least one tap, got {self.taps}")
         self.channels = self.inner + 2 * self.groups * self.n  # what passes the convolution: x | B | C
+        self.conv_unit = _conv_unit(self.channels)
         self.proj_rows = 2 * self.inner + 2 * self.groups * self.n + self.heads
         self.feature_width = self.inner
 
@@ -294,10 +295,13 @@ class SelectiveStateSpace(Part):
         h, g, n, dv, c, inner = self.heads, self.groups, self.n, self.dv, self.channels, self.inner
         state, conv = (cache if isinstance(cache, tuple) else (cache, None))
         proj = ops.linear(x, self.w_in, stream=ctx.stream, out=ctx.buffer("ssm.in", (t, self.w_in.shape[0]), dt, dev))
+        unit = self.conv_unit
+        if ops.ssm_features(out, proj, state.state, None if conv is None else conv.state, self.w_conv, self.w_conv_bias, self.w_dt_bias, self.decay_coef,
+                            self.w_skip, self.w_norm, ctx, h, dv, n, g, unit, self.norm_groups, self.eps, dt == torch.float32):
+            return
         xbc_in = proj[:, inner:inner + c]
         xbc = ctx.buffer("ssm.xbc", (t, c), torch.float32, dev)
         conv_state = conv.state if conv is not None else ctx.buffer("ssm.noconv", (1, 0, c), dt, dev)
-        unit = _conv_unit(c)
         ops.conv_silu_unit(xbc, xbc_in, conv_state, self.w_conv, ctx, 0, 1, c // unit, unit, 0.0, bias=self.w_conv_bias,
                            update=conv is not None)
         steps = ctx.buffer("ssm.dt", (2, t, h), torch.float32, dev)  # step sizes, then decays

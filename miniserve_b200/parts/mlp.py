@@ -316,32 +316,30 @@ class RoutedExperts(Part):
 
     def forward(self, x, ctx) -> torch.Tensor:
         t, dt, dev = x.shape[0], self.env.dtype, self.w_down.device
+        # bfloat16: both products on the tcgen05 kernel where it has the activation, over the tokens' inputs gathered into sorted order
+        if ops.experts.tc_experts_ok(dt, self.hidden, self.inter, self.activation) and x.stride(0) % 8 == 0:
+            shared = self.shared.forward(x, ctx) if self.shared is not None else None
+            gate = ctx.buffer("moe.shared_gate", (t,), torch.float32, dev) if self.shared_gated else None
+            return ops.experts.experts_forward(
+                x, ctx, self.w_router, self.w_correction, self.w_router_bias, self.w_shared_gate, gate, self.w_gate_up, self.w_down, shared, self.top,
+                self.group_count, self.group_keep, min(self.group_best, self.outputs // self.group_count), self.weight_scale, self.renormalize,
+                self.score, self.weigh == "input", self.renorm_eps, self.gated, not self.gated, self.clamps)
         slots, i32 = t * self.top, torch.int32
         idx, wgt = self.route(x, ctx)
         pos = ctx.buffer("moe.pos", (slots,), i32, dev)
         perm = ctx.buffer("moe.perm", (slots,), i32, dev)
         offsets = ctx.buffer("moe.offsets", (self.experts + 1,), i32, dev)
-        # bfloat16: both products on the tcgen05 kernel where it has the activation, over the tokens' inputs gathered into sorted order
-        tc = ops.experts.tc_experts_ok(dt, self.hidden, self.inter, self.activation) and x.stride(0) % 8 == 0
-        tile_rows = ops.experts.tc_tile_rows(slots, self.experts) if tc else ops.experts.TILE_ROWS
-        tiles = ctx.buffer("moe.tiles", (ops.experts.expert_max_tiles(slots, self.experts, tile_rows), 2), i32, dev)
+        tiles = ctx.buffer("moe.tiles", (ops.experts.expert_max_tiles(slots, self.experts), 2), i32, dev)
         meta = ctx.buffer("moe.meta", (2,), i32, dev)
-        ops.experts.expert_plan(pos, perm, offsets, tiles, meta, idx, self.experts, stream=ctx.stream, tile_rows=tile_rows)
+        ops.experts.expert_plan(pos, perm, offsets, tiles, meta, idx, self.experts, stream=ctx.stream)
         act = ctx.buffer("moe.act", (slots, self.inter), dt, dev)
         y = ctx.buffer("moe.y", (slots, self.hidden), torch.float32, dev)
-        if tc:
-            xs = ctx.buffer("moe.xs", (slots, self.hidden), dt, dev)
-            ops.experts.expert_gather(xs, x, perm, meta, self.top, stream=ctx.stream)
-            ops.experts.expert_products_tc(act, xs, self.w_gate_up, tiles, meta, offsets, self.gated, stream=ctx.stream,
-                                           relu_squared=not self.gated, clamps=self.clamps, tile_rows=tile_rows)
-            ops.experts.expert_products_tc(y, act, self.w_down, tiles, meta, offsets, False, stream=ctx.stream, tile_rows=tile_rows)
+        if self.gated:
+            ops.experts.expert_gate_up(act, x, self.w_gate_up, perm, self.top, tiles, meta, offsets, self.activation, stream=ctx.stream,
+                                       clamps=self.clamps)
         else:
-            if self.gated:
-                ops.experts.expert_gate_up(act, x, self.w_gate_up, perm, self.top, tiles, meta, offsets, self.activation, stream=ctx.stream,
-                                           clamps=self.clamps)
-            else:
-                ops.experts.expert_up(act, x, self.w_gate_up, perm, self.top, tiles, meta, offsets, self.activation, stream=ctx.stream)
-            ops.experts.expert_down(y, act, self.w_down, tiles, meta, offsets, stream=ctx.stream)
+            ops.experts.expert_up(act, x, self.w_gate_up, perm, self.top, tiles, meta, offsets, self.activation, stream=ctx.stream)
+        ops.experts.expert_down(y, act, self.w_down, tiles, meta, offsets, stream=ctx.stream)
         out = ctx.buffer("moe.out", (t, self.hidden), dt, dev)
         shared = self.shared.forward(x, ctx) if self.shared is not None else None
         gate = ctx.buffer("moe.shared_gate", (t,), torch.float32, dev) if self.shared_gated else None  # written by the router's kernel

@@ -119,3 +119,74 @@ def test_float32_convolutions_of_a_token_are_the_same_bits_in_any_step(c, unit, 
         ops.conv_silu_unit(out, x[:n], state, w, _rows((n,), (0,)), unit, dk, c // dk - unit, dk, 1e-6)
         outs.append(out)
     assert all(torch.equal(o, outs[0][:o.shape[0]]) for o in outs)
+
+
+def _held(ctx, decode):
+    kept = {}
+    ctx.decode_only, ctx.step_cache = decode, {}
+    ctx.buffer = lambda role, shape, dtype, dev: kept.setdefault((role, shape, dtype), torch.empty(shape, dtype=dtype, device=dev))
+    return ctx
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, dv, n, groups, taps, parts", [(4, 32, 64, 2, 4, 2), (6, 20, 20, 3, 1, 1), (3, 7, 32, 1, 3, 1), (8, 64, 128, 8, 2, 4), (2, 6, 18, 1, 4, 1)])
+@pytest.mark.parametrize("lens, started", [((1, 1, 1), (0, 3, 1)), ((5, 1, 8, 40), (0, 9, 2, 1)), ((3, 2), (1, 0))])
+def test_state_space_features_in_one_call(dtype, heads, dv, n, groups, taps, parts, lens, started):
+    """The one native call against the single ones, bit for bit, and only for the steps that it takes."""
+    gen = torch.Generator().manual_seed(heads + taps)
+    t, inner, decode = sum(lens), heads * dv, all(k == 1 for k in lens)
+    c = inner + 2 * groups * n
+    proj = torch.randn(t, -(-(inner + c + heads) // 8) * 8, generator=gen).to(dtype).to(DEV)
+    f = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)  # noqa: E731
+    w_conv, conv_bias, dt_bias, coef, skip, norm = f(c, taps), f(c), f(heads), f(heads).exp(), f(heads), f(inner)
+    state, conv = f(len(lens), heads, dv, n), f(len(lens), taps - 1, c).to(dtype)
+    unit = max(u for u in range(1, 129) if c % u == 0)
+    ctx = _held(_rows(lens, started), decode)
+    ctx.leading_single_rows, ctx.sm_count = next((i for i, k in enumerate(lens) if k != 1), len(lens)), 148
+    exact = dtype == torch.float32
+    out = torch.full((t, inner), float("nan"), dtype=dtype, device=DEV)
+    got_state, got_conv = state.clone(), conv.clone()
+    taken = ops.ssm_features(out, proj, got_state, got_conv if taps > 1 else None, w_conv, conv_bias, dt_bias, coef, skip, norm, ctx, heads, dv, n, groups, unit,
+                             parts, 1e-6, exact)
+    assert taken == ((decode and n % 4 == 0) or (not decode and not exact and t >= 16 and n in (32, 64, 128) and inner % 4 == 0))
+    if not taken:
+        assert torch.equal(got_state, state) and torch.equal(got_conv, conv)
+        return
+    xbc, steps, o, want = f(t, c), f(2, t, heads), f(t, heads, dv), torch.full((t, inner), float("nan"), dtype=dtype, device=DEV)
+    ops.conv_silu_unit(xbc, proj[:, inner:inner + c], conv, w_conv, ctx, 0, 1, c // unit, unit, 0.0, bias=conv_bias, update=taps > 1)
+    ops.ssm_step_decay(steps, proj[:, inner + c:inner + c + heads], dt_bias, coef)
+    xs, bs, cs = torch.split_with_sizes(xbc, (inner, groups * n, groups * n), 1)
+    ops.decay_scan(o, state, cs, bs, xs, steps[1], None, coef, 1.0, None, ctx, heads, n, dv, 1.0, delta=False, head_decay=True, v_scale=steps[0], exact=exact)
+    ops.gated_group_norm(want, o.view(t, inner), xs, skip, proj[:, :inner], norm, parts, dv, 1e-6)
+    assert torch.equal(out, want) and torch.equal(got_state, state) and torch.equal(got_conv, conv)
+
+
+@pytest.mark.parametrize("t, hidden, inter, experts, extra, top, kind", [(1, 64, 40, 5, 1, 2, "gated"), (9, 72, 64, 12, 0, 3, "clamped"), (300, 64, 48, 4, 2, 2, "plain"),
+                                                                        (40, 128, 136, 3, 1, 1, "shared")])
+def test_routed_feed_forward_in_one_call(t, hidden, inter, experts, extra, top, kind):
+    from miniserve_b200.ops import experts as xo
+
+    gen = torch.Generator().manual_seed(t)
+    f = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)  # noqa: E731
+    r, gated = experts + extra, kind != "plain"
+    x, router, correction = f(t, hidden).bfloat16(), f(r, hidden) * hidden ** -0.5, f(r) * 0.01
+    w_up, w_down = (f(experts, (2 if gated else 1) * inter, hidden) * hidden ** -0.5).bfloat16(), (f(experts, hidden, inter) * inter ** -0.5).bfloat16()
+    clamps = (2.0, 1.7, 1.0) if kind == "clamped" else None
+    shared, gate_w = (f(t, hidden).bfloat16(), f(hidden)) if kind == "shared" else (None, None)
+    gates = [None if gate_w is None else torch.empty(t, device=DEV) for _ in range(2)]
+    ctx = _held(_rows((t,), (0,)), False)
+    got = xo.experts_forward(x, ctx, router, correction, None, gate_w, gates[0], w_up, w_down, shared, top, 1, 1, 1, 1.5, True, "softmax", False, 0.0, gated,
+                             not gated, clamps)
+    slots, i32 = t * top, dict(dtype=torch.int32, device=DEV)
+    rows = xo.tc_tile_rows(slots, experts)
+    idx, wgt, pos, perm, offsets = torch.empty(t, top, **i32), f(t, top), torch.empty(slots, **i32), torch.empty(slots, **i32), torch.empty(experts + 1, **i32)
+    tiles, meta = torch.empty(xo.expert_max_tiles(slots, experts, rows), 2, **i32), torch.empty(2, **i32)
+    xs, act, y, want = torch.zeros(slots, hidden, dtype=x.dtype, device=DEV), torch.empty(slots, inter, dtype=x.dtype, device=DEV), f(slots, hidden), torch.empty_like(x)
+    xo.expert_route(idx, wgt, x, router, correction, top, 1, 1, 1.5, True, gate_w=gate_w, gate_out=gates[1])
+    xo.expert_plan(pos, perm, offsets, tiles, meta, idx, experts, tile_rows=rows)
+    xo.expert_gather(xs, x, perm, meta, top)
+    xo.expert_products_tc(act, xs, w_up, tiles, meta, offsets, gated, relu_squared=not gated, clamps=clamps, tile_rows=rows)
+    xo.expert_products_tc(y, act, w_down, tiles, meta, offsets, False, tile_rows=rows)
+    xo.expert_combine(want, y, x, idx, wgt, pos, experts, shared=shared, shared_gate=gates[1])
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and ops.device_status("cuda").item() == 0 and (gate_w is None or torch.equal(*gates))
