@@ -24,7 +24,7 @@
 
 namespace ms {
 
-constexpr int TC_BM = 128, TC_BK = 64;
+constexpr int TC_BM = 128, TC_BK = 64, TC_FEW_ROWS = 32;
 constexpr int TC_THREADS = 192;
 
 enum TcEpilogue : int { TC_OUT_BF16 = 0, TC_OUT_F32 = 1, TC_SILU_MUL = 2, TC_QKV_ROPE = 3, TC_RELU2 = 4, TC_CLAMPED_GLU = 5 };
@@ -168,8 +168,8 @@ struct TcGroups {
 // (gate rows, then up rows), BN is 256 and a CTA computes 128 gate and the matching 128 up columns.
 // GROUPED: blockIdx.y walks the plan's row tiles instead (the grid has as many as a step can have at most, the
 // surplus CTAs leave at once); a tile's rows beyond its run are computed with the run's matrix and not stored.
-template <int BN, int STAGES, int EPI, bool GROUPED = false, int AROWS = TC_BM>
-__global__ void __launch_bounds__(TC_THREADS, (STAGES * (AROWS + BN) * TC_BK * 2 + (TC_BM - AROWS) * TC_BK * 2 + 2048 <= 112 * 1024) ? 2 : 1)
+template <int BN, int STAGES, int EPI, bool GROUPED = false>
+__global__ void __launch_bounds__(TC_THREADS, STAGES * TcSmem<BN>::stage_bytes + 2048 <= 112 * 1024 ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, void* __restrict__ out,
                int M, int N_out, int K, int up_row_offset, int* __restrict__ status, const TcGroups grp) {
   extern __shared__ unsigned char smem_dyn[];
@@ -190,7 +190,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if ((int)blockIdx.y >= grp.meta[0]) return;
     const int e = grp.tiles[2 * blockIdx.y];
     m0 = grp.tiles[2 * blockIdx.y + 1];
-    M = min(min(M, grp.offsets[e + 1]), m0 + AROWS);
+    M = min(min(M, grp.offsets[e + 1]), m0 + TC_BM);
     w0 = e * grp.w_rows + n0;
   }
   const int k_iters = (K + TC_BK - 1) / TC_BK;
@@ -227,13 +227,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           gave_up = 1;
           break;
         }
-        unsigned char* a_tile = smem + (size_t)s * TcSmem<BN, AROWS>::stage_bytes;
-        unsigned char* b_tile = a_tile + TcSmem<BN, AROWS>::a_bytes;
-        mbar_expect_tx(&full_bar[s], TcSmem<BN, AROWS>::stage_bytes);
+        unsigned char* a_tile = smem + (size_t)s * TcSmem<BN>::stage_bytes;
+        unsigned char* b_tile = a_tile + TcSmem<BN>::a_bytes;
+        mbar_expect_tx(&full_bar[s], TcSmem<BN>::stage_bytes);
         tma_load_2d(a_tile, &map_a, &full_bar[s], it * TC_BK, m0);
         if (tc_gated(EPI)) {
           tma_load_2d(b_tile, &map_w, &full_bar[s], it * TC_BK, w0);
-          tma_load_2d(b_tile + TcSmem<BN, AROWS>::b_bytes / 2, &map_w, &full_bar[s], it * TC_BK, up_row_offset + w0);
+          tma_load_2d(b_tile + TcSmem<BN>::b_bytes / 2, &map_w, &full_bar[s], it * TC_BK, up_row_offset + w0);
         } else {
           tma_load_2d(b_tile, &map_w, &full_bar[s], it * TC_BK, w0);
         }
@@ -252,8 +252,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const unsigned char* a_tile = smem + (size_t)s * TcSmem<BN, AROWS>::stage_bytes;
-        const unsigned char* b_tile = a_tile + TcSmem<BN, AROWS>::a_bytes;
+        const unsigned char* a_tile = smem + (size_t)s * TcSmem<BN>::stage_bytes;
+        const unsigned char* b_tile = a_tile + TcSmem<BN>::a_bytes;
         const uint64_t da = make_smem_desc(a_tile), db = make_smem_desc(b_tile);
 #pragma unroll
         for (int k = 0; k < TC_BK / 16; ++k) {
@@ -506,6 +506,142 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(2 * ACC_COLS) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------- grouped products of a few rows per matrix
+// The grouped form for decode steps (tiles of 32 sorted rows): a stream of weights, so the CTAs stay. Two CTAs an SM walk the plan's row tiles
+// x 64 columns of W, each with a ring that keeps running from one tile into the next and two accumulators, so that neither a tile's start nor
+// its end leaves the memory idle. Both products of 8 tokens x 4 choices, 14 experts, us: of 1536 at width 2048 60.7 with a CTA per tile, two an
+// SM (4.4 TB/s of weights), 55.2 with one CTA an SM that stays, 16 stages, 52.3 with two, 8 stages each (5.05 TB/s); of 768 at 1024 25.1 / 23.5 /
+// 21.4; 128 experts of 768 at 2048 98 / 82 / 79. Stages of 8 or 16 rows of A instead of 32 are no faster: the weights bound it.
+constexpr int FEW_THREADS = 96, FEW_BN = 64, FEW_STAGES = 8, FEW_CTAS = 2;  // warp 0: the epilogue (a tile's rows are tensor-memory lanes 0 .. 31, warp 0's), 1: MMA, 2: TMA
+template <int STAGES, int EPI>
+__global__ void __launch_bounds__(FEW_THREADS, FEW_CTAS)
+gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, void* __restrict__ out,
+                   int M, int N_out, int K, int up_row_offset, int* __restrict__ status, const TcGroups grp) {
+  constexpr int AROWS = TC_FEW_ROWS, BN = FEW_BN, COLS = tc_gated(EPI) ? BN / 2 : BN;
+  using S = TcSmem<BN, AROWS>;
+  extern __shared__ unsigned char smem_dyn[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base_slot;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k_iters = (K + TC_BK - 1) / TC_BK, n_tiles = (N_out + COLS - 1) / COLS;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base_slot)), "r"(2u * BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem_base = tmem_base_slot;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int num_tiles = grp.meta[0] * n_tiles;  // (the plan is an earlier kernel's)
+
+  if (warp == 2) {
+    if (elect_one()) {
+      int kb = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        const int n0 = (tile % n_tiles) * COLS, at = tile / n_tiles;
+        const int w0 = grp.tiles[2 * at] * grp.w_rows + n0, m0 = grp.tiles[2 * at + 1];
+        for (int it = 0; it < k_iters; ++it, ++kb) {
+          const int s = kb % STAGES;
+          if (kb >= STAGES && !mbar_wait(&empty_bar[s], ((kb / STAGES) - 1) & 1)) {
+            atomicExch(status, 11);
+            ok = false;
+            break;
+          }
+          unsigned char* a_tile = smem + (size_t)s * S::stage_bytes;
+          unsigned char* b_tile = a_tile + S::a_bytes;
+          mbar_expect_tx(&full_bar[s], S::stage_bytes);
+          tma_load_2d(b_tile, &map_w, &full_bar[s], it * TC_BK, w0);
+          if (tc_gated(EPI)) tma_load_2d(b_tile + S::b_bytes / 2, &map_w, &full_bar[s], it * TC_BK, up_row_offset + w0);
+          tma_load_2d(a_tile, &map_a, &full_bar[s], it * TC_BK, m0);
+        }
+      }
+      // (after a wait that gave up) copies in flight end before the CTA does
+      if (!ok)
+        for (int i = max(0, kb - STAGES); i < kb; ++i) mbar_wait_bounded(smem_u32(&full_bar[i % STAGES]), (i / STAGES) & 1, MS_WAIT_NS / 64);
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc(TC_BM, BN);
+      int kb = 0, tc = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tc) {
+        const int buf = tc & 1;
+        if (tc >= 2 && !mbar_wait(&acc_empty[buf], ((tc >> 1) - 1) & 1)) {
+          atomicExch(status, 14);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const uint32_t tmem_acc = tmem_base + (uint32_t)buf * BN;
+        for (int it = 0; it < k_iters; ++it, ++kb) {
+          const int s = kb % STAGES;
+          if (!mbar_wait(&full_bar[s], (kb / STAGES) & 1)) {
+            atomicExch(status, 12);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          // (the instruction's rows 32 .. 127 read what lies behind the stage's 32; they are not stored)
+          const unsigned char* a_tile = smem + (size_t)s * S::stage_bytes;
+          const uint64_t da = make_smem_desc(a_tile), db = make_smem_desc(a_tile + S::a_bytes);
+#pragma unroll
+          for (int k = 0; k < TC_BK / 16; ++k) umma_bf16(tmem_acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (it | k) != 0);
+          umma_commit(&empty_bar[s]);
+        }
+        if (ok) umma_commit(&acc_full[buf]);
+      }
+      // arrivals that nobody waits for must not outlive the CTA
+      for (int i = max(0, kb - STAGES); i < kb && ok; ++i) ok = mbar_wait(&empty_bar[i % STAGES], (i / STAGES) & 1);
+    }
+  } else {
+    int tc = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++tc) {
+      const int buf = tc & 1, n0 = (tile % n_tiles) * COLS, at = tile / n_tiles;
+      const int row = grp.tiles[2 * at + 1] + lane, rows_end = min(M, grp.offsets[grp.tiles[2 * at] + 1]);
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (tc >> 1) & 1))) {
+        if (lane == 0) atomicExch(status, 13);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t acc_addr = tmem_base + (uint32_t)buf * BN;
+      uint32_t acc[BN];
+#pragma unroll
+      for (int c = 0; c < BN; c += 32) tmem_ld32(acc_addr + (uint32_t)c, *reinterpret_cast<uint32_t(*)[32]>(acc + c));
+      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);  // the accumulator is free for the tile after the next
+      if (row < rows_end) {
+        uint32_t(&lo)[32] = *reinterpret_cast<uint32_t(*)[32]>(acc);
+        uint32_t(&hi)[32] = *reinterpret_cast<uint32_t(*)[32]>(acc + 32);
+        store_chunk<EPI>(out, lo, hi, row, n0, N_out, grp.glu);
+        if (!tc_gated(EPI)) store_chunk<EPI>(out, hi, hi, row, n0 + 32, N_out, grp.glu);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(2u * BN) : "memory");
   }
 }
 
@@ -1200,14 +1336,14 @@ static int launch_tc(void* out, const void* A, const void* W, int M, int N_out, 
 }
 
 // The grouped form: A [rows, K] sorted by matrix, W [matrices * w_rows, K], the plan on the device.
-template <int BN, int STAGES, int EPI, int AROWS = TC_BM>
+template <int BN, int STAGES, int EPI>
 static int launch_tc_grouped(void* out, const void* A, const void* W, int rows, int N_out, int matrices, int w_rows, int K,
                              int up_row_offset, const TcGroups& grp, int max_tiles, int* status, cudaStream_t stream) {
   CUtensorMap map_a, map_w;
-  if (int rc = make_map(&map_a, A, rows, K, AROWS)) return rc;
+  if (int rc = make_map(&map_a, A, rows, K, TC_BM)) return rc;
   if (int rc = make_map(&map_w, W, (long long)matrices * w_rows, K, tc_gated(EPI) ? BN / 2 : BN)) return rc;
-  constexpr size_t smem = (size_t)STAGES * TcSmem<BN, AROWS>::stage_bytes + TcSmem<BN, AROWS>::overread + 1024;
-  auto kernel = gemm_tc_kernel<BN, STAGES, EPI, true, AROWS>;
+  constexpr size_t smem = (size_t)STAGES * TcSmem<BN>::stage_bytes + 1024;
+  auto kernel = gemm_tc_kernel<BN, STAGES, EPI, true>;
   static bool configured = false;
   if (!configured) {
     MS_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1216,6 +1352,24 @@ static int launch_tc_grouped(void* out, const void* A, const void* W, int rows, 
   constexpr int COLS = tc_gated(EPI) ? BN / 2 : BN;
   dim3 grid(ceil_div(N_out, COLS), max_tiles);
   MS_LAUNCH(kernel, grid, TC_THREADS, smem, stream, map_a, map_w, out, rows, N_out, K, up_row_offset, status, grp);
+  return 0;
+}
+
+template <int EPI>
+static int launch_tc_few(void* out, const void* A, const void* W, int rows, int N_out, int matrices, int w_rows, int K, int up_row_offset,
+                         const TcGroups& grp, int max_tiles, int* status, cudaStream_t stream) {
+  constexpr int AROWS = TC_FEW_ROWS, STAGES = FEW_STAGES, COLS = tc_gated(EPI) ? FEW_BN / 2 : FEW_BN;
+  CUtensorMap map_a, map_w;
+  if (int rc = make_map(&map_a, A, rows, K, AROWS)) return rc;
+  if (int rc = make_map(&map_w, W, (long long)matrices * w_rows, K, COLS)) return rc;
+  constexpr size_t smem = (size_t)STAGES * TcSmem<FEW_BN, AROWS>::stage_bytes + TcSmem<FEW_BN, AROWS>::overread + 1024;
+  static_assert(FEW_CTAS * (smem + 1024 + 512) <= 227 * 1024, "the rings do not fit shared memory");
+  auto kernel = gemm_tc_few_kernel<STAGES, EPI>;
+  static std::atomic<unsigned long long> allowed{0};
+  MS_CHECK_CUDA(allow_shared_memory((const void*)kernel, (int)smem, allowed));
+  const long long tiles = (long long)ceil_div(N_out, COLS) * max_tiles, ctas = (sm_count() > 0 ? sm_count() : 148) * FEW_CTAS;
+  MS_CHECK_ARG(tiles < (1LL << 30), "gemm_tc: too many tiles (%lld)", tiles);
+  MS_LAUNCH(kernel, (unsigned)(tiles < ctas ? tiles : ctas), FEW_THREADS, smem, stream, map_a, map_w, out, rows, N_out, K, up_row_offset, status, grp);
   return 0;
 }
 
@@ -1456,9 +1610,8 @@ MS_EXPORT int ms_gemm_tc_bf16(void* out, const void* A, const void* W, int M, in
   }
 }
 
-// Rows per tile: 256, taken by pairs of CTAs, where the caller's plan has such tiles; 128; or 32 where an expert has a few rows (decode steps): then a CTA takes 64 columns of W, so that the weights are spread over
-// all SMs, and fetches 32 rows of A a stage.
-constexpr int TC_FEW_ROWS = 32, TC_PAIR_ROWS = 2 * TC_BM;
+// Rows per tile: 256, taken by pairs of CTAs, where the caller's plan has such tiles; 128; or 32 where an expert has a few rows (decode steps).
+constexpr int TC_PAIR_ROWS = 2 * TC_BM;
 // (Steps of many rows per expert are planned in tiles of 256: ops/experts.py has the line and both sides.)
 // Tiles of the grouped products of 128 rows: 1: 256 columns of W (gated) or 128, one CTA an SM; 2: 128, a shorter ring, two CTAs an SM, so that one CTA's
 // epilogue hides behind the other's products. 0: chosen from the rows per expert (measured on B200 with 16 experts, both products: 2,048 tokens x 3
@@ -1470,7 +1623,7 @@ template <int EPI>
 static int launch_grouped_gated(void* out, const void* A, const void* W, int rows, int N, int experts, int K, const TcGroups& grp, int tile_rows,
                                 int max_tiles, int* status, cudaStream_t stream) {
   if (tile_rows == TC_PAIR_ROWS) return launch_tc_pair_grouped<EPI>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
-  if (tile_rows == TC_FEW_ROWS) return launch_tc_grouped<64, 7, EPI, TC_FEW_ROWS>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
+  if (tile_rows == TC_FEW_ROWS) return launch_tc_few<EPI>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
   const bool narrow = g_grouped_config ? g_grouped_config == 2 : rows >= 128 * experts;
   if (narrow) return launch_tc_grouped<128, 3, EPI>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
   return launch_tc_grouped<256, 4, EPI>(out, A, W, rows, N, experts, 2 * N, K, N, grp, max_tiles, status, stream);
@@ -1480,7 +1633,7 @@ template <int EPI>
 static int launch_grouped_plain(void* out, const void* A, const void* W, int rows, int N, int experts, int K, const TcGroups& grp, int tile_rows,
                                 int max_tiles, int* status, cudaStream_t stream) {
   if (tile_rows == TC_PAIR_ROWS) return launch_tc_pair_grouped<EPI>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
-  if (tile_rows == TC_FEW_ROWS) return launch_tc_grouped<64, 7, EPI, TC_FEW_ROWS>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
+  if (tile_rows == TC_FEW_ROWS) return launch_tc_few<EPI>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
   const bool narrow = g_grouped_config ? g_grouped_config == 2 : rows >= 128 * experts;
   if (narrow) return launch_tc_grouped<128, 3, EPI>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);
   return launch_tc_grouped<128, 5, EPI>(out, A, W, rows, N, experts, N, K, 0, grp, max_tiles, status, stream);

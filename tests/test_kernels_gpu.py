@@ -759,8 +759,8 @@ def test_a_wait_that_nothing_answers_gives_up_raises_the_status_word_and_leaves_
 @pytest.mark.parametrize("n, k", [(128, 64), (200, 72), (72, 136), (392, 320)])
 @pytest.mark.parametrize("counts", [[256, 128, 512], [0, 1, 127, 129, 0, 255, 257, 640, 300], [700], [0, 0, 130]])
 @pytest.mark.parametrize("mode", ["silu", "clamped", "relu2", "plain"])
-def test_grouped_products_by_pairs_of_ctas(n, k, counts, mode):
-    """Tiles of 256 sorted rows against tiles of 128 (which the models' tests hold against the oracle): the same sums in the same
+def test_grouped_products_by_pairs_of_ctas_and_by_few_rows(n, k, counts, mode):
+    """Tiles of 256 and of 32 sorted rows, whose CTAs walk many, against tiles of 128 (which the models' tests hold against the oracle): the same sums in the same
     order. Runs that end inside a tile, inside its first half and at its edge; widths that are no whole tiles; rows of no run stay as they are."""
     from miniserve_b200.ops import experts as xo
 
@@ -772,7 +772,7 @@ def test_grouped_products_by_pairs_of_ctas(n, k, counts, mode):
     a = torch.randn(rows, k, device=DEV).bfloat16()
     w = (torch.randn(e, (2 if gated else 1) * n, k, device=DEV) * k ** -0.5).bfloat16()
     outs = []
-    for tile_rows in (xo.TC_TILE_ROWS, xo.TC_PAIR_ROWS):
+    for tile_rows in (xo.TC_TILE_ROWS, xo.TC_PAIR_ROWS, xo.TC_FEW_ROWS):
         pos, perm, offsets = torch.empty(rows, **i32), torch.empty(rows, **i32), torch.empty(e + 1, **i32)
         tiles, meta = torch.empty(xo.expert_max_tiles(rows, e, tile_rows), 2, **i32), torch.empty(2, **i32)
         xo.expert_plan(pos, perm, offsets, tiles, meta, idx, e, tile_rows=tile_rows)
@@ -783,4 +783,4 @@ def test_grouped_products_by_pairs_of_ctas(n, k, counts, mode):
         outs.append(out)
     torch.cuda.synchronize()
     assert ops.device_status("cuda").item() == 0
-    assert torch.equal(outs[0], outs[1]) and not torch.any(outs[1][:sum(counts)] == 32768.0) and torch.all(outs[1][sum(counts):] == 32768.0)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and not torch.any(outs[1][:sum(counts)] == 32768.0) and torch.all(outs[1][sum(counts):] == 32768.0)
