@@ -15,6 +15,7 @@
 // the same one scales the sum).
 // Every mbarrier wait is bounded; on a timeout the kernel raises the status word and winds down.
 #include <cfloat>
+#include <climits>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -306,10 +307,10 @@ __device__ __noinline__ float at_softmax_masked(uint32_t t_s, uint32_t t_o, int 
 }
 
 // What one work item (a tile of 2 x 128 query rows, one group of heads, one split of the keys)
-// has to do. The scheduler warp computes it from the item's index and hands it to the other roles
-// through a ring of two in shared memory; it also tells empty items from real ones.
+// has to do. The scheduler warp finds it from the item's number and hands it to the other roles
+// through a ring of two in shared memory.
 struct AtItem {
-  int r, rank, tok0, q_len, m0, start, kv_len, head0, split;
+  int r, tile, tok0, q_len, m0, start, kv_len, head0, split;
   int n_tiles[2], q_first[2], q_last[2], lo_g[2], lo_max[2], shares[2];
   int tile_begin, n_all;
   // Kept first keys: the walk over key tiles runs over virtual tiles; those below `first_tile` (the window's first
@@ -323,25 +324,18 @@ struct AtGrid {
   int q_tiles, rows, head_groups, splits, max_tiles_per_item, window, G;
   int chunk;  // > 0: a query sees only keys from the start of its own block of this many positions on
   int keep;   // > 0: the first `keep` keys of a request stay visible behind the window (the cache keeps their pages)
-  __device__ __forceinline__ int total() const { return q_tiles * rows * head_groups * splits; }
 };
 
-// Items are numbered so that the tiles with the most keys (the last tiles of the longest rows)
-// come first: tile rank, then row, then head group, then split.
-__device__ __forceinline__ bool at_item(AtItem& it, int idx, const AtGrid& gr, const int* __restrict__ cu_q,
-                                        const int* __restrict__ q_start) {
-  it.split = idx % gr.splits;
-  idx /= gr.splits;
-  it.head0 = (idx % gr.head_groups) * gr.G;
-  idx /= gr.head_groups;
-  it.r = idx % gr.rows;
-  it.rank = idx / gr.rows;
+// Tile `tile` of row r for one group of heads, its keys whole: how many key tiles that are (0: the row has no such tile).
+__device__ __forceinline__ int at_tile(AtItem& it, int r, int tile, const AtGrid& gr, const int* __restrict__ cu_q, const int* __restrict__ q_start) {
   const int tpc = AT_ROWS / gr.G;  // tokens per group
-  it.tok0 = cu_q[it.r];
-  it.q_len = cu_q[it.r + 1] - it.tok0;
-  it.m0 = (gr.q_tiles - 1 - it.rank) * 2 * tpc;
-  if (it.m0 >= it.q_len) return false;
-  it.start = q_start[it.r];
+  it.r = r;
+  it.tile = tile;
+  it.tok0 = cu_q[r];
+  it.q_len = cu_q[r + 1] - it.tok0;
+  it.m0 = tile * 2 * tpc;
+  if (tile < 0 || it.m0 >= it.q_len) return 0;
+  it.start = q_start[r];
   it.kv_len = it.start + it.q_len;
   // per group: the key tiles it needs (B needs at least as many as A; B may have no rows at all)
   it.has_b = it.m0 + tpc < it.q_len;
@@ -361,54 +355,134 @@ __device__ __forceinline__ bool at_item(AtItem& it, int idx, const AtGrid& gr, c
   it.tile_begin = it.walk_shift;
   it.n_tiles[0] = (min(it.kv_len, it.q_last[0] + 1) + AT_KEYS - 1) / AT_KEYS - it.tile_begin;
   it.n_tiles[1] = it.has_b ? (min(it.kv_len, it.q_last[1] + 1) + AT_KEYS - 1) / AT_KEYS - it.tile_begin : 0;
-  // Key ranges longer than `max_tiles_per_item` are cut into pieces of that length (the last one
-  // shorter; measured faster than equal pieces, whose items all start late in the queue's order)
-  // that other items take, at most `splits` of them: this one keeps `per_split` key tiles from its
-  // piece's first. A group whose keys lie in more than one piece leaves a partial result
-  // (unnormalised O, the maximum it is scaled by, the sum), and the last of them to finish adds
-  // the partial results up in the order of the pieces.
-  const int n_full = max(it.n_tiles[0], it.n_tiles[1]);
-  const int per_split = max(gr.max_tiles_per_item, (n_full + gr.splits - 1) / gr.splits);
-  if (it.split * per_split >= n_full) return false;
+  return max(it.n_tiles[0], it.n_tiles[1]);
+}
+// Key ranges longer than `max_tiles_per_item` are cut into pieces of that length (the last one
+// shorter; measured faster than equal pieces, whose items all start late in the queue's order)
+// that are items of their own, at most `splits` of them. A group whose keys lie in more than one piece leaves a partial result
+// (unnormalised O, the maximum it is scaled by, the sum), and the last of them to finish adds
+// the partial results up in the order of the pieces.
+__device__ __forceinline__ int at_piece_tiles(int n_full, const AtGrid& gr) { return max(gr.max_tiles_per_item, (n_full + gr.splits - 1) / gr.splits); }
+// Piece `split` of the tile: what at_tile left, cut down to it.
+__device__ __forceinline__ void at_piece(AtItem& it, int head0, int split, int per_split) {
+  it.head0 = head0;
+  it.split = split;
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
     it.shares[g] = (it.n_tiles[g] + per_split - 1) / per_split;  // in how many splits the group has keys
-    it.n_tiles[g] = min(max(it.n_tiles[g] - it.split * per_split, 0), per_split);
+    it.n_tiles[g] = min(max(it.n_tiles[g] - split * per_split, 0), per_split);
   }
-  it.tile_begin += it.split * per_split;
+  it.tile_begin += split * per_split;
   it.n_all = max(it.n_tiles[0], it.n_tiles[1]);
-  return true;
 }
 
-// The scheduler (all lanes of one warp): the CTA's first item is the one with its own number, the
-// others come off a counter in global memory. Empty items (tiles past a short row's end, splits
-// past a short key range) are stepped over: the lanes look at the 32 items from the claimed one
-// on, so a run of empty items costs one round trip. When nothing is left, the CTA signs off on a
-// second counter, and the last one to do so puts both back to zero for the next launch.
-// Lane 0's `item` is the one claimed.
-__device__ __forceinline__ bool at_claim(AtItem& item, int* __restrict__ queue, const AtGrid& gr, const int* __restrict__ cu_q,
-                                         const int* __restrict__ q_start, int lane, bool first) {
-  const int total = gr.total();
+// The order of the items is the longest first, so that the short ones even out the end. Where rows begin at different positions, tiles are ranked by
+// the position of their last key over all rows (rank 0 ends at pos_max; a row has one tile in each rank, while it has any), and all whole pieces of cut
+// key ranges come before the last pieces and the tiles that are not cut; the scheduler counts items along the pairs (rank, row). With every row ranked by
+// itself a portion of 900 tokens behind 4,096 had its last items of 28 tiles begin when its neighbours of 1,531 and 517 tokens were done: 89 us for
+// the three, 68 now; four rows of 17 to 900 tokens behind 0 to 4,096 84 -> 63. Counting takes half a microsecond for 32 pairs, once a CTA, so
+// rows that begin alike (whose order it would not change) and steps of many pairs (100 short rows behind up to 3,000 keys: 152 us, 235 by position) are
+// numbered by place: a tile's rank is its distance from the longest row's last one, then row, head group, split, empty ones among them.
+struct AtOrder {
+  int pairs, pos_max;  // ranks x rows (0: by place)
+};
+constexpr int AT_MOST_PAIRS = 256;
+__device__ __forceinline__ AtOrder at_order(const AtGrid& gr, const int* __restrict__ cu_q, const int* __restrict__ q_start, int lane) {
+  if (gr.rows < 2 || gr.rows > AT_MOST_PAIRS / 2) return {0, 0};
+  const int span = 2 * (AT_ROWS / gr.G);
+  int last = 0, first = INT_MAX, latest = 0;
+  for (int r = lane; r < gr.rows; r += 32) {
+    const int len = cu_q[r + 1] - cu_q[r], start = q_start[r];
+    if (len > 0) {
+      last = max(last, start + (len + span - 1) / span * span);
+      first = min(first, start);
+      latest = max(latest, start);
+    }
+  }
+  last = __reduce_max_sync(0xffffffffu, last);
+  latest = __reduce_max_sync(0xffffffffu, latest);
+  first = __reduce_min_sync(0xffffffffu, first);
+  if (first >= latest || (last - first) / span > AT_MOST_PAIRS / gr.rows) return {0, 0};
+  return {(last - first) / span * gr.rows, last};
+}
+
+// The scheduler (all lanes of one warp): the CTA's first item is the one with its own number, the others come off a counter in global
+// memory. When nothing is left, the CTA signs off on a second counter, and the last one to do so puts both back to zero for the next
+// launch. Lane 0's `item` is the one claimed.
+// By place, empty items (tiles past a short row's end, splits past a short key range) are stepped over: the lanes look at the 32 items from
+// the claimed one on, so a run of empty items costs one round trip. By position a CTA's numbers only grow, so it counts on from where it stood.
+struct AtCursor {
+  int entry, items;  // entries of the order (pairs, twice) passed, and the items in them
+};
+__device__ __forceinline__ bool at_claim(AtItem& item, AtCursor& at, int* __restrict__ queue, const AtGrid& gr, const AtOrder& order,
+                                         const int* __restrict__ cu_q, const int* __restrict__ q_start, int lane, bool first) {
+  const int span = 2 * (AT_ROWS / gr.G), total = gr.q_tiles * gr.rows * gr.head_groups * gr.splits;
   for (;;) {
     int idx = (int)blockIdx.x;
     if (!first) {
       if (lane == 0) idx = (int)gridDim.x + atomicAdd(queue, 1);
       idx = __shfl_sync(0xffffffffu, idx, 0);
     }
-    if (idx >= total) {
-      if (lane == 0 && atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
-        queue[0] = 0;
-        queue[1] = 0;
+    if (order.pairs == 0) {
+      if (idx >= total) break;
+      bool work = false;
+      if (idx + lane < total) {
+        int n = idx + lane;
+        const int split = n % gr.splits;
+        n /= gr.splits;
+        const int head = n % gr.head_groups;
+        n /= gr.head_groups;
+        const int n_full = at_tile(item, n % gr.rows, gr.q_tiles - 1 - n / gr.rows, gr, cu_q, q_start), per = at_piece_tiles(n_full, gr);
+        work = split * per < n_full;
+        if (work) at_piece(item, head * gr.G, split, per);
       }
-      return false;
+      const unsigned mask = __ballot_sync(0xffffffffu, work);
+      if (mask & 1u) return true;
+      const int run = mask ? __ffs(mask) - 1 : 32;  // this many items from idx on are empty
+      if (!first && lane == 0 && run > 1) atomicMax(queue, idx + run - (int)gridDim.x);
+      first = false;
+      continue;
     }
-    const bool work = idx + lane < total && at_item(item, idx + lane, gr, cu_q, q_start);
-    const unsigned mask = __ballot_sync(0xffffffffu, work);
-    if (mask & 1u) return true;
-    const int run = mask ? __ffs(mask) - 1 : 32;  // this many items from idx on are empty
-    if (!first && lane == 0 && run > 1) atomicMax(queue, idx + run - (int)gridDim.x);
-    first = false;
+    for (; at.entry < 2 * order.pairs; at.entry += 32) {
+      const int entry = at.entry + lane, phase = entry >= order.pairs, pair = entry - phase * order.pairs;
+      int r = 0, tile = -1, whole = 0, count = 0;
+      if (entry < 2 * order.pairs) {
+        const int rank = pair / gr.rows;
+        r = pair - rank * gr.rows;
+        const int before = order.pos_max - rank * span - q_start[r];
+        tile = before > 0 ? before / span - 1 : -1;
+        const int n_full = at_tile(item, r, tile, gr, cu_q, q_start);
+        if (n_full > 0) {
+          const int per = at_piece_tiles(n_full, gr);
+          whole = n_full / per;
+          count = gr.head_groups * (phase == 0 ? whole : whole * per < n_full);
+        }
+      }
+      int upto = count;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
+      }
+      const int sum = __shfl_sync(0xffffffffu, upto, 31);
+      if (idx < at.items + sum) {
+        const int l = __ffs(__ballot_sync(0xffffffffu, idx < at.items + upto)) - 1;
+        const int place = idx - at.items - __shfl_sync(0xffffffffu, upto - count, l), pieces = __shfl_sync(0xffffffffu, whole, l);
+        const int in_phase = __shfl_sync(0xffffffffu, phase, l);
+        const int n_full = at_tile(item, __shfl_sync(0xffffffffu, r, l), __shfl_sync(0xffffffffu, tile, l), gr, cu_q, q_start);
+        const int head = in_phase ? place : place / pieces, split = in_phase ? pieces : place - head * pieces;
+        at_piece(item, head * gr.G, split, at_piece_tiles(n_full, gr));
+        return true;
+      }
+      at.items += sum;
+    }
+    break;
   }
+  if (lane == 0 && atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
+    queue[0] = 0;
+    queue[1] = 0;
+  }
+  return false;
 }
 
 // Persistent: one CTA per SM takes items off a queue until none is left. EXTRAS: the instantiation that takes
@@ -495,9 +569,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
         return ok;
       };
+      const AtOrder order = at_order(gr, cu_q, q_start, lane);
+      AtCursor cursor = {0, 0};
       for (int i = 0; ok; ++i) {
         AtItem mine;
-        const bool alive = at_claim(mine, queue, gr, cu_q, q_start, lane, i == 0);
+        const bool alive = at_claim(mine, cursor, queue, gr, order, cu_q, q_start, lane, i == 0);
         if (!wait_free(&item_empty[i & 1], i >> 1)) break;
         AtItem& it = items[i & 1];
         if (lane == 0) {
@@ -707,7 +783,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         break;
       }
       const AtItem& it = items[i & 1];
-      const int r = it.r, rank = it.rank, tok0 = it.tok0, q_len = it.q_len, m0 = it.m0, start = it.start, kv_len = it.kv_len;
+      const int r = it.r, q_tile = it.tile, tok0 = it.tok0, q_len = it.q_len, m0 = it.m0, start = it.start, kv_len = it.kv_len;
       const int head0 = it.head0, split = it.split, tile_begin = it.tile_begin, first_tile = it.first_tile, walk_shift = it.walk_shift;
       const int lo_mine = it.lo_g[g], lo_max_mine = it.lo_max[g], q_first_mine = it.q_first[g], lo_item = it.lo_g[0];
       const int n_mine = it.n_tiles[g], n_all = it.n_all, shares = it.shares[g], alive = it.alive;
@@ -856,7 +932,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           // partial results up in the order of the splits, its own from tensor memory, and writes the
           // rows. Partial results are laid out [group of rows][split][4 columns][row], so that the 128
           // threads of a group (one row each) write and read whole 512-byte lines together.
-          const size_t unit = ((size_t)(rank * gr.rows + r) * gr.head_groups + head0 / G) * 2 + g;
+          const size_t unit = ((size_t)(q_tile * gr.rows + r) * gr.head_groups + head0 / G) * 2 + g;
           float4* po = reinterpret_cast<float4*>(part_o) + (unit * gr.splits + split) * (32 * 128) + row;
           float2* pml = part_ml + unit * gr.splits * 128 + row;
           int* ticket = tickets + unit;
@@ -980,7 +1056,8 @@ constexpr int AT_MIN_TILES = 8;  // the least number of key tiles that a split k
 // pieces of that length, at most *splits of them. One CTA fills an SM, so a step with at most one query tile per SM cannot even its load
 // out through the queue (nor can one with up to two): the last tiles of a long prompt, or the few tiles of a portion far into a
 // long context, walk many more keys than the rest while other SMs idle. Then key ranges longer
-// than about 1.2 times the work per SM are cut. With many more tiles than SMs the queue evens the
+// than about 1.2 times the work per SM are cut (1.1 where rows begin at different positions: us with 1.0 / 1.1 / 1.2 / 1.3, 1,531 tokens beside 517 behind
+// 1,024 and 900 behind 4,096 67 / 68 / 72 / 76, four rows of up to 1,100 behind up to 2,000 34 / 29.5 / 29.4 / 29.7). With many more tiles than SMs the queue evens the
 // load out by itself and splits only add partial results.
 // Measured on B200, 16 heads in 8 groups: 256 tokens behind 30,000: 645 us whole, 109 us cut;
 // 512 behind 8,192: 193 -> 72 us; one prompt of 2,048 (128 tiles, the last 16 key tiles long):
@@ -993,7 +1070,9 @@ MS_EXPORT void ms_attn_tc_plan(const int* q_start, const int* q_len, int num_row
   const int G = at_heads_per_cta(nq, nkv), span = 2 * (AT_ROWS / G), head_groups = nq / G;
   long long ctas = 0, steps = 0;
   int longest = 0;
+  bool alike = true;  // rows that begin alike are taken in an order of their own (at_order), which evens out less
   for (int r = 0; r < num_rows; ++r) {
+    alike = alike && q_start[r] == q_start[0];
     for (int m0 = 0; m0 < q_len[r]; m0 += span) {
       const int last = q_start[r] + (m0 + span < q_len[r] ? m0 + span : q_len[r]) - 1;
       const int lo = window > 0 && q_start[r] + m0 - window + 1 > 0 ? q_start[r] + m0 - window + 1 : 0;
@@ -1004,7 +1083,7 @@ MS_EXPORT void ms_attn_tc_plan(const int* q_start, const int* q_len, int num_row
     }
   }
   if (ctas == 0 || ctas > 2LL * sm_count) return;
-  const long long fair = (steps * 12 + 10LL * sm_count - 1) / (10LL * sm_count);  // 1.2 x the work per SM, rounded up
+  const long long fair = (steps * (alike ? 12 : 11) + 10LL * sm_count - 1) / (10LL * sm_count);  // 1.2 (1.1) x the work per SM, rounded up
   *min_tiles = (int)(fair < 4 ? 4 : fair);
   const int want = ceil_div(longest, *min_tiles);
   *splits = want < 1 ? 1 : (want > 16 ? 16 : want);
