@@ -105,8 +105,11 @@ __device__ __forceinline__ int wk_first(int row, const int* __restrict__ cu_q) {
 // Bound by instruction issue: 16 x 16 pairs over dk channels with a decay each. A warp takes four tokens j at once, eight lanes
 // over the channels of each (two channels an instruction), lets their keys decay from j on, and adds up over the lanes at the end (28
 // exchanges for four tokens). The sum over the lanes, products of decays and the triangular system in 64 bits (above).
+// With the delta rule the triangular system is a chain of 16 steps in 64 bits, in which a CTA's warps wait for one another: six CTAs an SM (80
+// registers a thread, 24 to 64 bytes of them spilled) cover it better than four. 2,048 tokens, both kernels: 16 heads of 64 x 64 139.9 -> 136.3
+// us, 32 heads 225.7 -> 209.8. Without it nothing waits so long, and six measured the same as four (108.2).
 template <typename TIn, typename TZ, bool DELTA, int N>
-__global__ void __launch_bounds__(WK_THREADS, 4)
+__global__ void __launch_bounds__(WK_THREADS, DELTA ? 6 : 4)
 walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float* __restrict__ k_out, float* __restrict__ last_out,
                     float* __restrict__ u0_out, float* __restrict__ pairs, const TIn* __restrict__ q, int ld_q, const TIn* __restrict__ k,
                     int ld_k, int qk_group, const TIn* __restrict__ v, int ld_v, const TZ* __restrict__ z, int ld_z,
