@@ -61,6 +61,22 @@ def test_convolution_in_fours(dtype, taps, unit, dk, others, dv, lens, started):
         _near(got, want, torch.float32)
 
 
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("lens", [(1, 1), (301, 9)])
+def test_convolution_with_taps_at_any_address(taps, lens):
+    """Four channels' taps are read as whole vectors where they are aligned: the same bits where they are not."""
+    gen = torch.Generator().manual_seed(taps)
+    ctx, t, c = _rows(lens, (0, 5)), sum(lens), 2052
+    x, state = torch.randn(t, c, generator=gen).bfloat16().to(DEV), torch.randn(len(lens), taps - 1, c, generator=gen).bfloat16().to(DEV)
+    w = torch.randn(c, taps, generator=gen).to(DEV)
+    moved = torch.empty(c * taps + 1, device=DEV)[1:].view(c, taps).copy_(w)
+    assert w.data_ptr() % 16 == 0 and moved.data_ptr() % 16 == 4
+    got, want = (torch.full((t, c), float("nan"), device=DEV) for _ in range(2))
+    ops.conv_silu_unit(got, x, state, w, ctx, 0, 1, c // 4, 4, 1e-6)
+    ops.conv_silu_unit(want, x, state, moved, ctx, 0, 1, c // 4, 4, 1e-6)
+    assert not torch.isnan(got).any() and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("t, heads, dv", [(1, 1, 64), (37, 3, 32), (130, 5, 128), (3, 7, 64)])
 @pytest.mark.parametrize("kind, own", [("silu", False), ("sigmoid", True)])
