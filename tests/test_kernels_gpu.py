@@ -468,6 +468,21 @@ def test_attention_bf16_decode_by_tensor_copies(nq, nkv, d, page, keys, extra, s
         assert torch.equal(o[filled], sums[0][filled])  # the same sums in the same order
 
 
+@pytest.mark.parametrize("rows, splits", [(1, 8), (7, 1), (7, 16), (8, 1), (8, 4), (1, 17), (2, 40)])
+def test_attention_bf16_decode_copies_by_rows_and_splits(rows, splits, monkeypatch):
+    """Around the rule that leaves a few rows to copies of 16 bytes a lane: the same bits on either side of it."""
+    torch.manual_seed(rows)
+    lens = [(2000 - 31 * i, 1) for i in range(rows)]
+    pb = PagedBatch(lens, 16, 2, 128, torch.bfloat16, seed=3)
+    pb.k_pool, pb.v_pool = (torch.randn(pb.k_pool.shape, device=DEV).bfloat16() for _ in range(2))
+    q = torch.randn(rows, 8, 128, device=DEV).bfloat16()
+    monkeypatch.setattr(attention_bf16, "choose_splits", lambda *a, **k: splits)
+    ctx, got, want = make_context(pb), torch.full_like(q, -7.0), torch.full_like(q, 7.0)
+    attention_bf16.run_decode(got, q, pb.k_pool, pb.v_pool, ctx, 0, 128 ** -0.5, None, rows)
+    attention_bf16.run_decode(want, q, pb.k_pool, pb.v_pool, ctx, 0, 128 ** -0.5, None, rows, form="general")
+    assert torch.equal(got, want) and ops.device_status("cuda").item() == 0
+
+
 @pytest.mark.parametrize("graph_kv_len", [0, 8192, 32768])
 def test_attention_bf16_decode_of_long_contexts_as_laid_out_inside_a_graph(graph_kv_len):
     """Inside a CUDA graph the launch follows the batch size and the graph's class of context length, not
