@@ -1250,6 +1250,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(out) + ((size_t)(m0 + rr) * N_out + col) * ITEM) =
                     *reinterpret_cast<const uint4*>(stage_out + rr * 128 + ((chunk ^ (rr & 7)) << 4));
             }
+            // an empty group: "one pending" above means the other tile's store only while every turn commits one (a whole tile's last
+            // store may still be reading when the next tile of the CTA leaves by rows)
+            if (issuer) asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
           }
           out_buf ^= 1;
         }

@@ -771,12 +771,9 @@ def test_a_wait_that_nothing_answers_gives_up_raises_the_status_word_and_leaves_
     assert torch.equal(out, table[:5])
 
 
-@pytest.mark.parametrize("n, k", [(128, 64), (200, 72), (72, 136), (392, 320)])
-@pytest.mark.parametrize("counts", [[256, 128, 512], [0, 1, 127, 129, 0, 255, 257, 640, 300], [700], [0, 0, 130]])
-@pytest.mark.parametrize("mode", ["silu", "clamped", "relu2", "plain"])
-def test_grouped_products_by_pairs_of_ctas_and_by_few_rows(n, k, counts, mode):
-    """Tiles of 256 and of 32 sorted rows, whose CTAs walk many, against tiles of 128 (which the models' tests hold against the oracle): the same sums in the same
-    order. Runs that end inside a tile, inside its first half and at its edge; widths that are no whole tiles; rows of no run stay as they are."""
+def _grouped_products(n, k, counts, mode, launches=1):
+    """Both grouped forms whose CTAs stay (tiles of 256 and of 32 sorted rows) against tiles of 128 (which the models' tests hold against the oracle): the
+    same sums in the same order. Rows of no run stay as they are."""
     from miniserve_b200.ops import experts as xo
 
     torch.manual_seed(n + len(counts))
@@ -786,16 +783,37 @@ def test_grouped_products_by_pairs_of_ctas_and_by_few_rows(n, k, counts, mode):
     idx = torch.tensor(sum(([i] * c for i, c in enumerate(counts)), []) + [e] * 40, **i32)[torch.randperm(rows, device=DEV)].view(-1, 1).contiguous()
     a = torch.randn(rows, k, device=DEV).bfloat16()
     w = (torch.randn(e, (2 if gated else 1) * n, k, device=DEV) * k ** -0.5).bfloat16()
-    outs = []
+    want = None
     for tile_rows in (xo.TC_TILE_ROWS, xo.TC_PAIR_ROWS, xo.TC_FEW_ROWS):
         pos, perm, offsets = torch.empty(rows, **i32), torch.empty(rows, **i32), torch.empty(e + 1, **i32)
         tiles, meta = torch.empty(xo.expert_max_tiles(rows, e, tile_rows), 2, **i32), torch.empty(2, **i32)
         xo.expert_plan(pos, perm, offsets, tiles, meta, idx, e, tile_rows=tile_rows)
         assert meta.tolist() == [sum(-(-c // tile_rows) for c in counts), sum(counts)]
-        out = torch.full((rows, n), 32768.0, device=DEV, dtype=torch.float32 if mode == "plain" else torch.bfloat16)
-        xo.expert_products_tc(out, a, w, tiles, meta, offsets, gated, relu_squared=mode == "relu2",
-                              clamps=(2.0, 1.7, 1.0) if mode == "clamped" else None, tile_rows=tile_rows)
-        outs.append(out)
-    torch.cuda.synchronize()
+        for _ in range(launches):
+            out = torch.full((rows, n), 32768.0, device=DEV, dtype=torch.float32 if mode == "plain" else torch.bfloat16)
+            xo.expert_products_tc(out, a, w, tiles, meta, offsets, gated, relu_squared=mode == "relu2",
+                                  clamps=(2.0, 1.7, 1.0) if mode == "clamped" else None, tile_rows=tile_rows)
+            want = out if want is None else want
+            assert torch.equal(out, want) and not torch.any(out[:sum(counts)] == 32768.0) and torch.all(out[sum(counts):] == 32768.0)
     assert ops.device_status("cuda").item() == 0
-    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and not torch.any(outs[1][:sum(counts)] == 32768.0) and torch.all(outs[1][sum(counts):] == 32768.0)
+
+
+@pytest.mark.parametrize("n, k", [(128, 64), (200, 72), (72, 136), (392, 320)])
+@pytest.mark.parametrize("counts", [[256, 128, 512], [0, 1, 127, 129, 0, 255, 257, 640, 300], [700], [0, 0, 130]])
+@pytest.mark.parametrize("mode", ["silu", "clamped", "relu2", "plain"])
+def test_grouped_products_by_pairs_of_ctas_and_by_few_rows(n, k, counts, mode):
+    """A tile or less a pair of CTAs: runs that end inside a tile, inside its first half and at its edge; widths that are no whole tiles."""
+    _grouped_products(n, k, counts, mode)
+
+
+@pytest.mark.parametrize("counts, k", [([384, 642], 64), ([130, 256, 511, 1, 640], 136)])
+@pytest.mark.parametrize("ragged", [0, 8])
+@pytest.mark.parametrize("mode", ["silu", "clamped", "relu2", "plain"])
+def test_grouped_products_of_many_tiles_a_pair(counts, k, ragged, mode):
+    """Every pair of CTAs takes five tiles of 256 rows and more, whole ones and ones that leave by rows in turn, over a short k, so that the turns of the
+    two accumulators and of the epilogue's two staging tiles run on from one kind of tile to the other."""
+    cols = 128 if mode in ("silu", "clamped") else 256
+    pairs, row_tiles = torch.cuda.get_device_properties(0).multi_processor_count // 2, sum(-(-c // 256) for c in counts)
+    n_tiles = 5 * pairs // row_tiles + 1
+    assert n_tiles * row_tiles > 5 * pairs and any(c % 256 == 0 or c > 256 for c in counts) and any(c % 128 for c in counts)
+    _grouped_products(cols * n_tiles - ragged, k, counts, mode, launches=6)
