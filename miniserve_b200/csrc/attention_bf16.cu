@@ -475,7 +475,10 @@ __device__ __forceinline__ void decode_slice(float (&o)[DTILES][4], float (&m_ru
   }
 }
 
-template <bool TMA, bool EX>
+// ORDER: the form that can take the longest requests' items first. Splits through scratch, which are never taken in that order, run the general
+// form without that code (a replayed step of one request, us, with it / without: 8,192 keys 1,157 / 1,146, 16,384 1,316 / 1,296, 32,768 1,621 / 1,602);
+// clusters of splits run the form with it, unasked (2 requests of 2,048 keys 912 / 919, 4 of 6,000 1,295 / 1,302).
+template <bool TMA, bool EX, bool ORDER>
 __global__ void __launch_bounds__(DC_THREADS)
 attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int* __restrict__ status,
                    __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
@@ -492,7 +495,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int split = blockIdx.x;
   int r = blockIdx.y, z = blockIdx.z;
-  if (longest_first) {
+  if (ORDER && longest_first) {
     // One CTA per item and more items than fit the GPU at once: CTAs start in the order of their index, so the longest
     // request's items come first and the shortest fill the end. Thread i finds request i's rank.
     __shared__ __align__(16) int lens[DC_THREADS];
@@ -856,8 +859,9 @@ static bool decode_takes_tma(const void* k_pool, const void* v_pool, long long p
   return DC_TMA && (num_rows >= 8 || (num_rows >= 2 && num_splits > 16)) && pool_pages > 0 && page_size >= DC_SLICE && status != nullptr && (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0;
 }
 static bool has_extras(const AttnExtras& ex) { return ex.cap_inv > 0.f || ex.chunk > 0 || ex.dist_r1 != nullptr || ex.keep_first > 0; }
-static DecodeKernel decode_form(bool tma, const AttnExtras& ex) {
-  return !tma ? attn_decode_kernel<false, true> : has_extras(ex) ? attn_decode_kernel<DC_TMA, true> : attn_decode_kernel<DC_TMA, !DC_TMA>;
+static DecodeKernel decode_form(bool tma, const AttnExtras& ex, bool order) {
+  if (!tma) return order ? attn_decode_kernel<false, true, true> : attn_decode_kernel<false, true, false>;
+  return has_extras(ex) ? attn_decode_kernel<DC_TMA, true, true> : attn_decode_kernel<DC_TMA, !DC_TMA, true>;
 }
 static constexpr size_t decode_smem(bool tma) { return tma ? DecodeSmem::bytes_tma : DecodeSmem::bytes; }
 
@@ -868,10 +872,11 @@ static int configure_decode() {
   MS_CHECK_CUDA(cudaGetDevice(&dev));
   MS_CHECK_ARG(dev >= 0 && dev < 64, "attention: device index %d is not supported", dev);
   if (!configured[dev]) {
-    MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes));
+    MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes));
+    MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes));
     if (DC_TMA) {
-      MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<DC_TMA, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes_tma));
-      MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<DC_TMA, !DC_TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes_tma));
+      MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<DC_TMA, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes_tma));
+      MS_CHECK_CUDA(cudaFuncSetAttribute(attn_decode_kernel<DC_TMA, !DC_TMA, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecodeSmem::bytes_tma));
     }
     configured[dev] = true;
   }
@@ -920,7 +925,7 @@ MS_EXPORT int MS_ATTN_FN(decode_fused)(void* out, void* part_o, void* part_ml, i
   // microsecond (64 requests, us: 1,025 to 3,986 keys 149 -> 119, 100 keys each 18.5 -> 20.5), so not where no row is long.
   // max_kv_len 0: not known, inside a graph, where that microsecond passes while the kernels before still run.
   const int longest_first = (max_kv_len == 0 || max_kv_len > 512) && num_splits == 1 && num_rows > 1 && num_rows <= DC_THREADS && num_rows * (int)grid.z > sm_count();
-  MS_LAUNCH(decode_form(tma, ex), grid, DC_THREADS, decode_smem(tma), stream,
+  MS_LAUNCH(decode_form(tma, ex, longest_first), grid, DC_THREADS, decode_smem(tma), stream,
       map_k, map_v, status, (__nv_bfloat16*)out, (float*)part_o, (float*)part_ml, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
       (const __nv_bfloat16*)v_pool, kv_len, page_indptr, page_indices, nq, nkv, scale * LOG2E, window, sink,
       shift_of(page_size), num_splits, counters, 0, longest_first, ex);
@@ -953,7 +958,7 @@ MS_EXPORT int MS_ATTN_FN(decode_cluster)(void* out, const void* q, const void* k
   const bool tma = decode_takes_tma(k_pool, v_pool, pool_pages, page_size, status, num_rows, num_splits);
   if (int rc = decode_maps(&map_k, &map_v, tma, k_pool, v_pool, pool_pages, nkv, page_size)) return rc;
   dim3 grid(num_splits, num_rows, nkv * ceil_div(group, 16));
-  MS_LAUNCH_CLUSTERED(decode_form(tma, ex), grid, DC_THREADS, decode_smem(tma), stream, num_splits,
+  MS_LAUNCH_CLUSTERED(decode_form(tma, ex, true), grid, DC_THREADS, decode_smem(tma), stream, num_splits,
       map_k, map_v, status, (__nv_bfloat16*)out, (float*)nullptr, (float*)nullptr, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
       (const __nv_bfloat16*)v_pool, kv_len, page_indptr, page_indices, nq, nkv, scale * LOG2E, window, sink,
       shift_of(page_size), num_splits, (int*)nullptr, 1, 0, ex);
@@ -983,7 +988,7 @@ MS_EXPORT int MS_ATTN_FN(decode_clusters_resident)(int num_splits, int* out) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    MS_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, decode_form(DC_TMA, AttnExtras{}), &cfg));
+    MS_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, decode_form(DC_TMA, AttnExtras{}, true), &cfg));
     cached[dev][num_splits] = n > 0 ? n : -1;
   }
   *out = cached[dev][num_splits] > 0 ? cached[dev][num_splits] : 0;
