@@ -846,17 +846,12 @@ MS_EXPORT int MS_ATTN_FN(decode_fused)(void* out, void* part_o, void* part_ml, i
                                        const float* sink_values, float softcap, int chunk, const float* dist_r1, const float* dist_r2,
                                        int keep_first, long long pool_pages, int* status, int max_kv_len);
 
-// Which form of the decode kernel a launch takes: slices by tensor copies where a slice lies in one page and the pool is known
-// (`pool_pages` > 0), else 16 bytes a lane; without extras the form that carries none of their code.
+// Which form of the decode kernel a launch takes: slices by tensor copies where the caller asks for them (`pool_pages` > 0; the rule is beside the
+// Python face) and a slice lies in one page of aligned pools, else 16 bytes a lane; without extras the form that carries none of their code.
 using DecodeKernel = void (*)(const CUtensorMap, const CUtensorMap, int*, __nv_bfloat16*, float*, float*, const __nv_bfloat16*, const __nv_bfloat16*,
                               const __nv_bfloat16*, const int*, const int*, const int*, int, int, float, int, int, int, int, int*, int, int, AttnExtras);
-// A few rows stay with the copies of 16 bytes a lane: their warps have a few slices each, of which the first comes sooner that way
-// (us, tensor copies against those: 1 row of 300 keys 4.84 / 4.47, of 2,048 8.72 / 8.38, 2 of 2,048 9.71 / 9.36, 4 of 300 5.34 / 5.07; from 8
-// rows on the other way round: 8 of 300 6.08 / 6.34, of 2,048 16.9 / 17.4, of 8,192 46.6 / 49.9, 64 of 2,048 86 / 93), unless several
-// long rows are cut many ways (2 of 8,192 19.9 / 20.4, of 32,768 51.5 / 53.0). One row of 32,768 takes the same alone (32.7), and its decode step,
-// where the kernels before hide the other form's start, 1,650 / 1,624.
-static bool decode_takes_tma(const void* k_pool, const void* v_pool, long long pool_pages, int page_size, const int* status, int num_rows, int num_splits) {
-  return DC_TMA && (num_rows >= 8 || (num_rows >= 2 && num_splits > 16)) && pool_pages > 0 && page_size >= DC_SLICE && status != nullptr && (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0;
+static bool decode_takes_tma(const void* k_pool, const void* v_pool, long long pool_pages, int page_size, const int* status) {
+  return DC_TMA && pool_pages > 0 && page_size >= DC_SLICE && status != nullptr && (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0;
 }
 static bool has_extras(const AttnExtras& ex) { return ex.cap_inv > 0.f || ex.chunk > 0 || ex.dist_r1 != nullptr || ex.keep_first > 0; }
 static DecodeKernel decode_form(bool tma, const AttnExtras& ex, bool order) {
@@ -918,7 +913,7 @@ MS_EXPORT int MS_ATTN_FN(decode_fused)(void* out, void* part_o, void* part_ml, i
   const int group = nq / nkv;
   if (int rc = configure_decode()) return rc;
   CUtensorMap map_k = {}, map_v = {};
-  const bool tma = decode_takes_tma(k_pool, v_pool, pool_pages, page_size, status, num_rows, num_splits);
+  const bool tma = decode_takes_tma(k_pool, v_pool, pool_pages, page_size, status);
   if (int rc = decode_maps(&map_k, &map_v, tma, k_pool, v_pool, pool_pages, nkv, page_size)) return rc;
   dim3 grid(num_splits, num_rows, nkv * ceil_div(group, 16));
   // By length where items wait for others to end: each CTA then compares all lengths, a thread a request, which takes about a
@@ -955,7 +950,7 @@ MS_EXPORT int MS_ATTN_FN(decode_cluster)(void* out, const void* q, const void* k
   const int group = nq / nkv;
   if (int rc = configure_decode()) return rc;
   CUtensorMap map_k = {}, map_v = {};
-  const bool tma = decode_takes_tma(k_pool, v_pool, pool_pages, page_size, status, num_rows, num_splits);
+  const bool tma = decode_takes_tma(k_pool, v_pool, pool_pages, page_size, status);
   if (int rc = decode_maps(&map_k, &map_v, tma, k_pool, v_pool, pool_pages, nkv, page_size)) return rc;
   dim3 grid(num_splits, num_rows, nkv * ceil_div(group, 16));
   MS_LAUNCH_CLUSTERED(decode_form(tma, ex, true), grid, DC_THREADS, decode_smem(tma), stream, num_splits,

@@ -12,7 +12,7 @@ from dataclasses import dataclass
 
 import torch
 
-from . import blas, experts, native
+from . import attention_bf16, blas, experts, native
 from .mixers import (act_mul, add_dyt, add_layernorm, add_normed_rmsnorm, add_rmsnorm_scaled, add_row_vector, axpby, channel_decay, channel_gate,  # noqa: F401
                      chunk_scan, chunk_scan_ok, clamped_glu, conv_bias, conv_silu_unit, conv_state_update, decay_scan, embed_sum, gate_relu_squared, gated_group_norm,
                      gelu_tanh, head_gate, head_norm_gate, latent_prepare, latent_rope_prepare, mlstm_gates, mlstm_output, qkv_prepare,
@@ -610,8 +610,6 @@ def attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: 
 
     float32 runs the row-wise kernel, prompts its tiled form (bit-identical however the step was cut). bfloat16 runs the
     tensor-core kernels when they take this head size, else the row-wise kernel too."""
-    from . import attention_bf16
-
     extras = extras if extras is not None and extras.any else None
     if attention_tiled_ok(out, q, k_pool, v_pool, ctx):
         attention_tiled(out, q, k_pool, v_pool, ctx, group, scale, window, sink, extras)

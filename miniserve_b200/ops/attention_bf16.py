@@ -9,6 +9,8 @@ from functools import lru_cache
 
 import torch
 
+import miniserve_b200.ops as ops
+
 from . import build, native
 
 _p, _i, _f, _ll = c_void_p, c_int, c_float, c_longlong
@@ -33,9 +35,12 @@ def takes_extras(head_dim: int, page_size: int) -> bool:
     return supports(head_dim, page_size)
 
 
+_NO_EXTRAS = (None, 0.0, 0, None, None, 0)
+
+
 def _extras_args(extras) -> tuple:
     if extras is None:
-        return (None, 0.0, 0, None, None, 0)
+        return _NO_EXTRAS
     sv, r1, r2 = extras.sink_values, extras.dist_r1, extras.dist_r2
     return (None if sv is None else sv.data_ptr(), float(extras.softcap or 0.0), int(extras.chunk or 0),
             None if r1 is None else r1.data_ptr(), None if r2 is None else r2.data_ptr(), int(extras.keep_first or 0))
@@ -119,6 +124,22 @@ def choose_splits(rows: int, head_chunks: int, max_kv_len: int | None, sm_count:
     return splits
 
 
+def takes_tensor_copies(rows: int, splits: int, head_dim: int, page_size: int) -> bool:
+    """Whether a decode launch brings its slices of keys by tensor copies (head sizes 64 and 128, pages that hold whole slices of 16).
+    A few rows stay with the copies of 16 bytes a lane: their warps have a few slices each, of which the first comes sooner that way
+    (us, tensor copies against those: 1 row of 300 keys 4.84 / 4.47, of 2,048 8.72 / 8.38, 2 of 2,048 9.71 / 9.36, 4 of 300 5.34 / 5.07;
+    from 8 rows on the other way round: 8 of 300 6.08 / 6.34, of 2,048 16.9 / 17.4, of 8,192 46.6 / 49.9, 64 of 2,048 86 / 93), unless
+    several long rows are cut many ways (2 of 8,192 19.9 / 20.4, of 32,768 51.5 / 53.0). One row of 32,768 takes the same alone (32.7), and
+    its decode step, where the kernels before hide the other form's start, 1,650 / 1,624."""
+    return head_dim in (64, 128) and page_size >= 16 and (rows >= 8 or (rows >= 2 and splits > 16))
+
+
+@lru_cache(maxsize=None)
+def _status_at(device_index: int) -> int:
+    """The address of the device's status word, which lives as long as the process."""
+    return ops.device_status(torch.device("cuda", device_index)).data_ptr()
+
+
 def _scratch(ctx, need: int, d: int, device) -> tuple[torch.Tensor, torch.Tensor]:
     """Partial results: ``need`` rows of d floats, and of two."""
     if ctx.graph_bucket:
@@ -160,17 +181,17 @@ def run_decode(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool:
     """Rows [0, rows) of the step, one new token each (so token i belongs to row i): keys split
     across CTAs, partial results merged by the last CTA of each (row, head group) to finish. ``form`` (tests):
     "general", copies of 16 bytes a lane, as head sizes other than 64 and 128 and pages of 8 tokens take."""
-    from . import device_status
-
     t, nq, d = q.shape
-    nkv, page_size = k_pool.shape[1], k_pool.shape[2]
+    pages, nkv, page_size, _ = k_pool.shape
     fns = _lib(d)
     indptr, indices = ctx.page_indptr[group], ctx.page_indices[group]
     chunks = nkv * -(-(nq // nkv) // 16)
     fit = (lambda n: clusters_resident(d, n, q.device.index or 0)) if CLUSTER_MERGE else None
     known = ctx.max_kv_len if not ctx.graph_bucket else (getattr(ctx, "graph_kv_len", 0) or None)
     splits = choose_splits(rows, chunks, known, ctx.sm_count, fit)
-    pool = (0 if form == "general" else k_pool.shape[0], device_status(q.device).data_ptr())
+    pool = (0, None)
+    if rows > 1 and takes_tensor_copies(rows, splits, d, page_size) and form != "general":
+        pool = (pages, _status_at(q.device.index))
     if CLUSTER_MERGE and 2 <= splits <= 8:
         # the splits as one thread-block cluster: merged through distributed shared memory
         _check(fns, fns["decode_cluster"](
@@ -178,15 +199,15 @@ def run_decode(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool:
             indices.data_ptr(), rows, nq, nkv, float(scale), int(window or 0), int(sink), page_size, splits, ctx.stream,
             *_extras_args(extras), *pool))
         return
-    part_o = part_ml = counters = None
+    merge = (None, None, None)
     if splits > 1:
         part_o, part_ml = _scratch(ctx, rows * nq * splits, d, q.device)
         counters = _counters(ctx, rows * chunks, q.device)
+        merge = (part_o.data_ptr(), part_ml.data_ptr(), counters.data_ptr())
     _check(fns, fns["decode_fused"](
-        out.data_ptr(), None if part_o is None else part_o.data_ptr(), None if part_ml is None else part_ml.data_ptr(),
-        None if counters is None else counters.data_ptr(), q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), ctx.kv_len.data_ptr(), indptr.data_ptr(),
+        out.data_ptr(), *merge, q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), ctx.kv_len.data_ptr(), indptr.data_ptr(),
         indices.data_ptr(), rows, nq, nkv, float(scale), int(window or 0), int(sink), page_size, splits, ctx.stream,
-        *_extras_args(extras), *pool, int(known or 0)), launches=1)
+        *_extras_args(extras), *pool, int(known or 0)))
 
 
 def run_prefill(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx, group: int,
