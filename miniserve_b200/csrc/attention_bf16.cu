@@ -962,19 +962,22 @@ MS_EXPORT int MS_ATTN_FN(decode_cluster)(void* out, const void* q, const void* k
 
 // How many clusters of `num_splits` CTAs of the decode kernel this device holds at a time (a cluster
 // lies within one GPC, so this is not SM count x 2 / num_splits). A launch with more (request, head
-// group) items than that runs in two rounds.
-MS_EXPORT int MS_ATTN_FN(decode_clusters_resident)(int num_splits, int* out) {
+// group) items than that runs in two rounds. `copies`: of the form that brings slices by tensor copies, whose stages take less shared
+// memory (at head size 64 four CTAs an SM where three of the general form fit).
+MS_EXPORT int MS_ATTN_FN(decode_clusters_resident)(int num_splits, int copies, int* out) {
   MS_CHECK_ARG(num_splits >= 1 && num_splits <= 8, "attention: a cluster takes up to 8 splits, not %d", num_splits);
-  static int cached[64][9] = {};
+  static int cached[64][2][9] = {};
   int dev = 0;
   MS_CHECK_CUDA(cudaGetDevice(&dev));
   MS_CHECK_ARG(dev >= 0 && dev < 64, "attention: device index %d is not supported", dev);
-  if (cached[dev][num_splits] == 0) {
+  const bool tma = DC_TMA && copies;
+  int& held = cached[dev][tma][num_splits];
+  if (held == 0) {
     if (int rc = configure_decode()) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_splits, 1024, 1);
     cfg.blockDim = dim3(DC_THREADS);
-    cfg.dynamicSmemBytes = decode_smem(DC_TMA);  // (the padded stages are no smaller; the registers of both forms allow as many)
+    cfg.dynamicSmemBytes = decode_smem(tma);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = num_splits;
@@ -983,10 +986,10 @@ MS_EXPORT int MS_ATTN_FN(decode_clusters_resident)(int num_splits, int* out) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    MS_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, decode_form(DC_TMA, AttnExtras{}, true), &cfg));
-    cached[dev][num_splits] = n > 0 ? n : -1;
+    MS_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, decode_form(tma, AttnExtras{}, true), &cfg));
+    held = n > 0 ? n : -1;
   }
-  *out = cached[dev][num_splits] > 0 ? cached[dev][num_splits] : 0;
+  *out = held > 0 ? held : 0;
   return 0;
 }
 

@@ -63,7 +63,7 @@ def _lib(head_dim: int):
         ("decode", [_p] * 9 + [_i, _i, _i, _f, _i, _i, _i, _i, _p], c_int),
         ("decode_fused", [_p] * 10 + [_i, _i, _i, _f, _i, _i, _i, _i, _p, _p, _f, _i, _p, _p, _i, _ll, _p, _i], c_int),
         ("decode_cluster", [_p] * 7 + [_i, _i, _i, _f, _i, _i, _i, _i, _p, _p, _f, _i, _p, _p, _i, _ll, _p], c_int),
-        ("decode_clusters_resident", [_i, ctypes.POINTER(c_int)], c_int),
+        ("decode_clusters_resident", [_i, _i, ctypes.POINTER(c_int)], c_int),
     ):
         fn = getattr(lib, pre + name)
         fn.argtypes, fn.restype = args, res
@@ -82,13 +82,14 @@ def _check(fns, rc: int, launches: int = 1) -> None:
 
 
 @lru_cache(maxsize=None)
-def clusters_resident(head_dim: int, splits: int, device_index: int = 0) -> int:
+def clusters_resident(head_dim: int, splits: int, device_index: int = 0, copies: bool = True) -> int:
     """How many thread-block clusters of ``splits`` decode CTAs the device holds at a time (a cluster
-    lies within one GPC: on a B200 with head size 128, 71 clusters of 4 and 33 of 8, not 74 and 37)."""
+    lies within one GPC: on a B200 with head size 128, 71 clusters of 4 and 33 of 8, not 74 and 37). ``copies``: of the form that
+    brings its slices by tensor copies (``takes_tensor_copies``), else of the general one."""
     fns = _lib(head_dim)
     out = c_int(0)
     with torch.cuda.device(device_index):
-        rc = fns["decode_clusters_resident"](splits, ctypes.byref(out))
+        rc = fns["decode_clusters_resident"](splits, int(copies), ctypes.byref(out))
     if rc != 0:
         raise native.NativeError(fns["last_error"]().decode())
     return out.value
@@ -186,7 +187,9 @@ def run_decode(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool:
     fns = _lib(d)
     indptr, indices = ctx.page_indptr[group], ctx.page_indices[group]
     chunks = nkv * -(-(nq // nkv) // 16)
-    fit = (lambda n: clusters_resident(d, n, q.device.index or 0)) if CLUSTER_MERGE else None
+    fit = None
+    if CLUSTER_MERGE:
+        fit = lambda n: clusters_resident(d, n, q.device.index or 0, form != "general" and takes_tensor_copies(rows, n, d, page_size))  # noqa: E731
     known = ctx.max_kv_len if not ctx.graph_bucket else (getattr(ctx, "graph_kv_len", 0) or None)
     splits = choose_splits(rows, chunks, known, ctx.sm_count, fit)
     pool = (0, None)

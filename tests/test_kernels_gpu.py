@@ -522,6 +522,24 @@ def test_the_device_says_how_many_clusters_of_decode_ctas_it_holds():
     assert 1 <= splits <= 8 and (splits == 1 or attention_bf16.clusters_resident(128, splits) >= 64)
 
 
+@pytest.mark.parametrize("d, page, rows", [(64, 16, 2), (64, 8, 30), (64, 16, 30), (128, 16, 4), (128, 16, 30)])
+def test_clusters_are_counted_of_the_form_that_runs(d, page, rows, monkeypatch):
+    """The general form's stages take more shared memory than those of tensor copies (57,600 against 53,248 bytes at head size 64: three CTAs an SM
+    against four), so fewer of its clusters are resident."""
+    counted, sms = [], torch.cuda.get_device_properties(0).multi_processor_count
+    real = attention_bf16.clusters_resident
+    monkeypatch.setattr(attention_bf16, "clusters_resident", lambda *a: counted.append(a) or real(*a))
+    pb, q, ref, scale = _attention_case(torch.bfloat16, [(300 + i, 1) for i in range(rows)], 4, 2, d, page)
+    out = torch.full_like(q, float("nan"))
+    attention_bf16.run_decode(out, q, pb.k_pool, pb.v_pool, make_context(pb), 0, scale, None, rows)
+    assert torch.allclose(out.float(), ref, **BF16_TOL)
+    copies = rows >= 8 and page >= 16
+    assert counted and all(c[3] == copies == attention_bf16.takes_tensor_copies(rows, c[1], d, page) for c in counted)
+    for n in range(2, 9):
+        assert real(d, n, 0, False) <= real(d, n, 0, True)
+        assert d != 64 or real(d, n, 0, False) * n <= 3 * sms
+
+
 @pytest.mark.parametrize("window", [1, 16, 17, 100])
 def test_attention_bf16_decode_window_edge(window):
     rows = [(200, 1), (5, 1), (99, 1), (100, 1)]
