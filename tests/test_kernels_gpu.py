@@ -436,6 +436,14 @@ def test_attention_bf16_decode(nq, nkv, d, page, splits, monkeypatch):
     assert torch.allclose(out.float()[1:3], ref[1:3], **BF16_TOL)
 
 
+def _forms_that_run(monkeypatch, d):
+    """A list that tells of every decode launch of head size d from here on whether it was given a pool to make tensor copies from."""
+    fns, ran = attention_bf16._lib(d), []
+    for name, at in (("decode_fused", -3), ("decode_cluster", -2)):
+        monkeypatch.setitem(fns, name, lambda *a, run=fns[name], at=at: ran.append(a[at] > 0 and a[at + 1] is not None) or run(*a))
+    return ran
+
+
 @pytest.mark.parametrize("nq, nkv, d, page", [(16, 8, 128, 16), (32, 1, 64, 32), (6, 2, 64, 64), (20, 4, 128, 128)])
 @pytest.mark.parametrize("keys", [1, 17, 700, 2500])
 @pytest.mark.parametrize("extra", ["plain", "window", "shaped", "kept"])
@@ -455,32 +463,45 @@ def test_attention_bf16_decode_by_tensor_copies(nq, nkv, d, page, keys, extra, s
                                       keep_first=21)}.get(extra)
     window = {"window": 100, "kept": 40}.get(extra)
     monkeypatch.setattr(attention_bf16, "choose_splits", lambda *a, **k: splits)
+    ran = _forms_that_run(monkeypatch, d)
     ctx = make_context(pb)
     ctx.kv_len[5] = 0  # (a row of a graph that no request fills)
     outs = []
     for form in ("general", None, None):
         outs.append(torch.full_like(q, -7.0))
         attention_bf16.run_decode(outs[-1], q, pb.k_pool, pb.v_pool, ctx, 0, d ** -0.5, window, len(rows), extra == "window", extras, form)
-    assert ops.device_status("cuda").item() == 0
+    assert ops.device_status("cuda").item() == 0 and ran == [False, True, True]
     sums = [o.float() for o in outs]
     filled = torch.arange(len(rows), device=DEV) != 5
     for o in sums[1:]:
         assert torch.equal(o[filled], sums[0][filled])  # the same sums in the same order
 
 
-@pytest.mark.parametrize("rows, splits", [(1, 8), (7, 1), (7, 16), (8, 1), (8, 4), (1, 17), (2, 40)])
-def test_attention_bf16_decode_copies_by_rows_and_splits(rows, splits, monkeypatch):
-    """Around the rule that leaves a few rows to copies of 16 bytes a lane: the same bits on either side of it."""
-    torch.manual_seed(rows)
+@pytest.mark.parametrize("rows, splits, page, copies", [(1, 8, 16, False), (7, 1, 16, False), (7, 16, 16, False), (8, 1, 16, True), (8, 4, 16, True), (1, 17, 16, False),
+                                                        (2, 40, 16, True), (2, 16, 16, False), (30, 1, 8, False)])
+def test_attention_bf16_decode_copies_by_rows_and_splits(rows, splits, page, copies, monkeypatch):
+    """Around the rule that leaves a few rows to copies of 16 bytes a lane: the form that it says runs, and finds what the float32 reference does."""
     lens = [(2000 - 31 * i, 1) for i in range(rows)]
-    pb = PagedBatch(lens, 16, 2, 128, torch.bfloat16, seed=3)
-    pb.k_pool, pb.v_pool = (torch.randn(pb.k_pool.shape, device=DEV).bfloat16() for _ in range(2))
-    q = torch.randn(rows, 8, 128, device=DEV).bfloat16()
+    pb, q, ref, scale = _attention_case(torch.bfloat16, lens, 8, 2, 128, page, seed=rows)
     monkeypatch.setattr(attention_bf16, "choose_splits", lambda *a, **k: splits)
+    ran = _forms_that_run(monkeypatch, 128)
     ctx, got, want = make_context(pb), torch.full_like(q, -7.0), torch.full_like(q, 7.0)
-    attention_bf16.run_decode(got, q, pb.k_pool, pb.v_pool, ctx, 0, 128 ** -0.5, None, rows)
-    attention_bf16.run_decode(want, q, pb.k_pool, pb.v_pool, ctx, 0, 128 ** -0.5, None, rows, form="general")
-    assert torch.equal(got, want) and ops.device_status("cuda").item() == 0
+    attention_bf16.run_decode(got, q, pb.k_pool, pb.v_pool, ctx, 0, scale, None, rows)
+    attention_bf16.run_decode(want, q, pb.k_pool, pb.v_pool, ctx, 0, scale, None, rows, form="general")
+    assert ran == [copies, False] and torch.equal(got, want) and ops.device_status("cuda").item() == 0
+    assert torch.allclose(got.float(), ref, **BF16_TOL)
+
+
+@pytest.mark.parametrize("nq, nkv, d, page, copies", [(8, 8, 64, 16, True), (8, 8, 128, 16, True), (8, 8, 128, 8, False), (8, 8, 48, 16, False)])
+def test_attention_bf16_decode_takes_the_longest_rows_first(nq, nkv, d, page, copies, monkeypatch):
+    """More items than multiprocessors, one CTA each, of rows of all lengths (some alike) in no order: every row comes out once, as the reference has it."""
+    rows = [((733 * i) % 901 if i % 5 else 600, 1) for i in range(45)]
+    pb, q, ref, scale = _attention_case(torch.bfloat16, rows, nq, nkv, d, page, seed=d)
+    assert len(rows) * nkv > torch.cuda.get_device_properties(0).multi_processor_count
+    monkeypatch.setattr(attention_bf16, "choose_splits", lambda *a, **k: 1)
+    ran, out = _forms_that_run(monkeypatch, d), torch.full_like(q, float("nan"))
+    attention_bf16.run_decode(out, q, pb.k_pool, pb.v_pool, make_context(pb), 0, scale, None, len(rows))
+    assert ran == [copies] and torch.allclose(out.float(), ref, **BF16_TOL)
 
 
 @pytest.mark.parametrize("graph_kv_len", [0, 8192, 32768])
