@@ -14,13 +14,10 @@
 //
 // Stands where the reference calls F.linear on cuBLAS (miniserve/model/qwen3.py:115-131) and, for
 // the fused epilogue, flashinfer.silu_and_mul after the gate_up product (miniserve/model/fused.py:195).
-#include <cuda.h>
 
-#include <map>
-#include <mutex>
-#include <tuple>
 
 #include "common.cuh"
+#include "tensor_map.cuh"
 
 namespace ms {
 
@@ -1274,27 +1271,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 // ---------------------------------------------------------------- host side
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                              const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static int get_encode(EncodeFn* out) {
-  static EncodeFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    MS_CHECK_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres));
-    MS_CHECK_ARG(ptr != nullptr && qres == cudaDriverEntryPointSuccess, "gemm_tc: the driver has no cuTensorMapEncodeTiled");
-    fn = reinterpret_cast<EncodeFn>(ptr);
-  }
-  *out = fn;
-  return 0;
-}
-
 // A 2-D bfloat16 tensor [rows, cols] (cols contiguous), boxes of box_rows x 64 columns, 128-byte swizzle.
 static int make_map(CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows) {
-  EncodeFn encode;
-  if (int rc = get_encode(&encode)) return rc;
+  TensorMapEncodeFn encode;
+  if (int rc = tensor_map_encoder(&encode)) return rc;
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
   const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
@@ -1308,8 +1288,8 @@ static int make_map(CUtensorMap* map, const void* base, long long rows, long lon
 
 // A 2-D float32 tensor to store to, boxes of 128 rows x 32 columns.
 static int make_map_f32(CUtensorMap* map, const void* base, long long rows, long long cols) {
-  EncodeFn encode;
-  if (int rc = get_encode(&encode)) return rc;
+  TensorMapEncodeFn encode;
+  if (int rc = tensor_map_encoder(&encode)) return rc;
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
   const cuuint32_t box[2] = {32, (cuuint32_t)TC_BM};
@@ -1619,8 +1599,9 @@ MS_EXPORT int ms_gemm_tc_bf16(void* out, const void* A, const void* W, int M, in
 constexpr int TC_PAIR_ROWS = 2 * TC_BM;
 // (Steps of many rows per expert are planned in tiles of 256: ops/experts.py has the line and both sides.)
 // Tiles of the grouped products of 128 rows: 1: 256 columns of W (gated) or 128, one CTA an SM; 2: 128, a shorter ring, two CTAs an SM, so that one CTA's
-// epilogue hides behind the other's products. 0: chosen from the rows per expert (measured on B200 with 16 experts, both products: 2,048 tokens x 3
-// choices at 768 of 1024: 75.6 us with 2, 87.7 with 1; at 1536 of 2048: 182 against 202; 8 tokens: 39.5 against 35.6 and 94 against 65).
+// epilogue hides behind the other's products. 0: by the rows per expert. Steps that this package plans have tiles of 128 between 16 and 112 rows an
+// expert, where form 1 runs; form 2 is left to plans of 128-row tiles over more rows than that, which only a caller of the single products makes
+// (16 experts, both products, us with 2 / 1: 2,048 tokens x 3 choices at 768 of 1024 75.6 / 87.7, at 1536 of 2048 182 / 202; 8 tokens 39.5 / 35.6, 94 / 65).
 static int g_grouped_config = 0;
 MS_EXPORT void ms_gemm_tc_set_grouped(int config) { g_grouped_config = config; }
 

@@ -11,7 +11,7 @@ using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint
                                        const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                        CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-static int tensor_map_encoder(TensorMapEncodeFn* out) {
+inline int tensor_map_encoder(TensorMapEncodeFn* out) {
   static TensorMapEncodeFn fn = nullptr;
   if (fn == nullptr) {
     void* ptr = nullptr;
@@ -27,7 +27,7 @@ static int tensor_map_encoder(TensorMapEncodeFn* out) {
 // A bfloat16 cache [pages, kv heads, page_size, d] (d = 64 or 128) as [groups of 8 rows][d / 64 parts of a row][8 rows][64]: one
 // copy brings `box_rows` rows (a multiple of 8) of one page and head, each part of a group a block swizzled in 128 bytes. Coordinates: 0, 0, 0 and the
 // group of rows that the copy begins with; groups past the pool's end read as zeros.
-static int cache_tensor_map(CUtensorMap* map, const void* pool, long long rows, int d, int box_rows) {
+inline int cache_tensor_map(CUtensorMap* map, const void* pool, long long rows, int d, int box_rows) {
   TensorMapEncodeFn encode;
   if (int rc = tensor_map_encoder(&encode)) return rc;
   const cuuint64_t dims[4] = {64, 8, (cuuint64_t)(d / 64), (cuuint64_t)(rows / 8)};
