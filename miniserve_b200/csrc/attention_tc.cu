@@ -14,12 +14,7 @@
 // only when the maximum has grown by more than 2^8 (the stale maximum is exact in the end because
 // the same one scales the sum).
 // Every mbarrier wait is bounded; on a timeout the kernel raises the status word and winds down.
-#include <cfloat>
 #include <climits>
-#include <cstdlib>
-#include <map>
-#include <mutex>
-#include <tuple>
 
 #include "common.cuh"
 #include "tensor_map.cuh"
@@ -381,8 +376,11 @@ __device__ __forceinline__ void at_piece(AtItem& it, int head0, int split, int p
 // key ranges come before the last pieces and the tiles that are not cut; the scheduler counts items along the pairs (rank, row). With every row ranked by
 // itself a portion of 900 tokens behind 4,096 had its last items of 28 tiles begin when its neighbours of 1,531 and 517 tokens were done: 89 us for
 // the three, 68 now; four rows of 17 to 900 tokens behind 0 to 4,096 84 -> 63. Counting takes half a microsecond for 32 pairs, once a CTA, so
-// rows that begin alike (whose order it would not change) and steps of many pairs (100 short rows behind up to 3,000 keys: 152 us, 235 by position) are
-// numbered by place: a tile's rank is its distance from the longest row's last one, then row, head group, split, empty ones among them.
+// rows that begin alike (whose order it would not change) and steps of many pairs are numbered by place: a tile's rank is its distance from the longest
+// row's last one, then row, head group, split, empty ones among them. Us by place / by position: 2 rows behind 5,102 and 6,076 65 / 59, 4 behind 3,030
+// to 3,860 82 / 68, 8 behind up to 3,000 46 / 42, 16 behind up to 2,000 45 / 44 and up to 4,000 86 / 87, 32 behind up to 1,500 42 / 50, 64 behind up to
+// 1,000 57 / 74 and up to 3,000 107 / 156, 100 behind up to 3,000 152 / 235. The bound on the pairs lies where the two meet for 16 rows; it also leaves
+// two rows that begin more than 16,384 positions apart by place, where by position they would take less (0 and 20,000 110 / 107, 1,024 and 24,000 113 / 102).
 struct AtOrder {
   int pairs, pos_max;  // ranks x rows (0: by place)
 };
@@ -1057,7 +1055,9 @@ constexpr int AT_MIN_TILES = 8;  // the least number of key tiles that a split k
 // out through the queue (nor can one with up to two): the last tiles of a long prompt, or the few tiles of a portion far into a
 // long context, walk many more keys than the rest while other SMs idle. Then key ranges longer
 // than about 1.2 times the work per SM are cut (1.1 where rows begin at different positions: us with 1.0 / 1.1 / 1.2 / 1.3, 1,531 tokens beside 517 behind
-// 1,024 and 900 behind 4,096 67 / 68 / 72 / 76, four rows of up to 1,100 behind up to 2,000 34 / 29.5 / 29.4 / 29.7). With many more tiles than SMs the queue evens the
+// 1,024 and 900 behind 4,096 67 / 68 / 72 / 76, four rows of up to 1,100 behind up to 2,000 34 / 29.5 / 29.4 / 29.7; also where such rows
+// are too far apart to be ranked by position, with 1.1 / 1.2: 600 tokens beside 500 behind 20,000 111 / 106, 700 behind 1,024 beside 300 behind 24,000
+// 114 / 121, four of 200 to 400 behind up to 9,000 63 / 64, eight of 100 behind up to 4,900 47 / 47). With many more tiles than SMs the queue evens the
 // load out by itself and splits only add partial results.
 // Measured on B200, 16 heads in 8 groups: 256 tokens behind 30,000: 645 us whole, 109 us cut;
 // 512 behind 8,192: 193 -> 72 us; one prompt of 2,048 (128 tiles, the last 16 key tiles long):

@@ -44,9 +44,12 @@ struct SkinnyExtras {
   int tanh_from;
   float limit, alpha, shift;
 };
+// Three CTAs an SM for the gated forms: with 86 registers two fit, and 3,072 outputs are 384 CTAs where 296 were on the GPU at once. They keep 80
+// registers and spill 24 bytes (of 16 rows: 40). The others stay at two CTAs an SM; a stated least of one leaves them 94 and 104 registers where none
+// stated gave 86 and 94 (a replayed step at Qwen3-0.6B sizes, us, none / one: 4 requests of 2,048 keys 1,007 / 997, one of 8,192 1,168 / 1,162, one of
+// 2,048 900 / 897, 16 of 300 991 / 992). The step with two / three CTAs of the gated forms: 8 requests of 2,048 keys 1,159 / 1,102, 16 of 300 1,054 / 992,
+// one of 300 854 / 802.
 template <int MT, int MODE>
-// (Three CTAs an SM for the gated forms: with 86 registers two fit, and 3,072 outputs are 384 CTAs where 296 were on the GPU at once; the others gain
-// nothing by it. A decode step at Qwen3-0.6B sizes: 8 requests 1,151 -> 1,097 us, 16 of 100 keys 987 -> 922, 1 unchanged.)
 __global__ void __launch_bounds__(SK_THREADS, MODE == 3 || MODE == 6 ? 3 : 1)
 gemm_skinny_kernel(void* __restrict__ out, const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ W,
                    int M, int N, int K, const SkinnyExtras ex) {
