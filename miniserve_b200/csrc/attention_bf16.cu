@@ -335,9 +335,9 @@ struct DecodeSmem {
 };
 constexpr bool DC_TMA = D == 64 || D == 128;  // head sizes whose slices tensor copies can bring
 
-// One warp's ring of stages filled by tensor copies, two a slice (a page's 16 keys of one head), instead of 16 bytes a lane: the copies
-// were 300 of the 520 instructions that a slice took, and the warps' instructions were what the kernel waited for (64 requests of
-// 2,048 keys: 0.34 instructions a cycle and scheduler with two warps each; 97.7 us at 5.5 TB/s, now 89.4 at 6.05). The page of the
+// One warp's ring of stages filled by tensor copies, two a slice (a page's 16 keys of one head), instead of 16 bytes a lane: two instructions of one
+// lane where every lane had some sixteen, and addresses to make. 64 requests of 2,048 keys: 29.5 M warp instructions a launch before, 24.2 M now (the polls of the waits
+// among them), 0.35 instructions a cycle and scheduler before, 0.30 now; 93.4 us at 5.75 TB/s, now 86.4 at 6.22. The page of the
 // next slice is looked up a slice ahead. Waits are bounded.
 struct DecodeRing {
   uint32_t stages, bars;  // shared-memory addresses

@@ -130,8 +130,9 @@ def takes_tensor_copies(rows: int, splits: int, head_dim: int, page_size: int) -
     A few rows stay with the copies of 16 bytes a lane: their warps have a few slices each, of which the first comes sooner that way
     (us, tensor copies against those: 1 row of 300 keys 4.84 / 4.47, of 2,048 8.72 / 8.38, 2 of 2,048 9.71 / 9.36, 4 of 300 5.34 / 5.07;
     from 8 rows on the other way round: 8 of 300 6.08 / 6.34, of 2,048 16.9 / 17.4, of 8,192 46.6 / 49.9, 64 of 2,048 86 / 93), unless
-    several long rows are cut many ways (2 of 8,192 19.9 / 20.4, of 32,768 51.5 / 53.0). One row of 32,768 takes the same alone (32.7), and
-    its decode step, where the kernels before hide the other form's start, 1,650 / 1,624."""
+    several long rows are cut many ways (2 of 8,192 19.9 / 20.4, of 32,768 51.5 / 53.0). One row takes the same alone (of 8,192 14.9 / 14.9,
+    of 32,768 32.7 / 33.0, of 131,072 97.8 / 102); of its decode step, where the kernels before hide the other form's start, 8,192 keys
+    1,153 / 1,148, 32,768 1,610 / 1,597, 65,536 2,184 / 2,222, 131,072 3,385 / 3,496: the general form up to the commoner lengths."""
     return head_dim in (64, 128) and page_size >= 16 and (rows >= 8 or (rows >= 2 and splits > 16))
 
 
