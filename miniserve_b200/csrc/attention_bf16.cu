@@ -319,6 +319,7 @@ attn_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __rest
 // warps' partials of all splits from there, each CTA its share of the output; otherwise the CTA
 // merges its warps and writes one partial per split, or the final output when there is a single split.
 constexpr int DC_WARPS = 4, DC_THREADS = DC_WARPS * 32, DC_STAGES = 3, DC_SLICE = 16;
+constexpr int DC_LONG = 512;  // keys from which on a request is long enough for its items' order to matter
 
 struct DecodeSmem {
   static constexpr int q_elems = 16 * DPAD;
@@ -497,23 +498,24 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   int r = blockIdx.y, z = blockIdx.z;
   if (ORDER && longest_first) {
     // One CTA per item and more items than fit the GPU at once: CTAs start in the order of their index, so the longest
-    // request's items come first and the shortest fill the end. Thread i finds request i's rank.
+    // request's items come first and the shortest fill the end. Thread i finds request i's rank. Where no request is long the grid's own order does.
     __shared__ __align__(16) int lens[DC_THREADS];
     __shared__ int found;
-    const int rows = gridDim.y, index = blockIdx.z * rows + blockIdx.y, rank = index / (int)gridDim.z;
-    z = index - rank * gridDim.z;
-    const int mine = tid < rows ? kv_len_ptr[tid] : -1;
+    const int rows = gridDim.y, mine = tid < rows ? kv_len_ptr[tid] : -1;
     lens[tid] = mine;
-    __syncthreads();
-    int ahead = 0;
-    for (int i = 0; i < rows; i += 4) {
-      const int4 v = *reinterpret_cast<const int4*>(lens + i);
-      ahead += (v.x > mine || (v.x == mine && i < tid)) + (v.y > mine || (v.y == mine && i + 1 < tid)) +
-               (v.z > mine || (v.z == mine && i + 2 < tid)) + (v.w > mine || (v.w == mine && i + 3 < tid));
+    if (__syncthreads_or(mine > DC_LONG)) {
+      const int index = blockIdx.z * rows + blockIdx.y, rank = index / (int)gridDim.z;
+      z = index - rank * gridDim.z;
+      int ahead = 0;
+      for (int i = 0; i < rows; i += 4) {
+        const int4 v = *reinterpret_cast<const int4*>(lens + i);
+        ahead += (v.x > mine || (v.x == mine && i < tid)) + (v.y > mine || (v.y == mine && i + 1 < tid)) +
+                 (v.z > mine || (v.z == mine && i + 2 < tid)) + (v.w > mine || (v.w == mine && i + 3 < tid));
+      }
+      if (tid < rows && ahead == rank) found = tid;
+      __syncthreads();
+      r = found;
     }
-    if (tid < rows && ahead == rank) found = tid;
-    __syncthreads();
-    r = found;
   }
   const int kvh = z / chunks_per_group, head0 = kvh * group + (z % chunks_per_group) * 16;
   const int heads_here = min(16, kvh * group + group - head0);
@@ -918,8 +920,9 @@ MS_EXPORT int MS_ATTN_FN(decode_fused)(void* out, void* part_o, void* part_ml, i
   dim3 grid(num_splits, num_rows, nkv * ceil_div(group, 16));
   // By length where items wait for others to end: each CTA then compares all lengths, a thread a request, which takes about a
   // microsecond (64 requests, us: 1,025 to 3,986 keys 149 -> 119, 100 keys each 18.5 -> 20.5), so not where no row is long.
-  // max_kv_len 0: not known, inside a graph, where that microsecond passes while the kernels before still run.
-  const int longest_first = (max_kv_len == 0 || max_kv_len > 512) && num_splits == 1 && num_rows > 1 && num_rows <= DC_THREADS && num_rows * (int)grid.z > sm_count();
+  // max_kv_len 0: not known, inside a graph: the CTAs look for themselves whether a row is long (a replayed step of 64 requests of 50 to 100 keys 1,363 us
+  // without the order, 1,390 with lengths compared whatever they are, 1,369 so; of 200 to 400 1,661, 1,671, 1,662).
+  const int longest_first = (max_kv_len == 0 || max_kv_len > DC_LONG) && num_splits == 1 && num_rows > 1 && num_rows <= DC_THREADS && num_rows * (int)grid.z > sm_count();
   MS_LAUNCH(decode_form(tma, ex, longest_first), grid, DC_THREADS, decode_smem(tma), stream,
       map_k, map_v, status, (__nv_bfloat16*)out, (float*)part_o, (float*)part_ml, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
       (const __nv_bfloat16*)v_pool, kv_len, page_indptr, page_indices, nq, nkv, scale * LOG2E, window, sink,

@@ -493,14 +493,19 @@ def test_attention_bf16_decode_copies_by_rows_and_splits(rows, splits, page, cop
 
 
 @pytest.mark.parametrize("nq, nkv, d, page, copies", [(8, 8, 64, 16, True), (8, 8, 128, 16, True), (8, 8, 128, 8, False), (8, 8, 48, 16, False)])
-def test_attention_bf16_decode_takes_the_longest_rows_first(nq, nkv, d, page, copies, monkeypatch):
-    """More items than multiprocessors, one CTA each, of rows of all lengths (some alike) in no order: every row comes out once, as the reference has it."""
-    rows = [((733 * i) % 901 if i % 5 else 600, 1) for i in range(45)]
+@pytest.mark.parametrize("longest", [900, 513, 512, 40])
+@pytest.mark.parametrize("known", [True, False])
+def test_attention_bf16_decode_takes_the_longest_rows_first(nq, nkv, d, page, copies, longest, known, monkeypatch):
+    """More items than multiprocessors, one CTA each, of rows of all lengths (some alike) in no order: every row comes out once, as the reference has it. Up to
+    512 keys the grid's order stays, which the kernel sees for itself where the host does not know the lengths (inside a graph)."""
+    rows = [((733 * i) % longest if i % 5 else min(600, longest - 1), 1) for i in range(45)]
+    rows[7] = (longest - 1, 1)
     pb, q, ref, scale = _attention_case(torch.bfloat16, rows, nq, nkv, d, page, seed=d)
     assert len(rows) * nkv > torch.cuda.get_device_properties(0).multi_processor_count
     monkeypatch.setattr(attention_bf16, "choose_splits", lambda *a, **k: 1)
-    ran, out = _forms_that_run(monkeypatch, d), torch.full_like(q, float("nan"))
-    attention_bf16.run_decode(out, q, pb.k_pool, pb.v_pool, make_context(pb), 0, scale, None, len(rows))
+    ran, out, ctx = _forms_that_run(monkeypatch, d), torch.full_like(q, float("nan")), make_context(pb)
+    ctx.graph_bucket = 0 if known else len(rows)
+    attention_bf16.run_decode(out, q, pb.k_pool, pb.v_pool, ctx, 0, scale, None, len(rows))
     assert ran == [copies] and torch.allclose(out.float(), ref, **BF16_TOL)
 
 
