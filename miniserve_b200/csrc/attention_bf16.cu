@@ -478,7 +478,8 @@ __device__ __forceinline__ void decode_slice(float (&o)[DTILES][4], float (&m_ru
 
 // ORDER: the form that can take the longest requests' items first. Splits through scratch, which are never taken in that order, run the general
 // form without that code (a replayed step of one request, us, with it / without: 8,192 keys 1,157 / 1,146, 16,384 1,316 / 1,296, 32,768 1,621 / 1,602);
-// clusters of splits run the form with it, unasked (2 requests of 2,048 keys 912 / 919, 4 of 6,000 1,295 / 1,302).
+// clusters of splits run the form with it, unasked (2 requests of 2,048 keys 912 / 919, 4 of 6,000 1,295 / 1,302). One more form in the library is not
+// free for the others: the step of 8 requests around 2,048 keys, whose kernel is the same, takes 1,094 us without it and 1,095 to 1,106 with it.
 template <bool TMA, bool EX, bool ORDER>
 __global__ void __launch_bounds__(DC_THREADS)
 attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int* __restrict__ status,
