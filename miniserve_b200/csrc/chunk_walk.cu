@@ -1,4 +1,4 @@
-// The recurrences of ``recurrence.cu`` over a prompt by chunks of 16 tokens, in float32.
+// The recurrences of ``recurrence.cu`` over a prompt by chunks of 16 tokens, in float32; the decay rule over long rows goes to ``tile_walk.cu``.
 //
 //   decay rule:  S <- diag(d_t) S + k_t v_t^T;                                                   o_t = S^T q_t
 //   delta rule:  S <- diag(d_t) S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;           o_t = S^T q_t
@@ -33,6 +33,8 @@
 #include <cfloat>
 
 #include "chunk_mma.cuh"
+#include "float_pairs.cuh"
+#include "tile_walk.cuh"
 
 namespace ms {
 
@@ -41,29 +43,6 @@ constexpr int WK_CHAIN = 2, WK_OUT = 4, WK_OWN = 8;          // warps of the wal
 enum WalkMode : int { WALK_CHANNEL = 0, WALK_DELTA = 1, WALK_HEAD = 2 };
 
 __device__ __forceinline__ float wk_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
-
-// two neighbouring floats in a register pair: each half rounds as the plain instruction does
-using wk_f2 = unsigned long long;
-__device__ __forceinline__ void wk_fma2(wk_f2& d, wk_f2 a, wk_f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
-__device__ __forceinline__ wk_f2 wk_mul2(wk_f2 a, wk_f2 b) {
-  wk_f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ wk_f2 wk_pair(float x, float y) {
-  wk_f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float2 wk_halves(wk_f2 x) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
-  return r;
-}
-__device__ __forceinline__ float wk_sum2(wk_f2 x) {
-  const float2 h = wk_halves(x);
-  return h.x + h.y;
-}
 
 // ---------------------------------------------------------------- the chunks of a step
 // A row of n tokens has ceil(n / 16) chunks, numbered row by row. Every warp finds its own by adding up over the rows, 32 at a time: a table
@@ -153,27 +132,27 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
   const size_t item = (size_t)chunk * H + h;
   {
     const int cl = lane & 7, j = warp * 4 + (lane >> 3);
-    wk_f2 p[2 * N] = {};
+    f2 p[2 * N] = {};
     double val[32];
 #pragma unroll
     for (int i = 0; i < WK_TOK; ++i) {
-      wk_f2 a = 0ull, b = 0ull;
+      f2 a = 0ull, b = 0ull;
 #pragma unroll
       for (int m = 0; m < N; ++m) {
         const ulonglong2 fk = *reinterpret_cast<const ulonglong2*>(&ks[i][cl * 4 + 32 * m]);
         const ulonglong2 fq = *reinterpret_cast<const ulonglong2*>(&qs[i][cl * 4 + 32 * m]);
         const ulonglong2 fd = *reinterpret_cast<const ulonglong2*>(&ds[i][cl * 4 + 32 * m]);
-        p[2 * m] = i == j ? fk.x : wk_mul2(p[2 * m], fd.x);  // (nothing ahead of token j)
-        p[2 * m + 1] = i == j ? fk.y : wk_mul2(p[2 * m + 1], fd.y);
+        p[2 * m] = i == j ? fk.x : f2_mul(p[2 * m], fd.x);  // (nothing ahead of token j)
+        p[2 * m + 1] = i == j ? fk.y : f2_mul(p[2 * m + 1], fd.y);
         if (DELTA) {
-          wk_fma2(a, fk.x, p[2 * m]);
-          wk_fma2(a, fk.y, p[2 * m + 1]);
+          f2_fma(a, fk.x, p[2 * m]);
+          f2_fma(a, fk.y, p[2 * m + 1]);
         }
-        wk_fma2(b, fq.x, p[2 * m]);
-        wk_fma2(b, fq.y, p[2 * m + 1]);
+        f2_fma(b, fq.x, p[2 * m]);
+        f2_fma(b, fq.y, p[2 * m + 1]);
       }
-      val[i] = wk_sum2(a);
-      val[16 + i] = wk_sum2(b);
+      val[i] = f2_sum(a);
+      val[16 + i] = f2_sum(b);
     }
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
@@ -263,9 +242,9 @@ __device__ __forceinline__ void wk_cp(float* dst, const float* src, bool in) {
 
 // a lane's 2 N channels of a row of DKP in shared memory: two for N = 1, else fours that are 64 apart
 template <int N>
-__device__ __forceinline__ void wk_row(wk_f2 (&x)[N], const float* row, int l) {
+__device__ __forceinline__ void wk_row(f2 (&x)[N], const float* row, int l) {
   if constexpr (N == 1) {
-    x[0] = *reinterpret_cast<const wk_f2*>(row + 2 * l);
+    x[0] = *reinterpret_cast<const f2*>(row + 2 * l);
   } else {
 #pragma unroll
     for (int m = 0; m < N / 2; ++m) {
@@ -283,18 +262,18 @@ __device__ __forceinline__ int wk_channel(int l, int pair, int half) {
 // The products of a lane's columns with ROWS rows, summed over the column's lanes: lane l comes back with row l's. (Eight rows: lanes l and l ^ 8
 // with two parts of row l & 7's.) A lane takes row i ^ l as its i-th, so that what it keeps of an exchange is always the first half of its sums.
 template <int N, int C, int ROWS>
-__device__ __forceinline__ void wk_against(float (&d)[C], const wk_f2 (&S)[C][N], const float* rows, int l) {
+__device__ __forceinline__ void wk_against(float (&d)[C], const f2 (&S)[C][N], const float* rows, int l) {
   float val[C][ROWS];
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
-    wk_f2 x[N], a[C] = {};
+    f2 x[N], a[C] = {};
     wk_row<N>(x, rows + (i ^ (l & (ROWS - 1))) * (32 * N), l);
 #pragma unroll
     for (int p = 0; p < N; ++p)
 #pragma unroll
-      for (int c = 0; c < C; ++c) wk_fma2(a[c], S[c][p], x[p]);
+      for (int c = 0; c < C; ++c) f2_fma(a[c], S[c][p], x[p]);
 #pragma unroll
-    for (int c = 0; c < C; ++c) val[c][i] = wk_sum2(a[c]);
+    for (int c = 0; c < C; ++c) val[c][i] = f2_sum(a[c]);
   }
 #pragma unroll
   for (int o = ROWS / 2; o > 0; o >>= 1)
@@ -377,7 +356,7 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
 #pragma unroll
     for (int s = 0; s < ST - 1; ++s) fetch(c0 + s);
   }
-  wk_f2 S[C][N];
+  f2 S[C][N];
   float* slot = state + ((size_t)state_slot[r] * H + h) * (size_t)dv * dk;
   // the chain's state into shared memory for the outputs, and from there
   auto leave = [&](int buf) {
@@ -386,7 +365,7 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
 #pragma unroll
       for (int p = 0; p < N; p += 2) {
         float* to = states + (buf * COLS + e) * DKP + wk_channel<N>(l, p, 0);
-        if constexpr (N == 1) *reinterpret_cast<wk_f2*>(to) = S[e][0];
+        if constexpr (N == 1) *reinterpret_cast<f2*>(to) = S[e][0];
         else *reinterpret_cast<ulonglong2*>(to) = make_ulonglong2(S[e][p], S[e][p + 1]);
       }
   };
@@ -402,12 +381,12 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
           const int col = v0 + mine + e, ch = wk_channel<N>(l, p, half);
           x[half] = !fresh && col < dv && ch < dk ? slot[(size_t)col * dk + ch] : 0.f;
         }
-        S[e][p] = wk_pair(x[0], x[1]);
+        S[e][p] = f2_pair(x[0], x[1]);
       }
     leave(0);
   }
   float out[C] = {};
-  wk_f2 P[WK_OWN / 2] = {};
+  f2 P[WK_OWN / 2] = {};
   const int tk0 = warp >= 2 * WK_CHAIN ? WK_OWN : 0, tk = tk0 + (l & 7), j0 = l & 8;  // an output lane's token, of whose earlier ones it takes j0 .. j0 + 7
 
 #pragma unroll 1
@@ -448,11 +427,11 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
         for (int e = 0; e < C; ++e) decayed[e * WK_TOK + l] = u[e] * f;
         uk = decayed;
       }
-      wk_f2 keep[N];
+      f2 keep[N];
       if constexpr (MODE == WALK_HEAD) {
         const float f = st[I::last + 2 * WK_TOK];
 #pragma unroll
-        for (int p = 0; p < N; ++p) keep[p] = wk_pair(f, f);
+        for (int p = 0; p < N; ++p) keep[p] = f2_pair(f, f);
       } else {
         wk_row<N>(keep, st + I::last, l);
       }
@@ -460,32 +439,32 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
       // the first half of the tokens by itself, then the state ahead of the chunk, then the other tokens one by one: half the roundings
       // of a long-lived state, and none more of one that decays fast (whose last token, then, must come behind it)
       const bool half = row_end - tok0 <= WK_TOK / 2;
-      wk_f2 next[C][N];
+      f2 next[C][N];
 #pragma unroll
       for (int e = 0; e < C; ++e)
 #pragma unroll
-        for (int p = 0; p < N; ++p) next[e][p] = half ? wk_mul2(S[e][p], keep[p]) : 0ull;
+        for (int p = 0; p < N; ++p) next[e][p] = half ? f2_mul(S[e][p], keep[p]) : 0ull;
 #pragma unroll
       for (int j = 0; j < WK_TOK; j += 4) {
         if (j == WK_TOK / 2 && !half) {
 #pragma unroll
           for (int e = 0; e < C; ++e)
 #pragma unroll
-            for (int p = 0; p < N; ++p) wk_fma2(next[e][p], S[e][p], keep[p]);
+            for (int p = 0; p < N; ++p) f2_fma(next[e][p], S[e][p], keep[p]);
         }
         float4 uj[C];
 #pragma unroll
         for (int e = 0; e < C; ++e) uj[e] = *reinterpret_cast<const float4*>(uk + e * WK_TOK + j);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          wk_f2 x[N];
+          f2 x[N];
           wk_row<N>(x, st + I::k + (j + i) * DKP, l);
 #pragma unroll
           for (int e = 0; e < C; ++e) {
             const float f = i == 0 ? uj[e].x : i == 1 ? uj[e].y : i == 2 ? uj[e].z : uj[e].w;
-            const wk_f2 twice = wk_pair(f, f);
+            const f2 twice = f2_pair(f, f);
 #pragma unroll
-            for (int p = 0; p < N; ++p) wk_fma2(next[e][p], twice, x[p]);
+            for (int p = 0; p < N; ++p) f2_fma(next[e][p], twice, x[p]);
           }
         }
       }
@@ -504,23 +483,23 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
         for (int e = 0; e < C; ++e) finite = finite && fabsf(uc[e * WK_TOK + l]) <= FLT_MAX;
         finite = __all_sync(0xffffffffu, finite);
         if (finite) {
-          wk_f2 a[C];
+          f2 a[C];
 #pragma unroll
-          for (int e = 0; e < C; ++e) a[e] = wk_pair(out[e], 0.f);
+          for (int e = 0; e < C; ++e) a[e] = f2_pair(out[e], 0.f);
 #pragma unroll
           for (int j = 0; j < WK_OWN; j += 4)
 #pragma unroll
             for (int e = 0; e < C; ++e) {
               const ulonglong2 uj = *reinterpret_cast<const ulonglong2*>(uc + e * WK_TOK + j0 + j);
-              wk_fma2(a[e], P[j / 2], uj.x);
-              wk_fma2(a[e], P[j / 2 + 1], uj.y);
+              f2_fma(a[e], P[j / 2], uj.x);
+              f2_fma(a[e], P[j / 2 + 1], uj.y);
             }
 #pragma unroll
-          for (int e = 0; e < C; ++e) out[e] = wk_sum2(a[e]);
+          for (int e = 0; e < C; ++e) out[e] = f2_sum(a[e]);
         } else {  // (zero times a later token's infinity is no zero)
 #pragma unroll
           for (int j = 0; j < WK_OWN; ++j) {
-            const float2 x = wk_halves(P[j / 2]);
+            const float2 x = f2_halves(P[j / 2]);
 #pragma unroll
             for (int e = 0; e < C; ++e)
               if (j0 + j <= tk) out[e] = fmaf(j & 1 ? x.y : x.x, uc[e * WK_TOK + j0 + j], out[e]);
@@ -555,7 +534,7 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
   for (int e = 0; e < C; ++e)
 #pragma unroll
     for (int p = 0; p < N; ++p) {
-      const float2 x = wk_halves(S[e][p]);
+      const float2 x = f2_halves(S[e][p]);
       const int col = v0 + mine + e, ch = wk_channel<N>(l, p, 0);
       if (col < dv && ch < dk) slot[(size_t)col * dk + ch] = x.x;
       if (col < dv && ch + 1 < dk) slot[(size_t)col * dk + ch + 1] = x.y;
@@ -594,22 +573,22 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
   __syncthreads();
   {  // a thread's two dot products: token i with j and with j + 8
     const int i = tid >> 3, j = tid & 7;
-    wk_f2 s0[16] = {}, s1[16] = {};  // (sums of DK / 32 products, added up in 64 bits)
+    f2 s0[16] = {}, s1[16] = {};  // (sums of DK / 32 products, added up in 64 bits)
 #pragma unroll 1
     for (int c = 0; c < DK; c += 32)
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&qs[i][c + 4 * e]), b = *reinterpret_cast<const ulonglong2*>(&ks[j][c + 4 * e]),
                          d = *reinterpret_cast<const ulonglong2*>(&ks[j + 8][c + 4 * e]);
-        wk_fma2(s0[2 * e], a.x, b.x);
-        wk_fma2(s0[2 * e + 1], a.y, b.y);
-        wk_fma2(s1[2 * e], a.x, d.x);
-        wk_fma2(s1[2 * e + 1], a.y, d.y);
+        f2_fma(s0[2 * e], a.x, b.x);
+        f2_fma(s0[2 * e + 1], a.y, b.y);
+        f2_fma(s1[2 * e], a.x, d.x);
+        f2_fma(s1[2 * e + 1], a.y, d.y);
       }
     double x0 = 0.0, x1 = 0.0;
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
-      const float2 a = wk_halves(s0[e]), b = wk_halves(s1[e]);
+      const float2 a = f2_halves(s0[e]), b = f2_halves(s1[e]);
       x0 += (double)a.x + (double)a.y;
       x1 += (double)b.x + (double)b.y;
     }
@@ -721,11 +700,17 @@ using namespace ms;
 // The most chunks that a step of so many tokens in so many rows can have.
 static inline int walk_max(int tokens, int rows) { return tokens / WK_TOK + rows; }
 
-// Floats of scratch for a step of so many tokens in so many rows. per_head: one decay per head.
-MS_EXPORT long long ms_walk_scratch(int tokens, int rows, int H, int dk, int dv, int delta, int per_head) {
+// Floats of scratch for a step of so many tokens in so many rows. groups: of heads that share q and k, with one decay per head; 0: a decay per key channel.
+MS_EXPORT long long ms_walk_scratch(int tokens, int rows, int H, int dk, int dv, int delta, int groups) {
+  if (!delta && tile_walk_takes(tokens, rows, H, dk, dv, groups)) return tile_walk_scratch(tokens, rows, H, dk, dv, groups);
   const long long items = (long long)walk_max(tokens, rows) * H, dkp = dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
-  if (per_head) return items * (WK_TOK * WK_TOK + 3 * WK_TOK);
+  if (groups) return items * (WK_TOK * WK_TOK + 3 * WK_TOK);
   return items * (WK_TOK * dkp * (delta ? 3 : 2) + dkp + WK_TOK * WK_TOK + (long long)WK_TOK * (ceil_div(dv, WK_COLS) * WK_COLS));
+}
+
+// Kernels that such a step launches.
+MS_EXPORT int ms_walk_kernels(int tokens, int rows, int H, int dk, int dv, int delta, int groups) {
+  return !delta && tile_walk_takes(tokens, rows, H, dk, dv, groups) ? 3 : 2;
 }
 
 // The decay rule (delta 0) or the delta rule with a decay per key channel; operands as ms_decay_scan's, dk up to 128. o [T, H, dv] float32.
@@ -733,17 +718,21 @@ MS_EXPORT int ms_walk_scan(float* o, float* state, const void* q, int ld_q, cons
                            const void* z, int ld_z, const float* z_bias, const float* decay_coef, float z_sign, const void* beta, int ld_beta,
                            const float* v_scale, float* scratch, const int* cu_q, const int* q_start, const int* state_slot,
                            int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, int delta, int in_dtype, int z_dtype,
-                           cudaStream_t stream) {
+                           int* status, cudaStream_t stream) {
   if (num_rows == 0 || num_tokens == 0) return 0;
   MS_CHECK_ARG(dk >= 1 && dk <= 128 && dv >= 1 && H >= 1 && H <= 65535 && num_rows <= 65535, "walk_scan: %d heads of %d x %d, %d rows", H, dk, dv, num_rows);
   MS_CHECK_ARG(qk_group > 0 && H % qk_group == 0, "walk_scan: %d heads are not a multiple of the group of %d", H, qk_group);
   MS_CHECK_ARG(!delta || beta != nullptr, "walk_scan: the delta rule needs beta");
   MS_CHECK_ARG((uintptr_t)scratch % 16 == 0, "walk_scan: scratch must start on 16 bytes");
   const int max_chunks = walk_max(num_tokens, num_rows);
-#define MS_WALK(TIN, TZZ)                                                                                                                      \
-  return launch_walk_for<TIN, TZZ>(delta, dk, o, state, (const TIN*)q, ld_q, (const TIN*)k, ld_k, qk_group, (const TIN*)v, ld_v, (const TZZ*)z, ld_z, \
-                                   z_bias, decay_coef, z_sign, (const TZZ*)beta, ld_beta, v_scale, scratch, cu_q, q_start,      \
-                                   state_slot, num_rows, max_chunks, H, dk, dv, q_scale, stream)
+  const bool tiles = !delta && tile_walk_takes(num_tokens, num_rows, H, dk, dv, 0);
+#define MS_WALK(TIN, TZZ)                                                                                                                       \
+  return tiles ? tile_walk_channel<TIN, TZZ>(o, state, (const TIN*)q, ld_q, (const TIN*)k, ld_k, qk_group, (const TIN*)v, ld_v, (const TZZ*)z,   \
+                                             ld_z, z_bias, decay_coef, z_sign, v_scale, scratch, cu_q, q_start, state_slot, num_tokens,         \
+                                             num_rows, H, dk, dv, q_scale, status, stream)                                                      \
+               : launch_walk_for<TIN, TZZ>(delta, dk, o, state, (const TIN*)q, ld_q, (const TIN*)k, ld_k, qk_group, (const TIN*)v, ld_v,        \
+                                           (const TZZ*)z, ld_z, z_bias, decay_coef, z_sign, (const TZZ*)beta, ld_beta, v_scale, scratch, cu_q,  \
+                                           q_start, state_slot, num_rows, max_chunks, H, dk, dv, q_scale, stream)
   if (in_dtype == MS_F32 && z_dtype == MS_F32) MS_WALK(float, float);
   if (in_dtype == MS_F32 && z_dtype == MS_BF16) MS_WALK(float, __nv_bfloat16);
   if (in_dtype == MS_BF16 && z_dtype == MS_F32) MS_WALK(__nv_bfloat16, float);
@@ -756,12 +745,15 @@ MS_EXPORT int ms_walk_scan(float* o, float* state, const void* q, int ld_q, cons
 // bytes.
 MS_EXPORT int ms_walk_scan_head(float* o, float* state, const float* q, int ld_q, const float* k, int ld_k, int qk_group, const float* v, int ld_v,
                                 const float* decay, int ld_decay, const float* v_scale, float* scratch, const int* cu_q, const int* q_start,
-                                const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, cudaStream_t stream) {
+                                const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, int* status, cudaStream_t stream) {
   if (num_rows == 0 || num_tokens == 0) return 0;
   MS_CHECK_ARG((dk == 32 || dk == 64 || dk == 128) && dv >= 1 && H >= 1 && H <= 65535 && num_rows <= 65535, "walk_scan_head: %d heads of %d x %d", H, dk, dv);
   MS_CHECK_ARG(qk_group > 0 && H % qk_group == 0, "walk_scan_head: %d heads are not a multiple of the group of %d", H, qk_group);
   MS_CHECK_ARG((uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 && ld_q % 4 == 0 && ld_k % 4 == 0 && (uintptr_t)scratch % 16 == 0,
                "walk_scan_head: rows of q and k must start on 16 bytes");
+  if (tile_walk_takes(num_tokens, num_rows, H, dk, dv, H / qk_group))
+    return tile_walk_head(o, state, q, ld_q, k, ld_k, qk_group, v, ld_v, decay, ld_decay, v_scale, scratch, cu_q, q_start, state_slot, num_tokens, num_rows, H, dk,
+                          dv, q_scale, status, stream);
   const int max_chunks = walk_max(num_tokens, num_rows);
 #define MS_WALK(N)                                                                                                                            \
   return launch_walk_head<N>(o, state, q, ld_q, k, ld_k, qk_group, v, ld_v, decay, ld_decay, v_scale, scratch, cu_q, q_start, \

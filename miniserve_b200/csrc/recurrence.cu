@@ -1100,11 +1100,11 @@ MS_EXPORT long long ms_ssm_work(int tokens, int H, int dv, int n, int groups) {
 }
 MS_EXPORT int ms_walk_scan_head(float* o, float* state, const float* q, int ld_q, const float* k, int ld_k, int qk_group, const float* v, int ld_v,
                                 const float* decay, int ld_decay, const float* v_scale, float* scratch, const int* cu_q, const int* q_start,
-                                const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, cudaStream_t stream);
+                                const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, int* status, cudaStream_t stream);
 MS_EXPORT int ms_ssm_features(void* out, int ld_out, const void* proj, int ld_proj, float* work, float* walk_scratch, float* state, void* conv_state,
                               const float* w_conv, const float* conv_bias, const float* dt_bias, const float* coef, const float* skip, const float* norm,
                               const int* row_of_token, const int* cu_q, const int* q_start, const int* state_slot, int num_tokens, int num_rows, int H,
-                              int dv, int n, int groups, int taps, int conv_unit, int norm_parts, int decode, float eps, int dtype, cudaStream_t stream) {
+                              int dv, int n, int groups, int taps, int conv_unit, int norm_parts, int decode, float eps, int dtype, int* status, cudaStream_t stream) {
   if (num_tokens == 0) return 0;
   MS_CHECK_ARG(work != nullptr && (uintptr_t)work % 16 == 0 && groups >= 1 && H % groups == 0 && conv_unit >= 1, "ssm_features: scratch must start on 16 bytes");
   const int inner = H * dv, keys = groups * n, channels = inner + 2 * keys, item = dtype == MS_F32 ? 4 : 2;
@@ -1122,7 +1122,7 @@ MS_EXPORT int ms_ssm_features(void* out, int ld_out, const void* proj, int ld_pr
                                1.f, steps, dv, MS_F32, stream)) return rc;
   } else {
     if (int rc = ms_walk_scan_head(o, state, queries, channels, keys_at, channels, H / groups, xbc, channels, decays, H, steps, walk_scratch, cu_q, q_start, state_slot,
-                                   num_tokens, num_rows, H, n, dv, 1.f, stream)) return rc;
+                                   num_tokens, num_rows, H, n, dv, 1.f, status, stream)) return rc;
   }
   return ms_gated_group_norm(out, ld_out, o, xbc, channels, skip, in, ld_proj, norm, num_tokens, inner, norm_parts, dv, eps, dtype, stream);
 }

@@ -242,4 +242,4 @@ class StepFunction:
         if code:
             self.reset_after_fault()
             raise StepError(f"a kernel reported a fault it caught itself (code {code}: 2-3 inconsistent cache "
-                            f"metadata; 11-13, 21-24, 31-34 a bounded wait in a tensor-core pipeline ran out)")
+                            f"metadata; 11-13, 21-24, 31-34, 41-42 a bounded wait in a tensor-core pipeline ran out)")

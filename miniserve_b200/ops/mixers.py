@@ -208,7 +208,7 @@ def sum_bias(out, a, b=None, vec=None, stream=None) -> None:
 def decay_scan(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign: float, beta, ctx, heads: int, dk: int, dv: int,
                q_scale: float, delta: bool, head_decay: bool = False, v_scale=None, ones_column: bool = False, bonus=None,
                exact: bool = False) -> None:
-    """The recurrence of every row of the step, token by token (``csrc/recurrence.cu``) or by chunks of 16 (``walk_ok``), from each
+    """The recurrence of every row of the step, token by token (``csrc/recurrence.cu``) or by chunks of 16 or 64 (``walk_ok``), from each
     request's slot of ``state`` [slots, heads, dv, dk] float32 (zero where a row starts at position 0)
     and back into it; o_out [T, heads, dv] float32. q, k [T, groups*dk], v [T, heads*dv], z [T, heads*dk]
     and beta [T, heads] are 2-d views; z_bias [heads*dk], decay_coef [heads] float32.
@@ -292,7 +292,8 @@ WALK_MIN_TOKENS = 16
 
 
 def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool = False, bonus=None) -> bool:
-    """Whether ``decay_scan`` walks the step by chunks of 16 tokens (``csrc/chunk_walk.cu``): a step that is not all single tokens, heads of up
+    """Whether ``decay_scan`` walks the step by chunks of 16 tokens (``csrc/chunk_walk.cu``; long rows under
+    the decay rule of 64, ``csrc/tile_walk.cu``): a step that is not all single tokens, heads of up
     to 128 key channels, no more rows than a grid's last dimension; with one decay per head float32 operands whose rows start on 16 bytes, 32, 64
     or 128 key channels, else rows long enough."""
     t = q.shape[0]
@@ -308,25 +309,36 @@ def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool =
 
 
 @lru_cache(maxsize=256)
-def _walk_floats(*sizes) -> int:
-    return int(native.recurrence().ms_walk_scratch(*map(int, sizes)))
+def _walk_plan(*sizes) -> tuple[int, int]:
+    """(floats of scratch, kernels) of a walk over (tokens, rows, heads, dk, dv, delta, groups of heads that share a decay's q and k; 0: a
+    decay per key channel)."""
+    lib, sizes = native.recurrence(), tuple(map(int, sizes))
+    return int(lib.ms_walk_scratch(*sizes)), int(lib.ms_walk_kernels(*sizes))
+
+
+def _status(device) -> int:
+    """The device's status word (raised by a walk whose copies or products do not come)."""
+    from . import device_status
+
+    return device_status(device).data_ptr()
 
 
 def _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx, heads, dk, dv, q_scale, delta, head_decay, v_scale) -> None:
     t, rows = o_out.shape[0], ctx.num_rows
     lib = native.recurrence()
-    scratch = ctx.buffer("walk.scratch", (_walk_floats(t, rows, heads, dk, dv, delta, head_decay),), torch.float32, o_out.device)
     groups = q.shape[1] // dk
+    floats, kernels = _walk_plan(t, rows, heads, dk, dv, delta, groups if head_decay else 0)
+    scratch, status = ctx.buffer("walk.scratch", (floats,), torch.float32, o_out.device), _status(o_out.device)
     rest = (_ptr(v_scale), _ptr(scratch), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.state_slot), t, rows, heads, dk, dv, float(q_scale))
     if head_decay:
         native.recurrence_check(lib.ms_walk_scan_head(
             _ptr(o_out), _ptr(state), _ptr(q), _rows(q), _ptr(k), _rows(k), heads // groups, _ptr(v), _rows(v), _ptr(z), _rows(z), *rest,
-            ctx.stream), launches=2)
+            status, ctx.stream), launches=kernels)
         return
     native.recurrence_check(lib.ms_walk_scan(
         _ptr(o_out), _ptr(state), _ptr(q), _rows(q), _ptr(k), _rows(k), heads // groups, _ptr(v), _rows(v), _ptr(z), _rows(z), _ptr(z_bias),
-        _ptr(decay_coef), float(z_sign), _ptr(beta), 0 if beta is None else _rows(beta), *rest, int(delta), _dt(q.dtype), _dt(z.dtype), ctx.stream),
-        launches=2)
+        _ptr(decay_coef), float(z_sign), _ptr(beta), 0 if beta is None else _rows(beta), *rest, int(delta), _dt(q.dtype), _dt(z.dtype), status,
+        ctx.stream), launches=kernels)
 
 
 # The decay rule is linear in the state with a diagonal factor, so the rows of a step with many tokens that ``walk_ok`` leaves are cut into
@@ -456,12 +468,13 @@ def ssm_features(out, proj, state, conv_state, w_conv, conv_bias, dt_bias, coef,
     assert conv_state is None or (conv_state.shape[1:] == (taps - 1, channels) and conv_state.dtype == proj.dtype and conv_state.is_contiguous())
     assert conv_state is not None or taps == 1
     work = ctx.buffer("ssm.work", (_ssm_floats(t, heads, dv, n, groups),), torch.float32, proj.device)
-    walk = None if decode else ctx.buffer("walk.scratch", (_walk_floats(t, ctx.num_rows, heads, n, dv, False, True),), torch.float32, proj.device)
+    floats, kernels = (0, 1) if decode else _walk_plan(t, ctx.num_rows, heads, n, dv, False, groups)
+    walk = None if decode else ctx.buffer("walk.scratch", (floats,), torch.float32, proj.device)
     native.recurrence_check(native.recurrence().ms_ssm_features(
         out.data_ptr(), _rows(out), proj.data_ptr(), _rows(proj), work.data_ptr(), _ptr(walk), state.data_ptr(), _ptr(conv_state), w_conv.data_ptr(),
         conv_bias.data_ptr(), dt_bias.data_ptr(), coef.data_ptr(), skip.data_ptr(), norm.data_ptr(), ctx.row_of_token.data_ptr(), ctx.cu_q.data_ptr(),
         ctx.q_start.data_ptr(), ctx.state_slot.data_ptr(), t, ctx.num_rows, heads, dv, n, groups, taps, conv_unit, norm_parts, decode, eps,
-        _dt(proj.dtype), ctx.stream), launches=4 if decode else 5 + (conv_state is not None))
+        _dt(proj.dtype), _status(proj.device), ctx.stream), launches=4 if decode else 3 + kernels + (conv_state is not None))
     return True
 
 

@@ -175,7 +175,7 @@ def recurrence():
     _declare(lib, "ms_ssm_step_decay", [_p, _p, _i, _p, _p, _i, _i, _i, _p])
     _declare(lib, "ms_gated_group_norm", [_p, _i, _p, _p, _i, _p, _p, _i, _p, _i, _i, _i, _i, _f, _i, _p])
     _declare(lib, "ms_ssm_work", [_i] * 5, _ll)
-    _declare(lib, "ms_ssm_features", [_p, _i, _p, _i] + [_p] * 14 + [_i] * 10 + [_f, _i, _p])
+    _declare(lib, "ms_ssm_features", [_p, _i, _p, _i] + [_p] * 14 + [_i] * 10 + [_f, _i, _p, _p])
     _declare(lib, "ms_conv_state_update", [_p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _p])
     _declare(lib, "ms_head_norm_gate", [_p, _i, _p, _p, _p, _i, _i, _i, _i, _f, _f, _i, _i, _i, _p])
     _declare(lib, "ms_mlstm_gates", [_p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _i, _i, _i, _f, _i, _i, _p])
@@ -183,8 +183,9 @@ def recurrence():
     _declare(lib, "ms_conv_bias", [_p, _p, _i, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p])
     _declare(lib, "ms_chunk_max", [_i, _i])
     _declare(lib, "ms_walk_scratch", [_i] * 7, _ll)
-    _declare(lib, "ms_walk_scan", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p, _f, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _i, _i, _i, _p])
-    _declare(lib, "ms_walk_scan_head", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _p])
+    _declare(lib, "ms_walk_kernels", [_i] * 7)
+    _declare(lib, "ms_walk_scan", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p, _f, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _i, _i, _i, _p, _p])
+    _declare(lib, "ms_walk_scan_head", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _p, _p])
     _declare(lib, "ms_chunk_supports", [_i, _i])
     _declare(lib, "ms_chunk_table", [_p, _p, _p, _i, _p])
     _declare(lib, "ms_chunk_scan", [_p, _i, _p, _p, _i, _p, _i, _i, _p, _i] + [_p] * 11 + [_i] * 5 + [_f, _i, _p])
