@@ -39,7 +39,7 @@
 namespace ms {
 
 constexpr int WK_TOK = 16, WK_THREADS = 128, WK_COLS = 16;  // (WK_THREADS: of the kernels ahead of the walk; WK_COLS: what u0 is padded to)
-constexpr int WK_CHAIN = 2, WK_OUT = 4, WK_OWN = 8;          // warps of the walk's chain, of its outputs, an output warp's tokens
+constexpr int WK_CHAIN = 2, WK_OUT = 4, WK_FETCH = 2, WK_OWN = 8;  // warps of the walk's chain, of its outputs, of its copies; an output warp's tokens
 enum WalkMode : int { WALK_CHANNEL = 0, WALK_DELTA = 1, WALK_HEAD = 2 };
 
 __device__ __forceinline__ float wk_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
@@ -285,14 +285,14 @@ __device__ __forceinline__ void wk_against(float (&d)[C], const f2 (&S)[C][N], c
   for (int c = 0; c < C; ++c) d[c] = val[c][0];
 }
 
-template <int MODE, int N, int C>
-__global__ void __launch_bounds__((WK_CHAIN + WK_OUT) * 32, C == 4 ? 2 : 1)
+template <int MODE, int N, int C, bool APART>
+__global__ void __launch_bounds__((WK_CHAIN + WK_OUT + (APART ? WK_FETCH : 0)) * 32, C == 4 ? 2 : 1)
 walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __restrict__ qp, int ld_q, const float* __restrict__ wp,
             const float* __restrict__ kp, int ld_k, int qk_group, const float* __restrict__ dec, const float* __restrict__ v, int ld_v,
             const float* __restrict__ v_scale, const float* __restrict__ pairs, const int* __restrict__ cu_q, const int* __restrict__ q_start,
             const int* __restrict__ state_slot, int H, int dk, int dv) {
   using I = WalkStage<MODE, N, C>;
-  constexpr int DKP = I::dkp, COLS = I::cols, ST = I::stages, FETCHERS = WK_OUT * 32;
+  constexpr int DKP = I::dkp, COLS = I::cols, ST = I::stages, FETCHERS = (APART ? WK_FETCH : WK_OUT) * 32;
   extern __shared__ __align__(16) float wk_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = lane & 15;
   const int v0 = blockIdx.x * COLS, h = blockIdx.y, r = blockIdx.z;
@@ -306,7 +306,7 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
   float* us = wk_smem + ST * I::floats + I::states + mine * WK_TOK;       // [2][COLS][16]: u of a chunk
   float* decayed = wk_smem + ST * I::floats + I::states + I::us + mine * WK_TOK;  // (head mode) [COLS][16]: u decayed to the chunk's end
 
-  const int ft = tid - WK_CHAIN * 32;  // (the output warps fetch)
+  const int ft = tid - (APART ? WK_CHAIN + WK_OUT : WK_CHAIN) * 32;  // (APART: warps that only fetch; else the output warps do)
   auto fetch = [&](int c) {  // (nothing behind the row's last chunk; the group is committed all the same)
     if (c < c1) {
       float* st = wk_smem + (size_t)((c - c0) % ST) * I::floats;
@@ -352,9 +352,18 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
     cs_commit();
   };
 
-  if (!chain) {
+  if (APART ? warp >= WK_CHAIN + WK_OUT : !chain) {
 #pragma unroll
     for (int s = 0; s < ST - 1; ++s) fetch(c0 + s);
+  }
+  if (APART && warp >= WK_CHAIN + WK_OUT) {
+#pragma unroll 1
+    for (int c = c0; c <= c1; ++c) {
+      cs_wait<ST - 2>();
+      __syncthreads();  // (the one below)
+      if (c < c1) fetch(c + ST - 1);
+    }
+    return;
   }
   f2 S[C][N];
   float* slot = state + ((size_t)state_slot[r] * H + h) * (size_t)dv * dk;
@@ -392,7 +401,7 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
 #pragma unroll 1
   for (int c = c0; c <= c1; ++c) {  // (one more trip for the last chunk's outputs)
     const int buf = (c - c0) & 1, tok0 = row_begin + (c - c0) * WK_TOK;
-    if (!chain) cs_wait<ST - 2>();
+    if (!APART && !chain) cs_wait<ST - 2>();
     __syncthreads();  // the chunk has come, and every warp is done with the stage that the next fetch fills
     const float* st = wk_smem + (size_t)((c - c0) % ST) * I::floats;
     if (chain) {
@@ -475,7 +484,7 @@ walk_kernel(float* __restrict__ o, float* __restrict__ state, const float* __res
       leave(buf ^ 1);
       __syncwarp();  // (u is read to the end before the next chunk's takes its place)
     } else {
-      fetch(c + ST - 1);
+      if (!APART) fetch(c + ST - 1);
       if (c > c0) {  // the chunk before: P U
         const float* uc = us + (buf ^ 1) * COLS * WK_TOK;
         bool finite = true;
@@ -624,22 +633,26 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
 
 // Dynamic shared memory beyond 48 KB is asked for once per kernel and device. Not a dependent launch: CTAs that become resident while the kernel
 // before drains gather on the SMs that are free first, and two chains on one SM walk at half the rate.
-#define MS_WALK_LAUNCH(MODE, N, C, ...)                                                                                     \
+#define MS_WALK_LAUNCH(MODE, N, C, APART, ...)                                                                                     \
   do {                                                                                                                      \
-    auto walk = walk_kernel<MODE, N, C>;                                                                                    \
+    auto walk = walk_kernel<MODE, N, C, APART>;                                                                                    \
     constexpr size_t bytes = WalkStage<MODE, N, C>::bytes;                                                                  \
     static std::atomic<unsigned long long> allowed{0};                                                                      \
     MS_CHECK_CUDA(allow_shared_memory((const void*)walk, (int)bytes, allowed));                                             \
-    MS_LAUNCH_APART(walk, dim3(ceil_div(dv, WalkStage<MODE, N, C>::cols), H, num_rows), (WK_CHAIN + WK_OUT) * 32, bytes, stream, __VA_ARGS__); \
+    MS_LAUNCH_APART(walk, dim3(ceil_div(dv, WalkStage<MODE, N, C>::cols), H, num_rows), (WK_CHAIN + WK_OUT + (APART ? WK_FETCH : 0)) * 32, bytes, stream, __VA_ARGS__); \
   } while (0)
 // Four columns a lane take half the reads from shared memory of two, but half the CTAs too: two until 16 columns a CTA leave two SMs of three
 // one. Both kernels, 2,048 tokens, two columns against four, us: 64 CTAs of 16 columns (16 heads of 64 x 64, delta rule) 140 / 169, (8 of 64 x 128,
 // decay rule) 107 / 126; 128 of them (32 of 64 x 64, delta rule) 242 / 221, (32 of 128 x 64, a decay per head) 219 / 191; 768 (three rows, 64
 // of 128 x 64) 396 / 254.
+// Where every CTA has a multiprocessor of its own (two columns), two more warps fetch: the output warps, which fetch elsewhere, were what a chunk waited for
+// (1,640 cycles against 1,330 of the chain): 16 heads of 64 x 64, 2,048 tokens 136 -> 127, 8 of 64 x 128, 300 tokens 23.2 -> 21.5. With several CTAs a
+// multiprocessor they only take issue slots (64 of 128 x 64, 64 rows of 32 tokens 319 -> 371).
 #define MS_WALK_LAUNCH_FOR(MODE, N, ...)                                                                                            \
   do {                                                                                                                              \
-    if (3ll * num_rows * H * ceil_div(dv, WalkStage<MODE, N, 4>::cols) >= 2ll * sms) MS_WALK_LAUNCH(MODE, N, 4, __VA_ARGS__);       \
-    else MS_WALK_LAUNCH(MODE, N, 2, __VA_ARGS__);                                                                                   \
+    if (3ll * num_rows * H * ceil_div(dv, WalkStage<MODE, N, 4>::cols) >= 2ll * sms) MS_WALK_LAUNCH(MODE, N, 4, false, __VA_ARGS__); \
+    else if (1ll * num_rows * H * ceil_div(dv, WalkStage<MODE, N, 2>::cols) <= sms) MS_WALK_LAUNCH(MODE, N, 2, true, __VA_ARGS__);  \
+    else MS_WALK_LAUNCH(MODE, N, 2, false, __VA_ARGS__);                                                                            \
   } while (0)
 
 template <typename TIn, typename TZ, bool DELTA, int N>
