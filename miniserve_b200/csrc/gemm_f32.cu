@@ -64,33 +64,41 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
   }
 }
 
-// The same products in larger tiles: BM x 128 outputs a CTA, 8 x 8 a thread, k in steps of 16 through two shared-memory buffers, the next
-// step's operands on their way in registers, two neighbouring columns a multiply-add instruction (fma.rn.f32x2: each half rounds as fmaf
-// does). The order of an element's sum is the same. Needs rows that start on 16 bytes.
+// The same products in tiles of BM x BN outputs a CTA, TM x TN a thread, k in steps of GK through two shared-memory buffers, the next step's
+// operands on their way in registers, two neighbouring columns a multiply-add instruction (fma.rn.f32x2: each half rounds as fmaf does).
+// The order of an element's sum is the same in all of them. Needs rows that start on 16 bytes.
 // Bound by FFMA issue (34 TFMA/s on the whole GPU) beside shared-memory reads: a thread's 16 operands for 64 products are what keeps
-// the two even; at 4 x 4 the reads take twice the products' time. 700 rows: 1024 -> 4096
-// columns 151 us against 262 at 4 x 4, 2048 -> 1024 113 / 208, 1024 -> 6144 207 / 401, 3072 -> 1024 165 / 311; one column an instruction: 184, 172,
-// 224, 255 (a warp alone on its scheduler issues every second cycle).
-constexpr int GK = 16, GBN2 = 128;
-template <int BM>
-__global__ void __launch_bounds__(BM * 2, BM == 128 ? 2 : 3)
+// the two even; at 4 x 4 the reads take twice the products' time. Where there are fewer tiles than multiprocessors a product takes as long as
+// one CTA does, so the tile's own outputs count: at 80 x 64 and k in steps of 32 (16: the next step's loads come back after the products of
+// this one, 87 us) 700 rows 2048 -> 1024 columns 82 us against 111 at 64 x 128 and 281 at 4 x 4 in one buffer, 3072 -> 1024 122 / 160 / 421;
+// 1024 -> 4096 146, 1024 -> 6144 191 (tiles of 128 x 128: 203). 32 x 64 and 32 x 32 for some hundred outputs a multiprocessor (100 rows
+// 2048 -> 1024 39 us, 64 x 128: 111), 8 x 64 for the few rows of a decode step (8 rows 1024 -> 151936 184 us, 32 x 64: 357).
+template <int BM, int BN, int TM, int TN, int GK>
+struct GfTile {
+  static constexpr int tx = BN / TN, ty = BM / TM, threads = tx * ty;
+  static constexpr int blocks = TM * TN >= 40 ? 3 : threads >= 128 ? 5 : 8;  // a multiprocessor's
+  static_assert((TM == 8 || TM == 5 || TM == 4) && (TN == 8 || TN == 4) && BM % TM == 0 && BN % TN == 0 && threads % (GK / 4) == 0);
+};
+template <int BM, int BN, int TM, int TN, int GK>
+__global__ void __launch_bounds__((GfTile<BM, BN, TM, TN, GK>::threads), (GfTile<BM, BN, TM, TN, GK>::blocks))
 gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K, int lda, int ldw, int ldc,
                       long long stride_a, long long stride_w, long long stride_c) {
-  constexpr int THREADS = BM * 2, LA = BM * GK / 4 / THREADS, LW = GBN2 * GK / 4 / THREADS;  // pieces of 16 bytes a thread
-  static_assert(LA * THREADS * 4 == BM * GK && LW * THREADS * 4 == GBN2 * GK, "whole pieces a thread");
-  __shared__ __align__(16) float as[2][GK][BM + 4], ws[2][GK][GBN2 + 4];
+  using I = GfTile<BM, BN, TM, TN, GK>;
+  constexpr int THREADS = I::threads, PA = BM * GK / 4, PW = BN * GK / 4, LA = (PA + THREADS - 1) / THREADS, LW = (PW + THREADS - 1) / THREADS;  // pieces of 16 bytes
+  __shared__ __align__(16) float as[2][GK][BM + 4], ws[2][GK][BN + 4];
   pdl_prologue();
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * GBN2;
+  const int tid = threadIdx.x, tx = tid % I::tx, ty = tid / I::tx;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   A += blockIdx.z * stride_a;
   W += blockIdx.z * stride_w;
   C += blockIdx.z * stride_c;
-  const int pr = tid >> 2, pk = (tid & 3) * 4;
+  const int pk = tid % (GK / 4) * 4;  // (THREADS is a multiple of GK / 4: the same for all of a thread's pieces)
+  auto row_of = [&](int i) { return (tid + i * THREADS) / (GK / 4); };
   const float *ap[LA], *wp[LW];  // (rows behind the end read the last one: what comes of them is not stored)
 #pragma unroll
-  for (int i = 0; i < LA; ++i) ap[i] = A + (size_t)min(m0 + pr + i * (THREADS / 4), M - 1) * lda + pk;
+  for (int i = 0; i < LA; ++i) ap[i] = A + (size_t)min(m0 + min(row_of(i), BM - 1), M - 1) * lda + pk;
 #pragma unroll
-  for (int i = 0; i < LW; ++i) wp[i] = W + (size_t)min(n0 + pr + i * (THREADS / 4), N - 1) * ldw + pk;
+  for (int i = 0; i < LW; ++i) wp[i] = W + (size_t)min(n0 + min(row_of(i), BN - 1), N - 1) * ldw + pk;
   float4 ra[LA], rw[LW];
   auto load = [&](int k0) {
     if (k0 + GK <= K) {
@@ -112,20 +120,22 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
   auto put = [&](int buf) {
 #pragma unroll
     for (int i = 0; i < LA; ++i) {
-      float* p = &as[buf][pk][pr + i * (THREADS / 4)];
+      if (PA % THREADS != 0 && i == LA - 1 && tid + i * THREADS >= PA) break;
+      float* p = &as[buf][pk][row_of(i)];
       p[0] = ra[i].x; p[BM + 4] = ra[i].y; p[2 * (BM + 4)] = ra[i].z; p[3 * (BM + 4)] = ra[i].w;
     }
 #pragma unroll
     for (int i = 0; i < LW; ++i) {
-      float* p = &ws[buf][pk][pr + i * (THREADS / 4)];
-      p[0] = rw[i].x; p[GBN2 + 4] = rw[i].y; p[2 * (GBN2 + 4)] = rw[i].z; p[3 * (GBN2 + 4)] = rw[i].w;
+      if (PW % THREADS != 0 && i == LW - 1 && tid + i * THREADS >= PW) break;
+      float* p = &ws[buf][pk][row_of(i)];
+      p[0] = rw[i].x; p[BN + 4] = rw[i].y; p[2 * (BN + 4)] = rw[i].z; p[3 * (BN + 4)] = rw[i].w;
     }
   };
-  unsigned long long acc[8][4];  // two columns each
+  unsigned long long acc[TM][TN / 2];  // two columns each
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
   load(0);
   put(0);
   __syncthreads();
@@ -135,19 +145,23 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
     if (more) load(k0 + GK);
 #pragma unroll
     for (int kk = 0; kk < GK; ++kk) {
-      float a[8];
-      ulonglong2 w[2];
+      float a[TM];
+      unsigned long long wj[TN / 2];
       *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&as[buf][kk][ty * 4]);
-      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&as[buf][kk][BM / 2 + ty * 4]);
-      w[0] = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][tx * 4]);
-      w[1] = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][GBN2 / 2 + tx * 4]);
-      const unsigned long long wj[4] = {w[0].x, w[0].y, w[1].x, w[1].y};
+      if constexpr (TM == 8) *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&as[buf][kk][BM / 2 + ty * 4]);
+      else if constexpr (TM == 5) a[4] = as[buf][kk][4 * I::ty + ty];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int h = 0; h < TN / 4; ++h) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][h * (4 * BN / TN) + tx * 4]);
+        wj[2 * h] = w.x;
+        wj[2 * h + 1] = w.y;
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
         unsigned long long twice;
         asm("mov.b64 %0, {%1, %1};" : "=l"(twice) : "f"(a[i]));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(twice), "l"(wj[j]));
+        for (int j = 0; j < TN / 2; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(twice), "l"(wj[j]));
       }
     }
     if (more) put(buf ^ 1);
@@ -155,12 +169,12 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
   }
   const bool wide = ldc % 4 == 0 && stride_c % 4 == 0 && (uintptr_t)C % 16 == 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int m = m0 + (i >> 2) * (BM / 2) + ty * 4 + (i & 3);
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + (i < 4 ? ty * 4 + i : TM == 8 ? BM / 2 + ty * 4 + i - 4 : 4 * I::ty + ty);
     if (m >= M) continue;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int n = n0 + half * (GBN2 / 2) + tx * 4;
+    for (int half = 0; half < TN / 4; ++half) {
+      const int n = n0 + half * (4 * BN / TN) + tx * 4;
       float f[4];
       asm("mov.b64 {%0, %1}, %2;" : "=f"(f[0]), "=f"(f[1]) : "l"(acc[i][2 * half]));
       asm("mov.b64 {%0, %1}, %2;" : "=f"(f[2]), "=f"(f[3]) : "l"(acc[i][2 * half + 1]));
@@ -176,29 +190,41 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
   }
 }
 
-// The rows of a tile: what leaves the busiest SM the fewest outputs. GBM x GBN (4 x 4 a thread, half the rate) where there are few rows
-// or columns, or rows that do not start on 16 bytes.
+// The tile: what is over first. `each` is what one more tile on the busiest multiprocessor takes and `alone` what the first takes besides (its
+// loads and barriers have nothing to run beside), both in tenths of a microsecond for 1024 k; measured over 1 to 2048 rows and 16 to 151936
+// columns they give the time to within a tenth. gemm_f32_kernel where rows do not start on 16 bytes and where the products are over before the
+// larger tiles' start is made up for: 300 rows 64 -> 1024 columns 6.6 us against 5.9.
 inline int launch_gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int batch, long long stride_a,
                            long long stride_w, long long stride_c, cudaStream_t stream) {
   const int known = sm_count(), sms = known > 0 ? known : 148;
   const bool rows16 = lda % 4 == 0 && ldw % 4 == 0 && stride_a % 4 == 0 && stride_w % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
-  auto cost = [&](int bm, int bn) {
-    const long long tiles = (long long)ceil_div(M, bm) * ceil_div(N, bn) * batch;
-    return (tiles + sms - 1) / sms * bm * bn;
-  };
-  const long long large = cost(128, GBN2), small = cost(64, GBN2);
-  // (and where the products are over before the larger tiles' start is made up for: 33 to 128 rows 64 -> 1024 columns 5.8 us against 5.2)
   const bool brief = K <= 64 && 2LL * ceil_div(M, GBM) * ceil_div(N, GBN) * batch <= sms;
-  if (!rows16 || M <= 32 || brief || 2 * cost(GBM, GBN) < (large < small ? large : small)) {
+  if (!rows16 || brief) {
     MS_LAUNCH(gemm_f32_kernel, dim3(ceil_div(N, GBN), ceil_div(M, GBM), batch), 256, 0, stream, C, A, W, M, N, K, lda, ldw, ldc, stride_a, stride_w,
               stride_c);
     return 0;
   }
-#define MS_GEMM_F32(BM)                                                                                                                         \
-  MS_LAUNCH_APART(gemm_f32_tiled_kernel<BM>, dim3(ceil_div(N, GBN2), ceil_div(M, BM), batch), BM * 2, 0, stream, C, A, W, M, N, K, lda, ldw, ldc, \
-                  stride_a, stride_w, stride_c)
-  if (large <= small) MS_GEMM_F32(128);
-  else MS_GEMM_F32(64);
+  int tile = 0;
+  long long least = -1;
+  auto weigh = [&](int which, int bm, int bn, int each, int alone) {
+    const long long tiles = (long long)ceil_div(M, bm) * ceil_div(N, bn) * batch, cost = (tiles + sms - 1) / sms * each + alone;
+    if (ceil_div(M, bm) > 65535 || (least >= 0 && cost >= least)) return;
+    tile = which;
+    least = cost;
+  };
+  weigh(0, 64, 128, 450, 110);
+  weigh(1, 80, 64, 350, 80);
+  weigh(2, 32, 64, 200, 90);
+  weigh(3, 32, 32, 115, 90);
+  weigh(4, 8, 64, 95, 140);
+#define MS_GEMM_F32(BM, BN, TM, TN, GK)                                                                                                      \
+  MS_LAUNCH_APART((gemm_f32_tiled_kernel<BM, BN, TM, TN, GK>), dim3(ceil_div(N, BN), ceil_div(M, BM), batch),                                \
+                  (GfTile<BM, BN, TM, TN, GK>::threads), 0, stream, C, A, W, M, N, K, lda, ldw, ldc, stride_a, stride_w, stride_c)
+  if (tile == 0) MS_GEMM_F32(64, 128, 8, 8, 16);
+  else if (tile == 1) MS_GEMM_F32(80, 64, 5, 8, 32);
+  else if (tile == 2) MS_GEMM_F32(32, 64, 4, 4, 32);
+  else if (tile == 3) MS_GEMM_F32(32, 32, 4, 4, 32);
+  else MS_GEMM_F32(8, 64, 4, 4, 32);
 #undef MS_GEMM_F32
   return 0;
 }
