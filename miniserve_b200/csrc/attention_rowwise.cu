@@ -126,15 +126,19 @@ attention_rowwise_kernel(T* __restrict__ out,            // [T, nq, d]
   }
 }
 
-// ---------------------------------------------------------------- the same for prompts, 64 query rows of a request at a time
+// ---------------------------------------------------------------- the same for prompts, ROWS query rows of a request at a time
 // The arithmetic of every (token, head) is the one above, operation by operation (the same bits); what differs is who does it: a CTA
-// takes 64 query rows (tokens of one request times the query heads of a kv head) and walks the key tiles once for all of them, keys and
-// values staged in shared memory by asynchronous copies a tile ahead. A warp has 16 rows from the scores to the output: a lane 4 x 4
-// scores, then the rows one after the other with a lane per key (the same exchanges as above), then 4 rows x 4 MD columns of the output.
+// takes ROWS query rows (tokens of one request times the query heads of a kv head) and walks the key tiles once for all of them, two tiles a
+// step. A warp has 8 rows from the scores to the output: a lane 4 x 4 scores (of 64 keys), then the rows of both tiles at once with a lane per key
+// (the same exchanges as above; the second tile goes on from the first one's maximum), then 4 rows x 2 MD columns of the output, tile by tile.
 // A tile in which a row sees nothing leaves the row as it is (alpha = 1, p = 0), so all rows may walk the tiles that any of them sees.
-// Bound by shared-memory reads (32 floats read for 64 products of a score tile): 700 tokens of 16 heads of 128 on 8
-// kv heads take 254 us where a warp per token and head takes 2,291, both inside a layer (every lane walking its own key's row in global memory).
-constexpr int TW_ROWS = 64, TW_KEYS = 32, TW_THREADS = 128, TW_LDS = TW_KEYS + 4;
+// Keys and values have one buffer each: the next keys come by asynchronous copies while the values are summed, the next values beside the scores.
+// Bound by a warp's chain of instructions (two CTAs a multiprocessor by shared memory, 1.7 warps a scheduler, 45 % of the issue slots), shared
+// memory's reads at a third (32 floats read for 64 products of a score tile, 12 for 32 of the output). 700 tokens of 16 heads of 128 on 8 kv heads
+// 102 us (4 warps of 16 rows, one tile a step, in the order of the grid: 255), 2048 tokens 580. On the way: 8 rows a warp and two tiles a step
+// 146; softcap and distance out of the unrolled scores and the values' loop not unrolled over the tiles (instruction fetches) 124; the order
+// of the grid 102.
+constexpr int TW_ROWS = 64, TW_KEYS = 32, TW_LDS = 2 * TW_KEYS + 4;
 
 __device__ __forceinline__ void tw_cp16(void* dst, const void* src, bool in) {
   const int bytes = in ? 16 : 0;
@@ -164,28 +168,33 @@ __device__ __forceinline__ unsigned long long tw_twice(float x) {
 }
 __device__ __forceinline__ int tw_row(int lane) { return lane >> 1; }
 
-template <int MD>  // head sizes of up to 32 MD, whole fours
-__global__ void __launch_bounds__(TW_THREADS)
+template <int MD, int ROWS>  // head sizes of up to 32 MD, whole fours
+__global__ void __launch_bounds__(ROWS * 4, 128 / (ROWS * 2))
 attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
                            const int* __restrict__ cu_q, const int* __restrict__ q_start, const int* __restrict__ page_indptr,
                            const int* __restrict__ page_indices, int num_rows, int nq, int nkv, int d, float scale, int window, int sink,
                            int page_shift, int num_pages, int* __restrict__ status, const float* __restrict__ sink_values, float softcap, int chunk,
-                           const float* __restrict__ dist_r1, const float* __restrict__ dist_r2, int keep_first) {
-  constexpr int LD = 32 * MD + 4;
+                           const float* __restrict__ dist_r1, const float* __restrict__ dist_r2, int keep_first, int sms) {
+  constexpr int LD = 32 * MD + 4, WARPS = ROWS / 8, MC = (MD + 1) / 2, MINE = 2 * TW_KEYS / WARPS;  // MINE: keys of a step that a warp stages
+  static_assert(MINE <= 32);
   extern __shared__ __align__(16) float tw_smem[];
-  float* qs = tw_smem;                        // [64][LD]
-  float* ks = qs + TW_ROWS * LD;              // [2][32][LD]
-  float* vs = ks + 2 * TW_KEYS * LD;          // [2][32][LD]
-  float* ss = vs + 2 * TW_KEYS * LD;          // [64][TW_LDS]
-  float* alphas = ss + TW_ROWS * TW_LDS;      // [64]
-  unsigned* seen = reinterpret_cast<unsigned*>(alphas + TW_ROWS);  // [64]
+  float* qs = tw_smem;                  // [ROWS][LD]
+  float* ks = qs + ROWS * LD;           // [64][LD]
+  float* vs = ks + 2 * TW_KEYS * LD;    // [64][LD] (read to column 64 MC: what lies behind a row is not stored)
+  float* ss = vs + 2 * TW_KEYS * LD;    // [ROWS][TW_LDS]
+  float* alphas = ss + ROWS * TW_LDS;   // [2][ROWS]
+  unsigned* seen = reinterpret_cast<unsigned*>(alphas + 2 * ROWS);  // [2][ROWS]
   __shared__ int s_row, s_tile;
-  __shared__ int usable[2][TW_KEYS];
+  __shared__ int usable[2][2 * TW_KEYS];
   pdl_prologue();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int group = nq / nkv, per_tile = TW_ROWS / group, kvh = blockIdx.y;
-  if (warp == 0) {  // which request and which of its tiles: the late (long) tiles first
-    int want = gridDim.x - 1 - blockIdx.x, row = -1, base = 0;
+  const int group = nq / nkv, per_tile = ROWS / group;
+  // The late (long) tiles first, all kv heads of one tile side by side; those that share a multiprocessor with the first `sms` the other way
+  // round, so that the longest has the shortest of them beside it.
+  const int place_in_grid = (int)blockIdx.x >= sms && (int)blockIdx.x < 2 * sms && 2 * sms <= (int)gridDim.x ? 3 * sms - 1 - (int)blockIdx.x : (int)blockIdx.x;
+  const int kvh = place_in_grid % nkv;
+  if (warp == 0) {  // which request and which of its tiles
+    int want = (int)gridDim.x / nkv - 1 - place_in_grid / nkv, row = -1, base = 0;
     for (int r0 = 0; r0 < num_rows && row < 0; r0 += 32) {
       const int r = r0 + lane;
       const int mine = r < num_rows ? (cu_q[r + 1] - cu_q[r] + per_tile - 1) / per_tile : 0;
@@ -214,10 +223,11 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
   if (row < 0) return;
   const int t0 = cu_q[row] + s_tile * per_tile, n_tok = min(per_tile, cu_q[row + 1] - t0);
   const int pos0 = q_start[row] + s_tile * per_tile, pos_last = pos0 + n_tok - 1;
-  const int rows = n_tok * group;  // of the 64
+  const int rows = n_tok * group;  // of the ROWS
   const int* pages = page_indices + page_indptr[row];
   const int page_size = 1 << page_shift;
   const float inv_cap = softcap > 0.f ? 1.0f / softcap : 0.f;
+  const bool extras = softcap > 0.f || dist_r1;
   auto first_key = [&](int pos) {
     int lo = window > 0 ? max(0, pos - window + 1) : 0;
     if (chunk > 0) lo = max(lo, (pos / chunk) * chunk);
@@ -226,172 +236,221 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
   const int lo_tile = (first_key(pos0) >> 5) << 5;  // (the first token's window begins first)
   const int kept_end = keep_first > 0 ? min((keep_first + 31) & ~31, lo_tile) : 0;
   const int vec = d / 4;
-  for (int idx = tid; idx < TW_ROWS * vec; idx += TW_THREADS) {
+  for (int idx = tid; idx < ROWS * vec; idx += ROWS * 4) {
     const int r = idx / vec, c = (idx - r * vec) * 4;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < rows) x = *reinterpret_cast<const float4*>(q + ((size_t)(t0 + r / group) * nq + kvh * group + r % group) * d + c);
     *reinterpret_cast<float4*>(qs + r * LD + c) = x;
   }
-  auto stage = [&](int tile, int buf) {
-    if (tile <= pos_last) {
-      for (int idx = tid; idx < TW_KEYS * vec; idx += TW_THREADS) {
-        const int j = idx / vec, c = (idx - j * vec) * 4, kj = tile + j;
-        bool in = kj <= pos_last;
-        const int page = in ? pages[kj >> page_shift] : -1;
-        in = page >= 0;
-        MS_DEBUG_ONLY(if (in && page >= num_pages) {
-          atomicExch(status, 5);
-          in = false;
-        })
-        const size_t base = in ? (((size_t)page * nkv + kvh) * page_size + (kj & (page_size - 1))) * d + c : 0;
-        tw_cp16(ks + (buf * TW_KEYS + j) * LD + c, k_pool + base, in);
-        tw_cp16(vs + (buf * TW_KEYS + j) * LD + c, v_pool + base, in);
-        if (c == 0) usable[buf][j] = in;
-      }
+  auto next_tile = [&](int tile) { return tile + TW_KEYS == kept_end ? lo_tile : tile + TW_KEYS; };
+  // Key `lane` of the warp's own MINE (warp * MINE + lane of the step's 64): its page, asked for a step ahead, and its place in the pools;
+  // negative where there is none.
+  const int mine = warp * MINE + lane;
+  auto key_of = [&](int a, int b) { return (mine < TW_KEYS ? a : b - TW_KEYS) + mine; };
+  auto page_of = [&](int a, int b) {
+    const int kj = key_of(a, b);
+    return lane < MINE && kj <= pos_last ? pages[kj >> page_shift] : -1;
+  };
+  auto place_of = [&](int page, int a, int b) -> long long {
+    MS_DEBUG_ONLY(if (page >= num_pages) {
+      atomicExch(status, 5);
+      return -1;
+    })
+    return page < 0 ? -1 : (((long long)page * nkv + kvh) * page_size + (key_of(a, b) & (page_size - 1))) * d;
+  };
+  auto stage = [&](float* to, const float* pool, long long place) {
+    const int c = lane * 4;
+#pragma unroll
+    for (int j = 0; j < MINE; ++j) {
+      const long long at = __shfl_sync(0xffffffffu, place, j);
+      if (c < d) tw_cp16(to + (warp * MINE + j) * LD + c, pool + (at >= 0 ? at + c : 0), at >= 0);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  auto next_tile = [&](int tile) { return tile + TW_KEYS == kept_end ? lo_tile : tile + TW_KEYS; };
 
-  const int r0 = warp * 16;            // the warp's rows
-  const int qg = lane >> 3, kg = lane & 7;  // a lane's four rows r0 + 4 qg + i; its keys kg + 8 jj, its columns 4 kg + 32 m
-  float m = -INFINITY, l = 0.f;        // of row r0 + tw_row(lane)
-  unsigned long long acc[4][MD][2];    // two columns each: fma.rn.f32x2 rounds each half as fmaf does
+  const int r0 = warp * 8;                    // the warp's rows
+  const int rg = lane >> 4, kg = lane & 15;   // a lane's four rows r0 + 4 rg + i; its keys kg + 16 jj, its columns 4 kg + 64 m
+  const bool second = lane >= 16;             // of the lane's fold: row r0 + own of the step's first or second tile
+  const int own = tw_row(lane) & 7;
+  const int row_last = min(r0 + 8, rows) - 1;
+  const int see_all = pos0 + r0 / group, see_from = first_key(pos0 + row_last / group);  // keys see_from .. see_all are seen by all the warp's rows
+  float m = -INFINITY, l = 0.f;               // of row r0 + own
+  unsigned long long acc[4][MC][2];           // two columns each: fma.rn.f32x2 rounds each half as fmaf does
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int mm = 0; mm < MD; ++mm)
+    for (int mm = 0; mm < MC; ++mm)
 #pragma unroll
       for (int e = 0; e < 2; ++e) acc[i][mm][e] = 0ull;
 
-  int tile = kept_end > 0 ? 0 : lo_tile, buf = 0;
-  stage(tile, 0);
+  int tile = kept_end > 0 ? 0 : lo_tile, tile2 = next_tile(tile), after = next_tile(tile2), after2 = next_tile(after), buf = 0;
+  long long place = place_of(page_of(tile, tile2), tile, tile2);
+  if (lane < MINE) usable[0][mine] = place >= 0;
+  stage(ks, k_pool, place);
+  stage(vs, v_pool, place);
+  int page = page_of(after, after2);
 #pragma unroll 1
-  for (; tile <= pos_last; tile = next_tile(tile), buf ^= 1) {
-    stage(next_tile(tile), buf ^ 1);
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  for (; tile <= pos_last; buf ^= 1) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the keys
     __syncthreads();
     if (r0 < rows) {
-      const float* kb = ks + buf * TW_KEYS * LD;
-      const float* vb = vs + buf * TW_KEYS * LD;
-      {
-        float s[4][4] = {};
-        const float* qp = qs + (r0 + 4 * qg) * LD;
+      float s[4][4] = {};
+      const float* qp = qs + (r0 + 4 * rg) * LD;
 #pragma unroll 4
-        for (int c = 0; c < d; c += 4) {
-          float4 a[4], b[4];
+      for (int c = 0; c < d; c += 4) {
+        float4 a[4], b[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qp + i * LD + c);
+        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qp + i * LD + c);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(kb + (kg + 8 * j) * LD + c);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
-              s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
-              s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
-              s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
-            }
-        }
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (kg + 16 * j) * LD + c);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) ss[(r0 + 4 * qg + i) * TW_LDS + kg + 8 * j] = s[i][j];
+          for (int j = 0; j < 4; ++j) {
+            s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+            s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+            s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+            s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+          }
       }
-      __syncwarp();
-      const int kj = tile + lane;
-      const bool there = kj <= pos_last && usable[buf][lane];
-      float sc[16];
-      bool all_see = true, missing = false;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int r = r0 + i;
-        const int qpos = pos0 + r / group, h = kvh * group + r % group, lo = first_key(qpos);
-        const bool sees = r < rows && kj <= qpos && (kj >= lo || kj < keep_first);
-        float s = -INFINITY;
-        if (sees && there) {
-          s = ss[r * TW_LDS + lane] * scale;
-          if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
-          if (dist_r1) s -= dist_r1[h] * logf(1.0f + dist_r2[h] * (float)(qpos - kj));
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ss[(r0 + 4 * rg + i) * TW_LDS + kg + 16 * j] = s[i][j];
+    }
+    __syncthreads();  // the keys' buffer is free
+    place = place_of(page, after, after2);
+    if (lane < MINE) usable[buf ^ 1][mine] = place >= 0;
+    stage(ks, k_pool, place);
+    const int later = next_tile(after2), later2 = next_tile(later);
+    page = page_of(later, later2);
+    unsigned hidden = 0;  // bit t: a row of the warp does not see all of tile t
+    if (r0 < rows) {
+      float sc[16];
+      bool missing = false;
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int begin = t ? tile2 : tile, kj = begin + lane;
+        const bool there = kj <= pos_last && usable[buf][t * TW_KEYS + lane];
+        float* st = ss + r0 * TW_LDS + t * TW_KEYS + lane;
+        if (extras) {  // (by itself: beside the plain scores its instructions would be fetched past in every step)
+#pragma unroll 1
+          for (int i = 0; i < 8; ++i) {
+            const int r = r0 + i, h = kvh * group + r % group;
+            if (r >= rows) break;
+            float x = st[i * TW_LDS] * scale;
+            if (softcap > 0.f) x = softcap * tanhf(x * inv_cap);
+            if (dist_r1) x -= dist_r1[h] * logf(1.0f + dist_r2[h] * (float)(pos0 + r / group - kj));
+            st[i * TW_LDS] = x;
+          }
         }
-        missing = missing || (sees && !there);
-        all_see = all_see && (r >= rows || s != -INFINITY);
-        sc[i] = s;
+        const float times = extras ? 1.f : scale;
+        if (begin + TW_KEYS - 1 <= see_all && begin >= see_from) {
+          missing = missing || !there;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sc[8 * t + i] = there ? st[i * TW_LDS] * times : -INFINITY;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = r0 + i, qpos = pos0 + r / group;
+            const bool sees = r < rows && kj <= qpos && (kj >= first_key(qpos) || kj < keep_first);
+            missing = missing || (sees && !there);
+            sc[8 * t + i] = sees && there ? st[i * TW_LDS] * times : -INFINITY;
+          }
+        }
+        bool all_see = true;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) all_see = all_see && (r0 + i >= rows || sc[8 * t + i] != -INFINITY);
+        if (!__all_sync(0xffffffffu, all_see)) {
+          hidden |= 1u << t;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const unsigned mask = __ballot_sync(0xffffffffu, sc[8 * t + i] != -INFINITY);
+            if (lane == i) seen[t * ROWS + r0 + i] = mask;
+          }
+        }
       }
       if (missing) atomicExch(status, 3);
-      all_see = __all_sync(0xffffffffu, all_see);
-      if (!all_see) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const unsigned mask = __ballot_sync(0xffffffffu, sc[i] != -INFINITY);
-          if (lane == i) seen[r0 + i] = mask;
-        }
-      }
       float v[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = sc[i];
-      const float m_new = fmaxf(m, tw_fold16(v, [](float x, float y) { return fmaxf(x, y); }));
-      const float alpha = (m == -INFINITY) ? 0.f : expf(m - m_new);
+      const float top = tw_fold16(v, [](float x, float y) { return fmaxf(x, y); }), other = __shfl_xor_sync(0xffffffffu, top, 16);
+      const float m_first = fmaxf(m, second ? other : top), m_second = fmaxf(m_first, second ? top : other);
+      const float before = second ? m_first : m, m_new = second ? m_second : m_first;
+      const float alpha = (before == -INFINITY) ? 0.f : expf(before - m_new);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float mi = __shfl_sync(0xffffffffu, m_new, 2 * i);
         v[i] = (sc[i] == -INFINITY) ? 0.f : expf(sc[i] - mi);
-        ss[(r0 + i) * TW_LDS + lane] = v[i];
+        ss[(r0 + (i & 7)) * TW_LDS + (i >> 3) * TW_KEYS + lane] = v[i];
       }
-      l = l * alpha + tw_fold16(v, [](float x, float y) { return x + y; });
-      m = m_new;
-      if (!(lane & 1)) alphas[r0 + tw_row(lane)] = alpha;
-      __syncwarp();
-      float al[4];
-      unsigned mk[4];
+      const float sum = tw_fold16(v, [](float x, float y) { return x + y; });
+      const float l_first = __shfl_sync(0xffffffffu, l * alpha + sum, lane & 15);
+      l = __shfl_sync(0xffffffffu, l_first * alpha + sum, lane | 16);
+      m = m_second;
+      if (!(lane & 1)) alphas[(second ? ROWS : 0) + r0 + own] = alpha;
+    }
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the values
+    __syncthreads();
+    if (r0 < rows) {
+#pragma unroll 1
+      for (int t = 0; t < 2; ++t) {
+        if (t == 1 && tile2 > pos_last) break;
+        unsigned mk[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = r0 + 4 * qg + i;
-        al[i] = alphas[r];
-        mk[i] = all_see ? 0xffffffffu : seen[r];
-        const unsigned long long twice = tw_twice(al[i]);
+        for (int i = 0; i < 4; ++i) {
+          const int r = t * ROWS + r0 + 4 * rg + i;
+          mk[i] = (hidden >> t) & 1u ? seen[r] : 0xffffffffu;
+          const unsigned long long twice = tw_twice(alphas[r]);
 #pragma unroll
-        for (int mm = 0; mm < MD; ++mm)
+          for (int mm = 0; mm < MC; ++mm)
 #pragma unroll
-          for (int e = 0; e < 2; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][mm][e]) : "l"(twice));
-      }
-      const float* pr = ss + (r0 + 4 * qg) * TW_LDS;
-      auto values = [&](auto whole) {
+            for (int e = 0; e < 2; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][mm][e]) : "l"(twice));
+        }
+        const float* pr = ss + (r0 + 4 * rg) * TW_LDS + t * TW_KEYS;
+        const float* vt = vs + t * TW_KEYS * LD + 4 * kg;
+        auto values = [&](auto whole) {
 #pragma unroll 2
-        for (int j0 = 0; j0 < TW_KEYS; j0 += 4) {
-          float4 p[4];
+          for (int j0 = 0; j0 < TW_KEYS; j0 += 4) {
+            float4 p[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pr + i * TW_LDS + j0);
+            for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pr + i * TW_LDS + j0);
 #pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            ulonglong2 v[MD];
+            for (int jj = 0; jj < 4; ++jj) {
+              ulonglong2 v[MC];
 #pragma unroll
-            for (int mm = 0; mm < MD; ++mm) v[mm] = *reinterpret_cast<const ulonglong2*>(vb + (j0 + jj) * LD + 4 * kg + 32 * mm);
+              for (int mm = 0; mm < MC; ++mm) v[mm] = *reinterpret_cast<const ulonglong2*>(vt + (j0 + jj) * LD + 64 * mm);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
-              // (a key that a row does not see may hold anything: the row's sums must not meet it)
-              if (whole.value || ((mk[i] >> (j0 + jj)) & 1u)) {
-                const unsigned long long twice = tw_twice(pj);
+              for (int i = 0; i < 4; ++i) {
+                const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
+                // (a key that a row does not see may hold anything: the row's sums must not meet it)
+                if (whole.value || ((mk[i] >> (j0 + jj)) & 1u)) {
+                  const unsigned long long twice = tw_twice(pj);
 #pragma unroll
-                for (int mm = 0; mm < MD; ++mm) {
-                  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][mm][0]) : "l"(twice), "l"(v[mm].x));
-                  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][mm][1]) : "l"(twice), "l"(v[mm].y));
+                  for (int mm = 0; mm < MC; ++mm) {
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][mm][0]) : "l"(twice), "l"(v[mm].x));
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][mm][1]) : "l"(twice), "l"(v[mm].y));
+                  }
                 }
               }
             }
           }
-        }
-      };
-      if (all_see) values(std::true_type());
-      else values(std::false_type());
+        };
+        if ((hidden >> t) & 1u) values(std::false_type());
+        else values(std::true_type());
+      }
     }
-    __syncthreads();
+    __syncthreads();  // the values' buffer is free
+    stage(vs, v_pool, place);
+    tile = after;
+    tile2 = after2;
+    after = later;
+    after2 = later2;
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   if (r0 >= rows) return;
-  {  // the sink's term of the lane's row, as above
-    const int r = r0 + tw_row(lane);
+  if (lane < 16) {  // the sink's term of the lane's row, as above
+    const int r = r0 + own;
     float a = 1.f;
     if (sink) {
       const float s0 = sink_values ? sink_values[kvh * group + r % group] : 0.f;
@@ -407,13 +466,13 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
   __syncwarp();
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int r = r0 + 4 * qg + i;
+    const int r = r0 + 4 * rg + i;
     if (r >= rows) continue;
     const float a = alphas[r], sum = ss[r * TW_LDS];
     float* o = out + ((size_t)(t0 + r / group) * nq + kvh * group + r % group) * d;
 #pragma unroll
-    for (int mm = 0; mm < MD; ++mm) {
-      const int c = 4 * kg + 32 * mm;
+    for (int mm = 0; mm < MC; ++mm) {
+      const int c = 4 * kg + 64 * mm;
       if (c < d) {
         float4 x;
         asm("mov.b64 {%0, %1}, %2;" : "=f"(x.x), "=f"(x.y) : "l"(acc[i][mm][0]));
@@ -486,19 +545,31 @@ MS_EXPORT int ms_attention_tiled_f32(float* out, const float* q, const float* k_
                "attention: operands must start on 16 bytes");
   int page_shift = 0;
   while ((1 << page_shift) < page_size) ++page_shift;
-  const dim3 grid(num_tokens / (TW_ROWS / (nq / nkv)) + num_rows, nkv);
-#define MS_TILED_LAUNCH(MD)                                                                                                                     \
+#define MS_TILED_LAUNCH(MD, ROWS)                                                                                                               \
   do {                                                                                                                                          \
-    auto kernel = attention_tiled_f32_kernel<MD>;                                                                                               \
-    constexpr size_t smem = ((TW_ROWS + 4 * TW_KEYS) * (32 * MD + 4) + TW_ROWS * TW_LDS + 2 * TW_ROWS) * 4;                                     \
+    auto kernel = attention_tiled_f32_kernel<MD, ROWS>;                                                                                         \
+    constexpr size_t smem = ((ROWS + 4 * TW_KEYS) * (32 * MD + 4) + ROWS * TW_LDS + 4 * ROWS) * 4;                                              \
     static std::atomic<unsigned long long> allowed{0};                                                                                          \
     MS_CHECK_CUDA(allow_shared_memory((const void*)kernel, (int)smem, allowed));                                                                \
-    MS_LAUNCH_APART(kernel, grid, TW_THREADS, smem, stream, out, q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, num_rows, nq, nkv, \
-                    head_dim, scale, window, sink, page_shift, num_pages, status, sink_values, softcap, chunk, dist_r1, dist_r2, keep_first);                   \
+    const long long grid = ((long long)num_tokens / (ROWS / (nq / nkv)) + num_rows) * nkv;                                                      \
+    MS_CHECK_ARG(grid <= 0x7fffffffll, "attention: %d tokens of %d kv heads are too many for one launch", num_tokens, nkv);                     \
+    MS_LAUNCH_APART(kernel, (unsigned)grid, ROWS * 4, smem, stream, out, q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, num_rows, nq, nkv,  \
+                    head_dim, scale, window, sink, page_shift, num_pages, status, sink_values, softcap, chunk, dist_r1, dist_r2, keep_first,    \
+                    ROWS == 32 ? sms : 1 << 29);                                                                                                \
   } while (0)
-  if (head_dim <= 32) MS_TILED_LAUNCH(1);
-  else if (head_dim <= 64) MS_TILED_LAUNCH(2);
-  else MS_TILED_LAUNCH(4);
+#define MS_TILED_ROWS(MD)                     \
+  do {                                        \
+    if (small) MS_TILED_LAUNCH(MD, 32);       \
+    else MS_TILED_LAUNCH(MD, 64);             \
+  } while (0)
+  const int group = nq / nkv, known = sm_count(), sms = known > 0 ? known : 148;
+  // 64 rows only where 32 would leave more of them without a token (one CTA a multiprocessor then, and twice the chain): 700 tokens of 16 heads
+  // of 128 on 8 kv heads 146 us at 32 rows, 158 at 64, both in the plain order of the grid; 100 tokens behind 1000 170 / 228.
+  const bool small = group <= 32 && 2 * (32 / group) >= 64 / group;
+  if (head_dim <= 32) MS_TILED_ROWS(1);
+  else if (head_dim <= 64) MS_TILED_ROWS(2);
+  else MS_TILED_ROWS(4);
+#undef MS_TILED_ROWS
 #undef MS_TILED_LAUNCH
   return 0;
 }

@@ -557,7 +557,7 @@ def attention_tiled_ok(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor,
 
 def attention_tiled(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ctx, group: int, scale: float,
                     window: int | None, sink: bool = False, extras: "AttentionExtras | None" = None) -> None:
-    """``attention_rowwise`` for a step of whole rows, 64 query rows of a request at a time: the same float32 operations in the same
+    """``attention_rowwise`` for a step of whole rows, 32 (or 64) query rows of a request at a time: the same float32 operations in the same
     order for every (token, head), so the same bits."""
     _check_dev(out, q, k_pool, v_pool)
     extras = extras or NO_EXTRAS
