@@ -469,6 +469,13 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+// the same as they lie in memory, and made float32 where they are used
+template <typename T> struct Four { using raw = float4; };
+template <> struct Four<__nv_bfloat16> { using raw = uint2; };
+__device__ __forceinline__ float4 float4_of(const float4& r) { return r; }
+__device__ __forceinline__ float4 float4_of(const uint2& r) {
+  return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
+}
 __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& f) {
   uint2 v;
   *reinterpret_cast<__nv_bfloat162*>(&v.x) = __floats2bfloat162_rn(f.x, f.y);
@@ -478,14 +485,16 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& f) {
 __device__ __forceinline__ void store4(float* p, const float4& f) { *reinterpret_cast<float4*>(p) = f; }
 
 // The same for channels in fours and TAPS taps: a thread takes four channels over a run of RUN tokens, the taps and the window of
-// inputs in registers, so an input is read once. Bound by memory (2 bytes in, 4 out per channel and token): 2,048 x 6,144 bfloat16 take 33 us
-// (2.3 TB/s) where a warp per token and head takes 97; 2,048 x 2,048 with unit heads of 64 15 against 40. Heads
+// inputs in registers, so an input is read once (and three more ahead of the run). Bound by the chain of a thread (loads, exponentials, quotients)
+// and what runs beside it: 2,048 x 6,144 bfloat16 take 23.6 us (3.2 TB/s: 2 bytes in, 4 out) in runs of 4 with eight CTAs a multiprocessor (64
+// registers: inputs stay as they lie in memory until they are used), 24.6 in runs of 8 with six, 32.0 in runs of 8 with four; a warp per token and
+// head takes 97. 2,048 x 2,048 with unit heads of 64 12.7 us, 14.7, 15.0 and 40. Heads
 // of dk channels that are divided by their length are dk / 4 neighbouring lanes (a power of two).
 // `update` (every row has one token): the thread that read a row's history leaves it one token further, which saves a decode step the
 // launch that does it for rows of any length.
-constexpr int CONV_RUN = 8, CONV_THREADS = 128;
+constexpr int CONV_RUN = 4, CONV_THREADS = 128;
 template <typename T, int TAPS, int RUN>
-__global__ void __launch_bounds__(CONV_THREADS)
+__global__ void __launch_bounds__(CONV_THREADS, RUN > 1 ? 8 : 1)
 conv_silu_unit_x4_kernel(float* __restrict__ out, const T* __restrict__ proj, int ld, T* conv_state, const float* __restrict__ w,
                          const int* __restrict__ row_of_token, const int* __restrict__ cu_q, const int* __restrict__ q_start,
                          const int* __restrict__ state_slot, int num_tokens, int C, int unit_channels, int lanes_per_head, float unit_eps,
@@ -516,12 +525,12 @@ conv_silu_unit_x4_kernel(float* __restrict__ out, const T* __restrict__ proj, in
       for (int j = 0; j < TAPS; ++j) tap[e][j] = w[(size_t)(c + e) * TAPS + j];
   }
   float4 b = bias ? load4(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 x[RUN];
+  typename Four<T>::raw x[RUN];
   int row[RUN];
 #pragma unroll
   for (int i = 0; i < RUN; ++i) {
     row[i] = t0 + i < num_tokens ? row_of_token[t0 + i] : -1;
-    if (t0 + i < num_tokens) x[i] = load4(proj + (size_t)(t0 + i) * ld + c);
+    if (t0 + i < num_tokens) x[i] = *reinterpret_cast<const typename Four<T>::raw*>(proj + (size_t)(t0 + i) * ld + c);
   }
   float4 win[TAPS];  // the last TAPS inputs, oldest first
   int current = -1;
@@ -553,7 +562,7 @@ conv_silu_unit_x4_kernel(float* __restrict__ out, const T* __restrict__ proj, in
     }
 #pragma unroll
     for (int j = 0; j + 1 < TAPS; ++j) win[j] = win[j + 1];
-    win[TAPS - 1] = x[i];
+    win[TAPS - 1] = float4_of(x[i]);
     if (update && in) {
       T* st = conv_state + (size_t)state_slot[current] * (TAPS - 1) * C + c;
 #pragma unroll
@@ -860,13 +869,13 @@ MS_EXPORT int ms_conv_silu_unit(float* out, const void* proj, int ld, void* conv
   // four channels a thread where heads and rows are whole fours (and a normed head is a power of two of lanes of one warp)
   const int item = dtype == MS_F32 ? 16 : 8, lanes = dk / 4;
   // One token a thread, which looks up its row and reads a window of its own, where those CTAs are on the GPU at once (decoding rows); runs of
-  // eight tokens, which read an input once, where they give every multiprocessor threads enough. Between the two a warp per token and head is
+  // four tokens, which read an input once, where they give every multiprocessor threads enough. Between the two a warp per token and head is
   // faster: with normed heads 201 tokens of 2,048 channels 5 us against 7 in runs and 8 one by one, 2,048 of 96 4 against 7 and 6; without, 64
   // of 6,144 7.2 against 5.7 and 7.2. (Not in float32: the forms add a head's squares up in different orders, and a token's bits must not hang
   // on how many tokens the step has.)
   const int sms = scan_sm_count();
   const bool single = (long long)ceil_div(C / 4, CONV_THREADS) * num_tokens <= 4LL * sms;
-  const bool runs = !single && (dtype == MS_F32 || (long long)(C / 4) * ceil_div(num_tokens, CONV_RUN) >= (long long)(unit_heads > 0 ? 128 : 64) * sms);
+  const bool runs = !single && (dtype == MS_F32 || (long long)(C / 4) * ceil_div(num_tokens, 2 * CONV_RUN) >= (long long)(unit_heads > 0 ? 128 : 64) * sms);
   if ((runs || single) && taps >= 2 && taps <= 4 && C % 4 == 0 && ld % 4 == 0 && (uintptr_t)proj % item == 0 && (uintptr_t)conv_state % item == 0 &&
       (uintptr_t)out % 16 == 0 && (!bias || (uintptr_t)bias % 16 == 0) &&
       (unit_heads == 0 || (dk % 4 == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0)) && num_tokens <= 65535) {
@@ -996,7 +1005,8 @@ gated_group_norm_kernel(T* __restrict__ out, int ld_out, const float* __restrict
 }
 
 // The same for parts of whole fours up to 128 ITER channels: a warp per (token, part), four channels a lane at a time, everything read
-// once and kept in registers. 2,048 tokens of 4,096 channels in 8 parts: 23 us (4.4 TB/s) against 61.
+// once and kept in registers, and asked for before the first of it is worked on. 2,048 tokens of 4,096 channels in 8 parts: 20 us (5.0 TB/s; 23 with
+// each step's loads behind the last step's exponentials) against 61.
 template <typename T, int ITER>
 __global__ void __launch_bounds__(GGN_THREADS)
 gated_group_norm_x4_kernel(T* __restrict__ out, int ld_out, const float* __restrict__ o, const float* __restrict__ x, int ld_x,
@@ -1006,19 +1016,33 @@ gated_group_norm_x4_kernel(T* __restrict__ out, int ld_out, const float* __restr
   const int item = blockIdx.x * (GGN_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (item >= num_items) return;
   const int t = item / parts, part = item - t * parts, size = width / parts, base = part * size;
-  float4 y[ITER];
+  typename Four<T>::raw gr[ITER];
+  float4 y[ITER], xv[ITER];
+  float sv[ITER];
+#pragma unroll
+  for (int i = 0; i < ITER; ++i) {  // all of it is asked for before the first is worked on
+    const int c = (i * 32 + lane) * 4, ch = base + c;
+    y[i] = xv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    gr[i] = {};
+    sv[i] = 0.f;
+    if (c < size) {
+      gr[i] = *reinterpret_cast<const typename Four<T>::raw*>(gate + (size_t)t * ld_gate + ch);
+      y[i] = load4(o + (size_t)t * width + ch);
+      if (skip) {
+        xv[i] = load4(x + (size_t)t * ld_x + ch);
+        sv[i] = skip[ch / dv];
+      }
+    }
+  }
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < ITER; ++i) {
-    const int c = (i * 32 + lane) * 4, ch = base + c;
-    y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c < size) {
-      const float4 g = load4(gate + (size_t)t * ld_gate + ch);
-      float4 v = load4(o + (size_t)t * width + ch);
+    if ((i * 32 + lane) * 4 < size) {
+      const float4 g = float4_of(gr[i]);
+      float4 v = y[i];
       if (skip) {
-        const float4 xv = load4(x + (size_t)t * ld_x + ch);
-        const float s = skip[ch / dv];
-        v = make_float4(fmaf(s, xv.x, v.x), fmaf(s, xv.y, v.y), fmaf(s, xv.z, v.z), fmaf(s, xv.w, v.w));
+        const float s = sv[i];
+        v = make_float4(fmaf(s, xv[i].x, v.x), fmaf(s, xv[i].y, v.y), fmaf(s, xv[i].z, v.z), fmaf(s, xv[i].w, v.w));
       }
       y[i] = make_float4(v.x * (g.x / (1.0f + expf(-g.x))), v.y * (g.y / (1.0f + expf(-g.y))), v.z * (g.z / (1.0f + expf(-g.z))),
                          v.w * (g.w / (1.0f + expf(-g.w))));
