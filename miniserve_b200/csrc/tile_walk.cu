@@ -268,7 +268,23 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
 // grid (chunks, H). q', k' [chunks, H, 64, dkp] float32 (dkp = 32 N >= dk, zeros behind dk). z: the decays' logits (bias, coef, sign as in
 // recurrence.cu). The pairs of a sixteen: a warp takes four tokens j at once, eight lanes over the channels of each, lets their keys decay from
 // j on, and adds up over the lanes at the end. Then a thread per sixteen and channel decays queries from the sixteen's start and keys to its
-// end, which make the pairs of different sixteens, the keys decayed on over the sixteens between them.
+// end, which make the pairs of different sixteens, the keys decayed on over the sixteens between them. Bound by a CTA's chain (two or three a
+// multiprocessor, 30 % of the issue slots): 2,048 tokens of 8 heads of 64 channels 22.7 us; 27.0 with the operands read one by one, four in flight, and
+// q' and k' read back from global memory for their images.
+template <typename T>
+__device__ __forceinline__ float4 tw_load4(const T* p) {
+  if constexpr (sizeof(T) == 4) {
+    return *reinterpret_cast<const float4*>(p);
+  } else {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
+  }
+}
+// whether rows `ld` apart of T in fours start where four are one load
+template <typename T>
+__device__ __forceinline__ bool tw_fours(const T* p, int ld) {
+  return (reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T))) == 0 && ld % 4 == 0;
+}
 template <typename TIn, typename TZ, int N>
 __global__ void __launch_bounds__(TW_FIRST, 2)
 tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, uint8_t* __restrict__ k_image, int* __restrict__ plain,
@@ -280,6 +296,8 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
   using F = TwFactors<TW_CHANNEL, DKP>;
   extern __shared__ __align__(16) float tw_smem[];
   float *qs = tw_smem, *ks = qs + TW_TOK * LD, *ds = ks + TW_TOK * LD;
+  constexpr bool KEEP = N <= 2;  // k' stays in shared memory as well (a fourth array; at N = 4 it would leave room for one CTA)
+  float* kf = KEEP ? ds + TW_TOK * LD : ks;
   __shared__ double whole[SUBS][DKP];  // a sixteen's decays
   __shared__ uint32_t most[DKP];
   pdl_prologue();
@@ -289,20 +307,48 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
   const int t0 = at.first, n = min(TW_TOK, at.end - t0);
   const size_t qk_at = (size_t)(h / qk_group) * dk, item = (size_t)at.chunk * H + h;
   const float coef = decay_coef[h];
-#pragma unroll 4
-  for (int e = 0; e < TW_TOK * DKP / TW_FIRST; ++e) {
-    const int idx = e * TW_FIRST + tid, i = idx / DKP, c = idx % DKP;
-    float fq = 0.f, fk = 0.f, fd = 1.f;
-    if (i < n && c < dk) {
-      const size_t t = (size_t)(t0 + i);
-      fq = Elem<TIn>::load(q + t * ld_q + qk_at + c) * q_scale;
-      fk = Elem<TIn>::load(k + t * ld_k + qk_at + c);
-      fd = Elem<TZ>::load(z + t * ld_z + (size_t)h * dk + c);
-      fd = expf(-coef * tw_softplus(z_sign * (fd + z_bias[(size_t)h * dk + c])));
+  auto decay = [&](float logit, int c) { return expf(-coef * tw_softplus(z_sign * (logit + z_bias[(size_t)h * dk + c]))); };
+  if (dk % 4 == 0 && tw_fours(q, ld_q) && tw_fours(k, ld_k) && tw_fours(z, ld_z)) {
+    constexpr int EACH = TW_TOK * DKP / 4 / TW_FIRST, AT_ONCE = EACH < 4 ? EACH : 4;
+#pragma unroll 1
+    for (int e0 = 0; e0 < EACH; e0 += AT_ONCE) {
+      float4 fq[AT_ONCE], fk[AT_ONCE], fd[AT_ONCE];
+#pragma unroll
+      for (int e = 0; e < AT_ONCE; ++e) {  // all of it is asked for before the first is worked on
+        const int idx = (e0 + e) * TW_FIRST + tid, i = idx / (DKP / 4), c = (idx % (DKP / 4)) * 4;
+        const bool in = i < n && c < dk;
+        const size_t t = in ? (size_t)(t0 + i) : (size_t)t0;
+        const int cc = in ? c : 0;
+        fq[e] = tw_load4(q + t * ld_q + qk_at + cc);
+        fk[e] = tw_load4(k + t * ld_k + qk_at + cc);
+        fd[e] = tw_load4(z + t * ld_z + (size_t)h * dk + cc);
+      }
+#pragma unroll
+      for (int e = 0; e < AT_ONCE; ++e) {
+        const int idx = (e0 + e) * TW_FIRST + tid, i = idx / (DKP / 4), c = (idx % (DKP / 4)) * 4;
+        const bool in = i < n && c < dk;
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(qs + i * LD + c) = in ? make_float4(fq[e].x * q_scale, fq[e].y * q_scale, fq[e].z * q_scale, fq[e].w * q_scale) : none;
+        *reinterpret_cast<float4*>(ks + i * LD + c) = in ? fk[e] : none;
+        *reinterpret_cast<float4*>(ds + i * LD + c) =
+            in ? make_float4(decay(fd[e].x, c), decay(fd[e].y, c + 1), decay(fd[e].z, c + 2), decay(fd[e].w, c + 3)) : make_float4(1.f, 1.f, 1.f, 1.f);
+      }
     }
-    qs[i * LD + c] = fq;
-    ks[i * LD + c] = fk;
-    ds[i * LD + c] = fd;
+  } else {
+#pragma unroll 4
+    for (int e = 0; e < TW_TOK * DKP / TW_FIRST; ++e) {
+      const int idx = e * TW_FIRST + tid, i = idx / DKP, c = idx % DKP;
+      float fq = 0.f, fk = 0.f, fd = 1.f;
+      if (i < n && c < dk) {
+        const size_t t = (size_t)(t0 + i);
+        fq = Elem<TIn>::load(q + t * ld_q + qk_at + c) * q_scale;
+        fk = Elem<TIn>::load(k + t * ld_k + qk_at + c);
+        fd = decay(Elem<TZ>::load(z + t * ld_z + (size_t)h * dk + c), c);
+      }
+      qs[i * LD + c] = fq;
+      ks[i * LD + c] = fk;
+      ds[i * LD + c] = fd;
+    }
   }
   float* fac = factors + item * F::floats;
   float* out = pairs + item * (TW_BLOCKS * TW_SUB * TW_SUB);
@@ -370,21 +416,25 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
       if (sub == 0) fac[F::last + c] = (float)all;
       double own = 1.0;
 #pragma unroll 4
+      for (int i = TW_SUB - 1; i >= 0; --i) {
+        const int t = sub * TW_SUB + i;
+        const double x = own * (double)ks[t * LD + c];
+        const float y = (float)(behind * x);
+        ks[t * LD + c] = (float)x;
+        if (KEEP) kf[t * LD + c] = y;
+        k_out[(item * TW_TOK + t) * DKP + c] = y;
+        own *= (double)ds[t * LD + c];
+      }
+      own = 1.0;
+#pragma unroll 4
       for (int i = 0; i < TW_SUB; ++i) {
         const int t = sub * TW_SUB + i;
         own *= (double)ds[t * LD + c];
         const double x = own * (double)qs[t * LD + c];
+        const float y = (float)(before * x);
         qs[t * LD + c] = (float)x;
-        q_out[(item * TW_TOK + t) * DKP + c] = (float)(before * x);
-      }
-      own = 1.0;
-#pragma unroll 4
-      for (int i = TW_SUB - 1; i >= 0; --i) {
-        const int t = sub * TW_SUB + i;
-        const double x = own * (double)ks[t * LD + c];
-        ks[t * LD + c] = (float)x;
-        k_out[(item * TW_TOK + t) * DKP + c] = (float)(behind * x);
-        own *= (double)ds[t * LD + c];
+        ds[t * LD + c] = y;  // (nobody asks for this decay any more)
+        q_out[(item * TW_TOK + t) * DKP + c] = y;
       }
     }
   }
@@ -436,14 +486,15 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
     }
     __syncthreads();
   }
-  for (int idx = tid; idx < TW_TOK * DKP / 4; idx += TW_FIRST) {  // (what this CTA has written above)
-    const int t = idx / (DKP / 4), c = (idx % (DKP / 4)) * 4;
-    *reinterpret_cast<float4*>(qs + t * LD + c) = *reinterpret_cast<const float4*>(q_out + (item * TW_TOK + t) * DKP + c);
-    *reinterpret_cast<float4*>(ks + t * LD + c) = *reinterpret_cast<const float4*>(k_out + (item * TW_TOK + t) * DKP + c);
+  if (!KEEP) {
+    for (int idx = tid; idx < TW_TOK * DKP / 4; idx += TW_FIRST) {  // (what this CTA has written above)
+      const int t = idx / (DKP / 4), c = (idx % (DKP / 4)) * 4;
+      *reinterpret_cast<float4*>(ks + t * LD + c) = *reinterpret_cast<const float4*>(k_out + (item * TW_TOK + t) * DKP + c);
+    }
+    __syncthreads();
   }
-  __syncthreads();
   const size_t bytes = (size_t)3 * (DKP / 64) * TW_TILE;
-  const bool bad = tw_images<DKP, LD>(q_image + item * bytes, k_image + item * bytes, qs, ks, most);
+  const bool bad = tw_images<DKP, LD>(q_image + item * bytes, k_image + item * bytes, ds, kf, most);
   const int any = __syncthreads_or(bad);
   if (tid == 0) plain[item] = any;
 }
@@ -1196,7 +1247,7 @@ static int launch_tile_channel(const TwPlan& plan, TwArgs g, float* scratch, con
   int* plain = (int*)(scratch + 2 * plan.images);
   float *pairs = scratch + 2 * plan.images + plan.flags, *factors = pairs + plan.pairs, *qp = factors + plan.factors, *kp = qp + plan.keys;
   auto prepare = tile_prepare_kernel<TIn, TZ, N>;
-  constexpr size_t bytes = (size_t)3 * TW_TOK * (DKP + 4) * 4;
+  constexpr size_t bytes = (size_t)(N <= 2 ? 4 : 3) * TW_TOK * (DKP + 4) * 4;
   static std::atomic<unsigned long long> allowed{0};
   MS_CHECK_CUDA(allow_shared_memory((const void*)prepare, (int)bytes, allowed));
   MS_LAUNCH(prepare, dim3(plan.chunks, g.H), TW_FIRST, bytes, stream, qp, kp, q_image, k_image, plain, factors, pairs, q, g.ld_q, k, g.ld_k, g.qk_group, z, ld_z,
