@@ -139,9 +139,10 @@ __device__ __forceinline__ float query_factor(const PrepareExtras& ex, int h, in
 // (token, head). ADJACENT: these are four rotation pairs, so the rotation needs no exchange. Otherwise channel i
 // turns with channel i + rot / 2 (rot a multiple of 16): the lane loads its partners' eight channels as well.
 // LANES lanes a head: 16 where a cached head has up to 128 channels, so that every lane has its 16 bytes (16 + 2 x 8 heads of 128,
-// 2,048 tokens: 20 us against 33 with half of every warp idle), else a warp.
-template <bool ADJACENT, int LANES>
-__global__ void qkv_prepare_bf16x8_kernel(
+// 2,048 tokens: 20 us against 33 with half of every warp idle), else a warp. Bound by instruction issue (72 %): with a head's channels kept from the
+// norm to the end (ONE) and the norm's weights read in 16 bytes 16.1 us, 19.0 read twice and one by one.
+template <bool ADJACENT, int LANES, bool ONE>
+__global__ void __launch_bounds__(256) qkv_prepare_bf16x8_kernel(
     __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool,
     const __nv_bfloat16* __restrict__ proj, int ld, int q_off, int k_off, int v_off, const float* __restrict__ q_norm_w,
     const float* __restrict__ k_norm_w, const float* __restrict__ cos_sin, const int* __restrict__ positions,
@@ -188,17 +189,43 @@ __global__ void qkv_prepare_bf16x8_kernel(
     if (bias) bias += (size_t)nq * dk + (is_v ? (size_t)nkv * dk + (size_t)kvh * dv : (size_t)kvh * dk);
   }
   const int own = is_v ? dv : dk;
-  // (a head of up to 256 channels: one trip; wider heads take more)
+  // Eight channels with their bias, and eight weights (one for none), in 16 bytes where they start on 16.
+  auto fetch = [&](float (&x)[8], int c) {
+    bf16x8_to_float(*reinterpret_cast<const uint4*>(src + c), x);
+    if (bias) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] += bias[c + e];
+    }
+  };
+  const bool whole = (reinterpret_cast<uintptr_t>(nw) & 15) == 0;
+  auto weigh = [&](float (&x)[8], int c, float inv) {
+    if (!nw) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] *= inv;
+    } else if (whole) {
+      const float4 w0 = *reinterpret_cast<const float4*>(nw + c), w1 = *reinterpret_cast<const float4*>(nw + c + 4);
+      const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = (x[e] * inv) * wv[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = (x[e] * inv) * nw[c + e];
+    }
+  };
+  // ONE: a head's channels are one trip of its lanes and stay in registers from the norm to the end.
+  float v[8] = {};
+  if (ONE && lane * 8 < own) fetch(v, lane * 8);
   float ss = 0.f;
   const bool normed = !is_v && (nw || ex.unit_norm);
   if (normed) {
-    for (int c = lane * 8; c < dk; c += 8 * LANES) {
-      float v[8];
-      bf16x8_to_float(*reinterpret_cast<const uint4*>(src + c), v);
+    if (ONE) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (bias) v[e] += bias[c + e];
-        ss += v[e] * v[e];
+      for (int e = 0; e < 8; ++e) ss += v[e] * v[e];  // (zeros behind the last)
+    } else {
+      for (int c = lane * 8; c < dk; c += 8 * LANES) {
+        fetch(v, c);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
       }
     }
 #pragma unroll
@@ -208,29 +235,20 @@ __global__ void qkv_prepare_bf16x8_kernel(
   const float qs = h < nq ? query_factor(ex, h, pos) : 1.f;
   const int half = rot >> 1;
   for (int c = lane * 8; c < d_pad; c += 8 * LANES) {
-    float v[8];
-    if (c < own) {
-      bf16x8_to_float(*reinterpret_cast<const uint4*>(src + c), v);
-      if (bias) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] += bias[c + e];
-      }
-      if (is_v && ex.v_other) {
-        const float share = *ex.v_share;
-        float o[8];
-        bf16x8_to_float(*reinterpret_cast<const uint4*>((const __nv_bfloat16*)ex.v_other + (size_t)t * ex.ld_other + (size_t)(h - nq - nkv) * dv + c), o);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = fmaf(share, o[e], (1.f - share) * v[e]);
-      }
-    } else {
+    if (!ONE) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = 0.f;
+      if (c < own) fetch(v, c);
+    }
+    if (is_v && ex.v_other && c < own) {
+      const float share = *ex.v_share;
+      float o[8];
+      bf16x8_to_float(*reinterpret_cast<const uint4*>((const __nv_bfloat16*)ex.v_other + (size_t)t * ex.ld_other + (size_t)(h - nq - nkv) * dv + c), o);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = fmaf(share, o[e], (1.f - share) * v[e]);
     }
     if (!is_v && c < dk) {
-      if (normed) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = (v[e] * inv) * (nw ? nw[c + e] : 1.f);
-      }
+      if (normed) weigh(v, c, inv);
       if (ADJACENT) {
         const int j0 = c >> 1;
         const bool fours = rot % 8 == 0 && (reinterpret_cast<uintptr_t>(cos_sin) & 15) == 0;  // whole groups of four pairs, on 16 bytes
@@ -260,15 +278,8 @@ __global__ void qkv_prepare_bf16x8_kernel(
         const bool first = c < half;  // this chunk holds the pairs' first members (u), its partner chunk the second (v)
         const int pc = first ? c + half : c - half, j0 = first ? c : c - half;
         float p[8];
-        bf16x8_to_float(*reinterpret_cast<const uint4*>(src + pc), p);
-        if (bias) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) p[e] += bias[pc + e];
-        }
-        if (normed) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) p[e] = (p[e] * inv) * (nw ? nw[pc + e] : 1.f);
-        }
+        fetch(p, pc);
+        if (normed) weigh(p, pc, inv);
         const float4 c0 = *reinterpret_cast<const float4*>(cos_sin + (size_t)t * rot + j0);
         const float4 c1 = *reinterpret_cast<const float4*>(cos_sin + (size_t)t * rot + j0 + 4);
         const float4 s0 = *reinterpret_cast<const float4*>(cos_sin + (size_t)t * rot + half + j0);
@@ -484,16 +495,18 @@ MS_EXPORT int ms_qkv_prepare(void* q_out, void* k_pool, void* v_pool, const void
       k_off % 8 == 0 && v_off % 8 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)q_out % 16 == 0 && (uintptr_t)k_pool % 16 == 0 &&
       (uintptr_t)v_pool % 16 == 0 && (uintptr_t)v_other % 16 == 0 && ld_other % 8 == 0) {
     // (the table's rows are rot floats wide: 16-byte loads of eight cosines need rot / 2 a multiple of 8, which rot % 16 gives)
-#define MS_PREPARE(ADJACENT, LANES)                                                                                                            \
-  MS_LAUNCH((qkv_prepare_bf16x8_kernel<ADJACENT, LANES>), (unsigned)((items * LANES + 255) / 256), 256, 0, stream, (__nv_bfloat16*)q_out,      \
+#define MS_PREPARE(ADJACENT, LANES, ONE)                                                                                                       \
+  MS_LAUNCH((qkv_prepare_bf16x8_kernel<ADJACENT, LANES, ONE>), (unsigned)((items * LANES + 255) / 256), 256, 0, stream, (__nv_bfloat16*)q_out,      \
             (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, (const __nv_bfloat16*)proj, ld, q_off, k_off, v_off, q_norm_w, k_norm_w, cos_sin,  \
             positions, row_of_token, page_indptr, page_indices, num_tokens, nq, nkv, dk, dv, d_pad, rot, eps, page_shift, num_pages, status, ex)
     if (adjacent || rot == 0) {
-      if (d_pad <= 128) MS_PREPARE(true, 16);
-      else MS_PREPARE(true, 32);
+      if (d_pad <= 128) MS_PREPARE(true, 16, true);
+      else if (d_pad <= 256) MS_PREPARE(true, 32, true);
+      else MS_PREPARE(true, 32, false);
     } else {
-      if (d_pad <= 128) MS_PREPARE(false, 16);
-      else MS_PREPARE(false, 32);
+      if (d_pad <= 128) MS_PREPARE(false, 16, true);
+      else if (d_pad <= 256) MS_PREPARE(false, 32, true);
+      else MS_PREPARE(false, 32, false);
     }
 #undef MS_PREPARE
     return 0;
