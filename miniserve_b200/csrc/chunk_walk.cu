@@ -77,6 +77,21 @@ __device__ __forceinline__ int wk_first(int row, const int* __restrict__ cu_q) {
   return __reduce_add_sync(0xffffffffu, sum);
 }
 
+template <typename T>
+__device__ __forceinline__ float4 wk_load4(const T* p) {
+  if constexpr (sizeof(T) == 4) {
+    return *reinterpret_cast<const float4*>(p);
+  } else {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
+  }
+}
+// whether rows `ld` apart of T in fours start where four are one load
+template <typename T>
+__device__ __forceinline__ bool wk_fours(const T* p, int ld) {
+  return (reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T))) == 0 && ld % 4 == 0;
+}
+
 // ---------------------------------------------------------------- what a chunk needs beside the state (a decay per key channel)
 // grid (chunks, H). W, q', k' [chunks, H, 16, dkp] and last [chunks, H, dkp] float32 (dkp = 32 N >= dk, zeros behind dk), u0
 // [chunks, H, 16, dvp] (dvp: dv in whole sixteens, zeros behind; without the delta rule v itself), pairs = P [chunks, H, 16, 16]. z: the
@@ -86,7 +101,8 @@ __device__ __forceinline__ int wk_first(int row, const int* __restrict__ cu_q) {
 // exchanges for four tokens). The sum over the lanes, products of decays and the triangular system in 64 bits (above).
 // With the delta rule the triangular system is a chain of 16 steps in 64 bits, in which a CTA's warps wait for one another: six CTAs an SM (80
 // registers a thread, 24 to 64 bytes of them spilled) cover it better than four. 2,048 tokens, both kernels: 16 heads of 64 x 64 139.9 -> 136.3
-// us, 32 heads 225.7 -> 209.8. Without it nothing waits so long, and six measured the same as four (108.2).
+// us, 32 heads 225.7 -> 209.8. Without it nothing waits so long, and six measured the same as four (108.2). Operands come in fours where rows
+// start on whole fours, all of a thread's loads ahead of its work: 2,048 tokens of 16 heads 32.0 us, 37.8 one by one.
 template <typename TIn, typename TZ, bool DELTA, int N>
 __global__ void __launch_bounds__(WK_THREADS, DELTA ? 6 : 4)
 walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float* __restrict__ k_out, float* __restrict__ last_out,
@@ -107,20 +123,48 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t qk_at = (size_t)(h / qk_group) * dk;
   const float coef = decay_coef[h];
+  auto decay = [&](float logit, int c) { return expf(-coef * wk_softplus(z_sign * (logit + z_bias[(size_t)h * dk + c]))); };
+  if (dk % 4 == 0 && wk_fours(q, ld_q) && wk_fours(k, ld_k) && wk_fours(z, ld_z)) {
+    constexpr int EACH = WK_TOK * DKP / 4 / WK_THREADS, AT_ONCE = EACH < 2 ? EACH : 2;
+#pragma unroll 1
+    for (int e0 = 0; e0 < EACH; e0 += AT_ONCE) {
+      float4 fq[AT_ONCE], fk[AT_ONCE], fd[AT_ONCE];
 #pragma unroll
-  for (int e = 0; e < WK_TOK * DKP / WK_THREADS; ++e) {
-    const int idx = e * WK_THREADS + tid, i = idx / DKP, c = idx % DKP;
-    float fq = 0.f, fk = 0.f, fd = 1.f;
-    if (i < n && c < dk) {
-      const size_t t = (size_t)(t0 + i);
-      fq = Elem<TIn>::load(q + t * ld_q + qk_at + c) * q_scale;
-      fk = Elem<TIn>::load(k + t * ld_k + qk_at + c);
-      fd = Elem<TZ>::load(z + t * ld_z + (size_t)h * dk + c);
-      fd = expf(-coef * wk_softplus(z_sign * (fd + z_bias[(size_t)h * dk + c])));
+      for (int e = 0; e < AT_ONCE; ++e) {  // all of it is asked for before the first is worked on
+        const int idx = (e0 + e) * WK_THREADS + tid, i = idx / (DKP / 4), c = (idx % (DKP / 4)) * 4;
+        const bool in = i < n && c < dk;
+        const size_t t = in ? (size_t)(t0 + i) : (size_t)t0;
+        const int cc = in ? c : 0;
+        fq[e] = wk_load4(q + t * ld_q + qk_at + cc);
+        fk[e] = wk_load4(k + t * ld_k + qk_at + cc);
+        fd[e] = wk_load4(z + t * ld_z + (size_t)h * dk + cc);
+      }
+#pragma unroll
+      for (int e = 0; e < AT_ONCE; ++e) {
+        const int idx = (e0 + e) * WK_THREADS + tid, i = idx / (DKP / 4), c = (idx % (DKP / 4)) * 4;
+        const bool in = i < n && c < dk;
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(&qs[i][c]) = in ? make_float4(fq[e].x * q_scale, fq[e].y * q_scale, fq[e].z * q_scale, fq[e].w * q_scale) : none;
+        *reinterpret_cast<float4*>(&ks[i][c]) = in ? fk[e] : none;
+        *reinterpret_cast<float4*>(&ds[i][c]) =
+            in ? make_float4(decay(fd[e].x, c), decay(fd[e].y, c + 1), decay(fd[e].z, c + 2), decay(fd[e].w, c + 3)) : make_float4(1.f, 1.f, 1.f, 1.f);
+      }
     }
-    qs[i][c] = fq;
-    ks[i][c] = fk;
-    ds[i][c] = fd;
+  } else {
+#pragma unroll 4
+    for (int e = 0; e < WK_TOK * DKP / WK_THREADS; ++e) {
+      const int idx = e * WK_THREADS + tid, i = idx / DKP, c = idx % DKP;
+      float fq = 0.f, fk = 0.f, fd = 1.f;
+      if (i < n && c < dk) {
+        const size_t t = (size_t)(t0 + i);
+        fq = Elem<TIn>::load(q + t * ld_q + qk_at + c) * q_scale;
+        fk = Elem<TIn>::load(k + t * ld_k + qk_at + c);
+        fd = decay(Elem<TZ>::load(z + t * ld_z + (size_t)h * dk + c), c);
+      }
+      qs[i][c] = fq;
+      ks[i][c] = fk;
+      ds[i][c] = fd;
+    }
   }
   if (tid < WK_TOK) {
     float b = 0.f;
