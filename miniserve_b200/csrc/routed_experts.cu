@@ -222,42 +222,84 @@ expert_route_kernel(int* __restrict__ idx_out, float* __restrict__ wgt_out, cons
 //   perm[row]   the slot of a sorted row
 //   offsets[e]  the first sorted row of expert e (E + 1 entries)
 //   tiles       (expert, first row) of every tile of `tile_rows` sorted rows; meta[0] = how many
-constexpr int PLAN_THREADS = 1024;
+// Bound by latency (one CTA): a thread's slots are asked for together and stay in registers to the end, a warp adds the counts up. 7,600 slots of
+// 14 experts 5.9 us (8.0 with slots read again and one thread going over the experts; 8.4 where a warp first finds its equal slots), 32 slots
+// 2.9 (3.2).
+constexpr int PLAN_THREADS = 1024, PLAN_EACH = 16;
 __global__ void __launch_bounds__(PLAN_THREADS)
 expert_plan_kernel(int* __restrict__ pos, int* __restrict__ perm, int* __restrict__ offsets, int* __restrict__ tiles,
                    int* __restrict__ meta, const int* __restrict__ idx, int S, int E, int tile_rows) {
   extern __shared__ int plan_smem[];
   int* cnt = plan_smem;     // [E]
   int* off = cnt + E;       // [E + 1]
+  int* first = cnt;         // [E]: an expert's first tile, once the counts are in the offsets
   pdl_prologue();
-  for (int e = threadIdx.x; e < E; e += PLAN_THREADS) cnt[e] = 0;
+  const int tid = threadIdx.x;
+  for (int e = tid; e < E; e += PLAN_THREADS) cnt[e] = 0;
+  int expert[PLAN_EACH], rank[PLAN_EACH];  // of the thread's first slots; steps with more read theirs again
+#pragma unroll
+  for (int i = 0; i < PLAN_EACH; ++i) {
+    const int slot = i * PLAN_THREADS + tid;
+    expert[i] = slot < S ? idx[slot] : -1;
+  }
   __syncthreads();
-  for (int slot = threadIdx.x; slot < S; slot += PLAN_THREADS) {
+#pragma unroll
+  for (int i = 0; i < PLAN_EACH; ++i) {
+    if (i * PLAN_THREADS >= S) break;
+    rank[i] = expert[i] >= 0 && expert[i] < E ? atomicAdd(&cnt[expert[i]], 1) : -1;
+  }
+  for (int slot = PLAN_EACH * PLAN_THREADS + tid; slot < S; slot += PLAN_THREADS) {
     const int e = idx[slot];
     pos[slot] = (e >= 0 && e < E) ? atomicAdd(&cnt[e], 1) : -1;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (tid < 32) {
     int at = 0, nt = 0;
-    for (int e = 0; e < E; ++e) {
-      off[e] = at;
-      for (int r0 = 0; r0 < cnt[e]; r0 += tile_rows) {
-        tiles[2 * nt] = e;
-        tiles[2 * nt + 1] = at + r0;
-        ++nt;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + tid, rows = e < E ? cnt[e] : 0, own = (rows + tile_rows - 1) / tile_rows;
+      int upto = rows, tiles_upto = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, o), y = __shfl_up_sync(0xffffffffu, tiles_upto, o);
+        if (tid >= o) {
+          upto += x;
+          tiles_upto += y;
+        }
       }
-      at += cnt[e];
+      if (e < E) {
+        off[e] = at + upto - rows;
+        first[e] = nt + tiles_upto - own;
+      }
+      at += __shfl_sync(0xffffffffu, upto, 31);
+      nt += __shfl_sync(0xffffffffu, tiles_upto, 31);
     }
-    off[E] = at;
-    meta[0] = nt;
-    meta[1] = at;
+    if (tid == 0) {
+      off[E] = at;
+      meta[0] = nt;
+      meta[1] = at;
+    }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e <= E; e += PLAN_THREADS) offsets[e] = off[e];
-  for (int slot = threadIdx.x; slot < S; slot += PLAN_THREADS) {
-    const int rank = pos[slot];
-    if (rank >= 0) {
-      const int p = off[idx[slot]] + rank;
+  for (int e = tid; e <= E; e += PLAN_THREADS) {
+    offsets[e] = off[e];
+    if (e < E)
+      for (int r0 = off[e], nt = first[e]; r0 < off[e + 1]; r0 += tile_rows, ++nt) {
+        tiles[2 * nt] = e;
+        tiles[2 * nt + 1] = r0;
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < PLAN_EACH; ++i) {
+    const int slot = i * PLAN_THREADS + tid;
+    if (slot >= S) break;
+    const int p = rank[i] >= 0 ? off[expert[i]] + rank[i] : -1;
+    pos[slot] = p;
+    if (p >= 0) perm[p] = slot;
+  }
+  for (int slot = PLAN_EACH * PLAN_THREADS + tid; slot < S; slot += PLAN_THREADS) {
+    const int r = pos[slot];
+    if (r >= 0) {
+      const int p = off[idx[slot]] + r;
       pos[slot] = p;
       perm[p] = slot;
     }
