@@ -107,6 +107,17 @@ __device__ __forceinline__ void pdl_prologue() {
   pdl_launch_dependents();
   pdl_wait();
 }
+// A kernel whose weights come from far (each layer's are read once in a decode step) asks for them between the two halves of the prologue: weights are
+// not written by kernels that may still run when its CTAs begin. weight_load16: 16 bytes, asked for where it stands (a plain load may move behind
+// the wait). Whatever earlier kernels write is then read through pointers that have gone through behind_wait(): the compiler takes loads through
+// `const __restrict__` parameters for constant and may otherwise move them ahead of the wait.
+template <typename P>
+__device__ __forceinline__ void behind_wait(P& p) { asm volatile("" : "+l"(p) : : "memory"); }
+__device__ __forceinline__ uint4 weight_load16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 
 // ---- bounded wait on an mbarrier
 // Waits for the phase of the given parity of the mbarrier at shared-memory address `bar`, for at

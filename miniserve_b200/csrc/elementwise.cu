@@ -82,13 +82,20 @@ add_rmsnorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ r
                           const int* __restrict__ rows, float eps, int hidden, int write_residual) {
   extern __shared__ float row_buf[];  // hidden floats, used only by rows wider than 8 * THREADS
   __shared__ float red[32];
-  pdl_prologue();
+  const int chunks = hidden >> 3;
+  const bool in_regs = chunks <= THREADS;
+  pdl_launch_dependents();
+  // A step of 8 requests with 57 of these: 1,101 -> 1,088 us, against weights asked for behind the sum of squares.
+  uint4 w_raw = make_uint4(0u, 0u, 0u, 0u);
+  if (in_regs && (int)threadIdx.x < chunks) w_raw = weight_load16(w + 8 * threadIdx.x);
+  pdl_wait();
+  behind_wait(residual);
+  behind_wait(delta);
+  behind_wait(rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
   const __nv_bfloat16* dl = delta ? delta + (size_t)r * hidden : nullptr;
-  const int chunks = hidden >> 3;
-  const bool in_regs = chunks <= THREADS;
   float h[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   float ss = 0.f;
   for (int c = threadIdx.x; c < chunks; c += THREADS) {
@@ -122,7 +129,7 @@ add_rmsnorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ r
       *reinterpret_cast<float4*>(sum_to + 8 * c + 4) = make_float4(h[4], h[5], h[6], h[7]);
     }
     float wv[8], y[8];
-    bf16x8_to_float(*reinterpret_cast<const uint4*>(w + 8 * c), wv);
+    bf16x8_to_float(in_regs ? w_raw : *reinterpret_cast<const uint4*>(w + 8 * c), wv);
 #pragma unroll
     for (int e = 0; e < 8; ++e) y[e] = (h[e] * inv) * wv[e];
     *reinterpret_cast<uint4*>(o + 8 * c) = float_to_bf16x8(y);

@@ -128,11 +128,29 @@ qk_norm_rope_kv_bf16_token_kernel(
   constexpr int HPW = 32 / LPH;   // heads per warp and pass
   constexpr int HALF = D / 2;
   constexpr int BATCH = 2;        // passes whose loads are issued together
-  pdl_prologue();
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int sub = lane % LPH, slot = lane / LPH, j0 = sub * 8;
-  const int pos = positions[t];
   const bool has_kv = k_pool != nullptr;
+  pdl_launch_dependents();
+  // the norm weights of this lane's elements, the same for every head of a kind, ahead of the wait: a step of 8 requests, 28 of these, 9 us shorter
+  const bool normed = q_norm_w != nullptr;
+  uint4 wq_lo = make_uint4(0u, 0u, 0u, 0u), wq_hi = wq_lo, wk_lo = wq_lo, wk_hi = wq_lo;
+  if (normed) {
+    wq_lo = weight_load16(q_norm_w + j0);
+    wq_hi = weight_load16(q_norm_w + HALF + j0);
+    if (has_kv) {
+      wk_lo = weight_load16(k_norm_w + j0);
+      wk_hi = weight_load16(k_norm_w + HALF + j0);
+    }
+  }
+  pdl_wait();
+  behind_wait(qkv);
+  behind_wait(cos_sin);
+  behind_wait(positions);
+  behind_wait(row_of_token);
+  behind_wait(page_indptr);
+  behind_wait(page_indices);
+  const int pos = positions[t];
   const int heads_total = nq + (has_kv ? 2 * nkv : 0);
   const __nv_bfloat16* row_in = qkv + (size_t)t * heads_total * D;
   // The page of the token hangs on a chain of three dependent loads; the first values of the
@@ -163,17 +181,6 @@ qk_norm_rope_kv_bf16_token_kernel(
   } else {
 #pragma unroll
     for (int i = 0; i < 8; ++i) sincosf((float)pos * inv_freq[j0 + i], &sn[i], &cs[i]);
-  }
-  // the norm weights of this lane's elements, the same for every head of a kind
-  const bool normed = q_norm_w != nullptr;
-  uint4 wq_lo = make_uint4(0u, 0u, 0u, 0u), wq_hi = wq_lo, wk_lo = wq_lo, wk_hi = wq_lo;
-  if (normed) {
-    wq_lo = *reinterpret_cast<const uint4*>(q_norm_w + j0);
-    wq_hi = *reinterpret_cast<const uint4*>(q_norm_w + HALF + j0);
-    if (has_kv) {
-      wk_lo = *reinterpret_cast<const uint4*>(k_norm_w + j0);
-      wk_hi = *reinterpret_cast<const uint4*>(k_norm_w + HALF + j0);
-    }
   }
   size_t slot_base = 0;
   if (has_kv) {
