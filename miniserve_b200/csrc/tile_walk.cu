@@ -970,12 +970,14 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
   const int end = min(at.end, at.first + g.unit), first = at.index * g.unit / TW_TOK, steps = first + (end - at.first + TW_TOK - 1) / TW_TOK;  // chunks of the row
   const int chunk0 = at.chunk - first;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + I::bars);
-  uint64_t *q_full = bars /* two */, *added_full = bars + 2 /* two */, *added_read = bars + 4 /* two */, *outputs_read = bars + 6 /* two */, *state_in = bars + 8, *done = bars + 9;
-  uint32_t* slot_at = reinterpret_cast<uint32_t*>(bars + 10);
-  int* plain_at = reinterpret_cast<int*>(bars + 11);             // [4]: a chunk's products with the state are plain sums
+  uint64_t *q_full = bars /* two */, *added_full = bars + 2 /* two */, *added_read = bars + 4 /* two */, *outputs_read = bars + 6 /* two */, *state_in = bars + 8, *done = bars + 9 /* two */;
+  // (done: two, since an output warp that still adds a chunk's outputs may find the products of the next two done. Those of one barrier would then be as many
+  // phases ahead, which reads as not done. With two, the third's products wait for outputs_read.)
+  uint32_t* slot_at = reinterpret_cast<uint32_t*>(bars + 11);
+  int* plain_at = reinterpret_cast<int*>(bars + 12);             // [4]: a chunk's products with the state are plain sums
   uint32_t* most = reinterpret_cast<uint32_t*>(smem + I::most);  // [3][64]: the state's largest, column by column
   if (tid == 0) {
-    for (int i = 0; i < 10; ++i) tw_bar_init(bars + i, i >= 4 && i <= 8 ? 8 : 1);
+    for (int i = 0; i < 11; ++i) tw_bar_init(bars + i, i >= 4 && i <= 8 ? 8 : 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == TW_WORKERS / 32) {
@@ -1018,12 +1020,12 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
               tw_mma_parts<true>(tmem + (k & 1) * 128, a + ((blk * TW_TILE + ks * 32) >> 4), NB * TW_TILE, b + ((blk * 4 + ks) * 2048 >> 4), DKP * 128, blk + ks > 0);
-          tw_commit(done);
+          tw_commit(done + (k & 1));
         }
         ok = ok && tw_wait(added_read + (c & 1), c >> 1);
         if (c + 2 < steps && ok) copy_added(c + 2);
         if (k >= 0) {
-          ok = ok && tw_wait(done, k);
+          ok = ok && tw_wait(done + (k & 1), k >> 1);
           if (c + 2 < steps && ok) copy_q(c + 2);
         }
       }
@@ -1071,7 +1073,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
         float* grids = reinterpret_cast<float*>(smem + I::grids) + c0;  // (the warps of these columns write the same)
         grids[lane] = tw_grid(tw_power(mx[c0 + lane]));
         __syncwarp();
-        if (k > 0) ok = ok && tw_wait(done, k - 1);
+        if (k > 0) ok = ok && tw_wait(done + ((k - 1) & 1), (k - 1) >> 1);
         if (was) asm volatile("bar.sync 3, 512;\n" ::: "memory");  // (the plain sums have read the state)
         if (plain) {
           float* Sf = reinterpret_cast<float*>(smem + I::s);
@@ -1127,7 +1129,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
       const size_t item = (size_t)(chunk0 + c) * g.H + h;
       const float* fac = g.factors + item * F::floats;
       const float by0 = MODE == TW_HEAD ? fac[F::from + row] : 1.f, by1 = MODE == TW_HEAD ? fac[F::from + row + 8] : 1.f;
-      ok = ok && tw_wait(done, k);
+      ok = ok && tw_wait(done + (k & 1), k >> 1);
       if (plain_at[k & 3]) {
         tw_arrive(outputs_read + (k & 1));
         const float* Sf = reinterpret_cast<const float*>(smem + I::s);
