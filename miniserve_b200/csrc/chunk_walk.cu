@@ -820,3 +820,17 @@ MS_EXPORT int ms_walk_scan_head(float* o, float* state, const float* q, int ld_q
   MS_WALK(4);
 #undef MS_WALK
 }
+
+// ms_walk_scan_head by chunks of 64 tokens, whatever the step, in which copies do not come: those of queries from chunk `no_queries` of a row on, those of what
+// chunks add to the state from `no_added` on. Each wait ends after limit_ns, the status word is raised, and the kernel ends by itself. For tests.
+MS_EXPORT int ms_tile_walk_selftest(float* o, float* state, const float* q, const float* k, const float* v, const float* decay, float* scratch, const int* cu_q,
+                                    const int* q_start, const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, int* status, int no_queries,
+                                    int no_added, long long limit_ns, cudaStream_t stream) {
+  MS_CHECK_ARG(status != nullptr && limit_ns > 0 && limit_ns <= 1000000000LL, "tile_walk_selftest: a limit of up to a second, and a status word");
+  MS_CHECK_ARG((dk == 32 || dk == 64 || dk == 128) && dv >= 1 && H >= 1 && H <= 65535 && num_rows >= 1 && num_tokens >= 1, "tile_walk_selftest: %d heads of %d x %d", H, dk, dv);
+  TwWaits waits;
+  waits.no_queries = no_queries, waits.no_added = no_added, waits.limit_ns = (unsigned long long)limit_ns;
+  return tile_walk_head(o, state, q, H * dk, k, H * dk, 1, v, H * dv, decay, H, nullptr, scratch, cu_q, q_start, state_slot, num_tokens, num_rows, H, dk, dv, 1.f,
+                        status, stream, waits);
+}
+MS_EXPORT long long ms_tile_walk_scratch(int tokens, int rows, int H, int dk, int dv, int groups) { return tile_walk_scratch(tokens, rows, H, dk, dv, groups); }

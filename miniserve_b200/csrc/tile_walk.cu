@@ -518,8 +518,8 @@ __device__ __forceinline__ void tw_arrive(uint64_t* bar) {  // a warp's lanes ha
   __syncwarp();
   if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(cs_smem(bar)) : "memory");
 }
-__device__ __forceinline__ bool tw_wait(uint64_t* bar, int use) {  // for the use of that number
-  const bool ok = mbar_wait_bounded(cs_smem(bar), use & 1);
+__device__ __forceinline__ bool tw_wait(uint64_t* bar, int use, unsigned long long limit_ns) {  // for the use of that number
+  const bool ok = mbar_wait_bounded(cs_smem(bar), use & 1, limit_ns);
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   return ok;
 }
@@ -605,6 +605,7 @@ struct TwArgs {
   const int *cu_q, *q_start, *state_slot;
   int* status;
   int ld_q, ld_k, qk_group, ld_v, unit, num_rows, H, dk, dv, tiles, o_quads;
+  TwWaits waits;
 };
 // outputs of a chunk that a warp read as tw_tmem_pairs has them: tokens tok and 8 on of the chunk's n, columns col, 8 on, ..
 __device__ __forceinline__ void tw_add_outputs(const TwArgs& g, const float (&r)[16], float by0, float by1, int tok0, int tok, int n, int h, int col) {
@@ -708,6 +709,8 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
   const uint32_t tmem = *slot_at, lanes = tmem + ((uint32_t)(32 * quad) << 16);
   const int row = 16 * quad + (lane >> 2), pcol = c0 + 2 * (lane & 3);
   bool ok = true;
+  // (what does not come in time gets as long again, since the CTA must not end while it is on its way)
+  auto come = [&](uint64_t* bar) { return tw_wait(bar, 0, g.waits.limit_ns) || (tw_wait(bar, 0, g.waits.limit_ns), false); };
   uint32_t worst = g.plain[image] ? 0xffffffffu : 0u;
   auto over = [&](int from, int to) {  // the decays of whole sixteens
     double x = 1.0;
@@ -762,12 +765,12 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
     for (int half = 0; half < NB; ++half) {
       if (tid == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        ok = tw_wait(k_full + half, 0) && ok;
+        ok = come(k_full + half) && ok;
         const uint64_t a = tw_desc(smem + I::a), b = tw_desc(smem + I::b);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) tw_mma_parts(tmem, a + (ks * 32 >> 4), TW_TILE, b + (ks * 32 >> 4), TW_TILE, ks > 0);
         tw_commit(done + half);
-        ok = tw_wait(done + half, 0) && ok;
+        ok = come(done + half) && ok;
         if (half + 1 < NB) copy_keys(half + 1);
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       }
@@ -929,7 +932,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
       }
     }
     if (tid == 0) {
-      ok = tw_wait(done, 0);
+      ok = come(done);
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     }
     __syncthreads();  // the products are there, and outputs to be added to
@@ -950,6 +953,8 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
 // grid (segments x column tiles, H). Eight warps carry the state (a thread: a channel's 32 columns), add what the chunks add, from the row's first chunk on, and
 // from the segment's first on hand it to the tensor cores as an operand; eight more scale the products with the queries and add them to the
 // outputs. One warp copies the images of queries and what the chunks add, and issues the products.
+// A role whose wait runs out raises the status word and waits for nothing more. The state's warps go on to their end, since they vote in every chunk; then
+// they agree on whether the state may be kept. The others leave their loops; the issuing thread once what it sent for has come.
 template <int MODE, int DKP>
 struct TwWalk {  // bytes
   static constexpr int image = 3 * (DKP / 64) * TW_TILE, sums = DKP * TW_COLS * 4;
@@ -970,14 +975,15 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
   const int end = min(at.end, at.first + g.unit), first = at.index * g.unit / TW_TOK, steps = first + (end - at.first + TW_TOK - 1) / TW_TOK;  // chunks of the row
   const int chunk0 = at.chunk - first;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + I::bars);
-  uint64_t *q_full = bars /* two */, *added_full = bars + 2 /* two */, *added_read = bars + 4 /* two */, *outputs_read = bars + 6 /* two */, *state_in = bars + 8, *done = bars + 9 /* two */;
+  uint64_t *q_full = bars /* two */, *added_full = bars + 2 /* two */, *added_read = bars + 4 /* two */, *outputs_read = bars + 6 /* two */, *state_in = bars + 8, *done = bars + 9 /* two */, *state_read = bars + 11;
   // (done: two, since an output warp that still adds a chunk's outputs may find the products of the next two done. Those of one barrier would then be as many
   // phases ahead, which reads as not done. With two, the third's products wait for outputs_read.)
-  uint32_t* slot_at = reinterpret_cast<uint32_t*>(bars + 11);
-  int* plain_at = reinterpret_cast<int*>(bars + 12);             // [4]: a chunk's products with the state are plain sums
+  uint32_t* slot_at = reinterpret_cast<uint32_t*>(bars + 12);
+  int* plain_at = reinterpret_cast<int*>(bars + 13);             // [4]: a chunk's products with the state are plain sums
   uint32_t* most = reinterpret_cast<uint32_t*>(smem + I::most);  // [3][64]: the state's largest, column by column
   if (tid == 0) {
-    for (int i = 0; i < 11; ++i) tw_bar_init(bars + i, i >= 4 && i <= 8 ? 8 : 1);
+    for (int i = 0; i < 12; ++i) tw_bar_init(bars + i, (i >= 4 && i <= 8) || i == 11 ? 8 : 1);
+    for (int i = 0; i < 4; ++i) plain_at[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == TW_WORKERS / 32) {
@@ -992,15 +998,22 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
   const int w = warp & 7, quad = w & 3, c0 = COLS * (w >> 2);  // of tensor memory's lanes, of the columns
   const size_t images = MODE == TW_HEAD ? g.H / g.qk_group : g.H, own = MODE == TW_HEAD ? h / g.qk_group : h;
   bool ok = true;
+  auto wait = [&](uint64_t* bar, int use) { return tw_wait(bar, use, g.waits.limit_ns); };
+  auto all_wait = [&](uint64_t* bar, int use) { return __all_sync(0xffffffffu, wait(bar, use)); };  // (a warp's lanes go on as one)
 
   if (warp == TW_WORKERS / 32) {
     // ---- copies and products
     if (tw_elect()) {
+      int q_sent = 0, added_sent = 0, products = 0;
       auto copy_q = [&](int c) {
+        if (c >= g.waits.no_queries) return;
+        ++q_sent;
         tw_expect(q_full + ((c - first) & 1), I::image);
         tw_bulk(smem + I::q + ((c - first) & 1) * I::image, g.q_image + ((size_t)(chunk0 + c) * images + own) * I::image, I::image, q_full + ((c - first) & 1));
       };
       auto copy_added = [&](int c) {
+        if (c >= g.waits.no_added) return;
+        ++added_sent;
         tw_expect(added_full + (c & 1), I::sums);
         tw_bulk(smem + I::added + (c & 1) * I::sums, g.added + (((size_t)(chunk0 + c) * g.H + h) * g.tiles + tile) * (TW_COLS * DKP), I::sums, added_full + (c & 1));
       };
@@ -1013,7 +1026,8 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
       for (int c = 0; c < steps && ok; ++c) {
         const int k = c - first;
         if (k >= 0) {
-          ok = tw_wait(state_in, k) && tw_wait(q_full + (k & 1), k >> 1) && (k < 2 || tw_wait(outputs_read + (k & 1), (k >> 1) - 1));
+          ok = wait(state_in, k) && wait(q_full + (k & 1), k >> 1) && (k < 2 || wait(outputs_read + (k & 1), (k >> 1) - 1));
+          if (!ok) break;
           const uint64_t a = tw_desc(smem + I::q + (k & 1) * I::image);
 #pragma unroll
           for (int blk = 0; blk < NB; ++blk)
@@ -1021,15 +1035,23 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
             for (int ks = 0; ks < 4; ++ks)
               tw_mma_parts<true>(tmem + (k & 1) * 128, a + ((blk * TW_TILE + ks * 32) >> 4), NB * TW_TILE, b + ((blk * 4 + ks) * 2048 >> 4), DKP * 128, blk + ks > 0);
           tw_commit(done + (k & 1));
+          ++products;
         }
-        ok = ok && tw_wait(added_read + (c & 1), c >> 1);
+        ok = wait(added_read + (c & 1), c >> 1);
         if (c + 2 < steps && ok) copy_added(c + 2);
         if (k >= 0) {
-          ok = ok && tw_wait(done + (k & 1), k >> 1);
+          ok = ok && wait(done + (k & 1), k >> 1);
           if (c + 2 < steps && ok) copy_q(c + 2);
         }
       }
-      if (!ok && g.status) atomicMax(g.status, 42);
+      if (!ok) {
+        if (g.status) atomicMax(g.status, 42);
+        for (int b = 0; b < 2; ++b) {  // the last use of each of the two
+          if (q_sent > b) wait(q_full + b, (q_sent - 1 - b) >> 1);
+          if (added_sent > b) wait(added_full + b, (added_sent - 1 - b) >> 1);
+          if (products > b) wait(done + b, (products - 1 - b) >> 1);
+        }
+      }
     }
     __syncwarp();
   } else if (warp < 8) {
@@ -1055,6 +1077,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
     float keep = last[0];
     int large = large_at[0];
     bool plain = false;
+    int plain_chunks = 0;
 #pragma unroll 1
     for (int c = 0; c < steps; ++c) {
       const int k = c - first;
@@ -1067,14 +1090,14 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
         const uint32_t mine = tw_largest(size, lane);
         if (has_ch) atomicMax(mx + c0 + lane, mine);
         const bool was = plain;
-        plain = tw_group_any(1, (has_ch && mine >= TW_MOST) || !ok || large);
+        plain = tw_group_any(1, (has_ch && mine >= TW_MOST) || large);
         if (tid == 0) plain_at[k & 3] = plain;
         if (tid < 64) most[(k + 2) % 3 * 64 + tid] = 0;  // (read before this chunk's barrier, used behind the next one's)
         float* grids = reinterpret_cast<float*>(smem + I::grids) + c0;  // (the warps of these columns write the same)
         grids[lane] = tw_grid(tw_power(mx[c0 + lane]));
         __syncwarp();
-        if (k > 0) ok = ok && tw_wait(done + ((k - 1) & 1), (k - 1) >> 1);
-        if (was) asm volatile("bar.sync 3, 512;\n" ::: "memory");  // (the plain sums have read the state)
+        if (k > 0) ok = ok && all_wait(done + ((k - 1) & 1), (k - 1) >> 1);
+        if (was) ok = ok && all_wait(state_read, plain_chunks++);  // (the plain sums have read the state)
         if (plain) {
           float* Sf = reinterpret_cast<float*>(smem + I::s);
           if (has_ch)
@@ -1104,7 +1127,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
         last += (size_t)g.H * F::floats, large_at += images;
         keep = last[0], large = large_at[0];
       }
-      ok = ok && tw_wait(added_full + (c & 1), c >> 1);
+      ok = ok && all_wait(added_full + (c & 1), c >> 1);
       const float* add = reinterpret_cast<const float*>(smem + I::added + (c & 1) * I::sums);
 #pragma unroll
       for (int j = 0; j < COLS; j += 4) {
@@ -1113,8 +1136,9 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
       }
       tw_arrive(added_read + (c & 1));
     }
-    if (plain) asm volatile("bar.sync 3, 512;\n" ::: "memory");
-    if (has_ch && at.index == at.count - 1 && ch < g.dk) {
+    if (!ok && lane == 0 && g.status) atomicMax(g.status, 42);
+    const bool lost = tw_group_any(1, !ok);  // (a part of it did not come)
+    if (!lost && has_ch && at.index == at.count - 1 && ch < g.dk) {
 #pragma unroll
       for (int j = 0; j < COLS; ++j)
         if (v0 + c0 + j < g.dv) slot[(size_t)(v0 + c0 + j) * g.dk + ch] = S[j];
@@ -1129,7 +1153,8 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
       const size_t item = (size_t)(chunk0 + c) * g.H + h;
       const float* fac = g.factors + item * F::floats;
       const float by0 = MODE == TW_HEAD ? fac[F::from + row] : 1.f, by1 = MODE == TW_HEAD ? fac[F::from + row + 8] : 1.f;
-      ok = ok && tw_wait(done + (k & 1), k >> 1);
+      ok = all_wait(done + (k & 1), k >> 1);
+      if (!ok) break;
       if (plain_at[k & 3]) {
         tw_arrive(outputs_read + (k & 1));
         const float* Sf = reinterpret_cast<const float*>(smem + I::s);
@@ -1141,7 +1166,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
           if (MODE == TW_HEAD) r *= fac[F::from + i];
           if (v0 + e < g.dv) atomicAdd(g.o + ((size_t)(tok0 + i) * g.H + h) * g.dv + v0 + e, r);
         }
-        asm volatile("bar.sync 3, 512;\n" ::: "memory");
+        tw_arrive(state_read);
         continue;
       }
       float r[16];
@@ -1149,6 +1174,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
       tw_arrive(outputs_read + (k & 1));
       tw_add_outputs(g, r, by0, by1, tok0, row, n, h, col);
     }
+    if (!ok && lane == 0 && g.status) atomicMax(g.status, 42);
   }
   __syncthreads();
   if (warp == TW_WORKERS / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem) : "memory");
@@ -1230,9 +1256,10 @@ static int launch_tile_head(const TwPlan& plan, TwArgs g, float* scratch, cudaSt
 
 int tile_walk_head(float* o, float* state, const float* q, int ld_q, const float* k, int ld_k, int qk_group, const float* v, int ld_v, const float* decay,
                    int ld_decay, const float* v_scale, float* scratch, const int* cu_q, const int* q_start, const int* state_slot, int num_tokens,
-                   int num_rows, int H, int dk, int dv, float q_scale, int* status, cudaStream_t stream) {
+                   int num_rows, int H, int dk, int dv, float q_scale, int* status, cudaStream_t stream, const TwWaits& waits) {
   const TwPlan plan(num_tokens, num_rows, H, dk, dv, H / qk_group);
   TwArgs g = {};
+  g.waits = waits;
   g.o = o, g.state = state, g.q = q, g.ld_q = ld_q, g.k = k, g.ld_k = ld_k, g.qk_group = qk_group, g.v = v, g.ld_v = ld_v, g.status = status;
   g.decay = decay, g.ld_decay = ld_decay, g.v_scale = v_scale, g.q_scale = q_scale;
   g.cu_q = cu_q, g.q_start = q_start, g.state_slot = state_slot, g.num_rows = num_rows, g.H = H, g.dk = dk, g.dv = dv;
@@ -1261,9 +1288,10 @@ static int launch_tile_channel(const TwPlan& plan, TwArgs g, float* scratch, con
 template <typename TIn, typename TZ>
 int tile_walk_channel(float* o, float* state, const TIn* q, int ld_q, const TIn* k, int ld_k, int qk_group, const TIn* v, int ld_v, const TZ* z, int ld_z,
                       const float* z_bias, const float* decay_coef, float z_sign, const float* v_scale, float* scratch, const int* cu_q, const int* q_start,
-                      const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, int* status, cudaStream_t stream) {
+                      const int* state_slot, int num_tokens, int num_rows, int H, int dk, int dv, float q_scale, int* status, cudaStream_t stream, const TwWaits& waits) {
   const TwPlan plan(num_tokens, num_rows, H, dk, dv, 0);
   TwArgs g = {};
+  g.waits = waits;
   g.o = o, g.state = state, g.ld_q = ld_q, g.ld_k = ld_k, g.qk_group = qk_group, g.v = v, g.ld_v = ld_v, g.status = status, g.v_scale = v_scale;
   g.cu_q = cu_q, g.q_start = q_start, g.state_slot = state_slot, g.num_rows = num_rows, g.H = H, g.dk = dk, g.dv = dv;
   if (dk <= 64) return launch_tile_channel<TIn, TZ, 2>(plan, g, scratch, q, k, z, ld_z, z_bias, decay_coef, z_sign, q_scale, stream);
@@ -1273,7 +1301,7 @@ int tile_walk_channel(float* o, float* state, const TIn* q, int ld_q, const TIn*
 #define MS_TW_CHANNEL(TIN, TZZ)                                                                                                                     \
   template int tile_walk_channel<TIN, TZZ>(float*, float*, const TIN*, int, const TIN*, int, int, const TIN*, int, const TZZ*, int, const float*,   \
                                            const float*, float, const float*, float*, const int*, const int*, const int*, int, int, int, int, int,  \
-                                           float, int*, cudaStream_t)
+                                           float, int*, cudaStream_t, const TwWaits&)
 MS_TW_CHANNEL(float, float);
 MS_TW_CHANNEL(float, __nv_bfloat16);
 MS_TW_CHANNEL(__nv_bfloat16, float);

@@ -184,6 +184,8 @@ def recurrence():
     _declare(lib, "ms_chunk_max", [_i, _i])
     _declare(lib, "ms_walk_scratch", [_i] * 7, _ll)
     _declare(lib, "ms_walk_kernels", [_i] * 7)
+    _declare(lib, "ms_tile_walk_scratch", [_i] * 6, _ll)
+    _declare(lib, "ms_tile_walk_selftest", [_p] * 10 + [_i] * 5 + [_p, _i, _i, _ll, _p])
     _declare(lib, "ms_walk_scan", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p, _f, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _i, _i, _i, _p, _p])
     _declare(lib, "ms_walk_scan_head", [_p, _p, _p, _i, _p, _i, _i, _p, _i, _p, _i, _p, _p] + [_p] * 3 + [_i] * 5 + [_f, _p, _p])
     _declare(lib, "ms_chunk_supports", [_i, _i])

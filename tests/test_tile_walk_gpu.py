@@ -128,3 +128,32 @@ def test_values_that_are_not_finite_stay_with_their_token_and_the_later_ones(rul
         assert torch.equal(torch.isfinite(g), torch.isfinite(w))
         own = (w - p).abs() <= 1e-5 * p.abs().max()  # (what the number does not reach; the walk says which)
         assert own.float().mean() > 0.5 and ((g - p).abs()[own] <= 2e-5 * p.abs().max()).all()
+
+
+@pytest.mark.parametrize("dk", [64, 128])
+@pytest.mark.parametrize("no_queries, no_added", [(0, 1 << 30), (2, 1 << 30), (1 << 30, 0), (1 << 30, 3), (1, 1)])
+def test_copies_that_do_not_come_end_the_walk_with_an_error(dk, no_queries, no_added):
+    """The walk ends by itself with the status word raised, whichever of its roles waits in vain; a state that lacks what a chunk adds is not kept."""
+    gen = torch.Generator().manual_seed(1)
+    heads, dv, rows = 2, 64, [(4, 300), (0, 400)]
+    t, lib, ctx = sum(n for _, n in rows), native.recurrence(), _ctx(rows, [1, 0])
+    q, k, v = (torch.randn(t, heads * d, generator=gen).to(DEV) for d in (dk, dk, dv))
+    decay, state = torch.rand(t, heads, generator=gen).to(DEV), torch.randn(2, heads, dv, dk, generator=gen).to(DEV)
+    scratch = torch.zeros(lib.ms_tile_walk_scratch(t, len(rows), heads, dk, dv, heads), device=DEV)
+
+    def go(none_q, none_added):
+        o, st, status = torch.zeros(t, heads, dv, device=DEV), state.clone(), torch.zeros(1, dtype=torch.int32, device=DEV)
+        native.recurrence_check(lib.ms_tile_walk_selftest(o.data_ptr(), st.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(),
+                                                          scratch.data_ptr(), ctx.cu_q.data_ptr(), ctx.q_start.data_ptr(), ctx.state_slot.data_ptr(), t, len(rows), heads,
+                                                          dk, dv, status.data_ptr(), none_q, none_added, 20_000_000, ctx.stream), launches=3)
+        torch.cuda.synchronize()
+        return o, st, status.item()
+
+    want = go(1 << 30, 1 << 30)
+    assert want[2] == 0 and torch.isfinite(want[0]).all() and not torch.equal(want[1], state)
+    _, st, status = go(no_queries, no_added)
+    assert status == 42
+    if no_added < 4:  # both rows have five chunks or more
+        assert torch.equal(st, state)
+    again = go(1 << 30, 1 << 30)
+    assert torch.equal(again[0], want[0]) and torch.equal(again[1], want[1]) and again[2] == 0
