@@ -13,17 +13,21 @@
 // rows leave multiprocessors idle, the third cuts rows into segments; each adds up the state from the row's first chunk on, in the same
 // steps, so that a segment's outputs have the bits of the whole row's.
 //
-// Accuracy: factors are three bfloat16 on common grids, whose products the tensor cores add up without rounding (below), 27 bits of a row's
-// largest number. Pairs of one sixteen tokens are float32 sums of multiply-adds. Products of decays are worked out in 64 bits and rounded once (a running
-// product of decays just below one is rounded down every time). A state is rounded twice in 64 tokens. Root mean squares of the errors over 2,048 tokens: 0.16 to
-// 0.96 of the token-by-token walk's (outputs), 0.13 to 1.0 (states), decays from 0.02 to 1. A token sees nothing of the tokens behind it, whatever they hold: chunks with
-// values that are not finite, or of 2^48 and more, are worked out in plain sums, every pair by itself. (With one decay per head the
+// Accuracy: a factor is the sum of three bfloat16 that hold all of its 24 bits, whatever its neighbours are (the splitting of Henry, Tang and Heinecke,
+// "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", 2019). Tensor cores cut sums off where float32 rounds them; so
+// pairs of one sixteen tokens and what a chunk's last eight tokens add to the state are float32 multiply-adds, and the sums of the rest are short. Products of
+// decays are worked out in 64 bits and rounded once (a running product of decays just below one is rounded down every time). A state is rounded twice in 64 tokens.
+// Root mean squares of the errors over 1,400 and 2,088 tokens, against the token-by-token walk's and the chunks of 16's, decays from 0.02 to 0.99999: outputs 0.28 to 0.96
+// and 0.36 to 1.07, states 0.13 to 1.02 and 0.25 to 1.00. With one channel, token or number in a hundred 1,024 to 16,384 times the others, or keys by 2^s and queries by 2^-s
+// (s from -12 to 12): outputs 0.27 to 1.1 of either, with exact decays none off by more than 8e-7 of its terms' sizes. A token sees nothing of the tokens behind it, whatever they hold:
+// chunks with values that are not finite, or of 2^48 and more, are worked out in plain sums, every pair by itself. (With one decay per head the
 // sums against the state are scaled behind the sum: a state within q's size of the largest float overflows.)
 //
-// What bounds it, 64 heads of 128 x 64, three rows of 1,037, 640 and 371 tokens, 263 us by chunks of 16 and 165 here: the second kernel (90 us) issues 19,000 instructions a
-// chunk and head at half the rate, most of them making operands and adding up results (tensor cores busy 26 %); the third (62) is a chain of 17 chunks of 2.5 us (the
-// products 1.1 of them, bound by shared memory; the state's parts 0.7), the first 19. Measured and not kept: the same products in float32
-// multiply-adds, 8 x 8 outputs a thread (332 us: both shared memory and the FMA pipe at 54 %); all three kernels' work on the chain (322).
+// What bounds it, 64 heads of 128 x 64, three rows of 1,037, 640 and 371 tokens, 263 us by chunks of 16 and 169 here: the second kernel (91 us) issues its instructions at
+// half the rate, most of them making operands and adding up results; the third (54) is a chain of 17 chunks, bound by shared memory and the state's parts; the first 23.
+// Measured and not kept: the same products in float32 multiply-adds, 8 x 8 outputs a thread (332 us: both shared memory and the FMA pipe at 54 %); all three kernels' work
+// on the chain (322); parts on a grid that a row shares, whose products add up without any cut (165, but a row's small numbers lose the bits that its largest takes: one
+// value channel of 1,024 made outputs 28 times as far off).
 #include <cfloat>
 
 #include "chunk_mma.cuh"
@@ -32,7 +36,10 @@
 
 namespace ms {
 
-constexpr int TW_FIRST = 256, TW_WORKERS = 512, TW_THREADS = TW_WORKERS + 32, TW_COLS = 64, TW_SUB = 16, TW_BLOCKS = 10;  // (TW_BLOCKS: of 16 x 16 pairs on and below a chunk's diagonal)
+constexpr int TW_FIRST = 256, TW_WORKERS = 512, TW_THREADS = TW_WORKERS + 32, TW_COLS = 64, TW_SUB = 16;
+// A chunk's pairs: the blocks of 16 x 16 below the diagonal, then those on it. With one decay per head these are not decayed yet, and in 64 bits: what they are
+// multiplied with is, and the product is rounded once.
+constexpr int TW_BLOCK = TW_SUB * TW_SUB, TW_DIAGONAL = 6 * TW_BLOCK;
 enum TileWalkMode : int { TW_CHANNEL = 0, TW_HEAD = 1 };
 
 __device__ __forceinline__ float tw_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
@@ -77,7 +84,8 @@ __device__ __forceinline__ TwPiece tw_piece(int at, int tokens, const int* __res
   return none;
 }
 
-__device__ __forceinline__ int tw_block(int i, int j) { return i * (i + 1) / 2 + j; }
+__device__ __forceinline__ int tw_below(int i, int j) { return (i * (i - 1) / 2 + j) * TW_BLOCK; }  // (floats)
+__host__ __device__ constexpr int tw_pairs(bool head) { return TW_DIAGONAL + 4 * TW_BLOCK * (head ? 2 : 1); }
 
 // A chunk's factors, for each head: the decays from the chunk's first token to each (times q's factor), where there is one per head; those of the whole chunk.
 template <int MODE, int DKP>
@@ -86,46 +94,32 @@ struct TwFactors {  // floats
 };
 
 // ---------------------------------------------------------------- numbers in three parts
-// A number x of a row whose largest is below 2^e is h + m + l: h a multiple of 2^(e - 8), m of 2^(e - 17), at most half a step of the part before
-// in size, l the rest rounded to eight bits (an error of 2^(e - 27) at most). All are bfloat16. Products of h's are multiples of one number, and
-// the sum of 128 of them stays below 2^24 of it: the tensor cores add them up without rounding, and what is left out (m l, l m, l l) is
-// below 2^-27 of the largest products.
-constexpr uint32_t TW_LEAST = (127u - 99u) << 23, TW_MOST = (127u + 48u) << 23,
-                   TW_MOST_PAIRS = (127u + 97u) << 23;  // (e from -99 on; numbers of 2^48 and more, pairs times values of 2^97, go to the plain sums)
-__device__ __forceinline__ uint32_t tw_power(uint32_t largest) {  // the bits of 2^e for the bits of the largest size of a row
-  return max((largest & 0x7f800000u) + 0x00800000u, TW_LEAST);
-}
-__device__ __forceinline__ float tw_grid(uint32_t power) { return __uint_as_float((power + (15u << 23)) | 0x00400000u); }  // 1.5 2^(e + 15)
+// A float32 number is the sum of three bfloat16, each what is left rounded to eight bits: of all its 24 bits, whatever its neighbours are. Their
+// products are exact; l l, below 2^-36 of a product, is left out. What the tensor cores lose is what falls off a sum that grows: they cut off where
+// float32 sums round. So the products of the first parts, where that counts, have a short chain and an accumulator of their own.
+constexpr uint32_t TW_MOST = (127u + 48u) << 23, TW_MOST_PAIRS = (127u + 72u) << 23;  // (numbers, pairs of 2^48, 2^72 and more go to the plain sums)
 __device__ __forceinline__ uint32_t tw_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ uint32_t tw_pack(f2 x) {
   uint32_t r;
   const float2 h = f2_halves(x);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(h.y), "f"(h.x));
   return r;
 }
-__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
+__device__ __forceinline__ f2 tw_less(f2 a, uint32_t b) {  // a - b, which is exact here
   f2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(f2_pair(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u))));
   return r;
 }
-// the parts of two numbers, each with a grid of its own
-__device__ __forceinline__ void tw_parts(uint32_t (&out)[3], f2 x, f2 grid) {
-  const f2 finer = f2_mul(grid, f2_pair(0x1p-9f, 0x1p-9f));
-  const f2 h = f2_sub(f2_add(x, grid), grid), r = f2_sub(x, h), m = f2_sub(f2_add(r, finer), finer);
-  out[0] = tw_pack(h);
-  out[1] = tw_pack(m);
-  out[2] = tw_pack(f2_sub(r, m));
+__device__ __forceinline__ void tw_parts(uint32_t (&out)[3], f2 x) {
+  out[0] = tw_pack(x);
+  const f2 r = tw_less(x, out[0]);
+  out[1] = tw_pack(r);
+  out[2] = tw_pack(tw_less(r, out[1]));
 }
-// eight numbers of one grid
-__device__ __forceinline__ void tw_parts8(uint4 (&out)[3], const float* x, float grid) {
+__device__ __forceinline__ void tw_parts8(uint4 (&out)[3], const float* x) {
   uint32_t w[4][3];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) tw_parts(w[i], f2_pair(x[2 * i], x[2 * i + 1]), f2_pair(grid, grid));
+  for (int i = 0; i < 4; ++i) tw_parts(w[i], f2_pair(x[2 * i], x[2 * i + 1]));
 #pragma unroll
   for (int p = 0; p < 3; ++p) out[p] = make_uint4(w[0][p], w[1][p], w[2][p], w[3][p]);
 }
@@ -134,26 +128,14 @@ constexpr int TW_TILE = TW_TOK * 128;
 __device__ __forceinline__ int tw_at(int row, int eight) { return row * 128 + ((eight ^ (row & 7)) << 4); }
 
 // Queries and keys of a chunk, [64][LD] in shared memory, as operand tiles in global memory: queries [part][channels / 64][64 tokens][64 channels],
-// keys [part][channels][64 tokens]. Returns whether a number is too large or none.
+// keys [part][channels][64 tokens]. Returns whether a thread's numbers are too large or none.
 template <int DK, int LD>
-__device__ __forceinline__ bool tw_images(uint8_t* q_to, uint8_t* k_to, const float* qs, const float* ks, uint32_t* most) {
+__device__ __forceinline__ bool tw_images(uint8_t* q_to, uint8_t* k_to, const float* qs, const float* ks) {
   constexpr int CP = DK < 64 ? 64 : DK, PARTS = TW_FIRST / CP, TOKENS = TW_TOK / PARTS, PART = CP / 64 * TW_TILE;  // (CP: channels with those behind the last)
   const int tid = threadIdx.x;
   uint32_t worst = 0;
   {  // four threads a token, every fourth run of eight channels each
     const int i = tid >> 2, part = tid & 3;
-    uint32_t largest = 0;
-#pragma unroll
-    for (int e = part * 8; e < DK; e += 32)
-#pragma unroll
-      for (int c = 0; c < 8; c += 4) {
-        const float4 y = *reinterpret_cast<const float4*>(qs + i * LD + e + c);
-        largest = max(max(max(largest, tw_bits(y.x)), tw_bits(y.y)), max(tw_bits(y.z), tw_bits(y.w)));
-      }
-    largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
-    largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
-    worst = largest;
-    const float grid = tw_grid(tw_power(largest));
 #pragma unroll
     for (int e = part * 8; e < CP; e += 32) {
       float x[8];
@@ -161,31 +143,25 @@ __device__ __forceinline__ bool tw_images(uint8_t* q_to, uint8_t* k_to, const fl
       for (int c = 0; c < 8; c += 4) {
         const float4 y = e < DK ? *reinterpret_cast<const float4*>(qs + i * LD + e + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         x[c] = y.x, x[c + 1] = y.y, x[c + 2] = y.z, x[c + 3] = y.w;
+        worst = max(max(max(worst, tw_bits(y.x)), tw_bits(y.y)), max(tw_bits(y.z), tw_bits(y.w)));
       }
       uint4 y[3];
-      tw_parts8(y, x, grid);
+      tw_parts8(y, x);
 #pragma unroll
       for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(q_to + p * PART + (e >> 6) * TW_TILE + tw_at(i, (e & 63) >> 3)) = y[p];
     }
   }
   const int ch = tid % CP, t0 = tid / CP * TOKENS;
-  if (tid < CP) most[tid] = 0;
-  __syncthreads();
-  uint32_t largest = 0;
-  if (ch < DK)
-#pragma unroll
-    for (int t = 0; t < TOKENS; ++t) largest = max(largest, tw_bits(ks[(t0 + t) * LD + ch]));
-  atomicMax(most + ch, largest);
-  __syncthreads();
-  worst = max(worst, most[ch]);
-  const float grid = tw_grid(tw_power(most[ch]));
 #pragma unroll
   for (int t = 0; t < TOKENS; t += 8) {
     float x[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = ch < DK ? ks[(t0 + t + e) * LD + ch] : 0.f;
+    for (int e = 0; e < 8; ++e) {
+      x[e] = ch < DK ? ks[(t0 + t + e) * LD + ch] : 0.f;
+      worst = max(worst, tw_bits(x[e]));
+    }
     uint4 y[3];
-    tw_parts8(y, x, grid);
+    tw_parts8(y, x);
 #pragma unroll
     for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(k_to + p * PART + tw_at(ch, (t0 + t) >> 3)) = y[p];
   }
@@ -194,7 +170,7 @@ __device__ __forceinline__ bool tw_images(uint8_t* q_to, uint8_t* k_to, const fl
 
 // ---------------------------------------------------------------- one decay per head: operands and dot products
 // grid (chunks, groups of heads that share q and k). A thread's 4 x 4 dot products (tokens wb * 16 + ty + 4 a against 32 half + tx + 8 b), sums of
-// sixteen products, added up in 64 bits: however much smaller than others a token's numbers are, its pairs are as precise.
+// eight products, added up in 64 bits: however much smaller than others a token's numbers are, its pairs are as precise.
 template <int DK>
 __global__ void __launch_bounds__(TW_FIRST, 2)
 tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_t* __restrict__ k_image, int* __restrict__ plain, const float* __restrict__ q,
@@ -202,7 +178,6 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
   constexpr int LD = DK + 4;
   extern __shared__ __align__(16) float tw_smem[];
   float *qs = tw_smem, *ks = qs + TW_TOK * LD;
-  __shared__ uint32_t most[DK < 64 ? 64 : DK];
   pdl_prologue();
   const int grp = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const TwPiece at = tw_piece(blockIdx.x, TW_TOK, cu_q, num_rows);
@@ -223,7 +198,7 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
   const size_t image = (size_t)at.chunk * gridDim.y + grp;
   {
     constexpr size_t bytes = (size_t)3 * (DK <= 64 ? 1 : 2) * TW_TILE;
-    const bool bad = tw_images<DK, LD>(q_image + image * bytes, k_image + image * bytes, qs, ks, most);
+    const bool bad = tw_images<DK, LD>(q_image + image * bytes, k_image + image * bytes, qs, ks);
     const int any = __syncthreads_or(bad);
     if (tid == 0) plain[image] = any;
   }
@@ -231,10 +206,10 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
   if (half != 0 && wb < 2) return;
   double sum[4][4] = {};
 #pragma unroll 1
-  for (int c0 = 0; c0 < DK; c0 += 16) {
+  for (int c0 = 0; c0 < DK; c0 += 8) {
     f2 part[4][4] = {};
 #pragma unroll
-    for (int c = 0; c < 16; c += 4) {
+    for (int c = 0; c < 8; c += 4) {
       ulonglong2 a[4], b[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -254,13 +229,17 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
 #pragma unroll
       for (int y = 0; y < 4; ++y) sum[x][y] += (double)f2_sum(part[x][y]);
   }
-  float* to = dots + image * (TW_BLOCKS * TW_SUB * TW_SUB);
+  float* to = dots + image * tw_pairs(true);
+  double* diagonal = reinterpret_cast<double*>(to + TW_DIAGONAL) + wb * TW_BLOCK;
 #pragma unroll
   for (int y = 0; y < 4; ++y) {
     const int j = half * 32 + tx + 8 * y;
-    if ((j >> 4) <= wb)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) to[(tw_block(wb, j >> 4) * TW_SUB + ty + 4 * x) * TW_SUB + (j & 15)] = (float)sum[x][y];
+    for (int x = 0; x < 4; ++x) {
+      const int at = (ty + 4 * x) * TW_SUB + (j & 15);
+      if ((j >> 4) < wb) to[tw_below(wb, j >> 4) + at] = (float)sum[x][y];
+      if ((j >> 4) == wb) diagonal[at] = sum[x][y];
+    }
   }
 }
 
@@ -299,7 +278,6 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
   constexpr bool KEEP = N <= 2;  // k' stays in shared memory as well (a fourth array; at N = 4 it would leave room for one CTA)
   float* kf = KEEP ? ds + TW_TOK * LD : ks;
   __shared__ double whole[SUBS][DKP];  // a sixteen's decays
-  __shared__ uint32_t most[DKP];
   pdl_prologue();
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const TwPiece at = tw_piece(blockIdx.x, TW_TOK, cu_q, num_rows);
@@ -351,7 +329,7 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
     }
   }
   float* fac = factors + item * F::floats;
-  float* out = pairs + item * (TW_BLOCKS * TW_SUB * TW_SUB);
+  float* out = pairs + item * tw_pairs(false);
   __syncthreads();
 #pragma unroll 1
   for (int sub = warp >> 2; sub < SUBS; sub += 2) {
@@ -385,7 +363,7 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int i = 2 * cl + e;
-      out[(tw_block(sub, sub) * TW_SUB + i) * TW_SUB + j] = i >= j ? (float)val[e] : 0.f;
+      out[TW_DIAGONAL + sub * TW_BLOCK + i * TW_SUB + j] = i >= j ? (float)val[e] : 0.f;
     }
   }
   __syncthreads();
@@ -478,7 +456,7 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
 #pragma unroll
           for (int y = 0; y < 2; ++y) sum[x][y] += (double)f2_sum(part[x][y]);
       }
-      float* to = out + tw_block(jb + far, jb) * TW_SUB * TW_SUB;
+      float* to = out + tw_below(jb + far, jb);
 #pragma unroll
       for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -494,7 +472,7 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
     __syncthreads();
   }
   const size_t bytes = (size_t)3 * (DKP / 64) * TW_TILE;
-  const bool bad = tw_images<DKP, LD>(q_image + item * bytes, k_image + item * bytes, ds, kf, most);
+  const bool bad = tw_images<DKP, LD>(q_image + item * bytes, k_image + item * bytes, ds, kf);
   const int any = __syncthreads_or(bad);
   if (tid == 0) plain[item] = any;
 }
@@ -553,14 +531,19 @@ __device__ __forceinline__ void tw_tmem_pairs(float (&r)[16], uint32_t at) {
                  "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
                : "r"(at));
 }
-// both accumulators' sum
+// the sum of SETS pairs of accumulators, 128 columns each
+template <int SETS>
 __device__ __forceinline__ void tw_tmem_sums(float (&r)[16], uint32_t at) {
-  float rest[16];
+  float more[2 * SETS - 1][16];
   tw_tmem_pairs(r, at);
-  tw_tmem_pairs(rest, at + 64);
+#pragma unroll
+  for (int i = 1; i < 2 * SETS; ++i) tw_tmem_pairs(more[i - 1], at + 64 * (i & 1) + 128 * (i >> 1));
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-  for (int j = 0; j < 16; ++j) r[j] += rest[j];
+  for (int j = 0; j < 16; ++j) {
+    if constexpr (SETS == 2) r[j] = (r[j] + more[1][j]) + (more[0][j] + more[2][j]);
+    else r[j] += more[0][j];
+  }
 }
 __device__ __forceinline__ bool tw_elect() {
   uint32_t pred;
@@ -574,24 +557,6 @@ __device__ __forceinline__ bool tw_group_any(int id, bool flag) {  // a barrier 
       : "=r"(res) : "r"(id), "r"((uint32_t)flag) : "memory");
   return res != 0;
 }
-// The largest of each of N numbers (bits of sizes) over a warp's lanes: lane l comes back with number l's (N < 32: l % N's).
-template <int N>
-__device__ __forceinline__ uint32_t tw_largest(uint32_t (&x)[N], int lane) {
-#pragma unroll
-  for (int o = N / 2; o > 0; o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const uint32_t send = up ? x[i] : x[i + o], keep = up ? x[i + o] : x[i];
-      x[i] = max(keep, __shfl_xor_sync(0xffffffffu, send, o));
-    }
-  }
-  uint32_t r = x[0];
-#pragma unroll
-  for (int o = 16; o >= N; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
-  return r;
-}
-
 struct TwArgs {
   float *o, *state;
   const uint8_t *q_image, *k_image;
@@ -629,10 +594,13 @@ __device__ __forceinline__ void tw_add_outputs(const TwArgs& g, const float (&r)
 // ---------------------------------------------------------------- a chunk by itself
 // grid (chunks x column tiles, H, 2): what the chunk adds to the state (z = 0), and the outputs that come of its own pairs (z = 1). A thread has one
 // column's 16 values, and 16 pairs of a token. Pairs of different sixteens are products of parts; those of one sixteen are plain sums, a column's in the
-// thread that has its values: where a token's own value is all that is left, it is as precise as any (a token's values share a grid).
-struct TwChunk {  // bytes
-  static constexpr int b = 0, a = 3 * TW_TILE, near = 6 * TW_TILE, runs = near + 4 * TW_SUB * TW_SUB * 4, fac = runs + 3 * TW_TOK * 8, most = fac + 2 * TW_TOK * 4,
-                       bars = most + TW_TOK * 4, all = bars + 64;
+// thread that has its values: where a token's own value is all that is left, it is as precise as any. So is what the last eight tokens add to the state, which
+// is most of it where decays are fast (with four, a state under decays from 0.7 to 0.99 is 1.14 times as far off as token by token).
+constexpr int TW_LAST = 8;
+struct TwChunk {  // bytes (last: where the pairs of one sixteen and, once they are in the values, products of decays are)
+  static constexpr int b = 0, a = 3 * TW_TILE, runs = 6 * TW_TILE, near = runs + 3 * TW_TOK * 8, last = runs, fac = last + TW_LAST * (TW_COLS + 128) * 4, bars = fac + 2 * TW_TOK * 4,
+                       all = bars + 64;
+  static_assert(near + 4 * TW_BLOCK * 4 <= fac, "pairs and products of decays end ahead of the factors");
 };
 template <int MODE, int DKP, typename TV>
 __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g) {
@@ -649,7 +617,6 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
   const size_t item = (size_t)at.chunk * g.H + h, image = MODE == TW_HEAD ? (size_t)at.chunk * (g.H / g.qk_group) + h / g.qk_group : item;
   uint64_t *k_full = reinterpret_cast<uint64_t*>(smem + I::bars), *done = k_full + 2;
   uint32_t* slot_at = reinterpret_cast<uint32_t*>(k_full + 4);
-  uint32_t* most = reinterpret_cast<uint32_t*>(smem + I::most);  // z = 0: of the columns' decayed values, z = 1: of the tokens'
   double *as = reinterpret_cast<double*>(smem + I::runs), *upto = as + TW_TOK, *after = upto + TW_TOK;  // decays; from a sixteen's start, to its end
   float *scale = reinterpret_cast<float*>(smem + I::fac), *behind = scale + TW_TOK;
   auto copy_keys = [&](int half) {
@@ -664,7 +631,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
   }
   const int quad = warp & 3, c0 = 32 * (warp >> 2), vcol = c0 + lane, vtok = 16 * quad, prow = tid >> 2, ppart = tid & 3;
   const bool has_col = v0 + vcol < g.dv;
-  const float* pairs = g.pairs + (MODE == TW_HEAD ? image : item) * (TW_BLOCKS * TW_SUB * TW_SUB);  // (one decay per head: not decayed yet)
+  const float* pairs = g.pairs + (MODE == TW_HEAD ? image : item) * tw_pairs(MODE == TW_HEAD);
   float u[16];
   {
     const TV* from = static_cast<const TV*>(g.v) + (size_t)(tok0 + vtok) * g.ld_v + (size_t)h * g.dv + v0 + vcol;
@@ -679,7 +646,6 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid < TW_TOK) {
-      most[tid] = 0;
       scale[tid] = g.v_scale && tid < n ? g.v_scale[(size_t)(tok0 + tid) * g.H + h] : 1.f;
       if constexpr (MODE == TW_HEAD) {
         const double a = tid < n ? (double)g.decay[(size_t)(tok0 + tid) * g.ld_decay + h] : 1.0;
@@ -701,7 +667,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; i += 4) {
-      const float4 by = *reinterpret_cast<const float4*>(scale + vtok + i);
+      const float4 by = MODE == TW_HEAD && adds ? make_float4(1.f, 1.f, 1.f, 1.f) : *reinterpret_cast<const float4*>(scale + vtok + i);
       u[i] = Elem<TV>::load(raw + i) * by.x, u[i + 1] = Elem<TV>::load(raw + i + 1) * by.y;
       u[i + 2] = Elem<TV>::load(raw + i + 2) * by.z, u[i + 3] = Elem<TV>::load(raw + i + 3) * by.w;
     }
@@ -721,7 +687,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
     if constexpr (MODE == TW_HEAD) {
       if (tid < TW_TOK) {
         const int b = tid >> 4;
-        behind[tid] = (float)(after[tid] * over(b + 1, 4));
+        behind[tid] = (float)((double)scale[tid] * (after[tid] * over(b + 1, 4)));  // (the values' factor with it: one rounding less)
         if (tile == 0) {  // (for the walk)
           float* fac = g.factors + item * F::floats;
           fac[F::from + tid] = (float)((double)g.q_scale * over(0, b) * upto[tid]);
@@ -743,23 +709,39 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
         to[idx] = v0 + col < g.dv && ch < g.dk ? slot[(size_t)(v0 + col) * g.dk + ch] : 0.f;
       }
     }
-    uint32_t col = 0;
+    float *u_last = reinterpret_cast<float*>(smem + I::last), *k_last = u_last + TW_LAST * TW_COLS;  // [8][64], [DKP][8]
+    for (int idx = tid; idx < TW_LAST * DKP; idx += TW_FIRST) {
+      const int t = n - TW_LAST + idx / DKP, ch = idx % DKP;
+      float x = 0.f;
+      if (MODE == TW_HEAD) {
+        if (t >= 0 && ch < g.dk) x = g.k[(size_t)(tok0 + t) * g.ld_k + (size_t)(h / g.qk_group) * g.dk + ch];
+      } else if (t >= 0) {
+        x = g.k[(item * TW_TOK + t) * DKP + ch];
+      }
+      k_last[ch * TW_LAST + idx / DKP] = x;
+    }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) col = max(col, tw_bits(u[i]));
-    atomicMax(most + vcol, col);
-    const bool plain = __syncthreads_or(max(worst, col) >= TW_MOST);
+    for (int i = 0; i < 16; ++i) {
+      worst = max(worst, tw_bits(u[i]));
+      const int t = vtok + i - (n - TW_LAST);
+      if (t >= 0 && t < TW_LAST) {
+        u_last[t * TW_COLS + vcol] = u[i];
+        u[i] = 0.f;
+      }
+    }
+    if (n < TW_LAST)
+      for (int idx = tid; idx < (TW_LAST - n) * TW_COLS; idx += TW_FIRST) u_last[idx] = 0.f;  // (rows ahead of the chunk's first token)
     {
       uint4 y[3];
-      const float grid = tw_grid(tw_power(most[vcol]));
 #pragma unroll
       for (int q = 0; q < 16; q += 8) {
-        tw_parts8(y, u + q, grid);
+        tw_parts8(y, u + q);
 #pragma unroll
         for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(smem + I::b + p * TW_TILE + tw_at(vcol, (vtok + q) >> 3)) = y[p];
       }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    __syncthreads();
+    const bool plain = __syncthreads_or(worst >= TW_MOST);
     float* added = g.added + (item * g.tiles + tile) * (TW_COLS * DKP);
 #pragma unroll 1
     for (int half = 0; half < NB; ++half) {
@@ -778,11 +760,27 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       if (!plain) {
         float r[16];
-        tw_tmem_sums(r, lanes + c0);
+        tw_tmem_sums<1>(r, lanes + c0);
+        f2 sum[8];
 #pragma unroll
-        for (int j = 0; j < 16; j += 2) {
-          const int col = pcol + 8 * (j >> 2), ch = 64 * half + row + 8 * ((j >> 1) & 1);
-          *reinterpret_cast<float2*>(added + ((col >> 2) * DKP + ch) * 4 + (col & 3)) = make_float2(r[j], r[j + 1]);
+        for (int j = 0; j < 8; ++j) sum[j] = f2_pair(r[2 * j], r[2 * j + 1]);
+#pragma unroll
+        for (int t = 0; t < TW_LAST; t += 4) {
+          float k0[4], k1[4];
+          *reinterpret_cast<float4*>(k0) = *reinterpret_cast<const float4*>(k_last + (64 * half + row) * TW_LAST + t);
+          *reinterpret_cast<float4*>(k1) = *reinterpret_cast<const float4*>(k_last + (64 * half + row + 8) * TW_LAST + t);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float* ut = u_last + (t + e) * TW_COLS + pcol;
+            const f2 by[2] = {f2_pair(k0[e], k0[e]), f2_pair(k1[e], k1[e])};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f2_fma(sum[j], by[j & 1], *reinterpret_cast<const f2*>(ut + 8 * (j >> 1)));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int col = pcol + 8 * (j >> 1), ch = 64 * half + row + 8 * (j & 1);
+          *reinterpret_cast<f2*>(added + ((col >> 2) * DKP + ch) * 4 + (col & 3)) = sum[j];
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -795,8 +793,8 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
         float r = 0.f;
         for (int j = 0; j < n; ++j) {
           const float x = MODE == TW_HEAD ? (ch < g.dk ? g.k[(size_t)(tok0 + j) * g.ld_k + (size_t)(h / g.qk_group) * g.dk + ch] : 0.f) : g.k[(item * TW_TOK + j) * DKP + ch];
-          const float y = v0 + col < g.dv ? Elem<TV>::load(from + (size_t)j * g.ld_v + col) * scale[j] : 0.f;
-          r = fmaf(x, MODE == TW_HEAD ? y * behind[j] : y, r);
+          const float y = v0 + col < g.dv ? Elem<TV>::load(from + (size_t)j * g.ld_v + col) * (MODE == TW_HEAD ? behind[j] : scale[j]) : 0.f;
+          r = fmaf(x, y, r);
         }
         added[idx] = r;
       }
@@ -806,7 +804,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
 #pragma unroll
     for (int i = 0; i < 16; ++i) pr[i] = 0.f;
     if (ppart < prow >> 4) {
-      const float* pf = pairs + (tw_block(prow >> 4, ppart) * TW_SUB + (prow & 15)) * TW_SUB;
+      const float* pf = pairs + tw_below(prow >> 4, ppart) + (prow & 15) * TW_SUB;
 #pragma unroll
       for (int i = 0; i < 16; i += 4) {
         const float4 x = *reinterpret_cast<const float4*>(pf + i);
@@ -816,8 +814,8 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
     float* near = reinterpret_cast<float*>(smem + I::near);
     if constexpr (MODE == TW_HEAD) {
       const int b = tid >> 6, iq = ((tid >> 4) & 3) * 4, j = tid & 15;
-      const float* from = pairs + (tw_block(b, b) * TW_SUB) * TW_SUB + j;
-      float d[4];
+      const double* from = reinterpret_cast<const double*>(pairs + TW_DIAGONAL) + b * TW_BLOCK + j;
+      double d[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) d[e] = from[(iq + e) * TW_SUB];
       double run = (double)g.q_scale;
@@ -825,7 +823,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         if (iq + e > j) run *= as[b * TW_SUB + iq + e];
-        near[(b * TW_SUB + iq + e) * TW_SUB + j] = iq + e >= j ? (float)((double)d[e] * run) : 0.f;
+        near[(b * TW_SUB + iq + e) * TW_SUB + j] = iq + e >= j ? (float)(d[e] * run) : 0.f;
       }
       if (ppart < prow >> 4) {
         const float f = (float)((double)g.q_scale * upto[prow] * over(ppart + 1, prow >> 4));
@@ -836,57 +834,28 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
         }
       }
     } else {
-      *reinterpret_cast<float4*>(near + tid * 4) = *reinterpret_cast<const float4*>(pairs + tw_block(tid >> 6, tid >> 6) * (TW_SUB * TW_SUB) + (tid & 63) * 4);
+      *reinterpret_cast<float4*>(near + tid * 4) = *reinterpret_cast<const float4*>(pairs + TW_DIAGONAL + tid * 4);
     }
-    {
-      uint32_t size[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) size[i] = tw_bits(u[i]);
-      const uint32_t mine = tw_largest(size, lane);
-      worst = max(worst, mine);
-      if (lane < 16) atomicMax(most + vtok + lane, mine);
-    }
-    __syncthreads();
-    float *power = reinterpret_cast<float*>(most), *inverse = scale;  // (the scale is in the values by now)
-    if (tid < TW_TOK) {
-      const uint32_t x = tw_power(most[tid]);
-      power[tid] = __uint_as_float(x), inverse[tid] = __uint_as_float((254u << 23) - x);
-    }
-    __syncthreads();
     {
       uint4 y[3];
-      float x[8];
 #pragma unroll
       for (int q = 0; q < 16; q += 8) {
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-          const float4 by = *reinterpret_cast<const float4*>(inverse + vtok + q + i);
-          x[i] = u[q + i] * by.x, x[i + 1] = u[q + i + 1] * by.y, x[i + 2] = u[q + i + 2] * by.z, x[i + 3] = u[q + i + 3] * by.w;
-        }
-        tw_parts8(y, x, tw_grid(127u << 23));
+        tw_parts8(y, u + q);
 #pragma unroll
         for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(smem + I::b + p * TW_TILE + tw_at(vcol, (vtok + q) >> 3)) = y[p];
       }
-      uint32_t largest = 0;
-#pragma unroll
-      for (int i = 0; i < 16; i += 4) {
-        const float4 by = *reinterpret_cast<const float4*>(power + 16 * ppart + i);
-        pr[i] *= by.x, pr[i + 1] *= by.y, pr[i + 2] *= by.z, pr[i + 3] *= by.w;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) largest = max(largest, tw_bits(pr[i + e]));
-      }
-      largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
-      largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
-      worst = max(worst, largest >= TW_MOST_PAIRS ? TW_MOST : 0u);
       if (ppart < 3) {  // (the last sixteen is in nobody's pairs)
-        const float pgrid = tw_grid(tw_power(largest));
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          tw_parts8(y, pr + 8 * q, pgrid);
+          tw_parts8(y, pr + 8 * q);
 #pragma unroll
           for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(smem + I::a + p * TW_TILE + tw_at(prow, 2 * ppart + q)) = y[p];
         }
       }
+      uint32_t far = 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) worst = max(worst, tw_bits(u[i])), far = max(far, tw_bits(pr[i]));
+      worst = max(worst, far >= TW_MOST_PAIRS ? TW_MOST : 0u);
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     const bool plain = __syncthreads_or(worst >= TW_MOST);
@@ -924,7 +893,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
         float sum = 0.f;
         for (int j = 0; j <= i; ++j) {
           const int jb = j >> 4;
-          float x = jb == ib ? near[(ib * TW_SUB + (i & 15)) * TW_SUB + (j & 15)] : pairs[(tw_block(ib, jb) * TW_SUB + (i & 15)) * TW_SUB + (j & 15)];
+          float x = jb == ib ? near[(ib * TW_SUB + (i & 15)) * TW_SUB + (j & 15)] : pairs[tw_below(ib, jb) + (i & 15) * TW_SUB + (j & 15)];
           if (MODE == TW_HEAD && jb != ib) x = (float)((double)x * ((double)g.q_scale * upto[i] * over(jb + 1, ib) * after[j]));
           sum = fmaf(x, Elem<TV>::load(from + (size_t)j * g.ld_v + col) * (g.v_scale ? g.v_scale[(size_t)(tok0 + j) * g.H + h] : 1.f), sum);
         }
@@ -939,7 +908,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (!plain) {
       float r[16];
-      tw_tmem_sums(r, lanes + c0);
+      tw_tmem_sums<1>(r, lanes + c0);
       tw_add_outputs(g, r, 1.f, 1.f, tok0, row, n, h, v0 + pcol);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -958,7 +927,7 @@ __global__ void __launch_bounds__(TW_FIRST, 4) tile_chunk_kernel(const TwArgs g)
 template <int MODE, int DKP>
 struct TwWalk {  // bytes
   static constexpr int image = 3 * (DKP / 64) * TW_TILE, sums = DKP * TW_COLS * 4;
-  static constexpr int q = 0, s = 2 * image, added = 3 * image, most = added + 2 * sums, grids = most + 3 * 64 * 4, bars = grids + 64 * 4, all = bars + 128;
+  static constexpr int q = 0, s = 2 * image, added = 3 * image, bars = added + 2 * sums, all = bars + 128;
   static_assert(all <= 227 * 1024, "shared memory");
   static_assert(image >= sums, "the plain sums' state lies where the state's parts are");
 };
@@ -980,17 +949,15 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
   // phases ahead, which reads as not done. With two, the third's products wait for outputs_read.)
   uint32_t* slot_at = reinterpret_cast<uint32_t*>(bars + 12);
   int* plain_at = reinterpret_cast<int*>(bars + 13);             // [4]: a chunk's products with the state are plain sums
-  uint32_t* most = reinterpret_cast<uint32_t*>(smem + I::most);  // [3][64]: the state's largest, column by column
   if (tid == 0) {
     for (int i = 0; i < 12; ++i) tw_bar_init(bars + i, (i >= 4 && i <= 8) || i == 11 ? 8 : 1);
     for (int i = 0; i < 4; ++i) plain_at[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == TW_WORKERS / 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;\n" ::"r"(cs_smem(slot_at)) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(cs_smem(slot_at)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  if (tid < 192) most[tid] = 0;
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -1033,7 +1000,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
           for (int blk = 0; blk < NB; ++blk)
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
-              tw_mma_parts<true>(tmem + (k & 1) * 128, a + ((blk * TW_TILE + ks * 32) >> 4), NB * TW_TILE, b + ((blk * 4 + ks) * 2048 >> 4), DKP * 128, blk + ks > 0);
+              tw_mma_parts<true>(tmem + (k & 1) * 256 + (ks & 1) * 128, a + ((blk * TW_TILE + ks * 32) >> 4), NB * TW_TILE, b + ((blk * 4 + ks) * 2048 >> 4), DKP * 128, blk * 4 + ks > 1);
           tw_commit(done + (k & 1));
           ++products;
         }
@@ -1082,20 +1049,13 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
     for (int c = 0; c < steps; ++c) {
       const int k = c - first;
       if (k >= 0) {
-        // the state as an operand: its largest column by column, then its parts, once the products over the one before are done
-        uint32_t* mx = most + k % 3 * 64;
-        uint32_t size[COLS];
+        // the state as an operand: its parts, once the products over the one before are done
+        uint32_t mine = 0;
 #pragma unroll
-        for (int j = 0; j < COLS; ++j) size[j] = tw_bits(S[j]);
-        const uint32_t mine = tw_largest(size, lane);
-        if (has_ch) atomicMax(mx + c0 + lane, mine);
+        for (int j = 0; j < COLS; ++j) mine = max(mine, tw_bits(S[j]));
         const bool was = plain;
         plain = tw_group_any(1, (has_ch && mine >= TW_MOST) || large);
         if (tid == 0) plain_at[k & 3] = plain;
-        if (tid < 64) most[(k + 2) % 3 * 64 + tid] = 0;  // (read before this chunk's barrier, used behind the next one's)
-        float* grids = reinterpret_cast<float*>(smem + I::grids) + c0;  // (the warps of these columns write the same)
-        grids[lane] = tw_grid(tw_power(mx[c0 + lane]));
-        __syncwarp();
         if (k > 0) ok = ok && all_wait(done + ((k - 1) & 1), (k - 1) >> 1);
         if (was) ok = ok && all_wait(state_read, plain_chunks++);  // (the plain sums have read the state)
         if (plain) {
@@ -1109,11 +1069,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
           for (int q = 0; q < COLS / 8; ++q) {
             uint32_t y[4][3];
 #pragma unroll
-            for (int j = 0; j < 4; j += 2) {
-              const ulonglong2 g2 = *reinterpret_cast<const ulonglong2*>(grids + 8 * q + 2 * j);
-              tw_parts(y[j], f2_pair(S[8 * q + 2 * j], S[8 * q + 2 * j + 1]), g2.x);
-              tw_parts(y[j + 1], f2_pair(S[8 * q + 2 * j + 2], S[8 * q + 2 * j + 3]), g2.y);
-            }
+            for (int j = 0; j < 4; ++j) tw_parts(y[j], f2_pair(S[8 * q + 2 * j], S[8 * q + 2 * j + 1]));
 #pragma unroll
             for (int p = 0; p < 3; ++p)
               *reinterpret_cast<uint4*>(to + p * DKP * 128 + ((((c0 >> 3) + q) ^ (ch & 7)) << 4)) = make_uint4(y[0][p], y[1][p], y[2][p], y[3][p]);
@@ -1170,14 +1126,14 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tile_walk_kernel(const TwArgs g
         continue;
       }
       float r[16];
-      tw_tmem_sums(r, lanes + (k & 1) * 128 + c0);
+      tw_tmem_sums<2>(r, lanes + (k & 1) * 256 + c0);
       tw_arrive(outputs_read + (k & 1));
       tw_add_outputs(g, r, by0, by1, tok0, row, n, h, col);
     }
     if (!ok && lane == 0 && g.status) atomicMax(g.status, 42);
   }
   __syncthreads();
-  if (warp == TW_WORKERS / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem) : "memory");
+  if (warp == TW_WORKERS / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
 }
 
 // ---------------------------------------------------------------- host
@@ -1203,7 +1159,7 @@ struct TwPlan {
     const long long items = (long long)chunks * H, own = (long long)chunks * (groups ? groups : H), state = (long long)tiles * TW_COLS * dkp;
     images = own * 3 * (dkp / 64) * (TW_TILE / 4);
     flags = (own + 3) / 4 * 4;
-    pairs = (groups ? own : items) * (TW_BLOCKS * TW_SUB * TW_SUB);
+    pairs = (groups ? own : items) * tw_pairs(groups > 0);
     factors = items * (groups ? TwFactors<TW_HEAD, 64>::floats : dkp);
     keys = groups ? 0 : items * TW_TOK * dkp;
     added = items * state;

@@ -84,6 +84,66 @@ def test_head_decays(heads, groups, dk, dv, scaled):
              rows, slots, q, *exact, state, heads, dv)
 
 
+def _spread(where, gen, q, k, v, state):
+    """[T, H, d] operands and [1, H, dv, dk] states with numbers far larger than the others, in place."""
+    if where == "a value channel":
+        v[:, :, 5] *= 1024
+    elif where == "a key channel":
+        k[:, :, 5] *= 1024
+        state[..., 5] *= 1024
+    elif where == "a query channel":
+        q[:, :, 5] *= 1024
+    elif where == "tokens":
+        k[::97] *= 1024
+        v[40::97] *= 4096
+    elif where == "some values":
+        v[torch.rand(v.shape, generator=gen, device=DEV) < 0.01] *= 16384
+    elif where == "keys against queries":  # the products are as large as without
+        by = torch.exp2(torch.randint(-12, 13, (k.shape[2],), generator=gen, device=DEV).float())
+        k *= by
+        q /= by
+        state *= by
+    else:
+        assert where == "everything"
+        for x in (q, k, v, state):
+            x *= torch.exp2(4 * torch.randn(x.shape, generator=gen, device=DEV))
+
+
+@pytest.mark.parametrize("rule, heads, dk, dv, t", [("decay", 3, 64, 72, 701), ("decay", 2, 128, 64, 701), ("head", 3, 128, 64, 431), ("head", 2, 32, 40, 431)])
+@pytest.mark.parametrize("low, high", [(0.02, 0.6), (0.9, 0.999), (0.9999, 0.99999)])
+@pytest.mark.parametrize("where", ["a value channel", "a key channel", "a query channel", "tokens", "some values", "keys against queries", "everything"])
+def test_numbers_of_very_different_sizes(rule, heads, dk, dv, t, low, high, where):
+    """The error of every output and of every number of the state against the size of its own terms: a large number takes no bits from others."""
+    gen = torch.Generator(device=DEV).manual_seed(dk + dv)
+    q, k, v, state = (torch.randn(s, generator=gen, device=DEV) for s in ((t, heads, dk), (t, heads, dk), (t, heads, dv), (1, heads, dv, dk)))
+    _spread(where, gen, q, k, v, state)
+    a = low + (high - low) * torch.rand(t, heads, dk if rule == "decay" else 1, generator=gen, device=DEV)
+    rows, st, o, flat = [(7, t)], state.clone(), torch.empty(t, heads, dv, device=DEV), [x.reshape(t, -1) for x in (q, k, v)]
+    assert _takes(rows, heads, dk, dv, heads if rule == "head" else 0)
+    if rule == "head":
+        ops.decay_scan(o, st, *flat, a.reshape(t, heads), None, None, 0.0, None, _ctx(rows, [0]), heads, dk, dv, 1.0, delta=False, head_decay=True)
+        a = a.double()
+    else:
+        z = torch.log(torch.expm1(-torch.log(a.double()))).float()
+        ops.decay_scan(o, st, *flat, z.reshape(t, -1), torch.zeros(heads * dk, device=DEV), torch.ones(heads, device=DEV), 1.0, None, _ctx(rows, [0]), heads, dk, dv,
+                       1.0, delta=False)
+        a = torch.exp(-torch.nn.functional.softplus(z.double(), threshold=1e9))
+    q, k, v, exact = q.double(), k.double(), v.double(), state[0].double()
+    size = exact.abs()
+    worst = torch.zeros((), dtype=torch.float64, device=DEV)
+    for i in range(t):
+        u = v[i][:, :, None] * k[i][:, None, :]
+        exact, size = exact * a[i][:, None, :] + u, size * a[i][:, None, :] + u.abs()
+        off = (o[i].double() - (exact * q[i][:, None, :]).sum(-1)).abs() / (size * q[i].abs()[:, None, :]).sum(-1)
+        worst = torch.maximum(worst, off.max())
+    behind = ((st[0].double() - exact).abs() / size).max().item()
+    # At most eight cuts of 2^-23 of a sum no larger than its terms' (9.5e-7), hardly ever one after the other. Decays made of logits come on top: each is
+    # off by up to 2^-24 (expf's last bit, below one), and as many of them are in a term as it has been kept for, on average no more than 1 / (1 - decay) tokens.
+    most = 1e-6 + (rule == "decay") * min(t, 1 / (1 - (low + high) / 2)) * 2.0 ** -24
+    assert worst.item() < most and behind < most, (worst.item(), behind)
+    assert ops.device_status(DEV).item() == 0
+
+
 @pytest.mark.parametrize("rule, dk, dv, n", [("decay", 64, 128, 1300), ("head", 128, 64, 1000)])
 def test_heads_that_fill_the_gpu_walk_rows_whole(rule, dk, dv, n):
     """Few heads: rows in segments. The same bits beside so many heads that rows stay whole, behind a state and from zero."""
