@@ -156,7 +156,7 @@ attn_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __rest
                     const int* __restrict__ cu_q, const int* __restrict__ q_start, const int* __restrict__ page_indptr,
                     const int* __restrict__ page_indices, int nq, int nkv, float scale_log2, int window,
                     int sink, int page_shift, AttnExtras ex) {
-  pdl_prologue();
+  pdl_prologue(q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices);
   const int r = blockIdx.y, head = blockIdx.z;
   const int tok0 = cu_q[r], q_len = cu_q[r + 1] - tok0;
   const int m0 = blockIdx.x * PF_BM;
@@ -585,7 +585,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   for (int idx = tid; idx < 16 * CHUNKS; idx += DC_THREADS) {
     const int row = idx / CHUNKS, chunk = idx - row * CHUNKS;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (row < heads_here) v = *reinterpret_cast<const uint4*>(q + ((size_t)r * nq + head0 + row) * D + chunk * 8);
+    if (row < heads_here) v = behind_load16(q + ((size_t)r * nq + head0 + row) * D + chunk * 8);
     *reinterpret_cast<uint4*>(qs + row * DPAD + chunk * 8) = v;
   }
   for (; issued < DC_STAGES - 1; ++issued) issue(issued);
@@ -777,7 +777,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
 // out[r, head] = sum_s w_s O_s / sum_s w_s l_s with w_s = 2^(m_s - max m)
 __global__ void attn_decode_merge_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ part_o,
                                          const float* __restrict__ part_ml, int num_splits, int sink, int nq, AttnExtras ex) {
-  pdl_prologue();
+  pdl_prologue(part_o, part_ml);
   const size_t item = blockIdx.x;  // r * nq + head
   const float* ml = part_ml + item * num_splits * 2;
   float m = -INFINITY;

@@ -35,7 +35,7 @@ attention_rowwise_kernel(T* __restrict__ out,            // [T, nq, d]
                          int num_pages, int* __restrict__ status, const float* __restrict__ sink_values, float softcap,
                          int chunk, const float* __restrict__ dist_r1, const float* __restrict__ dist_r2, int keep_first) {
   extern __shared__ float q_smem[];  // [warps][d]
-  pdl_prologue();
+  pdl_prologue(q, k_pool, v_pool, positions, row_of_token, page_indptr, page_indices, sink_values, dist_r1, dist_r2);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
   if (item >= (long long)num_tokens * nq) return;
@@ -186,7 +186,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
   unsigned* seen = reinterpret_cast<unsigned*>(alphas + 2 * ROWS);  // [2][ROWS]
   __shared__ int s_row, s_tile;
   __shared__ int usable[2][2 * TW_KEYS];
-  pdl_prologue();
+  pdl_prologue(q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, sink_values, dist_r1, dist_r2);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int group = nq / nkv, per_tile = ROWS / group;
   // The late (long) tiles first, all kv heads of one tile side by side; those that share a multiprocessor with the first `sms` the other way

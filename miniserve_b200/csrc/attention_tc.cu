@@ -531,7 +531,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncthreads();
   AT_FENCE_AFTER();
   const uint32_t tmem = tmem_slot;
-  pdl_wait();
+  pdl_wait(cu_q, q_start, page_indptr, page_indices, plan);
 
   // A launch that was captured into a CUDA graph takes what follows from the rows' lengths (tiles per
   // row, rows, key splits) from device memory, where the host puts it before every replay: the

@@ -37,7 +37,7 @@ add_layernorm_kernel(T* __restrict__ out, T* __restrict__ out2, float* __restric
                      const float* __restrict__ b2, const int* __restrict__ rows, float eps, int hidden, int write_residual) {
   extern __shared__ float ln_row[];  // hidden floats
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(delta, w, b, w2, b2, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -73,7 +73,7 @@ add_layernorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* __re
                             const float* __restrict__ b, const float* __restrict__ w2, const float* __restrict__ b2,
                             const int* __restrict__ rows, float eps, int hidden, int write_residual) {
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(delta, w, b, w2, b2, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -133,7 +133,7 @@ template <typename T>
 __global__ void token_shift_kernel(T* __restrict__ out, const T* __restrict__ h, T* __restrict__ state,
                                    const float* __restrict__ mix, const int* __restrict__ row_of_token, const int* __restrict__ cu_q,
                                    const int* __restrict__ q_start, const int* __restrict__ state_slot, int width, int update) {
-  pdl_prologue();
+  pdl_prologue(h, mix, row_of_token, cu_q, q_start, state_slot);
   const int t = blockIdx.x;
   const int row = row_of_token[t];
   const bool first = t == cu_q[row];
@@ -153,7 +153,7 @@ __global__ void token_shift_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const
                                           __nv_bfloat16* __restrict__ state, const float* __restrict__ mix,
                                           const int* __restrict__ row_of_token, const int* __restrict__ cu_q,
                                           const int* __restrict__ q_start, const int* __restrict__ state_slot, int width, int update) {
-  pdl_prologue();
+  pdl_prologue(h, mix, row_of_token, cu_q, q_start, state_slot);
   const int t = blockIdx.x;
   const int row = row_of_token[t];
   const bool first = t == cu_q[row];
@@ -178,7 +178,7 @@ template <typename T>
 __global__ void token_mixes_kernel(T* __restrict__ out, const T* __restrict__ h, T* __restrict__ state, const float* __restrict__ mix, int mixes,
                                    const int* __restrict__ row_of_token, const int* __restrict__ cu_q, const int* __restrict__ q_start,
                                    const int* __restrict__ state_slot, int width) {
-  pdl_prologue();
+  pdl_prologue(h, mix, row_of_token, cu_q, q_start, state_slot);
   const int t = blockIdx.x;
   const int row = row_of_token[t];
   const bool first = t == cu_q[row];
@@ -211,7 +211,7 @@ __global__ void token_mixes_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const
 #pragma unroll
     for (int m = 0; m < MIXES; ++m) factors(early[EARLY ? m : 0], m, c0);
   }
-  pdl_prologue();
+  pdl_prologue(h, mix, row_of_token, cu_q, q_start, state_slot);
   const int t0 = blockIdx.x * RUN;
   const __nv_bfloat16* prev[RUN];
   __nv_bfloat16* slot[RUN];  // where this token's CTA leaves the portion's last h
@@ -266,7 +266,7 @@ __global__ void token_mixes_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const
 template <typename T>
 __global__ void shift_state_update_kernel(T* __restrict__ state, const T* __restrict__ h, const int* __restrict__ cu_q,
                                           const int* __restrict__ state_slot, int width) {
-  pdl_prologue();
+  pdl_prologue(h, cu_q, state_slot);
   const int row = blockIdx.x;
   const int last = cu_q[row + 1] - 1;
   if (last < cu_q[row]) return;
@@ -278,7 +278,7 @@ __global__ void shift_state_update_kernel(T* __restrict__ state, const T* __rest
 template <typename T>
 __global__ void clamped_glu_kernel(T* __restrict__ out, const T* __restrict__ gate_up, const float* __restrict__ bias, int inter,
                                    long long total, float limit, float alpha, float shift) {
-  pdl_prologue();
+  pdl_prologue(gate_up, bias);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const long long t = idx / inter;
@@ -299,7 +299,7 @@ __global__ void clamped_glu_kernel(T* __restrict__ out, const T* __restrict__ ga
 __global__ void clamped_glu_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ gate_up,
                                           const float* __restrict__ bias, int inter8, long long total8, float limit, float alpha,
                                           float shift) {
-  pdl_prologue();
+  pdl_prologue(gate_up, bias);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total8) return;
   const long long t = idx / inter8;
@@ -329,7 +329,7 @@ __global__ void clamped_glu_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const
 template <typename T>
 __global__ void sum_bias_kernel(T* __restrict__ out, const T* __restrict__ a, const T* __restrict__ b, const float* __restrict__ vec,
                                 long long total, int width) {
-  pdl_prologue();
+  pdl_prologue(a, b, vec);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   float x = Elem<T>::load(a + i);
@@ -345,7 +345,7 @@ add_rmsnorm_scaled_kernel(T* __restrict__ out, float* __restrict__ residual, con
                           int write_residual) {
   extern __shared__ float row_buf[];  // hidden floats
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(delta, w, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -374,7 +374,7 @@ add_rmsnorm_scaled_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restr
                                  const __nv_bfloat16* __restrict__ delta, float delta_scale, const float* __restrict__ w,
                                  float w_offset, const int* __restrict__ rows, float eps, int hidden, int write_residual) {
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(delta, w, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -415,7 +415,7 @@ template <typename T>
 __global__ void stream_concat_kernel(T* __restrict__ out, const float* __restrict__ residual, const T* __restrict__ delta,
                                      float delta_scale, const T* __restrict__ table, const int* __restrict__ ids, int vocab,
                                      int hidden, int write_first, int write_second) {
-  pdl_prologue();
+  pdl_prologue(residual, delta, table, ids);
   const int t = blockIdx.x;
   T* o = out + (size_t)t * 2 * hidden;
   if (write_first) {
@@ -436,14 +436,14 @@ __global__ void stream_concat_kernel(T* __restrict__ out, const float* __restric
 }
 
 __global__ void add_row_vector_kernel(float* __restrict__ x, const float* __restrict__ vec, long long total, int width) {
-  pdl_prologue();
+  pdl_prologue(vec);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < total) x[i] += vec[(int)(i % width)];
 }
 
 template <typename T>
 __global__ void relu_squared_kernel(T* __restrict__ out, int ld_out, const T* __restrict__ x, int ld_x, long long total, int width) {
-  pdl_prologue();
+  pdl_prologue(x);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long t = i / width;
@@ -454,7 +454,7 @@ __global__ void relu_squared_kernel(T* __restrict__ out, int ld_out, const T* __
 
 __global__ void relu_squared_bf16x8_kernel(__nv_bfloat16* __restrict__ out, int ld_out, const __nv_bfloat16* __restrict__ x, int ld_x,
                                            long long total8, int width8) {
-  pdl_prologue();
+  pdl_prologue(x);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total8) return;
   const long long t = i / width8;
@@ -473,7 +473,7 @@ __global__ void relu_squared_bf16x8_kernel(__nv_bfloat16* __restrict__ out, int 
 template <typename T>
 __global__ void channel_gate_kernel(T* __restrict__ out, int ld_out, const T* __restrict__ attn, const T* __restrict__ gate,
                                     int ld_gate, long long items, int nq, int d_pad, int dv, float scale) {
-  pdl_prologue();
+  pdl_prologue(attn, gate);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const int c = (int)(idx % dv);
@@ -487,7 +487,7 @@ __global__ void channel_gate_kernel(T* __restrict__ out, int ld_out, const T* __
 __global__ void channel_gate_bf16x8_kernel(__nv_bfloat16* __restrict__ out, int ld_out, const __nv_bfloat16* __restrict__ attn,
                                            const __nv_bfloat16* __restrict__ gate, int ld_gate, long long items8, int nq, int d_pad,
                                            int dv8, float scale) {
-  pdl_prologue();
+  pdl_prologue(attn, gate);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items8) return;
   const int c = (int)(idx % dv8);
@@ -508,7 +508,7 @@ template <typename T>
 __global__ void gate_relu_squared_kernel(T* __restrict__ out, int ld_out, const T* __restrict__ attn, const T* __restrict__ gate,
                                          int ld_gate, const T* __restrict__ up, int ld_up, long long items, int nq, int d_pad, int dv,
                                          int inter) {
-  pdl_prologue();
+  pdl_prologue(attn, gate, up);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const int fa = nq * dv, width = fa + inter;
@@ -529,7 +529,7 @@ __global__ void gate_relu_squared_bf16x8_kernel(__nv_bfloat16* __restrict__ out,
                                                 const __nv_bfloat16* __restrict__ gate, int ld_gate,
                                                 const __nv_bfloat16* __restrict__ up, int ld_up, long long items8, int nq, int d_pad,
                                                 int dv, int inter) {
-  pdl_prologue();
+  pdl_prologue(attn, gate, up);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items8) return;
   const int fa = nq * dv, width8 = (fa + inter) >> 3;
@@ -556,7 +556,7 @@ __global__ void gate_relu_squared_bf16x8_kernel(__nv_bfloat16* __restrict__ out,
 
 __global__ void rope_table_scaled_kernel(float* __restrict__ table, const int* __restrict__ positions,
                                          const float* __restrict__ inv_freq, float factor, int num_tokens, int rot) {
-  pdl_prologue();
+  pdl_prologue(positions, inv_freq);
   const int half = rot >> 1;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)num_tokens * half) return;
@@ -574,7 +574,7 @@ __global__ void latent_prepare_kernel(T* __restrict__ pool,  // [pages, 1, page_
                                       const int* __restrict__ positions, const int* __restrict__ row_of_token,
                                       const int* __restrict__ page_indptr, const int* __restrict__ page_indices, int num_tokens,
                                       int rank, int d_pad, int page_shift, int num_pages, int* __restrict__ status) {
-  pdl_prologue();
+  pdl_prologue(proj, w, positions, row_of_token, page_indptr, page_indices);
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= num_tokens) return;
@@ -766,7 +766,7 @@ namespace ms {
 template <typename T>
 __global__ void row_rmsnorm_kernel(T* __restrict__ out, int ld_out, const T* __restrict__ x, int ld_x, const float* __restrict__ w,
                                    int rows, int n, float eps) {
-  pdl_prologue();
+  pdl_prologue(x, w);
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= rows) return;
@@ -792,7 +792,7 @@ __global__ void latent_rope_prepare_kernel(T* __restrict__ pool,  // [pages, 1, 
                                            const int* __restrict__ row_of_token, const int* __restrict__ page_indptr,
                                            const int* __restrict__ page_indices, int num_tokens, int rank, int rot, int d_pad,
                                            int page_shift, int num_pages, int* __restrict__ status) {
-  pdl_prologue();
+  pdl_prologue(kv, w, q, cos_sin, positions, row_of_token, page_indptr, page_indices);
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= (long long)num_tokens * (H + 1)) return;
@@ -885,7 +885,7 @@ MS_EXPORT int ms_latent_rope_prepare(void* pool, const void* kv, int ld_kv, cons
 namespace ms {
 __global__ void sum_bias_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ a,
                                        const __nv_bfloat16* __restrict__ b, const float* __restrict__ vec, long long total8, int width) {
-  pdl_prologue();
+  pdl_prologue(a, b, vec);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total8) return;
   float x[8], y[8];

@@ -28,7 +28,7 @@ constexpr int CS_KB = 32;  // key channels of the state staged at a time by the 
 // tab[c] = (row, first flat token) of chunk c, row_first[r] the row's first chunk (row_first[num_rows]: how many chunks there are)
 __global__ void __launch_bounds__(CS_THREADS)
 chunk_table_kernel(int2* __restrict__ tab, int* __restrict__ row_first, const int* __restrict__ cu_q, int num_rows) {
-  pdl_prologue();
+  pdl_prologue(cu_q);
   __shared__ int part[CS_THREADS];
   __shared__ int base;
   if (threadIdx.x == 0) base = 0;
@@ -122,7 +122,7 @@ chunk_states_kernel(float* __restrict__ ds, float* __restrict__ chunk_decay, con
                     int dv, int dk_tiles, int ones) {
   extern __shared__ __align__(16) unsigned char cs_raw[];
   StatesSmem& sm = *reinterpret_cast<StatesSmem*>(cs_raw);
-  pdl_prologue();
+  pdl_prologue(k, v, decay, write, tab, row_first, cu_q);
   const int chunk = blockIdx.x, h = blockIdx.y;
   if (chunk >= row_first[num_rows]) return;
   const int2 at = tab[chunk];
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(CS_THREADS)
 chunk_carry_kernel(float* __restrict__ state, __nv_bfloat16* __restrict__ before_hi, __nv_bfloat16* __restrict__ before_lo,
                    const float* __restrict__ ds, const float* __restrict__ chunk_decay, const int* __restrict__ row_first,
                    const int* __restrict__ q_start, const int* __restrict__ state_slot, int H, int per_head, int total4) {
-  pdl_prologue();
+  pdl_prologue(ds, chunk_decay, row_first, q_start, state_slot);
   const int i4 = blockIdx.x * CS_THREADS + threadIdx.x, r = blockIdx.y;
   if (i4 >= total4) return;
   const int h = i4 * 4 / per_head;
@@ -257,7 +257,7 @@ chunk_outputs_kernel(float* __restrict__ o, int ld_o, const __nv_bfloat16* __res
   __nv_bfloat16* ks = qs + CS_TOK * ldk;
   __nv_bfloat16* p_hi = ks;
   __nv_bfloat16* p_lo = p_hi + CS_TOK * CS_LDP;
-  pdl_prologue();
+  pdl_prologue(q, k, v, decay, write, before_hi, before_lo, tab, row_first, cu_q, q_start);
   const int chunk = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * CS_DV;
   if (chunk >= row_first[num_rows]) return;
   const int2 at = tab[chunk];

@@ -115,7 +115,7 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
   __shared__ __align__(16) float qs[WK_TOK][DKP], ks[WK_TOK][DKP], ds[WK_TOK][DKP];
   __shared__ __align__(16) double am[DELTA ? WK_TOK : 1][WK_TOK];  // A, a column j in am[j]
   __shared__ float bs[WK_TOK], vsc[WK_TOK];
-  pdl_prologue();
+  pdl_prologue(q, k, v, z, z_bias, decay_coef, beta, v_scale, cu_q);
   const int chunk = blockIdx.x, h = blockIdx.y;
   const int2 at = wk_at(chunk, cu_q, num_rows);
   if (at.x < 0) return;
@@ -606,7 +606,7 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
   __shared__ __align__(16) float qs[WK_TOK][DK + 4], ks[WK_TOK][DK + 4];
   __shared__ double dot[WK_TOK][WK_TOK + 1];
   __shared__ float as[WK_TOK][33];
-  pdl_prologue();
+  pdl_prologue(q, k, decay, cu_q);
   const int chunk = blockIdx.x, grp = blockIdx.y;
   const int2 at = wk_at(chunk, cu_q, num_rows);
   if (at.x < 0) return;

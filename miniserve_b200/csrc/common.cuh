@@ -95,24 +95,45 @@ __device__ __forceinline__ uint4 float_to_bf16x8(const float (&f)[8]) {
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // ---- programmatic dependent launch
-// Every kernel of this package starts with pdl_prologue(): it lets the next kernel in the stream
+// Every kernel of this package starts with pdl_prologue(its pointers): it lets the next kernel in the stream
 // begin launching (its CTAs become resident and may fetch what does not depend on earlier
 // kernels, i.e. weights), then waits until everything launched before it has completed and is
 // visible. Because every kernel waits before it touches activations or the cache, completion
 // order stays the launch order and no kernel reads or overwrites data too early. Launched
 // without the attribute (or when the switch below is off) both instructions do nothing.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_prologue() {
+// What earlier kernels write is read through pointers that are made behind the wait: the compiler takes what a `const __restrict__` parameter points
+// to for constant while the kernel runs and may load it ahead of the wait, whatever that clobbers (rows of the step before came out so). So the wait takes
+// a kernel's pointers and gives them back; it costs no instruction.
+template <typename P>
+__device__ __forceinline__ void behind_wait(P& p) {
+  asm volatile("" : "+l"(p) : : "memory");
+}
+template <typename... P>
+__device__ __forceinline__ void pdl_wait(P&... pointers) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (behind_wait(pointers), ...);
+}
+template <typename... P>
+__device__ __forceinline__ void pdl_prologue(P&... pointers) {
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait(pointers...);
+}
+// The first loads behind the wait of a decode step's short kernels: they stay where they stand, behind it, and need no such pointer (with one the compiler no longer knows
+// that it points to global memory, and every load looks for that: a step of 8 requests takes 1,095 us so, 1,082 like this).
+__device__ __forceinline__ uint4 behind_load16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int behind_load(const int* p) {
+  int v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
 }
 // A kernel whose weights come from far (each layer's are read once in a decode step) asks for them between the two halves of the prologue: weights are
 // not written by kernels that may still run when its CTAs begin. weight_load16: 16 bytes, asked for where it stands (a plain load may move behind
-// the wait). Whatever earlier kernels write is then read through pointers that have gone through behind_wait(): the compiler takes loads through
-// `const __restrict__` parameters for constant and may otherwise move them ahead of the wait.
-template <typename P>
-__device__ __forceinline__ void behind_wait(P& p) { asm volatile("" : "+l"(p) : : "memory"); }
+// the wait).
 __device__ __forceinline__ uint4 weight_load16(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));

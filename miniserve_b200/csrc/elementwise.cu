@@ -13,7 +13,7 @@ namespace ms {
 template <typename T>
 __global__ void embed_gather_kernel(float* __restrict__ residual, const T* __restrict__ table,
                                     const int* __restrict__ ids, int hidden, int vocab) {
-  pdl_prologue();
+  pdl_prologue(table, ids);
   const int t = blockIdx.x;
   int id = ids[t];
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);  // ids are validated on the host; stay in bounds anyway
@@ -25,7 +25,7 @@ __global__ void embed_gather_kernel(float* __restrict__ residual, const T* __res
 // bfloat16 rows that are a multiple of 8 wide: eight elements per thread (a 16-byte load, two 16-byte stores)
 __global__ void embed_gather_bf16x8_kernel(float* __restrict__ residual, const __nv_bfloat16* __restrict__ table,
                                            const int* __restrict__ ids, int hidden8, int vocab, int tokens) {
-  pdl_prologue();
+  pdl_prologue(table, ids);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)tokens * hidden8) return;
   const int t = (int)(idx / hidden8), c = (int)(idx - (long long)t * hidden8);
@@ -50,7 +50,7 @@ add_rmsnorm_kernel(T* __restrict__ out, float* __restrict__ residual, const T* _
                    int write_residual) {
   extern __shared__ float row_buf[];  // hidden floats
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(delta, w, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -88,10 +88,7 @@ add_rmsnorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ r
   // A step of 8 requests with 57 of these: 1,101 -> 1,088 us, against weights asked for behind the sum of squares.
   uint4 w_raw = make_uint4(0u, 0u, 0u, 0u);
   if (in_regs && (int)threadIdx.x < chunks) w_raw = weight_load16(w + 8 * threadIdx.x);
-  pdl_wait();
-  behind_wait(residual);
-  behind_wait(delta);
-  behind_wait(rows);
+  pdl_wait(residual, delta, w, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -139,7 +136,7 @@ add_rmsnorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ r
 // ---------------------------------------------------------------- SiLU(gate) * up
 template <typename T>
 __global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ gate_up, int inter, size_t total) {
-  pdl_prologue();
+  pdl_prologue(gate_up);
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const size_t t = idx / inter;
@@ -153,7 +150,7 @@ __global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ gate_
 // bfloat16, 8 elements per thread (inter % 8 == 0)
 __global__ void silu_mul_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ gate_up,
                                        int inter8, size_t total8) {
-  pdl_prologue();
+  pdl_prologue(gate_up);
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total8) return;
   const size_t t = idx / inter8;
@@ -179,7 +176,7 @@ __global__ void silu_mul_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __
 // ---------------------------------------------------------------- float32 <- T copy (logits of a bf16 GEMM)
 template <typename T>
 __global__ void to_float_kernel(float* __restrict__ out, const T* __restrict__ in, size_t n) {
-  pdl_prologue();
+  pdl_prologue(in);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = Elem<T>::load(in + i);
 }
@@ -188,7 +185,7 @@ __global__ void to_float_kernel(float* __restrict__ out, const T* __restrict__ i
 // been read back to the host (miniserve/engine/model_runner.py:263-277 does this with index_copy).
 __global__ void fill_tokens_kernel(int* __restrict__ token_ids, const int* __restrict__ dst, const int* __restrict__ tokens,
                                    const int* __restrict__ src, int n) {
-  pdl_prologue();
+  pdl_prologue(dst, tokens, src);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) token_ids[dst[i]] = tokens[src[i]];
 }

@@ -35,7 +35,7 @@ mlstm_gates_kernel(float* __restrict__ decay, float* __restrict__ write, float* 
                    const float* __restrict__ bias, float* __restrict__ m_state, const int* __restrict__ cu_q, const int* __restrict__ q_start,
                    const int* __restrict__ state_slot, int H, float cap) {
   __shared__ float wf[THREADS / 32], wm[THREADS / 32];
-  pdl_prologue();
+  pdl_prologue(raw, bias, cu_q, q_start, state_slot);
   const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int t0 = cu_q[r], len = cu_q[r + 1] - t0;
   if (len <= 0) return;
@@ -102,7 +102,7 @@ template <typename T>
 __global__ void mlstm_output_kernel(T* __restrict__ out, int ld_out, const float* __restrict__ o, int ld_o, const float* __restrict__ floor_,
                                     const float* __restrict__ w, const T* __restrict__ gate, int ld_gate, long long items, int H, int dv,
                                     float eps, float den_eps) {
-  pdl_prologue();
+  pdl_prologue(o, floor_, w, gate);
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= items) return;
@@ -127,7 +127,7 @@ __global__ void mlstm_output_kernel(T* __restrict__ out, int ld_out, const float
 __global__ void mlstm_output_bf16x8_kernel(__nv_bfloat16* __restrict__ out, int ld_out, const float* __restrict__ o, int ld_o,
                                            const float* __restrict__ floor_, const float* __restrict__ w, const __nv_bfloat16* __restrict__ gate,
                                            int ld_gate, long long items, int H, int dv, float eps, float den_eps) {
-  pdl_prologue();
+  pdl_prologue(o, floor_, w, gate);
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= items) return;
@@ -167,7 +167,7 @@ __global__ void conv_bias_kernel(T* __restrict__ u, const T* __restrict__ x, int
                                  const float* __restrict__ bias, const float* __restrict__ in_bias, const int* __restrict__ row_of_token,
                                  const int* __restrict__ cu_q, const int* __restrict__ q_start, const int* __restrict__ state_slot,
                                  long long items, int C, int taps, int single) {
-  pdl_prologue();
+  pdl_prologue(x, w, bias, in_bias, row_of_token, cu_q, q_start, state_slot);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const int groups = C / V;
@@ -212,7 +212,7 @@ __global__ void conv_bias_run_kernel(__nv_bfloat16* __restrict__ u, const __nv_b
                                      const __nv_bfloat16* __restrict__ conv_state, const float* __restrict__ w, const float* __restrict__ bias,
                                      const float* __restrict__ in_bias, const int* __restrict__ row_of_token, const int* __restrict__ cu_q,
                                      const int* __restrict__ q_start, const int* __restrict__ state_slot, int tokens, int C) {
-  pdl_prologue();
+  pdl_prologue(x, conv_state, w, bias, in_bias, row_of_token, cu_q, q_start, state_slot);
   const int groups = C >> 3;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int run = (int)(idx / groups), c = (int)(idx - (long long)run * groups) * 8;
@@ -305,7 +305,7 @@ rglru_scan_kernel(T* __restrict__ out, float* __restrict__ state, const float* _
   constexpr bool FAST = sizeof(T) == 2;
   __shared__ float wa[LRU_WARPS][32], wb[LRU_WARPS][32];
   __shared__ float ta[2][32], tb[2][32];  // this CTA's composed pair of the pass, in two buffers in turn
-  pdl_prologue();
+  pdl_prologue(z, u, y, bias_r, bias_i, coef, y_bias, cu_q, q_start, state_slot);
   cg::cluster_group cluster = cg::this_cluster();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rank = blockIdx.x % ctas, c = (blockIdx.x / ctas) * 32 + lane, r = blockIdx.y;
@@ -405,7 +405,7 @@ __global__ void rglru_step_kernel(T* __restrict__ out, float* __restrict__ state
                                   const T* __restrict__ y, int ld_y, const float* __restrict__ bias_r, const float* __restrict__ bias_i,
                                   const float* __restrict__ coef, const float* __restrict__ y_bias, const int* __restrict__ q_start,
                                   const int* __restrict__ state_slot, long long items, int C, int bs) {
-  pdl_prologue();
+  pdl_prologue(z, u, y, bias_r, bias_i, coef, y_bias, q_start, state_slot);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const int r = (int)(idx / C), c = (int)(idx - (long long)r * C);

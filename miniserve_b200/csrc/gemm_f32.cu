@@ -17,7 +17,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
   C += blockIdx.z * stride_c;
   __shared__ float As[GBK][GBM + 4];
   __shared__ float Ws[GBK][GBN + 4];
-  pdl_prologue();
+  pdl_prologue(A, W);
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * GBM, n0 = blockIdx.x * GBN;
   const int tx = tid & 15, ty = tid >> 4;  // 16 x 16 threads, each 4 x 4 outputs
@@ -86,7 +86,7 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
   using I = GfTile<BM, BN, TM, TN, GK>;
   constexpr int THREADS = I::threads, PA = BM * GK / 4, PW = BN * GK / 4, LA = (PA + THREADS - 1) / THREADS, LW = (PW + THREADS - 1) / THREADS;  // pieces of 16 bytes
   __shared__ __align__(16) float as[2][GK][BM + 4], ws[2][GK][BN + 4];
-  pdl_prologue();
+  pdl_prologue(A, W);
   const int tid = threadIdx.x, tx = tid % I::tx, ty = tid / I::tx;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   A += blockIdx.z * stride_a;

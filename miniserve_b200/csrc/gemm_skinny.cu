@@ -98,7 +98,7 @@ gemm_skinny_kernel(void* __restrict__ out, const __nv_bfloat16* __restrict__ X, 
   for (int idx = tid; idx < MT * 8 * chunks; idx += SK_THREADS) {
     const int row = idx / chunks, c = idx - row * chunks;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (row < M) v = *reinterpret_cast<const uint4*>(X + (size_t)row * K + c * 8);
+    if (row < M) v = behind_load16(X + (size_t)row * K + c * 8);
     *reinterpret_cast<uint4*>(xs + row * xs_stride + c * 8) = v;
   }
   __syncthreads();
@@ -236,7 +236,7 @@ gemm_skinny_stream_kernel(void* __restrict__ out, const __nv_bfloat16* __restric
   for (int idx = tid; idx < TOK * chunks; idx += SK_THREADS) {
     const int row = idx / chunks, c = idx - row * chunks;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (row < M) v = *reinterpret_cast<const uint4*>(X + (size_t)row * K + c * 8);
+    if (row < M) v = behind_load16(X + (size_t)row * K + c * 8);
     *reinterpret_cast<uint4*>(xs + row * xs_stride + c * 8) = v;
   }
   __syncthreads();

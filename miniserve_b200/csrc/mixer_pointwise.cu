@@ -22,7 +22,7 @@ template <typename T>
 __global__ void add_dyt_kernel(T* __restrict__ out, float* __restrict__ residual, const T* __restrict__ delta,
                                const float* __restrict__ w, const float* __restrict__ b, const float* __restrict__ alpha,
                                const int* __restrict__ rows, int hidden, int write_residual) {
-  pdl_prologue();
+  pdl_prologue(delta, w, b, alpha, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -41,7 +41,7 @@ __global__ void add_dyt_kernel(T* __restrict__ out, float* __restrict__ residual
 
 template <typename T>
 __global__ void gelu_tanh_kernel(T* __restrict__ out, const T* __restrict__ x, long long n) {
-  pdl_prologue();
+  pdl_prologue(x);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float z = Elem<T>::load(x + i);
@@ -49,7 +49,7 @@ __global__ void gelu_tanh_kernel(T* __restrict__ out, const T* __restrict__ x, l
 }
 
 __global__ void gelu_tanh_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ x, long long n8) {
-  pdl_prologue();
+  pdl_prologue(x);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   float v[8];
@@ -67,7 +67,7 @@ __global__ void scale_f32_kernel(float* __restrict__ x, float s, long long n) {
 
 template <typename T>
 __global__ void axpby_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ y, float a, float b, long long n) {
-  pdl_prologue();
+  pdl_prologue(x, y);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) Elem<T>::store(out + i, a * Elem<T>::load(x + i) + b * Elem<T>::load(y + i));
 }
@@ -76,7 +76,7 @@ __global__ void axpby_kernel(T* __restrict__ out, const T* __restrict__ x, const
 template <typename T>
 __global__ void head_gate_kernel(T* __restrict__ out, int ld_out, const T* __restrict__ attn, const T* __restrict__ gate,
                                  int ld_gate, long long items, int nq, int d_pad, int dv, float scale, int gated) {
-  pdl_prologue();
+  pdl_prologue(attn, gate);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const int c = (int)(idx % dv);
@@ -93,7 +93,7 @@ __global__ void head_gate_kernel(T* __restrict__ out, int ld_out, const T* __res
 __global__ void head_gate_bf16x8_kernel(__nv_bfloat16* __restrict__ out, int ld_out, const __nv_bfloat16* __restrict__ attn,
                                         const __nv_bfloat16* __restrict__ gate, int ld_gate, long long pairs, int nq, int d_pad,
                                         int dv, float scale) {
-  pdl_prologue();
+  pdl_prologue(attn, gate);
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= pairs) return;
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) qkv_prepare_bf16x8_kernel(
     const int* __restrict__ row_of_token, const int* __restrict__ page_indptr, const int* __restrict__ page_indices,
     int num_tokens, int nq, int nkv, int dk, int dv, int d_pad, int rot, float eps, int page_shift, int num_pages,
     int* __restrict__ status, PrepareExtras ex) {
-  pdl_prologue();
+  pdl_prologue(proj, q_norm_w, k_norm_w, cos_sin, positions, row_of_token, page_indptr, page_indices);
   const int lane = threadIdx.x % LANES;
   const unsigned group = LANES == 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16);  // the head's lanes
   const int heads_total = k_pool ? nq + 2 * nkv : nq;  // without pools the projection holds queries alone
@@ -309,7 +309,7 @@ __global__ void qkv_prepare_kernel(
     const int* __restrict__ positions, const int* __restrict__ row_of_token, const int* __restrict__ page_indptr,
     const int* __restrict__ page_indices, int num_tokens, int nq, int nkv, int dk, int dv, int d_pad, int rot,
     int adjacent, float eps, int page_shift, int num_pages, int* __restrict__ status, PrepareExtras ex) {
-  pdl_prologue();
+  pdl_prologue(proj, q_norm_w, k_norm_w, cos_sin, positions, row_of_token, page_indptr, page_indices);
   const int lane = threadIdx.x & 31;
   const int heads_total = k_pool ? nq + 2 * nkv : nq;  // without pools the projection holds queries alone
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -528,7 +528,7 @@ MS_EXPORT int ms_qkv_prepare(void* q_out, void* k_pool, void* v_pool, const void
 namespace ms {
 template <typename T>
 __global__ void act_mul_kernel(T* __restrict__ out, const T* __restrict__ gate_up, int inter, long long total, int act) {
-  pdl_prologue();
+  pdl_prologue(gate_up);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const long long t = idx / inter;

@@ -47,7 +47,7 @@ template <typename TZ>
 __global__ void decay_from_logits_kernel(float* __restrict__ out, const TZ* __restrict__ z, int ld_z, const float* __restrict__ z_bias,
                                          const float* __restrict__ decay_coef, float z_sign, const TZ* __restrict__ beta,
                                          int ld_beta, long long items, int H, int dk) {
-  pdl_prologue();
+  pdl_prologue(z, z_bias, decay_coef, beta);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const int width = H * dk + (beta ? H : 0);
@@ -81,7 +81,7 @@ decay_scan_kernel(float* __restrict__ o_out,   // [T, H, dv]
   // words a thread's channels take in shared memory: padded so that the 16-byte loads of a quarter warp's lanes fall on different banks
   constexpr int SCAN_SEG = SCAN_KPT == 4 ? 4 : SCAN_KPT + 4;
   extern __shared__ __align__(16) float smem[];
-  pdl_prologue();
+  pdl_prologue(q, k, v, z, z_bias, decay_coef, beta, cu_q, q_start, state_slot, v_scale, bonus);
   const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int threads = blockDim.x;
   const int cols = threads / L;
@@ -245,7 +245,7 @@ decay_step_kernel(float* __restrict__ o_out, float* __restrict__ state, const TI
                   int qk_group, const TIn* __restrict__ v, int ld_v, const float* __restrict__ z, int ld_z, const int* __restrict__ cu_q,
                   const int* __restrict__ q_start, const int* __restrict__ state_slot, int H, int dk, int dv, float q_scale,
                   const float* __restrict__ v_scale, int dv_in) {
-  pdl_prologue();
+  pdl_prologue(q, k, v, z, cu_q, q_start, state_slot, v_scale);
   constexpr int CPW = 32 / LPC;  // columns a warp takes at once
   const int r = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int l = lane % LPC, sub = lane / LPC;
@@ -310,7 +310,7 @@ decay_step_kernel(float* __restrict__ o_out, float* __restrict__ state, const TI
 // seg_cu[r * P + s]: first token of segment s of row r (segments of ceil(len / P) tokens; the last ones may be empty)
 __global__ void segment_setup_kernel(int* __restrict__ seg_cu, int* __restrict__ seg_zero, int* __restrict__ seg_slot,
                                      const int* __restrict__ cu_q, int num_rows, int P) {
-  pdl_prologue();
+  pdl_prologue(cu_q);
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx > num_rows * P) return;
   if (idx == num_rows * P) {
@@ -328,7 +328,7 @@ __global__ void segment_setup_kernel(int* __restrict__ seg_cu, int* __restrict__
 // c[t, ch] = product of decay[s, ch] over the tokens s of t's segment up to and including t. One thread per (segment, channel).
 __global__ void segment_cumprod_kernel(float* __restrict__ c, const float* __restrict__ decay, int ld_decay,
                                        const int* __restrict__ seg_cu, int num_segments, int width) {
-  pdl_prologue();
+  pdl_prologue(decay, seg_cu);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)num_segments * width) return;
   const int sg = (int)(idx / width), ch = (int)(idx - (long long)sg * width);
@@ -347,7 +347,7 @@ __global__ void segment_combine_kernel(float* __restrict__ state, const float* _
                                        const float* __restrict__ c, const int* __restrict__ seg_cu,
                                        const int* __restrict__ q_start, const int* __restrict__ state_slot, int num_rows, int P,
                                        int H, int dk, int dv, int dkz) {
-  pdl_prologue();
+  pdl_prologue(ends, c, seg_cu, q_start, state_slot);
   const long long per_row = (long long)H * dv * dk;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= num_rows * per_row) return;
@@ -375,7 +375,7 @@ segment_fixup_kernel(float* __restrict__ o, const TIn* __restrict__ q, int ld_q,
                      const float* __restrict__ before, const int* __restrict__ seg_cu, const int* __restrict__ q_start, int P,
                      int H, int dk, int dv, int cols, float q_scale, int dkz, int before_decay) {
   extern __shared__ float fix_smem[];
-  pdl_prologue();
+  pdl_prologue(q, c, before, seg_cu, q_start);
   const int sg = blockIdx.x, h = blockIdx.y;
   const int t0 = seg_cu[sg] + blockIdx.z * FIX_RUN, end = min(seg_cu[sg + 1], t0 + FIX_RUN);
   if (end <= t0) return;
@@ -427,7 +427,7 @@ __global__ void conv_silu_unit_kernel(float* __restrict__ out, const T* __restri
                                       const int* __restrict__ cu_q, const int* __restrict__ q_start,
                                       const int* __restrict__ state_slot, int num_tokens, int C, int taps, int unit_heads,
                                       int dk, int other_heads, int dv, float unit_eps, const float* __restrict__ bias) {
-  pdl_prologue();
+  pdl_prologue(proj, conv_state, w, row_of_token, cu_q, q_start, state_slot, bias);
   const int lane = threadIdx.x & 31;
   const int units = unit_heads + other_heads;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -499,7 +499,7 @@ conv_silu_unit_x4_kernel(float* __restrict__ out, const T* __restrict__ proj, in
                          const int* __restrict__ row_of_token, const int* __restrict__ cu_q, const int* __restrict__ q_start,
                          const int* __restrict__ state_slot, int num_tokens, int C, int unit_channels, int lanes_per_head, float unit_eps,
                          const float* __restrict__ bias, int update) {
-  pdl_prologue();
+  pdl_prologue(proj, w, row_of_token, cu_q, q_start, state_slot, bias);
   const int ch = (blockIdx.x * CONV_THREADS + threadIdx.x) * 4;
   const int t0 = blockIdx.y * RUN;
   const bool in = ch < C;
@@ -598,7 +598,7 @@ template <typename T>
 __global__ void conv_state_update_kernel(T* __restrict__ conv_state, const T* __restrict__ proj, int ld,
                                          const int* __restrict__ cu_q, const int* __restrict__ q_start,
                                          const int* __restrict__ state_slot, int num_rows, int C, int taps) {
-  pdl_prologue();
+  pdl_prologue(proj, cu_q, q_start, state_slot);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)num_rows * C) return;
   const int r = (int)(idx / C), ch = (int)(idx - (long long)r * C);
@@ -621,7 +621,7 @@ template <typename T>
 __global__ void head_norm_gate_kernel(T* __restrict__ out, int ld_out, const float* __restrict__ o, const float* __restrict__ w,
                                       const T* __restrict__ gate, int ld_gate, int num_tokens, int H, int dv, float eps,
                                       float scale, int gate_kind, int w_stride) {
-  pdl_prologue();
+  pdl_prologue(o, w, gate);
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= (long long)num_tokens * H) return;
@@ -645,7 +645,7 @@ template <typename T, int LANES>
 __global__ void __launch_bounds__(256)
 head_norm_gate_x4_kernel(T* __restrict__ out, int ld_out, const float* __restrict__ o, const float* __restrict__ w, const T* __restrict__ gate,
                          int ld_gate, int num_tokens, int H, float eps, float scale, int gate_kind, int w_stride) {
-  pdl_prologue();
+  pdl_prologue(o, w, gate);
   constexpr int DV = 4 * LANES;
   const long long item = ((long long)blockIdx.x * 256 + threadIdx.x) / LANES;
   const int c = (threadIdx.x % LANES) * 4;
@@ -960,7 +960,7 @@ namespace ms {
 template <typename T>
 __global__ void ssm_step_decay_kernel(float* __restrict__ out, const T* __restrict__ raw, int ld, const float* __restrict__ bias,
                                       const float* __restrict__ coef, long long items, int H) {
-  pdl_prologue();
+  pdl_prologue(raw, bias, coef);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const long long t = idx / H;
@@ -980,7 +980,7 @@ gated_group_norm_kernel(T* __restrict__ out, int ld_out, const float* __restrict
                         const float* __restrict__ skip, const T* __restrict__ gate, int ld_gate, const float* __restrict__ w,
                         int width, int parts, int dv, float eps) {
   __shared__ float scratch[32];
-  pdl_prologue();
+  pdl_prologue(o, x, skip, gate, w);
   const int t = blockIdx.x / parts, part = blockIdx.x - t * parts;
   const int size = width / parts, base = part * size;
   float ss = 0.f;
@@ -1012,7 +1012,7 @@ __global__ void __launch_bounds__(GGN_THREADS)
 gated_group_norm_x4_kernel(T* __restrict__ out, int ld_out, const float* __restrict__ o, const float* __restrict__ x, int ld_x,
                            const float* __restrict__ skip, const T* __restrict__ gate, int ld_gate, const float* __restrict__ w, int num_items,
                            int width, int parts, int dv, float eps) {
-  pdl_prologue();
+  pdl_prologue(o, x, skip, gate, w);
   const int item = blockIdx.x * (GGN_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (item >= num_items) return;
   const int t = item / parts, part = item - t * parts, size = width / parts, base = part * size;

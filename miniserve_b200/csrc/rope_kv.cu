@@ -27,7 +27,7 @@ __global__ void qk_norm_rope_kv_kernel(
     const int* __restrict__ positions, const int* __restrict__ row_of_token,
     const int* __restrict__ page_indptr, const int* __restrict__ page_indices,
     int num_tokens, int nq, int nkv, int d, int rot, float eps, int page_shift, int num_pages, int* __restrict__ status) {
-  pdl_prologue();
+  pdl_prologue(qkv, q_norm_w, k_norm_w, inv_freq, cos_sin, positions, row_of_token, page_indptr, page_indices);
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int heads_total = nq + (k_pool ? 2 * nkv : 0);
@@ -143,13 +143,7 @@ qk_norm_rope_kv_bf16_token_kernel(
       wk_hi = weight_load16(k_norm_w + HALF + j0);
     }
   }
-  pdl_wait();
-  behind_wait(qkv);
-  behind_wait(cos_sin);
-  behind_wait(positions);
-  behind_wait(row_of_token);
-  behind_wait(page_indptr);
-  behind_wait(page_indices);
+  pdl_wait(qkv, inv_freq, cos_sin, positions, row_of_token, page_indptr, page_indices);
   const int pos = positions[t];
   const int heads_total = nq + (has_kv ? 2 * nkv : 0);
   const __nv_bfloat16* row_in = qkv + (size_t)t * heads_total * D;
@@ -248,7 +242,7 @@ qk_norm_rope_kv_bf16_token_kernel(
 // table[t, rot/2 + j] = sin(...). Made once per step and read by every layer's q/k kernel.
 __global__ void rope_table_kernel(float* __restrict__ table, const int* __restrict__ positions,
                                   const float* __restrict__ inv_freq, int num_tokens, int rot) {
-  pdl_prologue();
+  pdl_prologue(positions, inv_freq);
   const int half = rot >> 1;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)num_tokens * half) return;
@@ -264,7 +258,7 @@ __global__ void rope_table_kernel(float* __restrict__ table, const int* __restri
 // tiled[tile of 128 tokens][eighth of the 64 pairs][cos, sin][token within the tile][pair within the eighth].
 // Tokens beyond the last one (the last tile's unused rows) are left as they are.
 __global__ void rope_table_tile_kernel(float* __restrict__ tiled, const float* __restrict__ table, int num_tokens) {
-  pdl_prologue();
+  pdl_prologue(table);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)num_tokens * 128) return;
   const int t = (int)(idx >> 7), col = (int)(idx & 127);

@@ -52,7 +52,7 @@ expert_route_kernel(int* __restrict__ idx_out, float* __restrict__ wgt_out, cons
   if (TOK == 1 && vec) {  // a few tokens: the router is fetched from memory, and asked for before the wait for the input
     for (size_t at = (size_t)threadIdx.x * 32; at < (size_t)R * K; at += ROUTE_THREADS * 32) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(router + at));
   }
-  pdl_prologue();
+  pdl_prologue(x, router, correction, logit_bias, gate_w);
   if (vec == 2) {  // bfloat16 rows of whole 16 bytes
     const int k8 = K >> 3;
     for (int i = threadIdx.x; i < TOK * k8; i += ROUTE_THREADS) {
@@ -240,7 +240,11 @@ expert_plan_kernel(int* __restrict__ pos, int* __restrict__ perm, int* __restric
 #pragma unroll
   for (int i = 0; i < PLAN_EACH; ++i) {
     const int slot = i * PLAN_THREADS + tid;
-    expert[i] = slot < S ? idx[slot] : -1;
+    expert[i] = -1;
+    if (i * PLAN_THREADS < S) {
+      const int e = behind_load(idx + min(slot, S - 1));
+      if (slot < S) expert[i] = e;
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -249,7 +253,7 @@ expert_plan_kernel(int* __restrict__ pos, int* __restrict__ perm, int* __restric
     rank[i] = expert[i] >= 0 && expert[i] < E ? atomicAdd(&cnt[expert[i]], 1) : -1;
   }
   for (int slot = PLAN_EACH * PLAN_THREADS + tid; slot < S; slot += PLAN_THREADS) {
-    const int e = idx[slot];
+    const int e = behind_load(idx + slot);
     pos[slot] = (e >= 0 && e < E) ? atomicAdd(&cnt[e], 1) : -1;
   }
   __syncthreads();
@@ -299,7 +303,7 @@ expert_plan_kernel(int* __restrict__ pos, int* __restrict__ perm, int* __restric
   for (int slot = PLAN_EACH * PLAN_THREADS + tid; slot < S; slot += PLAN_THREADS) {
     const int r = pos[slot];
     if (r >= 0) {
-      const int p = off[idx[slot]] + r;
+      const int p = off[behind_load(idx + slot)] + r;
       pos[slot] = p;
       perm[p] = slot;
     }
@@ -348,7 +352,7 @@ expert_gemm_kernel(void* __restrict__ out_, const T* __restrict__ A, int lda, co
   __shared__ float As[XG_BK][XG_BM + 4];
   __shared__ float Bg[XG_BK][XG_BN + 4];
   __shared__ float Bu[GATED ? XG_BK : 1][XG_BN + 4];
-  pdl_prologue();
+  pdl_prologue(A, perm, W, tiles, meta, offsets);
   if ((int)blockIdx.x >= meta[0]) return;
   const int e = tiles[2 * blockIdx.x], row0 = tiles[2 * blockIdx.x + 1];
   const int rows = min(XG_BM, offsets[e + 1] - row0);
@@ -434,7 +438,7 @@ expert_gemm_mma_kernel(void* __restrict__ out_, const __nv_bfloat16* __restrict_
   __shared__ __align__(16) __nv_bfloat16 As[2][XM_BM][XM_LD];
   __shared__ __align__(16) __nv_bfloat16 Bg[2][XM_BN][XM_LD];
   __shared__ __align__(16) __nv_bfloat16 Bu[GATED ? 2 : 1][GATED ? XM_BN : 1][XM_LD];
-  pdl_prologue();
+  pdl_prologue(A, perm, W, tiles, meta, offsets);
   if ((int)blockIdx.x >= meta[0]) return;
   const int e = tiles[2 * blockIdx.x], row0 = tiles[2 * blockIdx.x + 1];
   const int rows = min(XM_BM, offsets[e + 1] - row0);
@@ -538,7 +542,7 @@ __global__ void expert_combine_kernel(T* __restrict__ out, const float* __restri
                                       const int* __restrict__ idx, const float* __restrict__ wgt, const int* __restrict__ pos,
                                       long long total, int H, int top, int E, const T* __restrict__ shared,
                                       const float* __restrict__ shared_gate) {
-  pdl_prologue();
+  pdl_prologue(y, x, idx, wgt, pos, shared, shared_gate);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long t = i / H;
@@ -575,7 +579,7 @@ template <typename T>
 __global__ void expert_combine_x4_kernel(T* __restrict__ out, const float* __restrict__ y, const T* __restrict__ x, int ld_x,
                                          const int* __restrict__ idx, const float* __restrict__ wgt, const int* __restrict__ pos, int total4,
                                          int H4, int top, int E, const T* __restrict__ shared, const float* __restrict__ shared_gate) {
-  pdl_prologue();
+  pdl_prologue(y, x, idx, wgt, pos, shared, shared_gate);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total4) return;
   const int t = i / H4, c = (i - t * H4) * 4;
@@ -677,12 +681,22 @@ MS_EXPORT int ms_expert_plan_of(int* pos, int* perm, int* offsets, int* tiles, i
 // tile of rows is one box for TMA. One warp per row, 16 bytes a lane and trip. K % 8 == 0, rows 16-byte aligned.
 __global__ void expert_gather_kernel(__nv_bfloat16* __restrict__ xs, const __nv_bfloat16* __restrict__ x, int ld_x,
                                      const int* __restrict__ perm, const int* __restrict__ meta, int top, int slots, int K) {
-  pdl_prologue();
+  pdl_prologue(x);
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= slots || row >= meta[1]) return;
-  const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(perm[row] / top) * ld_x);
+  if (row >= slots) return;
+  const int rows = behind_load(meta + 1), slot = behind_load(perm + row);  // (both at once; a row behind the last has any slot)
+  if (row >= rows) return;
+  const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(slot / top) * ld_x);
   uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)row * K);
-  for (int c = lane; c < K / 8; c += 32) dst[c] = src[c];
+  const int last = K / 8 - 1;
+  for (int c = lane; c <= last; c += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = behind_load16(src + min(c + 32 * i, last));  // (four on their way at once)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (c + 32 * i <= last) dst[c + 32 * i] = v[i];
+  }
 }
 
 MS_EXPORT int ms_expert_gather(void* xs, const void* x, int ld_x, const int* perm, const int* meta, int top, int slots, int K,

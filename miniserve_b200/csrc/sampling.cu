@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(1024)
 nucleus_kernel(Nucleus* __restrict__ out, const float* __restrict__ logits, const float* __restrict__ temperature,
                const float* __restrict__ top_p, int vocab) {
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(logits, temperature, top_p);
   const int r = blockIdx.x;
   const float t = temperature[r], tp = top_p[r];
   Nucleus n;
@@ -134,7 +134,7 @@ sample_kernel(int* __restrict__ tokens, const float* __restrict__ logits, const 
               const Nucleus* __restrict__ nucleus, int vocab) {
   __shared__ Best scratch[32];
   __shared__ int tie_base[33];
-  pdl_prologue();
+  pdl_prologue(logits, temperature, seed, counter, nucleus);
   const int r = blockIdx.x;
   const float* lg = logits + (size_t)r * vocab;
   const float t = temperature ? temperature[r] : 0.f;
@@ -203,7 +203,7 @@ sample_partial_kernel(Best* __restrict__ partial, const float* __restrict__ logi
                       const float* __restrict__ temperature, const long long* __restrict__ seed,
                       const long long* __restrict__ counter, int vocab, int per_block) {
   __shared__ Best scratch[32];
-  pdl_prologue();
+  pdl_prologue(logits, temperature, seed, counter);
   const int r = blockIdx.y;
   const float* lg = logits + (size_t)r * vocab;
   const float t = temperature ? temperature[r] : 0.f;
@@ -230,7 +230,7 @@ sample_partial_kernel(Best* __restrict__ partial, const float* __restrict__ logi
 __global__ void __launch_bounds__(256)
 sample_final_kernel(int* __restrict__ tokens, const Best* __restrict__ partial, int num_partials) {
   __shared__ Best scratch[32];
-  pdl_prologue();
+  pdl_prologue(partial);
   const int r = blockIdx.x;
   Best b;
   b.val = -INFINITY;
@@ -308,7 +308,7 @@ sample_cluster_kernel(int* __restrict__ tokens, const float* __restrict__ logits
   const int ctas = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int r = blockIdx.x / ctas;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  pdl_prologue();
+  pdl_prologue(logits, temperature, top_p, seed, counter);
   const float* lg = logits + (size_t)r * vocab;
   const float t = temperature[r], tp = top_p[r];
   const int begin = min(rank * slice, vocab), n = min(slice, vocab - begin);

@@ -47,7 +47,7 @@ __global__ void embed_sum_kernel(float* __restrict__ residual, const T* __restri
                                  const int* __restrict__ ids, const int* __restrict__ positions, const int* __restrict__ row_of_token,
                                  const int* __restrict__ cu_q, const int* __restrict__ state_slot, int* __restrict__ prev_token,
                                  int hidden, int vocab, float scale) {
-  pdl_prologue();
+  pdl_prologue(table, inv_freq, ids, positions, row_of_token, cu_q, state_slot);
   const int t = blockIdx.x;
   int id = ids[t];
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
@@ -76,7 +76,7 @@ __global__ void embed_sum_bf16x8_kernel(float* __restrict__ residual, const __nv
                                         const float* __restrict__ inv_freq, const int* __restrict__ ids, const int* __restrict__ positions,
                                         const int* __restrict__ row_of_token, const int* __restrict__ cu_q,
                                         const int* __restrict__ state_slot, int* __restrict__ prev_token, int hidden, int vocab, float scale) {
-  pdl_prologue();
+  pdl_prologue(table, inv_freq, ids, positions, row_of_token, cu_q, state_slot);
   const int t = blockIdx.x;
   int id = ids[t];
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
@@ -127,7 +127,7 @@ add_normed_rmsnorm_kernel(T* __restrict__ out, float* __restrict__ residual, con
                           const int* __restrict__ rows, int hidden, int write_residual) {
   extern __shared__ float row_h[];  // hidden floats
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(delta, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(THREADS)
 add_normed_rmsnorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ residual, const __nv_bfloat16* __restrict__ delta,
                                  NormWeight nb, NormWeight n, const int* __restrict__ rows, int hidden, int write_residual) {
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(delta, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -240,7 +240,7 @@ stream_norm_kernel(T* __restrict__ out, float* dst, const float* src, int src_st
                    const float* __restrict__ w, float eps, const int* __restrict__ rows, int hidden, int write) {
   extern __shared__ float row_u[];  // hidden floats
   __shared__ float red[32];
-  pdl_prologue();
+  pdl_prologue(y, w, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   const float* xs = src + (size_t)r * src_streams * hidden;
@@ -284,7 +284,7 @@ stream_norm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* dst, const flo
 #pragma unroll
     for (int t = 0; t < S; ++t) mix[s][t] = y ? links.mix[s * S + t] : 0.f;
   }
-  pdl_prologue();
+  pdl_prologue(y, w, rows);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   const int c = threadIdx.x * 8;

@@ -178,7 +178,7 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
   constexpr int LD = DK + 4;
   extern __shared__ __align__(16) float tw_smem[];
   float *qs = tw_smem, *ks = qs + TW_TOK * LD;
-  pdl_prologue();
+  pdl_prologue(q, k, cu_q);
   const int grp = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const TwPiece at = tw_piece(blockIdx.x, TW_TOK, cu_q, num_rows);
   if (at.row < 0) return;
@@ -278,7 +278,7 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
   constexpr bool KEEP = N <= 2;  // k' stays in shared memory as well (a fourth array; at N = 4 it would leave room for one CTA)
   float* kf = KEEP ? ds + TW_TOK * LD : ks;
   __shared__ double whole[SUBS][DKP];  // a sixteen's decays
-  pdl_prologue();
+  pdl_prologue(q, k, z, z_bias, decay_coef, cu_q);
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const TwPiece at = tw_piece(blockIdx.x, TW_TOK, cu_q, num_rows);
   if (at.row < 0) return;

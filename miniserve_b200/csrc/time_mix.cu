@@ -27,7 +27,7 @@ __device__ __forceinline__ float channel_decay_of(float z) { return expf(-expf(z
 template <typename T>
 __global__ void channel_decay_kernel(float* __restrict__ out, const T* __restrict__ z, int ld_z, const float* __restrict__ w0, long long items,
                                      int width) {
-  pdl_prologue();
+  pdl_prologue(z, w0);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const long long t = idx / width;
@@ -72,7 +72,7 @@ time_step_kernel(T* __restrict__ out, float* __restrict__ state, Rows<T> r, Rows
     const char* w = reinterpret_cast<const char*>(w2 + (size_t)h * dk * rank);
     for (size_t at = (size_t)tid * 128; at < (size_t)dk * rank * sizeof(T); at += TS_THREADS * 128) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(w + at));
   }
-  pdl_prologue();
+  pdl_prologue(w2, w0, u, norm_w, cu_q, q_start, state_slot);
   const int t = cu_q[row];
   const bool fresh = q_start[row] == 0;
   constexpr int CPW = 32 / LPC;
@@ -300,7 +300,7 @@ tm_states_kernel(float* __restrict__ added, float* __restrict__ passed, const __
                  const ChunkPlace pl, int H, int dk, int dv) {
   extern __shared__ __align__(16) unsigned char cs_raw[];
   TmStatesSmem<DKT>& sm = *reinterpret_cast<TmStatesSmem<DKT>*>(cs_raw);
-  pdl_prologue();
+  pdl_prologue(k, v, z, w0);
   const int chunk = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * TC_DV;
   if (chunk >= pl.row_first[pl.num_rows]) return;
   const int2 at = pl.tab[chunk];
@@ -358,7 +358,7 @@ tm_states_kernel(float* __restrict__ added, float* __restrict__ passed, const __
 __global__ void __launch_bounds__(CS_THREADS)
 tm_carry_kernel(float* __restrict__ state, __nv_bfloat16* __restrict__ before_hi, __nv_bfloat16* __restrict__ before_lo,
                 const float* __restrict__ added, const float* __restrict__ passed, const ChunkPlace pl, int H, int dk, int dv) {
-  pdl_prologue();
+  pdl_prologue(added, passed);
   const int total = H * dv * dk;
   const int i = blockIdx.x * CS_THREADS + threadIdx.x, r = blockIdx.y;
   if (i >= total) return;
@@ -506,7 +506,7 @@ tm_outputs_kernel(float* __restrict__ o, const HeadGate hg, const __nv_bfloat16*
                   const ChunkPlace pl, int H, int dk, int dv) {
   extern __shared__ __align__(16) unsigned char cs_raw[];
   TmOutputsSmem<DKT>& sm = *reinterpret_cast<TmOutputsSmem<DKT>*>(cs_raw);
-  pdl_prologue();
+  pdl_prologue(r, k, v, z, w0, u, before_hi, before_lo);
   const int chunk = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * TC_DV;
   if (chunk >= pl.row_first[pl.num_rows]) return;
   const int2 at = pl.tab[chunk];
