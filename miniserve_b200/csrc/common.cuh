@@ -131,8 +131,8 @@ __device__ __forceinline__ int behind_load(const int* p) {
   asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
-// A kernel whose weights come from far (each layer's are read once in a decode step) asks for them between the two halves of the prologue: weights are
-// not written by kernels that may still run when its CTAs begin. weight_load16: 16 bytes, asked for where it stands (a plain load may move behind
+// A kernel whose weights come from far (each layer's are read once in a decode step) asks for them between the two halves of the prologue, where its caller says
+// (a product's weights: always) that no kernel that may still run when its CTAs begin writes them. weight_load16: 16 bytes, asked for where it stands (a plain load may move behind
 // the wait).
 __device__ __forceinline__ uint4 weight_load16(const void* p) {
   uint4 v;

@@ -75,7 +75,7 @@ add_rmsnorm_kernel(T* __restrict__ out, float* __restrict__ residual, const T* _
 // The same for bfloat16 activations whose rows are a multiple of 8 wide: eight elements per thread
 // and trip (two 16-byte loads of the residual, one of the addend), the sum kept in registers when
 // a row is at most 8 * THREADS wide, else in shared memory.
-template <int THREADS>
+template <int THREADS, bool AHEAD>
 __global__ void __launch_bounds__(THREADS)
 add_rmsnorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ residual,
                           const __nv_bfloat16* __restrict__ delta, const __nv_bfloat16* __restrict__ w,
@@ -87,8 +87,10 @@ add_rmsnorm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ r
   pdl_launch_dependents();
   // A step of 8 requests with 57 of these: 1,101 -> 1,088 us, against weights asked for behind the sum of squares.
   uint4 w_raw = make_uint4(0u, 0u, 0u, 0u);
-  if (in_regs && (int)threadIdx.x < chunks) w_raw = weight_load16(w + 8 * threadIdx.x);
+  const bool mine = in_regs && (int)threadIdx.x < chunks;
+  if (AHEAD && mine) w_raw = weight_load16(w + 8 * threadIdx.x);
   pdl_wait(residual, delta, w, rows);
+  if (!AHEAD && mine) w_raw = behind_load16(w + 8 * threadIdx.x);
   const int i = blockIdx.x;
   const int r = rows ? rows[i] : i;
   float* res = residual + (size_t)r * hidden;
@@ -218,9 +220,9 @@ MS_EXPORT int ms_embed_gather(void* residual_f32, const void* table, const int* 
 }
 
 // delta: an addend in the activation dtype, or null; it is added to the residual before the norm.
-MS_EXPORT int ms_add_rmsnorm(void* out, void* residual_f32, const void* delta, const void* weight, const int* rows,
-                             float eps, int num_out_rows, int hidden, int write_residual, int dtype,
-                             cudaStream_t stream) {
+// weights_ahead: no kernel that may still run writes the weight, so it may be asked for ahead of the wait.
+static int add_rmsnorm(void* out, void* residual_f32, const void* delta, const void* weight, const int* rows, float eps, int num_out_rows, int hidden,
+                       int write_residual, int weights_ahead, int dtype, cudaStream_t stream) {
   if (num_out_rows == 0) return 0;
   MS_CHECK_ARG(num_out_rows > 0 && hidden > 0, "add_rmsnorm: bad sizes rows=%d H=%d", num_out_rows, hidden);
   MS_CHECK_ARG(!(rows && write_residual), "add_rmsnorm: a gathered norm cannot write the residual back");
@@ -234,9 +236,10 @@ MS_EXPORT int ms_add_rmsnorm(void* out, void* residual_f32, const void* delta, c
   } else if (hidden % 8 == 0 && ((uintptr_t)out % 16 == 0) && ((uintptr_t)residual_f32 % 16 == 0) &&
              ((uintptr_t)delta % 16 == 0) && ((uintptr_t)weight % 16 == 0)) {
     if (hidden <= 8 * 128) {
-      MS_LAUNCH((add_rmsnorm_bf16x8_kernel<128>), num_out_rows, 128, 0, stream, (__nv_bfloat16*)out, (float*)residual_f32, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)weight, rows, eps, hidden, write_residual);
+      auto k = weights_ahead ? add_rmsnorm_bf16x8_kernel<128, true> : add_rmsnorm_bf16x8_kernel<128, false>;
+      MS_LAUNCH(k, num_out_rows, 128, 0, stream, (__nv_bfloat16*)out, (float*)residual_f32, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)weight, rows, eps, hidden, write_residual);
     } else {
-      auto k = add_rmsnorm_bf16x8_kernel<256>;
+      auto k = weights_ahead ? add_rmsnorm_bf16x8_kernel<256, true> : add_rmsnorm_bf16x8_kernel<256, false>;
       const size_t need = hidden <= 8 * 256 ? 0 : smem;
       if (need > 48 * 1024) MS_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
       MS_LAUNCH(k, num_out_rows, 256, need, stream, (__nv_bfloat16*)out, (float*)residual_f32, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)weight, rows, eps, hidden, write_residual);
@@ -247,6 +250,15 @@ MS_EXPORT int ms_add_rmsnorm(void* out, void* residual_f32, const void* delta, c
     MS_LAUNCH(k, num_out_rows, THREADS, smem, stream, (__nv_bfloat16*)out, (float*)residual_f32, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)weight, rows, eps, hidden, write_residual);
   }
   return 0;
+}
+
+MS_EXPORT int ms_add_rmsnorm(void* out, void* residual_f32, const void* delta, const void* weight, const int* rows, float eps, int num_out_rows, int hidden,
+                             int write_residual, int dtype, cudaStream_t stream) {
+  return add_rmsnorm(out, residual_f32, delta, weight, rows, eps, num_out_rows, hidden, write_residual, 0, dtype, stream);
+}
+MS_EXPORT int ms_add_rmsnorm_ahead(void* out, void* residual_f32, const void* delta, const void* weight, const int* rows, float eps, int num_out_rows, int hidden,
+                                   int write_residual, int dtype, cudaStream_t stream) {
+  return add_rmsnorm(out, residual_f32, delta, weight, rows, eps, num_out_rows, hidden, write_residual, 1, dtype, stream);
 }
 
 MS_EXPORT int ms_silu_mul(void* out, const void* gate_up, int tokens, int inter, int dtype, cudaStream_t stream) {

@@ -85,9 +85,10 @@ TC_ATTENTION = _flag("MINISERVE_TC_ATTENTION", "1")  # prompts on the tcgen05 at
 
 def add_rmsnorm(out: torch.Tensor, residual: torch.Tensor, delta: torch.Tensor | None,
                 weight: torch.Tensor, eps: float, rows: torch.Tensor | None = None, num_rows: int | None = None,
-                write_residual: bool = True, stream=None) -> None:
+                write_residual: bool = True, stream=None, weights_ahead: bool = False) -> None:
     """out[i] = rmsnorm(residual[r] + delta[r]) * weight with r = rows[i] (or i); the sum is
-    written back to ``residual`` when there is no gather. Statistics in float32."""
+    written back to ``residual`` when there is no gather. Statistics in float32. ``weights_ahead``: ``weight`` is a parameter, which no kernel
+    that may still run on the stream writes; it is read while the kernels before this one run."""
     _check_dev(out, residual, delta, weight, rows)
     assert residual.dtype == torch.float32 and out.dtype == weight.dtype
     assert delta is None or delta.dtype == out.dtype
@@ -97,7 +98,7 @@ def add_rmsnorm(out: torch.Tensor, residual: torch.Tensor, delta: torch.Tensor |
     if rows is None:
         assert residual.shape[0] >= n
     k = native.kernels()
-    native.kernel_check(k.ms_add_rmsnorm(_ptr(out), _ptr(residual), _ptr(delta), _ptr(weight), _ptr(rows),
+    native.kernel_check((k.ms_add_rmsnorm_ahead if weights_ahead else k.ms_add_rmsnorm)(_ptr(out), _ptr(residual), _ptr(delta), _ptr(weight), _ptr(rows),
                                          float(eps), n, hidden, int(write_residual and rows is None),
                                          dtype_code(out.dtype), _stream(stream)))
 
@@ -405,10 +406,10 @@ def qk_norm_rope_kv(q_out: torch.Tensor, k_pool: torch.Tensor | None, v_pool: to
                     qkv: torch.Tensor, q_norm_w: torch.Tensor | None, k_norm_w: torch.Tensor | None,
                     inv_freq: torch.Tensor | None, rotary_dim: int, eps: float, positions: torch.Tensor,
                     row_of_token: torch.Tensor, page_indptr: torch.Tensor, page_indices: torch.Tensor,
-                    page_size: int, status: torch.Tensor, stream=None, cos_sin: torch.Tensor | None = None) -> None:
+                    page_size: int, status: torch.Tensor, stream=None, cos_sin: torch.Tensor | None = None, weights_ahead: bool = False) -> None:
     """Per-head norm of q and k, rotation by position, q written to ``q_out`` [T, nq, d] and the
     new k, v written into their pages. ``k_pool``/``v_pool``: [pages, nkv, page_size, d], or None
-    when this entry only reads another entry's cache (then ``qkv`` holds q alone)."""
+    when this entry only reads another entry's cache (then ``qkv`` holds q alone). ``weights_ahead``: as ``add_rmsnorm``'s, for both norms."""
     _check_dev(q_out, k_pool, v_pool, qkv, q_norm_w, k_norm_w, inv_freq, positions, row_of_token, page_indptr,
                page_indices, status)
     t, nq, d = q_out.shape
@@ -423,7 +424,7 @@ def qk_norm_rope_kv(q_out: torch.Tensor, k_pool: torch.Tensor | None, v_pool: to
     assert inv_freq is None or (inv_freq.dtype == torch.float32 and inv_freq.numel() == rotary_dim // 2)
     assert cos_sin is None or (cos_sin.dtype == torch.float32 and cos_sin.shape == (t, rotary_dim) and cos_sin.is_contiguous())
     k = native.kernels()
-    native.kernel_check(k.ms_qk_norm_rope_kv(
+    native.kernel_check((k.ms_qk_norm_rope_kv_ahead if weights_ahead else k.ms_qk_norm_rope_kv)(
         _ptr(q_out), _ptr(k_pool), _ptr(v_pool), _ptr(qkv), _ptr(q_norm_w), _ptr(k_norm_w), _ptr(inv_freq),
         _ptr(cos_sin if inv_freq is not None else None), _ptr(positions), _ptr(row_of_token), _ptr(page_indptr), _ptr(page_indices), t, nq, nkv, d,
         rotary_dim if inv_freq is not None else 0, float(eps), page_size, 0 if k_pool is None else k_pool.shape[0],

@@ -96,7 +96,8 @@ def kernels():
     _declare(lib, "ms_wait_selftest", [_p, _ll, _i, _p])
     _declare(lib, "ms_fill_tokens", [_p, _p, _p, _p, _i, _p])
     _declare(lib, "ms_embed_gather", [_p, _p, _p, _i, _i, _i, _i, _p])
-    _declare(lib, "ms_add_rmsnorm", [_p, _p, _p, _p, _p, _f, _i, _i, _i, _i, _p])
+    for name in ("ms_add_rmsnorm", "ms_add_rmsnorm_ahead"):
+        _declare(lib, name, [_p, _p, _p, _p, _p, _f, _i, _i, _i, _i, _p])
     _declare(lib, "ms_gemm_skinny_gate_up_bf16", [_p, _p, _p, _i, _i, _i, _p])
     _declare(lib, "ms_gemm_skinny_bf16", [_p, _p, _p, _i, _i, _i, _i, _p])
     _declare(lib, "ms_gemm_skinny_gelu_bf16", [_p, _p, _p, _i, _i, _i, _p])
@@ -106,8 +107,9 @@ def kernels():
     _declare(lib, "ms_gemm_skinny_set_stream", [_i], None)
     _declare(lib, "ms_silu_mul", [_p, _p, _i, _i, _i, _p])
     _declare(lib, "ms_to_float", [_p, _p, _ll, _i, _p])
-    _declare(lib, "ms_qk_norm_rope_kv",
-             [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _i, _p])
+    for name in ("ms_qk_norm_rope_kv", "ms_qk_norm_rope_kv_ahead"):
+        _declare(lib, name,
+                 [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _i, _p])
     _declare(lib, "ms_rope_table", [_p, _p, _p, _i, _i, _p])
     _declare(lib, "ms_rope_table_tile", [_p, _p, _i, _p])
     _declare(lib, "ms_gemm_f32", [_p, _p, _p, _i, _i, _i, _i, _i, _i, _p])

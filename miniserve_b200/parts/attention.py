@@ -284,7 +284,7 @@ class GQAttention(Part):
                 q, cache.k if self.owns_cache else None, cache.v if self.owns_cache else None, qkv,
                 self.w_q_norm, self.w_k_norm, inv_freq, rotary_dim, self.qk_norm_eps, ctx.positions,
                 ctx.row_of_token, indptr, indices, cache.page_size, ctx.status, stream=ctx.stream,
-                cos_sin=self.position.step_table(ctx))
+                cos_sin=self.position.step_table(ctx), weights_ahead=True)
         out = ctx.buffer("attn.out", (t, self.heads, self.head_dim), dt, dev)
         ops.attention(out, q, cache.k, cache.v, ctx, cache.group, self.scale, self.window, self.sink)
         return ops.linear(out.view(t, self.heads * self.head_dim), self.w_o, stream=ctx.stream,

@@ -69,7 +69,7 @@ class RMSNorm(Part):
                                    rows=rows, num_rows=n, write_residual=write_residual, stream=ctx.stream)
             return out
         ops.add_rmsnorm(out, residual, delta, self.w_weight, self.eps, rows=rows, num_rows=n,
-                        write_residual=write_residual, stream=ctx.stream)
+                        write_residual=write_residual, stream=ctx.stream, weights_ahead=True)
         return out
 
 
