@@ -1168,14 +1168,32 @@ struct TwPlan {
   long long floats() const { return 2 * images + flags + pairs + factors + 2 * keys + added + start; }
 };
 
-// Three launches of some 25 us (one decay per head) or 30 and a chunk of 64 tokens for the shortest row, against a chain of chunks of 16. Measured on one B200,
-// tiles against chunks of 16 in us. One decay per head, 16 heads of 64 x 64 and 64 of 128 x 64: 2,048 tokens 52 / 133 and 157 / 288, 1,024 35 / 69 and 84 / 145,
-// 300 24.1 / 24.2 and 40 / 48, 200 21 / 18 and 36 / 34; 16 rows of 128 50 / 55 and 184 / 260, three of 150 27 / 21 and 62 / 72, 32 of 64 64 / 57 and 229 / 276,
-// one of 400 beside 16 of 17 46 / 37 and 148 / 130. A decay per channel, 8 heads of 64 x 128 and 32 of 128 x 128: 2,048 tokens 71 / 108 and 330 / 373, 1,024
-// 46 / 57 and 180 / 193, 700 40 / 42 and 144 / 125, 512 37 / 33 and 95 / 86; four rows of 512 60 / 60 and 325 / 347, eight of 256 59 / 61 and 341 / 348.
+// Three launches and a chunk of 64 tokens for the shortest row, against a chain of chunks of 16. Measured on one B200, 31 shapes of 2 to 128 heads, steps of 200 to
+// 4,096 tokens in 1 to 16 rows, tiles against chunks of 16 in us. Of several rows only their number is known here, not which of them is long.
+//
+// A decay per channel, one row: the time of either as a sum of what is launched, what all SMs do together and the row's chain, fitted to these steps (9 % off on the
+// mean, hence the 6 % that chunks of 16 are favoured by where heads are not few). 32 heads of 128 x 128: 300 tokens 69 / 53, 640 111 / 104, 800 121 / 131, 2,048 274 / 324; 8 of
+// 64 x 128: 640 36 / 34, 800 37 / 39, 2,048 65 / 91; 64 of 32 x 32 (half of whose channels are padding): 2,048 243 / 174. None of 136 such steps is more than an eighth slower than
+// by chunks of 16. Several rows from 640 tokens each on the mean: rows of one length lose at first (16 heads of 128 x 64, two of 650 96 / 77; 32 of 64 x 64, two of 1,024 132 / 142), one long
+// row beside short ones gains (16 of 128 x 64, 4,036 tokens and three of 20, 259 / 378).
+//
+// One decay per head, where tiles are nearly twice as fast over long rows: few heads over one row from 420 tokens, else from 300, and 96 more for every other row, whose
+// lengths may be next to nothing. 4 heads of 64 x 64: 300 tokens 21 / 18, 512 23 / 26, 2,048 34 / 82; 16 of 64 x 64: 300 24 / 18, 400 25 / 22, 512 26 / 26, 2,048 52 / 83;
+// 32 of 128 x 64: 300 34 / 34, 2,048 95 / 195; 64: 300 42 / 48, 1,024 88 / 144, 2,048 162 / 285. Several rows of few heads may lose some microseconds (16 of 64 x 64, four
+// of 160 tokens 27 / 22) for what one long row beside short ones gains (580 tokens and three of 20: 31 / 51).
+static bool tw_one_row_pays(int tokens, int H, int dk, int dv) {
+  const float p = dk <= 64 ? 1.f : 2.f, n = dk <= 32 ? 0.5f : p, chunks = tokens / 64.f + 1.f;
+  const int tiles = ceil_div(dv, TW_COLS), sms = sm_count();
+  const float units = (float)(tw_unit(tokens, H, tiles) / TW_TOK), segments = 2ll * H * tiles > sms ? 1.f : tokens / 64.f / units + 1.f;
+  const float rounds = fmaxf(1.f, segments * H * tiles / sms);
+  const float by_tiles = 21.3f + chunks * H * (0.053f * p + tiles * (0.0075f * p + 0.015f)) + tokens / 64.f * 0.42f + 1.7f * p * fminf(units, tokens / 64.f) * rounds;
+  const float by_sixteens = 7.f + (tokens / 16.f + 1.f) * H * 0.0098f * n + tokens / 16.f * (0.305f + 0.074f * n + H * dv / 64.f * (0.0114f + 0.0069f * n));
+  return (H * tiles < 8 ? 1.f : 1.06f) * by_tiles < by_sixteens;
+}
 bool tile_walk_takes(int tokens, int rows, int H, int dk, int dv, int groups) {
-  const bool longer = groups ? tokens >= 300 + 96ll * (rows - 1) : tokens >= 640ll * rows;
-  return longer && tile_walk_scratch(tokens, rows, H, dk, dv, groups) < (1ll << 28);
+  const bool few = rows == 1 && (long long)H * ceil_div(dv, TW_COLS) < 24;
+  const bool pays = groups ? tokens >= (few ? 420 : 300) + 96ll * (rows - 1) : rows == 1 ? tw_one_row_pays(tokens, H, dk, dv) : tokens >= 640ll * rows;
+  return pays && tile_walk_scratch(tokens, rows, H, dk, dv, groups) < (1ll << 28);
 }
 long long tile_walk_scratch(int tokens, int rows, int H, int dk, int dv, int groups) { return TwPlan(tokens, rows, H, dk, dv, groups).floats(); }
 

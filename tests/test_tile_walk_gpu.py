@@ -109,7 +109,7 @@ def _spread(where, gen, q, k, v, state):
             x *= torch.exp2(4 * torch.randn(x.shape, generator=gen, device=DEV))
 
 
-@pytest.mark.parametrize("rule, heads, dk, dv, t", [("decay", 3, 64, 72, 701), ("decay", 2, 128, 64, 701), ("head", 3, 128, 64, 431), ("head", 2, 32, 40, 431)])
+@pytest.mark.parametrize("rule, heads, dk, dv, t", [("decay", 3, 64, 72, 1301), ("decay", 2, 128, 64, 1301), ("head", 3, 128, 64, 431), ("head", 2, 32, 40, 431)])
 @pytest.mark.parametrize("low, high", [(0.02, 0.6), (0.9, 0.999), (0.9999, 0.99999)])
 @pytest.mark.parametrize("where", ["a value channel", "a key channel", "a query channel", "tokens", "some values", "keys against queries", "everything"])
 def test_numbers_of_very_different_sizes(rule, heads, dk, dv, t, low, high, where):
@@ -217,3 +217,25 @@ def test_copies_that_do_not_come_end_the_walk_with_an_error(dk, no_queries, no_a
         assert torch.equal(st, state)
     again = go(1 << 30, 1 << 30)
     assert torch.equal(again[0], want[0]) and torch.equal(again[1], want[1]) and again[2] == 0
+
+
+# us by chunks of 64 and of 16 on a B200: (heads, dk, dv), groups (0: a decay per channel), tokens, rows
+@pytest.mark.parametrize("shape, groups, tokens, rows, tiles", [
+    ((32, 128, 128), 0, 2048, 1, True),    # 274, 324
+    ((32, 128, 128), 0, 300, 1, False),    # 69, 53
+    ((16, 128, 128), 0, 512, 1, False),    # 54, 52
+    ((8, 64, 128), 0, 2048, 1, True),      # 65, 91
+    ((8, 64, 128), 0, 640, 1, False),      # 36, 34
+    ((16, 128, 64), 0, 640, 1, False),     # 65, 51
+    ((64, 64, 64), 0, 640, 1, False),      # 94, 83
+    ((64, 128, 128), 0, 512, 1, True),     # 147, 165
+    ((4, 64, 64), 0, 900, 1, True),        # 32, 41
+    ((64, 32, 32), 0, 2048, 1, False),     # 243, 174
+    ((64, 128, 64), 8, 300, 1, True),      # 42, 48
+    ((64, 128, 64), 8, 2048, 3, True),     # 160, 254
+    ((4, 64, 64), 1, 300, 1, False),       # 21, 18
+    ((16, 64, 64), 2, 400, 1, False),      # 25, 22
+    ((16, 64, 64), 2, 512, 1, True),       # 26, 26
+])
+def test_which_steps_go_by_chunks_of_64(shape, groups, tokens, rows, tiles):
+    assert (native.recurrence().ms_walk_kernels(tokens, rows, *shape, 0, groups) == 3) == tiles
