@@ -15,7 +15,7 @@ struct TwWaits {
 };
 
 // Whether a step goes there. It does not know its rows' lengths, only that the longest has at least their mean. (With 1 GB of scratch and more a step
-// stays on the chunks of 16.)
+// stays on the chunks of 16: the cache pool leaves as much for it.)
 bool tile_walk_takes(int tokens, int rows, int H, int dk, int dv, int groups);
 long long tile_walk_scratch(int tokens, int rows, int H, int dk, int dv, int groups);  // floats; groups: of heads that share queries and keys, 0: a decay per channel
 

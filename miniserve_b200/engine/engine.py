@@ -151,9 +151,10 @@ class Engine:
             return [want if b is None else min(want, b) for b in bound]
         free, _ = torch.cuda.mem_get_info(model.device)
         state_bytes = sum(max_running * torch.empty((), dtype=st.dtype).element_size() * _numel(st.shape) for st in states)
-        # activations of the largest step: a few [tokens, widest] buffers, and float32 logits of every row
+        # activations of the largest step: a few [tokens, widest] buffers, and float32 logits of every row; a gigabyte for the rest, and
+        # one for the scratch of recurrent layers over long rows (``csrc/tile_walk.cu`` takes no more)
         widest = max(model.spec.hidden_size * 8, 1)
-        reserve = step_tokens * widest * 4 * 4 + max_running * model.spec.vocab_size * 4 * 3 + (1 << 30)
+        reserve = step_tokens * widest * 4 * 4 + max_running * model.spec.vocab_size * 4 * 3 + (1 << 30) * (2 if states else 1)
         usable = int(fraction * (free - reserve - state_bytes))
         windowed = sum(b * pb for b, pb in zip(bound, page_bytes) if b is not None)
         whole = sum(pb for b, pb in zip(bound, page_bytes) if b is None)
