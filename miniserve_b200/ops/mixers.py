@@ -309,9 +309,9 @@ def walk_ok(q, k, v, dk: int, ctx, head_decay: bool = False, ones_column: bool =
 
 
 @lru_cache(maxsize=256)
-def _walk_plan(*sizes) -> tuple[int, int]:
+def _walk_plan(device: int | None, *sizes) -> tuple[int, int]:
     """(floats of scratch, kernels) of a walk over (tokens, rows, heads, dk, dv, delta, groups of heads that share a decay's q and k; 0: a
-    decay per key channel)."""
+    decay per key channel) on a device, whose multiprocessors decide how rows are cut."""
     lib, sizes = native.recurrence(), tuple(map(int, sizes))
     return int(lib.ms_walk_scratch(*sizes)), int(lib.ms_walk_kernels(*sizes))
 
@@ -327,7 +327,7 @@ def _decay_walk(o_out, state, q, k, v, z, z_bias, decay_coef, z_sign, beta, ctx,
     t, rows = o_out.shape[0], ctx.num_rows
     lib = native.recurrence()
     groups = q.shape[1] // dk
-    floats, kernels = _walk_plan(t, rows, heads, dk, dv, delta, groups if head_decay else 0)
+    floats, kernels = _walk_plan(o_out.device.index, t, rows, heads, dk, dv, delta, groups if head_decay else 0)
     scratch, status = ctx.buffer("walk.scratch", (floats,), torch.float32, o_out.device), _status(o_out.device)
     rest = (_ptr(v_scale), _ptr(scratch), _ptr(ctx.cu_q), _ptr(ctx.q_start), _ptr(ctx.state_slot), t, rows, heads, dk, dv, float(q_scale))
     if head_decay:
@@ -468,7 +468,7 @@ def ssm_features(out, proj, state, conv_state, w_conv, conv_bias, dt_bias, coef,
     assert conv_state is None or (conv_state.shape[1:] == (taps - 1, channels) and conv_state.dtype == proj.dtype and conv_state.is_contiguous())
     assert conv_state is not None or taps == 1
     work = ctx.buffer("ssm.work", (_ssm_floats(t, heads, dv, n, groups),), torch.float32, proj.device)
-    floats, kernels = (0, 1) if decode else _walk_plan(t, ctx.num_rows, heads, n, dv, False, groups)
+    floats, kernels = (0, 1) if decode else _walk_plan(proj.device.index, t, ctx.num_rows, heads, n, dv, False, groups)
     walk = None if decode else ctx.buffer("walk.scratch", (floats,), torch.float32, proj.device)
     native.recurrence_check(native.recurrence().ms_ssm_features(
         out.data_ptr(), _rows(out), proj.data_ptr(), _rows(proj), work.data_ptr(), _ptr(walk), state.data_ptr(), _ptr(conv_state), w_conv.data_ptr(),

@@ -1,9 +1,10 @@
-"""The cache pool leaves room for the scratch of the walks over long rows."""
+"""What the walks over long rows ask for beside their operands: the cache pool leaves room for their scratch, and a plan belongs to one device."""
 from types import SimpleNamespace
 
 import torch
 
 from miniserve_b200.engine.engine import Engine
+from miniserve_b200.ops import mixers, native
 from miniserve_b200.parts.base import FixedState, PagedKV
 from miniserve_b200.parts.decoder import EntryCache
 
@@ -28,3 +29,17 @@ def test_the_pool_leaves_room_for_the_walks_scratch(monkeypatch):
     assert recurrent - dense >= most - (1 << 20)  # (pages are whole)
     assert dense < 3 << 29  # (and a model without such layers gives up nothing)
 
+
+def test_a_plan_belongs_to_one_device(monkeypatch):
+    asked = []
+
+    def plan(*sizes):
+        asked.append(sizes)
+        return len(asked)
+
+    monkeypatch.setattr(native, "recurrence", lambda: SimpleNamespace(ms_walk_scratch=plan, ms_walk_kernels=plan))
+    mixers._walk_plan.cache_clear()
+    sizes = (2048, 1, HEADS, WIDTH, WIDTH, False, 0)
+    first, second = mixers._walk_plan(0, *sizes), mixers._walk_plan(1, *sizes)
+    assert first != second and mixers._walk_plan(0, *sizes) == first and len(asked) == 4
+    mixers._walk_plan.cache_clear()
