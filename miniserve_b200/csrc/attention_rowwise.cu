@@ -138,17 +138,17 @@ attention_rowwise_kernel(T* __restrict__ out,            // [T, nq, d]
 // 102 us (4 warps of 16 rows, one tile a step, in the order of the grid: 255), 2048 tokens 580. On the way: 8 rows a warp and two tiles a step
 // 146; softcap and distance out of the unrolled scores and the values' loop not unrolled over the tiles (instruction fetches) 124; the order
 // of the grid 102.
-constexpr int TW_ROWS = 64, TW_KEYS = 32, TW_LDS = 2 * TW_KEYS + 4;
+constexpr int AR_ROWS = 64, AR_KEYS = 32, AR_LDS = 2 * AR_KEYS + 4;
 
-__device__ __forceinline__ void tw_cp16(void* dst, const void* src, bool in) {
+__device__ __forceinline__ void ar_cp16(void* dst, const void* src, bool in) {
   const int bytes = in ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-// Folds 16 values over the lanes of a warp, all sixteen in one go: lane l comes back with the fold of v[tw_row(l)]. The pairs are those of
+// Folds 16 values over the lanes of a warp, all sixteen in one go: lane l comes back with the fold of v[ar_row(l)]. The pairs are those of
 // the exchange by 16, 8, 4, 2, 1 that folds one value (warp_sum), so the result is the same bit for bit.
 template <typename F>
-__device__ __forceinline__ float tw_fold16(float (&v)[16], F fold) {
+__device__ __forceinline__ float ar_fold16(float (&v)[16], F fold) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int n = 8; n > 0; n >>= 1) {
@@ -161,12 +161,12 @@ __device__ __forceinline__ float tw_fold16(float (&v)[16], F fold) {
   }
   return fold(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
 }
-__device__ __forceinline__ unsigned long long tw_twice(float x) {
+__device__ __forceinline__ unsigned long long ar_twice(float x) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ int tw_row(int lane) { return lane >> 1; }
+__device__ __forceinline__ int ar_row(int lane) { return lane >> 1; }
 
 template <int MD, int ROWS>  // head sizes of up to 32 MD, whole fours
 __global__ void __launch_bounds__(ROWS * 4, 128 / (ROWS * 2))
@@ -175,17 +175,17 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
                            const int* __restrict__ page_indices, int num_rows, int nq, int nkv, int d, float scale, int window, int sink,
                            int page_shift, int num_pages, int* __restrict__ status, const float* __restrict__ sink_values, float softcap, int chunk,
                            const float* __restrict__ dist_r1, const float* __restrict__ dist_r2, int keep_first, int sms) {
-  constexpr int LD = 32 * MD + 4, WARPS = ROWS / 8, MC = (MD + 1) / 2, MINE = 2 * TW_KEYS / WARPS;  // MINE: keys of a step that a warp stages
+  constexpr int LD = 32 * MD + 4, WARPS = ROWS / 8, MC = (MD + 1) / 2, MINE = 2 * AR_KEYS / WARPS;  // MINE: keys of a step that a warp stages
   static_assert(MINE <= 32);
-  extern __shared__ __align__(16) float tw_smem[];
-  float* qs = tw_smem;                  // [ROWS][LD]
+  extern __shared__ __align__(16) float ar_smem[];
+  float* qs = ar_smem;                  // [ROWS][LD]
   float* ks = qs + ROWS * LD;           // [64][LD]
-  float* vs = ks + 2 * TW_KEYS * LD;    // [64][LD] (read to column 64 MC: what lies behind a row is not stored)
-  float* ss = vs + 2 * TW_KEYS * LD;    // [ROWS][TW_LDS]
-  float* alphas = ss + ROWS * TW_LDS;   // [2][ROWS]
+  float* vs = ks + 2 * AR_KEYS * LD;    // [64][LD] (read to column 64 MC: what lies behind a row is not stored)
+  float* ss = vs + 2 * AR_KEYS * LD;    // [ROWS][AR_LDS]
+  float* alphas = ss + ROWS * AR_LDS;   // [2][ROWS]
   unsigned* seen = reinterpret_cast<unsigned*>(alphas + 2 * ROWS);  // [2][ROWS]
   __shared__ int s_row, s_tile;
-  __shared__ int usable[2][2 * TW_KEYS];
+  __shared__ int usable[2][2 * AR_KEYS];
   pdl_prologue(q, k_pool, v_pool, cu_q, q_start, page_indptr, page_indices, sink_values, dist_r1, dist_r2);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int group = nq / nkv, per_tile = ROWS / group;
@@ -242,11 +242,11 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
     if (r < rows) x = *reinterpret_cast<const float4*>(q + ((size_t)(t0 + r / group) * nq + kvh * group + r % group) * d + c);
     *reinterpret_cast<float4*>(qs + r * LD + c) = x;
   }
-  auto next_tile = [&](int tile) { return tile + TW_KEYS == kept_end ? lo_tile : tile + TW_KEYS; };
+  auto next_tile = [&](int tile) { return tile + AR_KEYS == kept_end ? lo_tile : tile + AR_KEYS; };
   // Key `lane` of the warp's own MINE (warp * MINE + lane of the step's 64): its page, asked for a step ahead, and its place in the pools;
   // negative where there is none.
   const int mine = warp * MINE + lane;
-  auto key_of = [&](int a, int b) { return (mine < TW_KEYS ? a : b - TW_KEYS) + mine; };
+  auto key_of = [&](int a, int b) { return (mine < AR_KEYS ? a : b - AR_KEYS) + mine; };
   auto page_of = [&](int a, int b) {
     const int kj = key_of(a, b);
     return lane < MINE && kj <= pos_last ? pages[kj >> page_shift] : -1;
@@ -263,7 +263,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
 #pragma unroll
     for (int j = 0; j < MINE; ++j) {
       const long long at = __shfl_sync(0xffffffffu, place, j);
-      if (c < d) tw_cp16(to + (warp * MINE + j) * LD + c, pool + (at >= 0 ? at + c : 0), at >= 0);
+      if (c < d) ar_cp16(to + (warp * MINE + j) * LD + c, pool + (at >= 0 ? at + c : 0), at >= 0);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
@@ -271,7 +271,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
   const int r0 = warp * 8;                    // the warp's rows
   const int rg = lane >> 4, kg = lane & 15;   // a lane's four rows r0 + 4 rg + i; its keys kg + 16 jj, its columns 4 kg + 64 m
   const bool second = lane >= 16;             // of the lane's fold: row r0 + own of the step's first or second tile
-  const int own = tw_row(lane) & 7;
+  const int own = ar_row(lane) & 7;
   const int row_last = min(r0 + 8, rows) - 1;
   const int see_all = pos0 + r0 / group, see_from = first_key(pos0 + row_last / group);  // keys see_from .. see_all are seen by all the warp's rows
   float m = -INFINITY, l = 0.f;               // of row r0 + own
@@ -316,7 +316,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ss[(r0 + 4 * rg + i) * TW_LDS + kg + 16 * j] = s[i][j];
+        for (int j = 0; j < 4; ++j) ss[(r0 + 4 * rg + i) * AR_LDS + kg + 16 * j] = s[i][j];
     }
     __syncthreads();  // the keys' buffer is free
     place = place_of(page, after, after2);
@@ -331,31 +331,31 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int begin = t ? tile2 : tile, kj = begin + lane;
-        const bool there = kj <= pos_last && usable[buf][t * TW_KEYS + lane];
-        float* st = ss + r0 * TW_LDS + t * TW_KEYS + lane;
+        const bool there = kj <= pos_last && usable[buf][t * AR_KEYS + lane];
+        float* st = ss + r0 * AR_LDS + t * AR_KEYS + lane;
         if (extras) {  // (by itself: beside the plain scores its instructions would be fetched past in every step)
 #pragma unroll 1
           for (int i = 0; i < 8; ++i) {
             const int r = r0 + i, h = kvh * group + r % group;
             if (r >= rows) break;
-            float x = st[i * TW_LDS] * scale;
+            float x = st[i * AR_LDS] * scale;
             if (softcap > 0.f) x = softcap * tanhf(x * inv_cap);
             if (dist_r1) x -= dist_r1[h] * logf(1.0f + dist_r2[h] * (float)(pos0 + r / group - kj));
-            st[i * TW_LDS] = x;
+            st[i * AR_LDS] = x;
           }
         }
         const float times = extras ? 1.f : scale;
-        if (begin + TW_KEYS - 1 <= see_all && begin >= see_from) {
+        if (begin + AR_KEYS - 1 <= see_all && begin >= see_from) {
           missing = missing || !there;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) sc[8 * t + i] = there ? st[i * TW_LDS] * times : -INFINITY;
+          for (int i = 0; i < 8; ++i) sc[8 * t + i] = there ? st[i * AR_LDS] * times : -INFINITY;
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int r = r0 + i, qpos = pos0 + r / group;
             const bool sees = r < rows && kj <= qpos && (kj >= first_key(qpos) || kj < keep_first);
             missing = missing || (sees && !there);
-            sc[8 * t + i] = sees && there ? st[i * TW_LDS] * times : -INFINITY;
+            sc[8 * t + i] = sees && there ? st[i * AR_LDS] * times : -INFINITY;
           }
         }
         bool all_see = true;
@@ -374,7 +374,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
       float v[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = sc[i];
-      const float top = tw_fold16(v, [](float x, float y) { return fmaxf(x, y); }), other = __shfl_xor_sync(0xffffffffu, top, 16);
+      const float top = ar_fold16(v, [](float x, float y) { return fmaxf(x, y); }), other = __shfl_xor_sync(0xffffffffu, top, 16);
       const float m_first = fmaxf(m, second ? other : top), m_second = fmaxf(m_first, second ? top : other);
       const float before = second ? m_first : m, m_new = second ? m_second : m_first;
       const float alpha = (before == -INFINITY) ? 0.f : expf(before - m_new);
@@ -382,9 +382,9 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
       for (int i = 0; i < 16; ++i) {
         const float mi = __shfl_sync(0xffffffffu, m_new, 2 * i);
         v[i] = (sc[i] == -INFINITY) ? 0.f : expf(sc[i] - mi);
-        ss[(r0 + (i & 7)) * TW_LDS + (i >> 3) * TW_KEYS + lane] = v[i];
+        ss[(r0 + (i & 7)) * AR_LDS + (i >> 3) * AR_KEYS + lane] = v[i];
       }
-      const float sum = tw_fold16(v, [](float x, float y) { return x + y; });
+      const float sum = ar_fold16(v, [](float x, float y) { return x + y; });
       const float l_first = __shfl_sync(0xffffffffu, l * alpha + sum, lane & 15);
       l = __shfl_sync(0xffffffffu, l_first * alpha + sum, lane | 16);
       m = m_second;
@@ -401,20 +401,20 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
         for (int i = 0; i < 4; ++i) {
           const int r = t * ROWS + r0 + 4 * rg + i;
           mk[i] = (hidden >> t) & 1u ? seen[r] : 0xffffffffu;
-          const unsigned long long twice = tw_twice(alphas[r]);
+          const unsigned long long twice = ar_twice(alphas[r]);
 #pragma unroll
           for (int mm = 0; mm < MC; ++mm)
 #pragma unroll
             for (int e = 0; e < 2; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][mm][e]) : "l"(twice));
         }
-        const float* pr = ss + (r0 + 4 * rg) * TW_LDS + t * TW_KEYS;
-        const float* vt = vs + t * TW_KEYS * LD + 4 * kg;
+        const float* pr = ss + (r0 + 4 * rg) * AR_LDS + t * AR_KEYS;
+        const float* vt = vs + t * AR_KEYS * LD + 4 * kg;
         auto values = [&](auto whole) {
 #pragma unroll 2
-          for (int j0 = 0; j0 < TW_KEYS; j0 += 4) {
+          for (int j0 = 0; j0 < AR_KEYS; j0 += 4) {
             float4 p[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pr + i * TW_LDS + j0);
+            for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pr + i * AR_LDS + j0);
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
               ulonglong2 v[MC];
@@ -425,7 +425,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
                 const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
                 // (a key that a row does not see may hold anything: the row's sums must not meet it)
                 if (whole.value || ((mk[i] >> (j0 + jj)) & 1u)) {
-                  const unsigned long long twice = tw_twice(pj);
+                  const unsigned long long twice = ar_twice(pj);
 #pragma unroll
                   for (int mm = 0; mm < MC; ++mm) {
                     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][mm][0]) : "l"(twice), "l"(v[mm].x));
@@ -460,7 +460,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
     }
     if (!(lane & 1)) {
       alphas[r] = a;
-      ss[r * TW_LDS] = l;
+      ss[r * AR_LDS] = l;
     }
   }
   __syncwarp();
@@ -468,7 +468,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
   for (int i = 0; i < 4; ++i) {
     const int r = r0 + 4 * rg + i;
     if (r >= rows) continue;
-    const float a = alphas[r], sum = ss[r * TW_LDS];
+    const float a = alphas[r], sum = ss[r * AR_LDS];
     float* o = out + ((size_t)(t0 + r / group) * nq + kvh * group + r % group) * d;
 #pragma unroll
     for (int mm = 0; mm < MC; ++mm) {
@@ -527,7 +527,7 @@ MS_EXPORT int ms_attention_rowwise(void* out, const void* q, const void* k_pool,
 
 // 1 if ms_attention_tiled_f32 takes these sizes: head sizes of whole fours up to 128, groups of up to 64 query heads.
 MS_EXPORT int ms_attention_tiled_f32_supports(int head_dim, int nq, int nkv) {
-  return head_dim >= 4 && head_dim <= 128 && head_dim % 4 == 0 && nkv > 0 && nq % nkv == 0 && nq / nkv <= TW_ROWS && nkv <= 65535;
+  return head_dim >= 4 && head_dim <= 128 && head_dim % 4 == 0 && nkv > 0 && nq % nkv == 0 && nq / nkv <= AR_ROWS && nkv <= 65535;
 }
 
 // ms_attention_rowwise for float32 and a step of whole rows: cu_q [rows + 1], q_start [rows]. The same results, bit for bit.
@@ -548,7 +548,7 @@ MS_EXPORT int ms_attention_tiled_f32(float* out, const float* q, const float* k_
 #define MS_TILED_LAUNCH(MD, ROWS)                                                                                                               \
   do {                                                                                                                                          \
     auto kernel = attention_tiled_f32_kernel<MD, ROWS>;                                                                                         \
-    constexpr size_t smem = ((ROWS + 4 * TW_KEYS) * (32 * MD + 4) + ROWS * TW_LDS + 4 * ROWS) * 4;                                              \
+    constexpr size_t smem = ((ROWS + 4 * AR_KEYS) * (32 * MD + 4) + ROWS * AR_LDS + 4 * ROWS) * 4;                                              \
     static std::atomic<unsigned long long> allowed{0};                                                                                          \
     MS_CHECK_CUDA(allow_shared_memory((const void*)kernel, (int)smem, allowed));                                                                \
     const long long grid = ((long long)num_tokens / (ROWS / (nq / nkv)) + num_rows) * nkv;                                                      \

@@ -42,8 +42,6 @@ constexpr int WK_TOK = 16, WK_THREADS = 128, WK_COLS = 16;  // (WK_THREADS: of t
 constexpr int WK_CHAIN = 2, WK_OUT = 4, WK_FETCH = 2, WK_OWN = 8;  // warps of the walk's chain, of its outputs, of its copies; an output warp's tokens
 enum WalkMode : int { WALK_CHANNEL = 0, WALK_DELTA = 1, WALK_HEAD = 2 };
 
-__device__ __forceinline__ float wk_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
-
 // ---------------------------------------------------------------- the chunks of a step
 // A row of n tokens has ceil(n / 16) chunks, numbered row by row. Every warp finds its own by adding up over the rows, 32 at a time: a table
 // made by a launch of its own costs a small step more on the host (4 us) than these sums cost on the device.
@@ -77,21 +75,6 @@ __device__ __forceinline__ int wk_first(int row, const int* __restrict__ cu_q) {
   return __reduce_add_sync(0xffffffffu, sum);
 }
 
-template <typename T>
-__device__ __forceinline__ float4 wk_load4(const T* p) {
-  if constexpr (sizeof(T) == 4) {
-    return *reinterpret_cast<const float4*>(p);
-  } else {
-    const uint2 r = *reinterpret_cast<const uint2*>(p);
-    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
-  }
-}
-// whether rows `ld` apart of T in fours start where four are one load
-template <typename T>
-__device__ __forceinline__ bool wk_fours(const T* p, int ld) {
-  return (reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T))) == 0 && ld % 4 == 0;
-}
-
 // ---------------------------------------------------------------- what a chunk needs beside the state (a decay per key channel)
 // grid (chunks, H). W, q', k' [chunks, H, 16, dkp] and last [chunks, H, dkp] float32 (dkp = 32 N >= dk, zeros behind dk), u0
 // [chunks, H, 16, dvp] (dvp: dv in whole sixteens, zeros behind; without the delta rule v itself), pairs = P [chunks, H, 16, 16]. z: the
@@ -123,8 +106,8 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t qk_at = (size_t)(h / qk_group) * dk;
   const float coef = decay_coef[h];
-  auto decay = [&](float logit, int c) { return expf(-coef * wk_softplus(z_sign * (logit + z_bias[(size_t)h * dk + c]))); };
-  if (dk % 4 == 0 && wk_fours(q, ld_q) && wk_fours(k, ld_k) && wk_fours(z, ld_z)) {
+  auto decay = [&](float logit, int c) { return expf(-coef * softplusf(z_sign * (logit + z_bias[(size_t)h * dk + c]))); };
+  if (dk % 4 == 0 && in_fours(q, ld_q) && in_fours(k, ld_k) && in_fours(z, ld_z)) {
     constexpr int EACH = WK_TOK * DKP / 4 / WK_THREADS, AT_ONCE = EACH < 2 ? EACH : 2;
 #pragma unroll 1
     for (int e0 = 0; e0 < EACH; e0 += AT_ONCE) {
@@ -135,9 +118,9 @@ walk_prepare_kernel(float* __restrict__ w_out, float* __restrict__ q_out, float*
         const bool in = i < n && c < dk;
         const size_t t = in ? (size_t)(t0 + i) : (size_t)t0;
         const int cc = in ? c : 0;
-        fq[e] = wk_load4(q + t * ld_q + qk_at + cc);
-        fk[e] = wk_load4(k + t * ld_k + qk_at + cc);
-        fd[e] = wk_load4(z + t * ld_z + (size_t)h * dk + cc);
+        fq[e] = load4(q + t * ld_q + qk_at + cc);
+        fk[e] = load4(k + t * ld_k + qk_at + cc);
+        fd[e] = load4(z + t * ld_z + (size_t)h * dk + cc);
       }
 #pragma unroll
       for (int e = 0; e < AT_ONCE; ++e) {

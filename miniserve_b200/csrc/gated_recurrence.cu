@@ -17,12 +17,12 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "float_pairs.cuh"
 
 namespace ms {
 
 namespace cg = cooperative_groups;
 
-__device__ __forceinline__ float softplus_of(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 __device__ __forceinline__ float sigmoid_of(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float gelu_tanh_of(float z) { return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
 
@@ -47,7 +47,7 @@ mlstm_gates_kernel(float* __restrict__ decay, float* __restrict__ write, float* 
   auto gates = [&](int t, float& i, float& f) {
     const T* p = raw + (size_t)(t0 + t) * ld;
     i = cap * tanhf((Elem<T>::load(p + h) + bi) * inv_cap);
-    f = -softplus_of(-cap * tanhf((Elem<T>::load(p + H + h) + bf) * inv_cap));
+    f = -softplusf(-cap * tanhf((Elem<T>::load(p + H + h) + bf) * inv_cap));
   };
   float F = 0.f, M = -INFINITY;
   for (int t = a; t < b; ++t) {

@@ -22,6 +22,7 @@
 // sign = -1, c_h = 1/tau gives sigmoid(z + bias)^(1/tau); sign = +1, c_h = exp(A_h) gives
 // exp(-exp(A_h) softplus(z + bias)).
 #include "common.cuh"
+#include "float_pairs.cuh"
 
 namespace ms {
 
@@ -38,7 +39,6 @@ inline int scan_sm_count() {
   return sm_count;
 }
 
-__device__ __forceinline__ float softplusf(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 __device__ __forceinline__ float decay_of(float z, float coef, float sign) { return expf(-coef * softplusf(sign * z)); }
 
 // decay[t, h * dk + i] = exp(-c_h softplus(sign (z[t, h * dk + i] + bias[h * dk + i]))) for every token of a step,
@@ -462,20 +462,7 @@ __global__ void conv_silu_unit_kernel(float* __restrict__ out, const T* __restri
   for (int c = lane; c < size; c += 32) out[(size_t)t * C + base + c] *= inv;
 }
 
-// four consecutive elements as float32 (an address that is a multiple of their size), and back
-__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
-  const uint2 v = *reinterpret_cast<const uint2*>(p);
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
-  return make_float4(a.x, a.y, b.x, b.y);
-}
-__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-// the same as they lie in memory, and made float32 where they are used
-template <typename T> struct Four { using raw = float4; };
-template <> struct Four<__nv_bfloat16> { using raw = uint2; };
-__device__ __forceinline__ float4 float4_of(const float4& r) { return r; }
-__device__ __forceinline__ float4 float4_of(const uint2& r) {
-  return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
-}
+// four elements from float32 (load4's way back)
 __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& f) {
   uint2 v;
   *reinterpret_cast<__nv_bfloat162*>(&v.x) = __floats2bfloat162_rn(f.x, f.y);

@@ -42,8 +42,6 @@ constexpr int TW_FIRST = 256, TW_WORKERS = 512, TW_THREADS = TW_WORKERS + 32, TW
 constexpr int TW_BLOCK = TW_SUB * TW_SUB, TW_DIAGONAL = 6 * TW_BLOCK;
 enum TileWalkMode : int { TW_CHANNEL = 0, TW_HEAD = 1 };
 
-__device__ __forceinline__ float tw_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
-
 // ---------------------------------------------------------------- pieces of a step's rows
 // A row of n tokens has ceil(n / tokens) pieces, numbered row by row. Every warp finds its own by adding up over the rows, 32 at a time.
 struct TwPiece {
@@ -250,20 +248,6 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
 // end, which make the pairs of different sixteens, the keys decayed on over the sixteens between them. Bound by a CTA's chain (two or three a
 // multiprocessor, 30 % of the issue slots): 2,048 tokens of 8 heads of 64 channels 22.7 us; 27.0 with the operands read one by one, four in flight, and
 // q' and k' read back from global memory for their images.
-template <typename T>
-__device__ __forceinline__ float4 tw_load4(const T* p) {
-  if constexpr (sizeof(T) == 4) {
-    return *reinterpret_cast<const float4*>(p);
-  } else {
-    const uint2 r = *reinterpret_cast<const uint2*>(p);
-    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
-  }
-}
-// whether rows `ld` apart of T in fours start where four are one load
-template <typename T>
-__device__ __forceinline__ bool tw_fours(const T* p, int ld) {
-  return (reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T))) == 0 && ld % 4 == 0;
-}
 template <typename TIn, typename TZ, int N>
 __global__ void __launch_bounds__(TW_FIRST, 2)
 tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, uint8_t* __restrict__ k_image, int* __restrict__ plain,
@@ -285,8 +269,8 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
   const int t0 = at.first, n = min(TW_TOK, at.end - t0);
   const size_t qk_at = (size_t)(h / qk_group) * dk, item = (size_t)at.chunk * H + h;
   const float coef = decay_coef[h];
-  auto decay = [&](float logit, int c) { return expf(-coef * tw_softplus(z_sign * (logit + z_bias[(size_t)h * dk + c]))); };
-  if (dk % 4 == 0 && tw_fours(q, ld_q) && tw_fours(k, ld_k) && tw_fours(z, ld_z)) {
+  auto decay = [&](float logit, int c) { return expf(-coef * softplusf(z_sign * (logit + z_bias[(size_t)h * dk + c]))); };
+  if (dk % 4 == 0 && in_fours(q, ld_q) && in_fours(k, ld_k) && in_fours(z, ld_z)) {
     constexpr int EACH = TW_TOK * DKP / 4 / TW_FIRST, AT_ONCE = EACH < 4 ? EACH : 4;
 #pragma unroll 1
     for (int e0 = 0; e0 < EACH; e0 += AT_ONCE) {
@@ -297,9 +281,9 @@ tile_prepare_kernel(float* q_out, float* k_out, uint8_t* __restrict__ q_image, u
         const bool in = i < n && c < dk;
         const size_t t = in ? (size_t)(t0 + i) : (size_t)t0;
         const int cc = in ? c : 0;
-        fq[e] = tw_load4(q + t * ld_q + qk_at + cc);
-        fk[e] = tw_load4(k + t * ld_k + qk_at + cc);
-        fd[e] = tw_load4(z + t * ld_z + (size_t)h * dk + cc);
+        fq[e] = load4(q + t * ld_q + qk_at + cc);
+        fk[e] = load4(k + t * ld_k + qk_at + cc);
+        fd[e] = load4(z + t * ld_z + (size_t)h * dk + cc);
       }
 #pragma unroll
       for (int e = 0; e < AT_ONCE; ++e) {
