@@ -86,7 +86,7 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
   using I = GfTile<BM, BN, TM, TN, GK>;
   constexpr int THREADS = I::threads, PA = BM * GK / 4, PW = BN * GK / 4, LA = (PA + THREADS - 1) / THREADS, LW = (PW + THREADS - 1) / THREADS;  // pieces of 16 bytes
   __shared__ __align__(16) float as[2][GK][BM + 4], ws[2][GK][BN + 4];
-  pdl_prologue(A, W);
+  pdl_prologue();
   const int tid = threadIdx.x, tx = tid % I::tx, ty = tid / I::tx;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   A += blockIdx.z * stride_a;
@@ -103,13 +103,14 @@ gemm_f32_tiled_kernel(float* __restrict__ C, const float* __restrict__ A, const 
   auto load = [&](int k0) {
     if (k0 + GK <= K) {
 #pragma unroll
-      for (int i = 0; i < LA; ++i) ra[i] = *reinterpret_cast<const float4*>(ap[i] + k0);
+      for (int i = 0; i < LA; ++i) ra[i] = behind_loadf4(ap[i] + k0);
 #pragma unroll
-      for (int i = 0; i < LW; ++i) rw[i] = *reinterpret_cast<const float4*>(wp[i] + k0);
+      for (int i = 0; i < LW; ++i) rw[i] = behind_loadf4(wp[i] + k0);
     } else {  // zeros behind the last k: fma(0, 0, x) is x
       auto piece = [&](const float* p) {
         const int k = k0 + pk;
-        return make_float4(k < K ? p[k0] : 0.f, k + 1 < K ? p[k0 + 1] : 0.f, k + 2 < K ? p[k0 + 2] : 0.f, k + 3 < K ? p[k0 + 3] : 0.f);
+        return make_float4(k < K ? behind_load(p + k0) : 0.f, k + 1 < K ? behind_load(p + k0 + 1) : 0.f, k + 2 < K ? behind_load(p + k0 + 2) : 0.f,
+                           k + 3 < K ? behind_load(p + k0 + 3) : 0.f);
       };
 #pragma unroll
       for (int i = 0; i < LA; ++i) ra[i] = piece(ap[i]);
