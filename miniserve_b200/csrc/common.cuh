@@ -136,6 +136,11 @@ __device__ __forceinline__ float behind_load(const float* p) {
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ float behind_load(const __nv_bfloat16* p) {
+  unsigned short v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return __uint_as_float((unsigned)v << 16);
+}
 __device__ __forceinline__ int behind_load(const int* p) {
   int v;
   asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));

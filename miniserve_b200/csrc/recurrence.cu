@@ -947,14 +947,15 @@ namespace ms {
 template <typename T>
 __global__ void ssm_step_decay_kernel(float* __restrict__ out, const T* __restrict__ raw, int ld, const float* __restrict__ bias,
                                       const float* __restrict__ coef, long long items, int H) {
-  pdl_prologue(raw, bias, coef);
+  pdl_prologue();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= items) return;
   const long long t = idx / H;
   const int h = (int)(idx - t * H);
-  const float dt = softplusf(Elem<T>::load(raw + t * ld + h) + bias[h]);
+  const float x = behind_load(raw + t * ld + h), b = behind_load(bias + h), c = behind_load(coef + h);
+  const float dt = softplusf(x + b);
   out[idx] = dt;
-  out[items + idx] = expf(-coef[h] * dt);
+  out[items + idx] = expf(-c * dt);
 }
 
 // y[c] = (o[t, c] + skip[c / dv] * x[t, c]) * silu(gate[t, c]); out[t, c] = y[c] / sqrt(mean over c's part of y^2 + eps) * w[c],
