@@ -233,7 +233,7 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
     if (chunk > 0) lo = max(lo, (pos / chunk) * chunk);
     return lo;
   };
-  const int lo_tile = (first_key(pos0) >> 5) << 5;  // (the first token's window begins first)
+  const int see_first = first_key(pos0), lo_tile = (see_first >> 5) << 5;  // (the first token's window begins first)
   const int kept_end = keep_first > 0 ? min((keep_first + 31) & ~31, lo_tile) : 0;
   const int vec = d / 4;
   for (int idx = tid; idx < ROWS * vec; idx += ROWS * 4) {
@@ -244,12 +244,13 @@ attention_tiled_f32_kernel(float* __restrict__ out, const float* __restrict__ q,
   }
   auto next_tile = [&](int tile) { return tile + AR_KEYS == kept_end ? lo_tile : tile + AR_KEYS; };
   // Key `lane` of the warp's own MINE (warp * MINE + lane of the step's 64): its page, asked for a step ahead, and its place in the pools;
-  // negative where there is none.
+  // negative where there is none. Keys of the first tile that lie ahead of the first token's window are not looked up: the table begins with the page ahead of
+  // the window's first, and a tile may begin further back.
   const int mine = warp * MINE + lane;
   auto key_of = [&](int a, int b) { return (mine < AR_KEYS ? a : b - AR_KEYS) + mine; };
   auto page_of = [&](int a, int b) {
     const int kj = key_of(a, b);
-    return lane < MINE && kj <= pos_last ? pages[kj >> page_shift] : -1;
+    return lane < MINE && kj <= pos_last && (kj >= see_first || kj < keep_first) ? pages[kj >> page_shift] : -1;
   };
   auto place_of = [&](int page, int a, int b) -> long long {
     MS_DEBUG_ONLY(if (page >= num_pages) {
