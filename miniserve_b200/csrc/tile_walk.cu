@@ -18,13 +18,14 @@
 // pairs of one sixteen tokens and what a chunk's last eight tokens add to the state are float32 multiply-adds, and the sums of the rest are short. Products of
 // decays are worked out in 64 bits and rounded once (a running product of decays just below one is rounded down every time). A state is rounded twice in 64 tokens.
 // Root mean squares of the errors over 1,400 and 2,088 tokens, against the token-by-token walk's and the chunks of 16's, decays from 0.02 to 0.99999: outputs 0.28 to 0.96
-// and 0.36 to 1.07, states 0.13 to 1.02 and 0.25 to 1.00. With one channel, token or number in a hundred 1,024 to 16,384 times the others, or keys by 2^s and queries by 2^-s
+// and 0.36 to 1.00, states 0.13 to 1.02 and 0.25 to 1.00. With one channel, token or number in a hundred 1,024 to 16,384 times the others, or keys by 2^s and queries by 2^-s
 // (s from -12 to 12): outputs 0.27 to 1.1 of either, with exact decays none off by more than 8e-7 of its terms' sizes. A token sees nothing of the tokens behind it, whatever they hold:
 // chunks with values that are not finite, or of 2^48 and more, are worked out in plain sums, every pair by itself. (With one decay per head the
 // sums against the state are scaled behind the sum: a state within q's size of the largest float overflows.)
 //
-// What bounds it, 64 heads of 128 x 64, three rows of 1,037, 640 and 371 tokens, 263 us by chunks of 16 and 169 here: the second kernel (91 us) issues its instructions at
-// half the rate, most of them making operands and adding up results; the third (54) is a chain of 17 chunks, bound by shared memory and the state's parts; the first 23.
+// What bounds it, 64 heads of 128 x 64, three rows of 1,037, 640 and 371 tokens, 263 us by chunks of 16 and 170 here: the second kernel (91 us) issues its instructions at
+// half the rate, most of them making operands and adding up results; the third (54) is a chain of 17 chunks, bound by shared memory and the state's parts; the first 24.6 (long scoreboard, 28 % of the issue slots; 23.6
+// with sums of eight products everywhere, and outputs under fast decays 1.07 times as far off as by chunks of 16, 26.8 with sums of four everywhere).
 // Measured and not kept: the same products in float32 multiply-adds, 8 x 8 outputs a thread (332 us: both shared memory and the FMA pipe at 54 %); all three kernels' work
 // on the chain (322); parts on a grid that a row shares, whose products add up without any cut (165, but a row's small numbers lose the bits that its largest takes: one
 // value channel of 1,024 made outputs 28 times as far off).
@@ -168,7 +169,7 @@ __device__ __forceinline__ bool tw_images(uint8_t* q_to, uint8_t* k_to, const fl
 
 // ---------------------------------------------------------------- one decay per head: operands and dot products
 // grid (chunks, groups of heads that share q and k). A thread's 4 x 4 dot products (tokens wb * 16 + ty + 4 a against 32 half + tx + 8 b), sums of
-// eight products, added up in 64 bits: however much smaller than others a token's numbers are, its pairs are as precise.
+// four (on the diagonal) or sixteen products, added up in 64 bits: however much smaller than others a token's numbers are, its pairs are as precise.
 template <int DK>
 __global__ void __launch_bounds__(TW_FIRST, 2)
 tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_t* __restrict__ k_image, int* __restrict__ plain, const float* __restrict__ q,
@@ -202,17 +203,18 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
   }
   const int wb = warp < 4 ? warp : 7 - warp, half = warp >> 2, ty = lane >> 3, tx = lane & 7;
   if (half != 0 && wb < 2) return;
+  const int flip = (wb & 1) << 1;  // the thread's columns 8 (y ^ flip) on: those of y < 2 are the block on the diagonal, if the warp has one
   double sum[4][4] = {};
 #pragma unroll 1
-  for (int c0 = 0; c0 < DK; c0 += 8) {
+  for (int c0 = 0; c0 < DK; c0 += 16) {
     f2 part[4][4] = {};
 #pragma unroll
-    for (int c = 0; c < 8; c += 4) {
+    for (int c = 0; c < 16; c += 4) {
       ulonglong2 a[4], b[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         a[e] = *reinterpret_cast<const ulonglong2*>(qs + (wb * TW_SUB + ty + 4 * e) * LD + c0 + c);
-        b[e] = *reinterpret_cast<const ulonglong2*>(ks + (half * 32 + tx + 8 * e) * LD + c0 + c);
+        b[e] = *reinterpret_cast<const ulonglong2*>(ks + (half * 32 + tx + 8 * (e ^ flip)) * LD + c0 + c);
       }
 #pragma unroll
       for (int x = 0; x < 4; ++x)
@@ -220,18 +222,26 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
         for (int y = 0; y < 4; ++y) {
           f2_fma(part[x][y], a[x].x, b[y].x);
           f2_fma(part[x][y], a[x].y, b[y].y);
+          if (c == 4 && y < 2) {
+            const float2 h = f2_halves(part[x][y]);
+            sum[x][y] += (double)h.x + (double)h.y;
+            part[x][y] = 0ull;
+          }
         }
     }
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int y = 0; y < 4; ++y) sum[x][y] += (double)f2_sum(part[x][y]);
+      for (int y = 0; y < 4; ++y) {
+        const float2 h = f2_halves(part[x][y]);
+        sum[x][y] += y < 2 ? (double)h.x + (double)h.y : (double)(h.x + h.y);
+      }
   }
   float* to = dots + image * tw_pairs(true);
   double* diagonal = reinterpret_cast<double*>(to + TW_DIAGONAL) + wb * TW_BLOCK;
 #pragma unroll
   for (int y = 0; y < 4; ++y) {
-    const int j = half * 32 + tx + 8 * y;
+    const int j = half * 32 + tx + 8 * (y ^ flip);
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       const int at = (ty + 4 * x) * TW_SUB + (j & 15);
