@@ -326,11 +326,11 @@ __device__ __forceinline__ int at_tile(AtItem& it, int r, int tile, const AtGrid
   const int tpc = AT_ROWS / gr.G;  // tokens per group
   it.r = r;
   it.tile = tile;
-  it.tok0 = cu_q[r];
-  it.q_len = cu_q[r + 1] - it.tok0;
+  it.tok0 = behind_load(cu_q + r);
+  it.q_len = behind_load(cu_q + r + 1) - it.tok0;
   it.m0 = tile * 2 * tpc;
   if (tile < 0 || it.m0 >= it.q_len) return 0;
-  it.start = q_start[r];
+  it.start = behind_load(q_start + r);
   it.kv_len = it.start + it.q_len;
   // per group: the key tiles it needs (B needs at least as many as A; B may have no rows at all)
   it.has_b = it.m0 + tpc < it.q_len;
@@ -390,7 +390,7 @@ __device__ __forceinline__ AtOrder at_order(const AtGrid& gr, const int* __restr
   const int span = 2 * (AT_ROWS / gr.G);
   int last = 0, first = INT_MAX, latest = 0;
   for (int r = lane; r < gr.rows; r += 32) {
-    const int len = cu_q[r + 1] - cu_q[r], start = q_start[r];
+    const int len = behind_load(cu_q + r + 1) - behind_load(cu_q + r), start = behind_load(q_start + r);
     if (len > 0) {
       last = max(last, start + (len + span - 1) / span * span);
       first = min(first, start);
@@ -447,7 +447,7 @@ __device__ __forceinline__ bool at_claim(AtItem& item, AtCursor& at, int* __rest
       if (entry < 2 * order.pairs) {
         const int rank = pair / gr.rows;
         r = pair - rank * gr.rows;
-        const int before = order.pos_max - rank * span - q_start[r];
+        const int before = order.pos_max - rank * span - behind_load(q_start + r);
         tile = before > 0 ? before / span - 1 : -1;
         const int n_full = at_tile(item, r, tile, gr, cu_q, q_start);
         if (n_full > 0) {
@@ -531,17 +531,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncthreads();
   AT_FENCE_AFTER();
   const uint32_t tmem = tmem_slot;
-  pdl_wait(cu_q, q_start, page_indptr, page_indices, plan);
+  pdl_wait();  // (what follows reads the step's metadata by loads that stay behind it)
 
   // A launch that was captured into a CUDA graph takes what follows from the rows' lengths (tiles per
   // row, rows, key splits) from device memory, where the host puts it before every replay: the
   // launch itself (a CTA per SM, these arguments) is then the same for every step of its size.
   AtGrid gr = gr_given;
   if (plan != nullptr) {
-    gr.q_tiles = plan[0];
-    gr.rows = plan[1];
-    gr.splits = plan[2];
-    gr.max_tiles_per_item = plan[3];
+    gr.q_tiles = behind_load(plan + 0);
+    gr.rows = behind_load(plan + 1);
+    gr.splits = behind_load(plan + 2);
+    gr.max_tiles_per_item = behind_load(plan + 3);
     part_ml = reinterpret_cast<float2*>(part_o + (size_t)gr.q_tiles * gr.rows * gr.head_groups * 2 * gr.splits * (AT_ROWS * AT_D));
   }
   const int G = gr.G, window = gr.window;
@@ -581,7 +581,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
         __syncwarp();
         if (!alive) break;
-        const int* pages = page_indices + page_indptr[it.r];
+        const int* pages = page_indices + behind_load(page_indptr + it.r);
         const int kv_len = it.kv_len, head0 = it.head0, kvh = head0 / (nq / nkv), n_all = it.n_all;
         auto load_q = [&](int g) {
           if (it.n_tiles[g] == 0 || !wait_free(&q_empty[g], queries[g])) return;
@@ -600,7 +600,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           int group8 = 0;  // where this lane's keys begin, in groups of 8 rows of the pool
           if (lane < boxes) {
             const int key = key0 + lane * box_rows;
-            const int page = pages[key >> page_shift];
+            const int page = behind_load(pages + (key >> page_shift));
             group8 = ((max(page, 0) * nkv + kvh) * page_size + (key & (page_size - 1))) >> 3;
           }
           const uint32_t bytes = (uint32_t)boxes * box_rows * (AT_D * 2);

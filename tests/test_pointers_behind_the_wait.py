@@ -11,7 +11,9 @@ SOURCES = sorted((Path(__file__).resolve().parent.parent / "miniserve_b200" / "c
 AHEAD = {"gemm_skinny_kernel": {"W"}, "gemm_skinny_stream_kernel": {"W"}, "qk_norm_rope_kv_bf16_token_kernel": {"q_norm_w", "k_norm_w"},
          "attn_decode_kernel": {"k_pool", "v_pool", "kv_len_ptr", "page_indptr", "page_indices"}}
 # Read through pointers made of them, whose loads are all written out: (the parameter, what is made of it)
-MADE = {"gemm_f32_tiled_kernel": {"A": "ap", "W": "wp"}}
+MADE = {"gemm_f32_tiled_kernel": {"A": "ap", "W": "wp"}, "attn_prefill_tc_kernel": {"page_indices": "pages"}}
+# Handed on to functions that read them by loads that are written out
+HANDED_ON = {"attn_prefill_tc_kernel": ({"cu_q", "q_start"}, {"at_tile", "at_order", "at_claim"})}
 
 
 def _closing(text, at, left, right):
@@ -48,7 +50,8 @@ def kernels(text):
 
 @pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
 def test_pointers_go_through_the_wait(path):
-    for name, params, body in kernels(re.sub(r"//[^\n]*", "", path.read_text())):
+    text = re.sub(r"//[^\n]*", "", path.read_text())
+    for name, params, body in kernels(text):
         waits = re.findall(r"pdl_(?:prologue|wait)\(([^)]*)\)", body)
         if not waits:
             continue  # launched behind everything before it
@@ -56,8 +59,14 @@ def test_pointers_go_through_the_wait(path):
         read_only = {re.search(r"(\w+)\s*$", p).group(1) for p in params if re.search(r"\bconst\b.*__restrict__", p)}
         for pointer, made in MADE.get(name, {}).items():
             assert not re.search(r"reinterpret_cast<[^>]*>\(%s\b|\*%s\b" % (made, made), body.replace("*" + made + "[LA]", "").replace("*" + made + "[LW]", ""))
+            assert made + "[" not in body.replace(made + "[LA]", "").replace(made + "[LW]", "").replace(made + "[i]", "")
             passed.add(pointer)
+        pointers, functions = HANDED_ON.get(name, ((), ()))
+        for function in functions:
+            begin = text.index("{", _closing(text, text.index(function + "("), "(", ")"))
+            assert not re.search(r"\b(%s)\[" % "|".join(pointers), text[begin:_closing(text, begin, "{", "}")]), function
+        passed |= set(pointers)
         for pointer in read_only - passed - AHEAD.get(name, set()):
-            rest = re.sub(r"behind_load\w*\(\s*%s\b" % pointer, "", body)
+            rest = re.sub(r"behind_load\w*\(\s*%s\b|\b%s != nullptr" % (pointer, pointer), "", body)
             uses = [u for u in re.findall(r"[^;{}]*\b%s\b[^;{}]*" % pointer, rest) if not re.fullmatch(r"\s*(?:if \([^;]*\) )?%s \+= [^;]*" % pointer, u)]
             assert not uses, (name, pointer, uses)
