@@ -600,7 +600,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           int group8 = 0;  // where this lane's keys begin, in groups of 8 rows of the pool
           if (lane < boxes) {
             const int key = key0 + lane * box_rows;
-            const int page = behind_load(pages + (key >> page_shift));
+            // (keys that every row's window has passed are not looked up: the table begins with the page ahead of the window's first)
+            const int page = key + box_rows > it.lo_g[0] || key < gr.keep ? behind_load(pages + (key >> page_shift)) : 0;
             group8 = ((max(page, 0) * nkv + kvh) * page_size + (key & (page_size - 1))) >> 3;
           }
           const uint32_t bytes = (uint32_t)boxes * box_rows * (AT_D * 2);
