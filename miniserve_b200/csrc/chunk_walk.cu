@@ -589,7 +589,7 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
   __shared__ __align__(16) float qs[WK_TOK][DK + 4], ks[WK_TOK][DK + 4];
   __shared__ double dot[WK_TOK][WK_TOK + 1];
   __shared__ float as[WK_TOK][33];
-  pdl_prologue(q, k, decay, cu_q);
+  pdl_prologue(decay, cu_q);
   const int chunk = blockIdx.x, grp = blockIdx.y;
   const int2 at = wk_at(chunk, cu_q, num_rows);
   if (at.x < 0) return;
@@ -600,8 +600,8 @@ walk_head_kernel(float* __restrict__ pairs, float* __restrict__ decays, const fl
     const int idx = e * WK_THREADS + tid, i = idx / (DK / 4), c = (idx % (DK / 4)) * 4;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     if (i < n) {
-      a = *reinterpret_cast<const float4*>(q + (size_t)(t0 + i) * ld_q + (size_t)grp * DK + c);
-      b = *reinterpret_cast<const float4*>(k + (size_t)(t0 + i) * ld_k + (size_t)grp * DK + c);
+      a = behind_loadf4(q + (size_t)(t0 + i) * ld_q + (size_t)grp * DK + c);
+      b = behind_loadf4(k + (size_t)(t0 + i) * ld_k + (size_t)grp * DK + c);
     }
     *reinterpret_cast<float4*>(&qs[i][c]) = a;
     *reinterpret_cast<float4*>(&ks[i][c]) = b;

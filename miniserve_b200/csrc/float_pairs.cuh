@@ -36,6 +36,13 @@ __device__ __forceinline__ float4 float4_of(const uint2& r) {
 }
 template <typename T>
 __device__ __forceinline__ float4 load4(const T* p) { return float4_of(*reinterpret_cast<const typename Four<T>::raw*>(p)); }
+// as they lie in memory, behind the wait on the kernels before (common.cuh)
+__device__ __forceinline__ float4 behind_four(const float* p) { return behind_loadf4(p); }
+__device__ __forceinline__ uint2 behind_four(const __nv_bfloat16* p) {
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
 // whether rows `ld` apart of T in fours start where four are one load
 template <typename T>
 __device__ __forceinline__ bool in_fours(const T* p, int ld) {

@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(GGN_THREADS)
 gated_group_norm_x4_kernel(T* __restrict__ out, int ld_out, const float* __restrict__ o, const float* __restrict__ x, int ld_x,
                            const float* __restrict__ skip, const T* __restrict__ gate, int ld_gate, const float* __restrict__ w, int num_items,
                            int width, int parts, int dv, float eps) {
-  pdl_prologue(o, x, skip, gate, w);
+  pdl_prologue();
   const int item = blockIdx.x * (GGN_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (item >= num_items) return;
   const int t = item / parts, part = item - t * parts, size = width / parts, base = part * size;
@@ -1014,11 +1014,11 @@ gated_group_norm_x4_kernel(T* __restrict__ out, int ld_out, const float* __restr
     gr[i] = {};
     sv[i] = 0.f;
     if (c < size) {
-      gr[i] = *reinterpret_cast<const typename Four<T>::raw*>(gate + (size_t)t * ld_gate + ch);
-      y[i] = load4(o + (size_t)t * width + ch);
+      gr[i] = behind_four(gate + (size_t)t * ld_gate + ch);
+      y[i] = behind_loadf4(o + (size_t)t * width + ch);
       if (skip) {
-        xv[i] = load4(x + (size_t)t * ld_x + ch);
-        sv[i] = skip[ch / dv];
+        xv[i] = behind_loadf4(x + (size_t)t * ld_x + ch);
+        sv[i] = behind_load(skip + ch / dv);
       }
     }
   }
@@ -1037,13 +1037,16 @@ gated_group_norm_x4_kernel(T* __restrict__ out, int ld_out, const float* __restr
     }
     ss += (y[i].x * y[i].x + y[i].y * y[i].y) + (y[i].z * y[i].z + y[i].w * y[i].w);
   }
+#pragma unroll
+  for (int i = 0; i < ITER; ++i)  // (the weights, on their way while the sum is made)
+    if ((i * 32 + lane) * 4 < size) xv[i] = behind_loadf4(w + base + (i * 32 + lane) * 4);
   ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)size + eps);
 #pragma unroll
   for (int i = 0; i < ITER; ++i) {
     const int c = (i * 32 + lane) * 4, ch = base + c;
     if (c < size) {
-      const float4 wv = load4(w + ch);
+      const float4 wv = xv[i];
       store4(out + (size_t)t * ld_out + ch, make_float4((y[i].x * inv) * wv.x, (y[i].y * inv) * wv.y, (y[i].z * inv) * wv.z, (y[i].w * inv) * wv.w));
     }
   }

@@ -177,7 +177,7 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
   constexpr int LD = DK + 4;
   extern __shared__ __align__(16) float tw_smem[];
   float *qs = tw_smem, *ks = qs + TW_TOK * LD;
-  pdl_prologue(q, k, cu_q);
+  pdl_prologue(cu_q);
   const int grp = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const TwPiece at = tw_piece(blockIdx.x, TW_TOK, cu_q, num_rows);
   if (at.row < 0) return;
@@ -187,8 +187,8 @@ tile_head_kernel(float* __restrict__ dots, uint8_t* __restrict__ q_image, uint8_
     const int idx = e * TW_FIRST + tid, i = idx / (DK / 4), c = (idx % (DK / 4)) * 4;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     if (i < n) {
-      a = *reinterpret_cast<const float4*>(q + (size_t)(t0 + i) * ld_q + (size_t)grp * DK + c);
-      b = *reinterpret_cast<const float4*>(k + (size_t)(t0 + i) * ld_k + (size_t)grp * DK + c);
+      a = behind_loadf4(q + (size_t)(t0 + i) * ld_q + (size_t)grp * DK + c);
+      b = behind_loadf4(k + (size_t)(t0 + i) * ld_k + (size_t)grp * DK + c);
     }
     *reinterpret_cast<float4*>(qs + i * LD + c) = a;
     *reinterpret_cast<float4*>(ks + i * LD + c) = b;

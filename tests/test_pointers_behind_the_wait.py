@@ -67,6 +67,7 @@ def test_pointers_go_through_the_wait(path):
             assert not re.search(r"\b(%s)\[" % "|".join(pointers), text[begin:_closing(text, begin, "{", "}")]), function
         passed |= set(pointers)
         for pointer in read_only - passed - AHEAD.get(name, set()):
-            rest = re.sub(r"behind_load\w*\(\s*%s\b|\b%s != nullptr" % (pointer, pointer), "", body)
+            rest = re.sub(r"behind_(?:load\w*|four)\(\s*%s\b|\b%s != nullptr|if \(%s\)" % (pointer, pointer, pointer), "", body)
+            rest = re.sub(r"threadIdx\.x|\b[a-z]\w*(?:\[i\])?\.[xyzw]\b", "", rest)
             uses = [u for u in re.findall(r"[^;{}]*\b%s\b[^;{}]*" % pointer, rest) if not re.fullmatch(r"\s*(?:if \([^;]*\) )?%s \+= [^;]*" % pointer, u)]
             assert not uses, (name, pointer, uses)
