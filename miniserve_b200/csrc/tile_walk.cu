@@ -24,8 +24,8 @@
 // sums against the state are scaled behind the sum: a state within q's size of the largest float overflows.)
 //
 // What bounds it, 64 heads of 128 x 64, three rows of 1,037, 640 and 371 tokens, 263 us by chunks of 16 and 170 here: the second kernel (91 us) issues its instructions at
-// half the rate, most of them making operands and adding up results; the third (54) is a chain of 17 chunks, bound by shared memory and the state's parts; the first 24.6 (long scoreboard, 28 % of the issue slots; 23.6
-// with sums of eight products everywhere, and outputs under fast decays 1.07 times as far off as by chunks of 16, 26.8 with sums of four everywhere).
+// half the rate, most of them making operands and adding up results; the third (54) is a chain of 17 chunks, bound by shared memory and the state's parts; the first 24 (long scoreboard, 28 % of the issue slots; a microsecond less
+// with sums of eight products everywhere, and outputs under fast decays 1.07 times as far off as by chunks of 16; two more with sums of four everywhere).
 // Measured and not kept: the same products in float32 multiply-adds, 8 x 8 outputs a thread (332 us: both shared memory and the FMA pipe at 54 %); all three kernels' work
 // on the chain (322); parts on a grid that a row shares, whose products add up without any cut (165, but a row's small numbers lose the bits that its largest takes: one
 // value channel of 1,024 made outputs 28 times as far off).
